@@ -1,0 +1,46 @@
+"""GPU tests of the lattice sweeps (label axes of at most 128 positions) against a float64
+evaluation at the edges of what they are cut into: blocks of 16 diagonals, the positions a lane
+owns (1, 2 or 4), tiles of 32 frames, empty and one-node lattices.  The exact SIMT kernels stand
+around the sweeps, so that what is compared is theirs."""
+import numpy as np
+import pytest
+import torch
+
+import abi
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("T,U", [(1, 1), (1, 2), (15, 1), (16, 1), (17, 16), (16, 17), (31, 2), (32, 33),
+                                 (33, 32), (64, 64), (47, 65), (130, 127), (128, 128), (5, 128), (400, 40)])
+def test_edges(T, U):
+    B, V = 4, 40
+    g = torch.Generator(device="cuda").manual_seed(100 * T + U)
+    E = torch.empty((B, T, V), device="cuda").normal_(generator=g)
+    P = torch.empty((B, U, V), device="cuda").normal_(generator=g)
+    labels = torch.randint(1, V, (B, U - 1), generator=g, device="cuda", dtype=torch.int32)
+    il = torch.randint(max(1, T // 2), T + 1, (B,), generator=g, device="cuda", dtype=torch.int32)
+    ll = torch.randint(0, U, (B,), generator=g, device="cuda", dtype=torch.int32)
+    il[0], ll[0], il[3] = T, U - 1, 0
+    abi.set_option("lognorm_path", 1)
+    abi.set_option("grads_path", 1)
+    try:
+        fwd = abi.loss_forward(E, P, labels, il, ll)
+        eg, pg = abi.loss_backward(E, P, labels, il, ll, fwd)
+        eg2, pg2 = abi.loss_backward(E, P, labels, il, ll, fwd)   # the saved state is not consumed
+        torch.cuda.synchronize()
+    finally:
+        abi.set_option("lognorm_path", 0)
+        abi.set_option("grads_path", 0)
+    assert torch.equal(eg, eg2) and torch.equal(pg, pg2)
+    n = lambda x: x.cpu().numpy()
+    ref = O.truth64(n(E), n(P), n(labels), n(il), n(ll))
+    # A stored alpha is below 1024 in magnitude and rounded to 2^-14, 2^-15 at most, which is what
+    # the T + U factors of a path carry, independently: 4 sigma.  1e-5: the fp32 contractions.
+    tol = 4.0 * np.sqrt(T + U) * 2.0 ** -15 + 1e-5
+    costs = n(fwd["costs"])
+    np.testing.assert_allclose(costs[:3], ref["costs"][:3], rtol=1e-6, atol=tol)
+    assert np.isposinf(costs[3])
+    assert abi.rel_to_max(n(eg), ref["egrads"]) < tol
+    assert abi.rel_to_max(n(pg), ref["pgrads"]) < tol

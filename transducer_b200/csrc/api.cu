@@ -85,41 +85,59 @@ struct LogNormWs {
 
 // What the forward call leaves for the backward call (opaque to the caller).
 struct SavedState {
-  float *alphasS, *LNs, *ELs, *ebl, *rowRef, *maxP;
-  float2* arcs;   // arc terms of the single-warp sweeps (label axis <= 128), else null
-  float* deltas;  // per-block offsets of their rebased alphas
+  float *rowRef, *maxP, *alphas;
+  float *LN = nullptr, *deltas = nullptr;                 // label axis <= 128
+  float2* arcs = nullptr;
+  float *LNs = nullptr, *ELs = nullptr, *ebl = nullptr;   // longer ones
   SavedState(Carver& c, const Dims& d) {
-    const SkewGeom g = skew_geom(d);
     const size_t B = d.B;
-    alphasS = c.take<float>(B * g.stride);
-    LNs = c.take<float>(B * g.stride);
-    ELs = c.take<float>(B * g.stride);
-    ebl = c.take<float>(B * d.maxT);
     rowRef = c.take<float>(B * d.maxT);
     maxP = c.take<float>(B * d.maxU);
-    arcs = c.take<float2>(lattice_warp_supported(d) ? B * g.stride : 0);
-    deltas = c.take<float>(lattice_warp_supported(d) ? lattice_warp_delta_floats(d) : 0);
-    if (!lattice_warp_supported(d)) arcs = nullptr;
+    if (sweep_supported(d)) {
+      const SweepGeom g = sweep_geom(d);
+      alphas = c.take<float>(B * g.stride);
+      arcs = c.take<float2>(B * g.stride);
+      LN = c.take<float>(B * d.maxT * d.maxU);
+      deltas = c.take<float>(B * g.nBlk);
+    } else {
+      const SkewGeom g = skew_geom(d);
+      alphas = c.take<float>(B * g.stride);
+      LNs = c.take<float>(B * g.stride);
+      ELs = c.take<float>(B * g.stride);
+      ebl = c.take<float>(B * d.maxT);
+    }
   }
 };
 
 struct ForwardWs {
-  float* LN;  // row-major log-normalisers before the re-layout
-  float* EL;  // row-major label emissions E[t,label_u] gathered by the log-normaliser pass
+  float *EL, *ebl;  // emissions E[t,label_u], E[t,blank] gathered by the log-normaliser pass
+  float* LN;        // row-major log-normalisers before the re-layout (label axis > 128)
   ForwardWs(Carver& c, const Dims& d) {
-    LN = c.take<float>((size_t)d.B * d.maxT * d.maxU);
-    EL = c.take<float>(lognorm_umma_gathers(d) ? (size_t)d.B * d.maxT * d.maxU : 0);
+    const size_t cells = (size_t)d.B * d.maxT * d.maxU;
+    EL = c.take<float>(lognorm_umma_gathers(d) ? cells : 0);
+    ebl = c.take<float>((size_t)d.B * d.maxT);
+    LN = c.take<float>(sweep_supported(d) ? 0 : cells);
   }
 };
 
 struct BackwardWs {
-  float *expP, *Ws, *EMs, *W, *em, *emT, *nref, *ebl, *eBlank, *pBlank, *pLabel, *maxPScratch;
+  float *expP, *W, *em, *emT, *nref, *ebl, *eBlank, *pBlank, *pLabel, *maxPScratch;
+  SweepScratch sweep{};                 // label axis <= 128
+  float *Ws = nullptr, *EMs = nullptr;  // longer ones
   BackwardWs(Carver& c, const Dims& d) {
-    const SkewGeom g = skew_geom(d);
     const size_t B = d.B, T = d.maxT, U = d.maxU, V = d.V;
     expP = c.take<float>(B * U * V);  // SIMT path only
-    Ws = c.take<float>(B * g.stride);
-    EMs = c.take<float>(B * g.stride);
+    if (sweep_supported(d)) {
+      const SweepGeom g = sweep_geom(d);
+      sweep.F = c.take<float2>(B * g.stride);
+      sweep.g = c.take<float>(B * g.stride);
+      sweep.ticket = c.take<unsigned>(B);
+      sweep.partial = c.take<float>(sweep_partial_floats(d));
+    } else {
+      const SkewGeom g = skew_geom(d);
+      Ws = c.take<float>(B * g.stride);
+      EMs = c.take<float>(B * g.stride);
+    }
     W = c.take<float>(B * T * ld_w(d));
     em = c.take<float>(B * T * U);            // SIMT path
     emT = c.take<float>(B * U * grads_umma_ld_t(d));  // tensor-core path
@@ -378,7 +396,7 @@ int loss_forward_any(const void* E, const void* P, const int* labels, const int*
   return guarded([&] {
     Dims d{B, maxT, maxU, V, blank, dtype};
     check_dims(d);
-    if (dtype != kDtypeF32 && !lattice_warp_supported(d))
+    if (dtype != kDtypeF32 && maxU > 128)
       throw std::invalid_argument("bf16 emissions: the label axis must not exceed 128 positions");
     need(workspaceBytes, tb200_loss_forward_workspace_bytes(B, maxT, maxU, V), workspace);
     need(savedBytes, tb200_loss_saved_bytes(B, maxT, maxU, V), saved);
@@ -387,24 +405,32 @@ int loss_forward_any(const void* E, const void* P, const int* labels, const int*
     Carver c(workspace);
     ForwardWs fw(c, d);
     LogNormWs ws(c, d);
-    const SkewGeom g = skew_geom(d);
+    // The shape alone decides which sweeps run (the backward call must pick the ones that match
+    // the saved state).
+    const bool sweep = sweep_supported(d);
+    float* LN = sweep ? st.LN : fw.LN;
+    float* ebl = sweep ? fw.ebl : st.ebl;
     // (nodes the tensor-core log-normaliser could not represent are recomputed by the re-layout)
-    const bool gathered = log_norms_impl(E, P, fw.LN, st.rowRef, st.maxP, inLens, labLens, d, ws,
-                                         /*fixup=*/false, labels, fw.EL, st.ebl);
-    launch_lattice_prep(E, P, fw.LN, st.LNs, st.arcs ? nullptr : st.ELs, st.ebl, st.arcs, labels,
-                        inLens, labLens, g, d, g_stream, gathered ? fw.EL : nullptr);
+    const bool gathered = log_norms_impl(E, P, LN, st.rowRef, st.maxP, inLens, labLens, d, ws,
+                                         /*fixup=*/false, labels, fw.EL, ebl);
     if (lossSum) {
       TB200_CUDA_CHECK(cudaMemsetAsync(ws.ticket, 0, sizeof(unsigned), g_stream));
       if (B == 0) TB200_CUDA_CHECK(cudaMemsetAsync(lossSum, 0, sizeof(float), g_stream));
     }
-    // The shape alone decides which pair of sweeps runs (the backward call must pick the
-    // reverse sweep that matches the format of the saved alphas).
-    if (lattice_warp_supported(d))
-      launch_alpha_warp(st.arcs, costs, st.alphasS, st.deltas, g, inLens, labLens, d, lossSum,
-                        lossSum ? ws.ticket : nullptr, device_status_word(), g_stream);
-    else
-      launch_alpha_skew(static_cast<const float*>(P), costs, st.alphasS, st.LNs, st.ELs, st.ebl, g,
-                        labels, inLens, labLens, d, lossSum, lossSum ? ws.ticket : nullptr, g_stream);
+    unsigned* ticket = lossSum ? ws.ticket : nullptr;
+    if (sweep) {
+      launch_sweep_forward(E, P, LN, gathered ? fw.EL : nullptr, gathered ? ebl : nullptr, st.arcs,
+                           st.alphas, st.deltas, costs, lossSum, ticket, labels, inLens, labLens,
+                           sweep_geom(d), d, g_stream);
+      return;
+    }
+    const SkewGeom g = skew_geom(d);
+    const float* Ef = static_cast<const float*>(E);
+    const float* Pf = static_cast<const float*>(P);
+    launch_lattice_prep(Ef, Pf, LN, st.LNs, st.ELs, ebl, labels, inLens, labLens, g, d, g_stream,
+                        gathered ? fw.EL : nullptr);
+    launch_alpha_skew(Pf, costs, st.alphas, st.LNs, st.ELs, ebl, g, labels, inLens, labLens, d,
+                      lossSum, ticket, g_stream);
   });
 }
 
@@ -450,7 +476,6 @@ int loss_backward_any(const void* E, const void* P, const int* labels, const int
     SavedState st(cs, d);
     Carver c(workspace);
     BackwardWs ws(c, d);
-    const SkewGeom g = skew_geom(d);
     const int ldW = ld_w(d);
     const int passes = g_opt.grad_passes;
     const bool can = grads_umma_supported(E, P, egrads, pgrads, d, passes);
@@ -459,11 +484,12 @@ int loss_backward_any(const void* E, const void* P, const int* labels, const int
           "tensor-core gradients need alphabetSize % 4 == 0, alphabetSize >= 32, "
           "maxLabelLength <= 256 and 16-byte aligned emissions and egrads");
     const bool tensorCore = can && g_opt.grads_path != 1;
-    if (dtype != kDtypeF32 && !(tensorCore && lattice_warp_supported(d)))
+    const bool oneLaunch = tensorCore && maxU <= 128;
+    if (dtype != kDtypeF32 && !oneLaunch)
       throw std::invalid_argument(
           "bf16 gradients need the tensor-core gradient kernel: alphabetSize % 8 == 0, "
           "maxLabelLength <= 128, grad_passes = 2, 16-byte aligned buffers");
-    if ((egrads == E || pgrads == P) && !(tensorCore && lattice_warp_supported(d)))   // (one launch only)
+    if ((egrads == E || pgrads == P) && !oneLaunch)
       throw std::invalid_argument(
           "gradients in place (egrads == emissions / pgrads == predictions) need the "
           "tensor-core gradient kernel: alphabetSize % 4 == 0, maxLabelLength <= 128");
@@ -471,37 +497,27 @@ int loss_backward_any(const void* E, const void* P, const int* labels, const int
     const float* Pf = static_cast<const float*>(P);
     float* egf = static_cast<float*>(egrads);
     float* pgf = static_cast<float*>(pgrads);
-    if (lattice_warp_supported(d)) {
-      // single-warp reverse sweep: blank/label arc occupancies to the skewed lattices
-      // ws.Ws / ws.EMs, then re-laid out for whichever gradient kernels follow
-      int* status = device_status_word();
-      launch_gamma_warp(st.arcs, st.alphasS, st.deltas, g, inLens, labLens, ws.Ws, ws.EMs, ws.pBlank,
-                        ws.pLabel, d, status, g_stream);
-      if (tensorCore) {
-        launch_unskew_round(ws.Ws, ws.EMs, st.LNs, st.rowRef, st.maxP, deltas, ws.W, ws.emT,
-                            ws.nref, ws.ebl, inLens, labLens, g, d, true, g_stream);
-        launch_grads_umma(E, P, st.maxP, ws.W, ws.emT, ws.nref, ws.ebl, ws.pBlank, ws.pLabel,
-                          labels, deltas, egrads, pgrads, inLens, labLens, d, passes, status,
-                          g_stream);
-        return;
-      }
-      launch_unskew_round(ws.Ws, ws.EMs, st.LNs, st.rowRef, st.maxP, nullptr, ws.W, ws.em,
-                          nullptr, ws.eBlank, inLens, labLens, g, d, false, g_stream);
+    if (sweep_supported(d)) {
+      launch_sweep_backward(ws.sweep, st.arcs, st.alphas, st.deltas, st.LN, st.rowRef, st.maxP,
+                            deltas, ws.W, tensorCore ? ws.emT : ws.em,
+                            tensorCore ? ws.nref : nullptr, tensorCore ? ws.ebl : ws.eBlank,
+                            ws.pBlank, ws.pLabel, inLens, labLens, sweep_geom(d), d, tensorCore,
+                            g_stream);
     } else {
-      launch_gamma_skew(Pf, st.alphasS, st.LNs, st.ELs, st.ebl, g, st.rowRef, st.maxP, labels,
+      const SkewGeom g = skew_geom(d);
+      launch_gamma_skew(Pf, st.alphas, st.LNs, st.ELs, st.ebl, g, st.rowRef, st.maxP, labels,
                         inLens, labLens, ws.Ws, ws.EMs, ws.eBlank, ws.pBlank, ws.pLabel, d,
                         g_stream);
       launch_lattice_unskew(ws.Ws, ws.EMs, ws.W, ldW, ws.em, inLens, labLens, g, d, g_stream);
-      if (tensorCore) {
-        // label axes of 129..256 positions: the block-wide sweep's outputs re-laid out as the
-        // tensor-core kernel's operands; the kernel runs once per half of the label axis
+      if (tensorCore)
         launch_tc_operands(ws.W, ws.em, ws.eBlank, st.rowRef, deltas, ws.emT, ws.nref, ws.ebl,
                            inLens, d, g_stream);
-        launch_grads_umma(E, P, st.maxP, ws.W, ws.emT, ws.nref, ws.ebl, ws.pBlank, ws.pLabel,
-                          labels, deltas, egrads, pgrads, inLens, labLens, d, passes,
-                          device_status_word(), g_stream);
-        return;
-      }
+    }
+    if (tensorCore) {   // (label axes of 129..256 positions: once per half of the axis)
+      launch_grads_umma(E, P, st.maxP, ws.W, ws.emT, ws.nref, ws.ebl, ws.pBlank, ws.pLabel, labels,
+                        deltas, egrads, pgrads, inLens, labLens, d, passes, device_status_word(),
+                        g_stream);
+      return;
     }
     launch_exp_rows(Pf, ws.expP, ws.maxPScratch, labLens, B, maxU, V, g_stream);
     launch_egrad_simt(Ef, st.rowRef, ws.W, ldW, ws.expP, ws.eBlank, ws.em, labels, deltas,

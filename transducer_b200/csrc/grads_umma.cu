@@ -648,112 +648,6 @@ int pow2_cols(int x) {
   return c;
 }
 
-// Re-layout after the reverse sweep (gamma_warp_kernel), one CTA per 32 frames of one utterance,
-// the (up to four) 32x32 lattice tiles of the label axis side by side.  With delta_b the upstream gradient:
-//   stayS + stepS (skewed) -> W [B,maxT,ldW] = delta_b * g * exp(ref(t) + maxP(u) - LN(t,u)),
-//                   g = stay + step, rounded to TF32 (round-to-nearest; the tensor core would
-//                   otherwise truncate), zero outside the valid lattice.  (The exponent is
-//                   clamped at 80: it only gets there where the factored log-normaliser had
-//                   underflowed.)
-//   stepS (skewed) -> emT [B,maxU,ldT] = delta_b * label-arc occupancies with the frames
-//                   contiguous, so a tile's slice for one label is one TMA row; zero outside;
-//   stayS          -> ebl [B,ldT] = delta_b * sum_u stay(t,u), added in a fixed order;
-//   rowRef         -> nref [B,ldT] = -rowRef * log2(e)   (row lengths: multiples of 4 floats
-//                   as TMA requires).
-// With delta_b folded in here the gradient kernel never multiplies by it per element, and
-// frames at or beyond T_b come out as exact zeros without a select.
-// TC = false serves the SIMT gradient kernels instead: W unrounded and unscaled, the label-arc
-// occupancies row-major [B,maxT,maxU] (through emT), the row sums with row length maxT
-// (through ebl), no nref.
-template <bool TC>
-__global__ void __launch_bounds__(1024, 2) unskew_round_kernel(
-    const float* __restrict__ stayS, const float* __restrict__ stepS,
-    const float* __restrict__ LNs, const float* __restrict__ rowRef,
-    const float* __restrict__ maxP, const float* __restrict__ deltas, float* __restrict__ W,
-    float* __restrict__ emT, float* __restrict__ nref, float* __restrict__ ebl,
-    const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT, int maxU, int ld,
-    i64 latStride, int ldW, int ldT) {
-  // 32 warps: 8 per 32-wide block of label positions (ldW <= 128), all four blocks at once
-  extern __shared__ float smemU[];
-  float (*tW)[32][33] = reinterpret_cast<float (*)[32][33]>(smemU);                // [4]
-  float (*tE)[32][33] = tW + 4;
-  float (*tS)[32][33] = tE + 4;
-  __shared__ float sRow[4][32];
-  const int b = blockIdx.y, t0 = blockIdx.x * 32;
-  const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
-  const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) & 7, ub = threadIdx.x >> 8;
-  const float delta = (TC && deltas) ? deltas[b] : 1.0f;
-  const int u0 = ub * 32, u = u0 + lane;
-  const bool inRange = u0 < ldW;
-  const bool live = inRange && t0 < T && u0 < U;
-  if (live) {
-    const int uc = min(u, U - 1);
-    const float mp = maxP[(i64)b * maxU + uc];
-    // Lane `lane` of local warp w holds the tile's diagonals ds = w + 8i with 0 <= ds - lane < 32:
-    // exactly four of them.  All their loads are issued before the first use (unconditional,
-    // clamped into the lattice).
-    const int i0 = (lane > w) ? (lane - w + 7) >> 3 : 0;
-    float vSt[4], vSp[4], vLn[4], vRef[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int tt = w + 8 * (i0 + j) - lane;
-      const int tc = min(t0 + tt, T - 1);
-      const i64 o = (i64)b * latStride + (i64)(tc + uc) * ld + uc;
-      vSt[j] = stayS[o];
-      vSp[j] = stepS[o];
-      vLn[j] = LNs[o];
-      vRef[j] = rowRef[(i64)b * maxT + tc];
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int tt = w + 8 * (i0 + j) - lane;
-      float a = 0.0f, c = 0.0f, st = 0.0f;
-      if (t0 + tt < T && u < U) {
-        st = vSt[j];
-        const float sh = fminf((vRef[j] + mp) - vLn[j], 80.0f);
-        a = (st + vSp[j]) * expf(sh) * delta;
-        c = vSp[j] * delta;
-      }
-      tW[ub][tt][lane] = a;
-      tE[ub][tt][lane] = c;
-      tS[ub][tt][lane] = st;
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int tt = w * 4 + k, t = t0 + tt;
-    if (inRange) {
-      if (t < maxT && u < ldW)
-        W[((i64)b * maxT + t) * ldW + u] = live ? (TC ? tf32_round(tW[ub][tt][lane]) : tW[ub][tt][lane]) : 0.0f;
-      if (TC) {  // transposed: lane <-> frame, row <-> label position
-        const int uu = u0 + tt, t2 = t0 + lane;
-        if (uu < maxU && t2 < ldT) emT[((i64)b * maxU + uu) * ldT + t2] = live ? tE[ub][lane][tt] : 0.0f;
-      } else if (t < maxT && u < maxU) {
-        emT[((i64)b * maxT + t) * maxU + u] = live ? tE[ub][tt][lane] : 0.0f;
-      }
-    }
-    float v = live ? tS[ub][tt][lane] : 0.0f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) sRow[ub][tt] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    const int t = t0 + lane;
-    const bool ok = t < T;
-    const float rs = ((sRow[0][lane] + sRow[1][lane]) + sRow[2][lane]) + sRow[3][lane];
-    if (TC) {
-      if (t < ldT) {
-        nref[(i64)b * ldT + t] = ok ? -rowRef[(i64)b * maxT + t] * kLog2e : 0.0f;
-        ebl[(i64)b * ldT + t] = ok ? rs * delta : 0.0f;
-      }
-    } else if (t < maxT) {
-      ebl[(i64)b * maxT + t] = ok ? rs : 0.0f;
-    }
-  }
-}
-
 // Label-arc terms that grads_umma_kernel does not stage: within one block of 128 vocabulary
 // columns it subtracts the occupancies of the first kMaxStagedLabels label positions (in
 // position order) whose label falls into the block; with a vocabulary of ten thousand entries a
@@ -926,31 +820,6 @@ bool grads_umma_supported(const void* E, const void* P, const void* egrads,
   const int n = std::min(d.maxU, 128);   // positions of the (first) launch
   return pick_tile((int)round_up64(n, 8), (int)round_up64(n, 32), (int)round_up64(n, 16), passes,
                    kStaticSmemBound, bf).TB > 0;
-}
-
-void launch_unskew_round(const float* stayS, const float* stepS, const float* LNs,
-                         const float* rowRef, const float* maxP, const float* deltas, float* W,
-                         float* emT, float* nref, float* ebl, const int* inLens,
-                         const int* labLens, SkewGeom g, Dims d, bool tensorCore,
-                         cudaStream_t stream) {
-  if (d.B <= 0 || d.maxT <= 0 || d.maxU <= 0) return;
-  const int ldW = grads_umma_ld_w(d), ldT = grads_umma_ld_t(d);
-  dim3 grid(div_up(ldT, 32), d.B);
-  ScopedKernel sk("lattice_unskew_round", stream);
-  const int smem = 12 * 32 * 33 * (int)sizeof(float);
-  // (a function attribute belongs to the device that is current when it is set: set it on every
-  // launch, it is a host-side table update)
-  TB200_CUDA_CHECK(cudaFuncSetAttribute(tensorCore ? unskew_round_kernel<true> : unskew_round_kernel<false>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  if (tensorCore)
-    unskew_round_kernel<true><<<grid, 1024, smem, stream>>>(stayS, stepS, LNs, rowRef, maxP, deltas, W,
-                                                        emT, nref, ebl, inLens, labLens, d.maxT,
-                                                        d.maxU, g.ld, g.stride, ldW, ldT);
-  else
-    unskew_round_kernel<false><<<grid, 1024, smem, stream>>>(stayS, stepS, LNs, rowRef, maxP, nullptr,
-                                                         W, emT, nullptr, ebl, inLens, labLens,
-                                                         d.maxT, d.maxU, g.ld, g.stride, ldW, ldT);
-  TB200_CHECK_LAUNCH();
 }
 
 void launch_tc_operands(float* W, const float* em, const float* eBlank, const float* rowRef,

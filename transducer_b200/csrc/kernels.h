@@ -46,23 +46,14 @@ struct SkewGeom {
 };
 SkewGeom skew_geom(Dims d);
 
-// "No such arc" in the skewed arc-term array of the single-warp sweeps: a large negative
-// finite float (-5.97e29) whose four bytes are equal, so that memset can write it.
-constexpr unsigned kNoArcBits = 0xF0F0F0F0u;
-constexpr int kNoArcByte = 0xF0;
-
-// LN (row-major) -> LNs (skewed); ELs[t,u] = E[t,label_u] (skewed, skipped if null);
-// ebl[b,t] = E[t,blank].  NaN entries of LN (nodes the tensor-core log-normaliser marked)
-// are recomputed here with the exact fp32 logsumexp.
-// If arcs is not null: arcs[t,u] (skewed, [B,nDiag,ld] float2) = log2-unit log-probabilities of
-// the blank arc and the label arc leaving node (t,u), kNoArcBits where there is none.
-// If ELrow is not null it holds E[t,label_u] as [B,maxU,maxT] (frames contiguous) and ebl is an
-// INPUT (both written by launch_lognorm_umma): nothing is gathered from E here.
-// E and P are of d.dtype.
-void launch_lattice_prep(const void* E, const void* P, const float* LN, float* LNs,
-                         float* ELs, float* ebl, float2* arcs, const int* labels,
-                         const int* inLens, const int* labLens, SkewGeom g, Dims d,
-                         cudaStream_t stream, const float* ELrow = nullptr);
+// Label axes of more than 128 positions (shorter ones: lattice_sweep.cu).
+// LN (row-major) -> LNs (skewed); ELs[t,u] = E[t,label_u] (skewed); ebl[b,t] = E[t,blank].  NaN
+// entries of LN (nodes the tensor-core log-normaliser marked) are recomputed here with the exact
+// fp32 logsumexp.  If ELrow is not null it holds E[t,label_u] as [B,maxU,maxT] (frames contiguous)
+// and ebl is an INPUT (both written by launch_lognorm_umma): nothing is gathered from E here.
+void launch_lattice_prep(const float* E, const float* P, const float* LN, float* LNs, float* ELs,
+                         float* ebl, const int* labels, const int* inLens, const int* labLens,
+                         SkewGeom g, Dims d, cudaStream_t stream, const float* ELrow);
 
 void launch_alpha_skew(const float* P, float* costs, float* alphasS, const float* LNs,
                        const float* ELs, const float* ebl, SkewGeom g, const int* labels,
@@ -134,22 +125,10 @@ int grads_umma_ld_w(Dims d);  // row length of W: maxU rounded up to 32
 int grads_umma_ld_t(Dims d);  // row length of nref / ebl / emT: maxT rounded up to 4
 bool grads_umma_supported(const void* E, const void* P, const void* egrads,
                           const void* pgrads, Dims d, int passes);
-// After the reverse sweep of lattice_warp.cu: stayS/stepS/LNs (skewed) ->
-//   tensorCore: W [B,maxT,ldW] rounded to TF32, emT [B,maxU,ldT], ebl [B,ldT] (row sums of
-//               stay); rowRef -> nref = -rowRef*log2(e) [B,ldT].  W, emT and ebl are scaled by
-//               deltas[b] (1 if deltas is null).  Operands of launch_grads_umma.
-//   otherwise:  W [B,maxT,ldW] unrounded and unscaled, em [B,maxT,maxU] (passed as emT),
-//               eBlank [B,maxT] (passed as ebl); nref and deltas unused.  Operands of the SIMT
-//               gradient kernels.
-void launch_unskew_round(const float* stayS, const float* stepS, const float* LNs,
-                         const float* rowRef, const float* maxP, const float* deltas, float* W,
-                         float* emT, float* nref, float* ebl, const int* inLens,
-                         const int* labLens, SkewGeom g, Dims d, bool tensorCore,
-                         cudaStream_t stream);
 // Operands of launch_grads_umma from the outputs of the block-wide reverse sweep
 // (launch_gamma_skew + launch_lattice_unskew; label axes of more than 128 positions): W is
 // scaled by deltas[b] and rounded to TF32 in place, em [B,maxT,maxU] becomes emT, eBlank becomes
-// ebl, rowRef becomes nref (layouts as written by launch_unskew_round with tensorCore = true).
+// ebl, rowRef becomes nref (layouts as written by launch_sweep_backward with tensorCore = true).
 void launch_tc_operands(float* W, const float* em, const float* eBlank, const float* rowRef,
                         const float* deltas, float* emT, float* nref, float* ebl,
                         const int* inLens, Dims d, cudaStream_t stream);
@@ -161,27 +140,50 @@ void launch_grads_umma(const void* E, const void* P, const float* maxP, const fl
                        void* pgrads, const int* inLens, const int* labLens, Dims d, int passes,
                        int* status, cudaStream_t stream);
 
-// ---- lattice_warp.cu -------------------------------------------------------------
-// Single-warp lattice sweeps on skewed lattices for label axes of at most 128 positions.
-bool lattice_warp_supported(Dims d);
-// alpha recursion from the arc terms; writes costs (and the loss sum, see launch_alpha_skew)
-// and alphasS -- in LOG2 units, for launch_gamma_warp only (the nodes of the stored diagonals
-// that lie outside the lattice receive large negative numbers).  status: device error word (a copy that never lands
-// is recorded there and the cost becomes NaN).
-// The stored alphas are REBASED: block k of 16 diagonals is relative to an offset of its own;
-// deltas [B, ceil(nDiag/16)] (lattice_warp_delta_floats(d) floats) receives, at index k >= 1, by
-// how much the carried state was lowered at the start of block k.
-size_t lattice_warp_delta_floats(Dims d);
-void launch_alpha_warp(const float2* arcs, float* costs, float* alphasS, float* deltas, SkewGeom g,
-                       const int* inLens, const int* labLens, Dims d, float* lossSum,
-                       unsigned* ticket, int* status, cudaStream_t stream);
-// Reverse sweep: blank-arc and label-arc occupancies of every valid node to the skewed
-// lattices stayS / stepS (the terminating blank counts as the blank arc of node (T-1,U-1)),
-// their sums over frames to pBlank / pLabel [B,maxU].
-void launch_gamma_warp(const float2* arcs, const float* alphasS, const float* deltas, SkewGeom g,
-                       const int* inLens, const int* labLens, float* stayS, float* stepS,
-                       float* pBlank, float* pLabel, Dims d, int* status, cudaStream_t stream);
+// ---- lattice_sweep.cu ------------------------------------------------------------
+// Sweeps for label axes of at most 128 positions (file comment there).  Lattices are skewed:
+// node (t,u) of utterance b at b*stride + (t+u)*ld + u (pairs: permuted within the row).
+bool sweep_supported(Dims d);
+struct SweepGeom {
+  int npl;      // adjacent label positions per lane of a sweep
+  int ld;       // positions per anti-diagonal row, 32 * npl
+  int nDiag;    // rows per utterance
+  int nBlk;     // blocks of 16 rows: entries of `deltas` per utterance
+  i64 stride;   // ld * nDiag
+};
+SweepGeom sweep_geom(Dims d);
+// Arc terms (NaN entries of LN [B,maxT,maxU] -- nodes the tensor-core log-normaliser marked --
+// are recomputed in place first, exactly), alphas, costs [B] (+inf for an empty utterance) and, if
+// lossSum is not null, their sum in index order.  ELrow [B,maxU,maxT] and ebl [B,maxT]: label and
+// blank emissions as written by launch_lognorm_umma, or both null, and they are gathered from E.
+// E and P are of d.dtype.  For the backward call: arcs and alphas [B,stride], deltas [B,nBlk].
+void launch_sweep_forward(const void* E, const void* P, float* LN, const float* ELrow,
+                          const float* ebl, float2* arcs, float* alphas, float* deltas, float* costs,
+                          float* lossSum, unsigned* ticket, const int* labels, const int* inLens,
+                          const int* labLens, SweepGeom g, Dims d, cudaStream_t stream);
+struct SweepScratch {   // of the backward call
+  float2* F;         // [B,stride]
+  float* g;          // [B,stride]
+  unsigned* ticket;  // [B]
+  float* partial;    // sweep_partial_floats(d)
+};
+size_t sweep_partial_floats(Dims d);
+// Reverse sweep, then the occupancies in the layout the gradient kernels read:
+//   tensorCore: W [B,maxT,ldW] rounded to TF32, emT [B,maxU,ldT], ebl [B,ldT] (sums over u of the
+//               blank-arc occupancies), nref [B,ldT] = -rowRef*log2(e); W, emT and ebl are scaled
+//               by deltas[b] (1 if deltas is null).  Operands of launch_grads_umma.
+//   otherwise:  W [B,maxT,ldW] unrounded and unscaled, label-arc occupancies [B,maxT,maxU] (passed
+//               as emT), eBlank [B,maxT] (passed as ebl); nref and deltas unused.  Operands of the
+//               SIMT gradient kernels.
+//   both:       pBlank / pLabel [B,maxU], sums over t of the two occupancies, unscaled.
+void launch_sweep_backward(const SweepScratch& w, const float2* arcs, const float* alphas,
+                           const float* alphaDeltas, const float* LN, const float* rowRef,
+                           const float* maxP, const float* deltas, float* W, float* emT, float* nref,
+                           float* ebl, float* pBlank, float* pLabel, const int* inLens,
+                           const int* labLens, SweepGeom g, Dims d, bool tensorCore,
+                           cudaStream_t stream);
 
+// ---- lattice_warp.cu -------------------------------------------------------------
 // Viterbi sweep in one warp per utterance (label axis <= 256): same results as
 // launch_viterbi_lattice.  `nodes` is scratch of viterbi_warp_nodes(d) float4, decBits of
 // viterbi_warp_decbits_words(d) words.

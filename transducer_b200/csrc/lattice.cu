@@ -599,39 +599,26 @@ void launch_gamma_skew(const float* P, const float* alphasS, const float* LNs,
 namespace {
 
 // One CTA per 32x32 (t,u) tile.  Reads LN row-major and gathers E[t,label_u]; writes
-// both skewed.  Column tile 0 also writes ebl[t] = E[t,blank].  With `arcs` it also writes,
-// skewed and in log2 units, the log-probabilities of the two arcs leaving every valid node:
-//   arcs[t,u].x = (E[t,blank]   + P[u,blank]   - LN[t,u]) * log2(e)
-//   arcs[t,u].y = (E[t,label_u] + P[u,label_u] - LN[t,u]) * log2(e),  u < U-1
-// (the caller pre-fills the array with a large negative number: nodes outside the lattice and
-// the label arc of the last position keep it).
+// both skewed.  Column tile 0 also writes ebl[t] = E[t,blank].
 // With ELrow ([B,maxU,maxT], frames contiguous, written by the tensor-core log-normaliser
 // together with ebl) the label and blank emissions are read from there, coalesced, instead of
 // being gathered from E one DRAM sector per node.
-template <typename TIn>
 __global__ void __launch_bounds__(256) lattice_prep_kernel(
-    const TIn* __restrict__ E, const TIn* __restrict__ P, const float* __restrict__ LN,
+    const float* __restrict__ E, const float* __restrict__ P, const float* __restrict__ LN,
     float* __restrict__ LNs, float* __restrict__ ELs, float* __restrict__ ebl,
-    float2* __restrict__ arcs, const float* __restrict__ ELrow, const int* __restrict__ labels,
+    const float* __restrict__ ELrow, const int* __restrict__ labels,
     const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT, int maxU, int V,
     int blank, int ld, i64 latStride) {
-  __shared__ float tLn[32][33], tEl[32][33], tEb[32];
+  __shared__ float tLn[32][33], tEl[32][33];
   const int b = blockIdx.z, t0 = blockIdx.y * 32, u0 = blockIdx.x * 32;
   const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
   if (t0 >= T || u0 >= U) return;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const TIn* e = E + (i64)b * maxT * V;
+  const float* e = E + (i64)b * maxT * V;
   const float* ln = LN + (i64)b * maxT * maxU;
   const float* elr = ELrow ? ELrow + (i64)b * maxU * maxT : nullptr;
   const int* lab = labels + (i64)b * (maxU - 1);
   const int u = u0 + lane;
-  const int myLab = (u < U - 1) ? lab[u] : blank;
-  float pbl = 0.0f, plab = 0.0f;
-  if (arcs != nullptr && u < U) {
-    const TIn* p = P + (i64)b * maxU * V;
-    pbl = to_f32(p[(i64)u * V + blank]);
-    plab = to_f32(p[(i64)u * V + myLab]);
-  }
   // all loads first (unconditional, clamped into the lattice): the gathers of the four rows
   // are in flight together
   float va[4], vc[4];
@@ -642,7 +629,7 @@ __global__ void __launch_bounds__(256) lattice_prep_kernel(
     for (int k = 0; k < 4; ++k) {
       const int tc = min(t0 + w * 4 + k, T - 1);
       va[k] = ln[(i64)tc * maxU + uc];
-      vc[k] = elr ? 0.0f : to_f32(e[(i64)tc * V + labc]);
+      vc[k] = elr ? 0.0f : e[(i64)tc * V + labc];
     }
   }
 #pragma unroll
@@ -659,14 +646,14 @@ __global__ void __launch_bounds__(256) lattice_prep_kernel(
     while (todo) {
       const int src = __ffs(todo) - 1;
       todo &= todo - 1;
-      const TIn* er = e + (i64)t * V;
-      const TIn* pr = P + ((i64)b * maxU + u0 + src) * V;
+      const float* er = e + (i64)t * V;
+      const float* pr = P + ((i64)b * maxU + u0 + src) * V;
       float m = neg_inf();
-      for (int v = lane; v < V; v += 32) m = fmaxf(m, to_f32(er[v]) + to_f32(pr[v]));
+      for (int v = lane; v < V; v += 32) m = fmaxf(m, er[v] + pr[v]);
       m = warp_max(m);
       float s = 0.0f;
       if (m != neg_inf() && m != pos_inf())
-        for (int v = lane; v < V; v += 32) s += expf((to_f32(er[v]) + to_f32(pr[v])) - m);
+        for (int v = lane; v < V; v += 32) s += expf((er[v] + pr[v]) - m);
       s = warp_sum(s);
       if (lane == src) a = logf(s) + m;
     }
@@ -681,27 +668,16 @@ __global__ void __launch_bounds__(256) lattice_prep_kernel(
       tEl[lane][w * 4 + k] = (uu < U - 1 && tl < T) ? v : 0.0f;
     }
   }
-  if (threadIdx.x < 32) {
-    float v = 0.0f;
-    if (t0 + lane < T) v = elr ? ebl[(i64)b * maxT + t0 + lane] : to_f32(e[(i64)(t0 + lane) * V + blank]);
-    tEb[lane] = v;
-    if (!elr && u0 == 0 && t0 + lane < T) ebl[(i64)b * maxT + t0 + lane] = v;
-  }
+  if (threadIdx.x < 32 && !elr && u0 == 0 && t0 + lane < T)
+    ebl[(i64)b * maxT + t0 + lane] = e[(i64)(t0 + lane) * V + blank];
   __syncthreads();
   // diagonal s = t + u of this tile: s - (t0+u0) in [0, 62]; lane <-> u
   for (int ds = w; ds < 63; ds += 8) {
     const int tt = ds - lane;
     if (tt >= 0 && tt < 32 && t0 + tt < T && u < U) {
       const i64 o = (i64)b * latStride + (i64)(t0 + u0 + ds) * ld + u;
-      const float lnv = tLn[tt][lane], elv = tEl[tt][lane];
-      LNs[o] = lnv;
-      if (ELs != nullptr) ELs[o] = elv;
-      if (arcs != nullptr) {
-        float2 f;
-        f.x = ((tEb[tt] + pbl) - lnv) * 1.4426950408889634f;
-        f.y = (u < U - 1) ? ((elv + plab) - lnv) * 1.4426950408889634f : __uint_as_float(kNoArcBits);
-        arcs[o] = f;
-      }
+      LNs[o] = tLn[tt][lane];
+      ELs[o] = tEl[tt][lane];
     }
   }
 }
@@ -746,23 +722,14 @@ __global__ void __launch_bounds__(256) lattice_unskew_kernel(
 
 }  // namespace
 
-void launch_lattice_prep(const void* E, const void* P, const float* LN, float* LNs,
-                         float* ELs, float* ebl, float2* arcs, const int* labels,
-                         const int* inLens, const int* labLens, SkewGeom g, Dims d,
-                         cudaStream_t stream, const float* ELrow) {
+void launch_lattice_prep(const float* E, const float* P, const float* LN, float* LNs, float* ELs,
+                         float* ebl, const int* labels, const int* inLens, const int* labLens,
+                         SkewGeom g, Dims d, cudaStream_t stream, const float* ELrow) {
   if (d.B <= 0 || d.maxT <= 0 || d.maxU <= 0) return;
-  if (arcs != nullptr)
-    TB200_CUDA_CHECK(cudaMemsetAsync(arcs, kNoArcByte, sizeof(float2) * (size_t)d.B * g.stride, stream));
   dim3 grid(div_up(d.maxU, 32), div_up(d.maxT, 32), d.B);
   ScopedKernel sk("lattice_prep", stream);
-  if (d.dtype == kDtypeBf16)
-    lattice_prep_kernel<bf16><<<grid, 256, 0, stream>>>(
-        static_cast<const bf16*>(E), static_cast<const bf16*>(P), LN, LNs, ELs, ebl, arcs, ELrow,
-        labels, inLens, labLens, d.maxT, d.maxU, d.V, d.blank, g.ld, g.stride);
-  else
-    lattice_prep_kernel<float><<<grid, 256, 0, stream>>>(
-        static_cast<const float*>(E), static_cast<const float*>(P), LN, LNs, ELs, ebl, arcs, ELrow,
-        labels, inLens, labLens, d.maxT, d.maxU, d.V, d.blank, g.ld, g.stride);
+  lattice_prep_kernel<<<grid, 256, 0, stream>>>(E, P, LN, LNs, ELs, ebl, ELrow, labels, inLens, labLens,
+                                                d.maxT, d.maxU, d.V, d.blank, g.ld, g.stride);
   TB200_CHECK_LAUNCH();
 }
 

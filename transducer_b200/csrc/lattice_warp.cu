@@ -1,23 +1,11 @@
-// Lattice sweeps for label axes of at most 128 positions: the recursion runs in ONE warp.
+// Viterbi sweep for label axes of at most 256 positions: the recursion runs in ONE warp.
 //
 // The wavefront kernels of lattice.cu spend a block barrier and a shared-memory exchange on
-// every anti-diagonal.  Here lane l of a single warp owns the label positions u = 4l .. 4l+3;
-// all nodes of a diagonal are independent, the one value per lane that crosses from the
-// neighbouring lane arrives by a warp shuffle, and nothing else sits on the dependent chain:
-//   * the arc log-probabilities of every node were combined once by lattice_prep_kernel into
-//     the skewed array arcs[d][u] = (blank arc, label arc) in log2 units, a large negative
-//     finite number where the arc or the node does not exist -- so the recursion needs no
-//     validity logic and no -inf special cases;
-//   * in the skewed layout (node (t,u) at (t+u)*ld + u, see lattice.cu) a block of 16
-//     diagonals is one contiguous range of memory: it is fetched by one bulk asynchronous
-//     copy into a shared-memory ring, several blocks ahead of its use.
-// alpha: a single warp per utterance does everything.  reverse sweep: the exponentials of the
-// arc terms do not depend on the recursion, so four helper warps prepare them for the block
-// ahead and write the results of the block behind, while the recursion warp is left with two
-// multiplies and an add per node.
-//
-//   alpha   transducer/transducer_cpu.cpp:30-79   (transducer_cuda.cu:32-97)
-//   reverse transducer/transducer_cpu.cpp:81-143  (transducer_cuda.cu:99-176)
+// every anti-diagonal.  Here lane l of a single warp owns adjacent label positions; all nodes of
+// a diagonal are independent, the one value per lane that crosses from the neighbouring lane
+// arrives by a warp shuffle, and a block of 16 diagonals of the skewed operand array (node (t,u)
+// at (t+u)*ld + u) is one contiguous range of memory, fetched by one bulk asynchronous copy into
+// a shared-memory ring several blocks ahead of its use.
 #include <algorithm>
 
 #include "kernels.h"
@@ -31,404 +19,6 @@ using namespace sm100;
 
 constexpr int kDiag = 16;   // diagonals per block
 constexpr int kRing = 4;    // blocks in flight
-constexpr float kLn2F = 0.6931471805599453f;
-
-__device__ __forceinline__ float lg2_approx(float x) {
-  float y;
-  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-__device__ __forceinline__ void finish_cost_w(float* costs, int b, float cost, int B,
-                                              float* lossSum, unsigned* ticket) {
-  costs[b] = cost;
-  if (lossSum == nullptr) return;
-  __threadfence();
-  const unsigned done = atomicAdd(ticket, 1u);
-  if (done == (unsigned)(B - 1)) {  // last utterance: add the costs in index order
-    __threadfence();
-    float s = 0.0f;
-    for (int k = 0; k < B; ++k) s += ((volatile float*)costs)[k];
-    *lossSum = s;
-    *ticket = 0u;
-  }
-}
-
-// ---------------------------------------------------------------------------
-// alpha
-// ---------------------------------------------------------------------------
-// One warp per utterance.  The recursion runs in log2 units,
-//   a(t,u) = log2( 2^(a(t-1,u) + blank arc) + 2^(a(t,u-1) + label arc) ),
-// so that the two transcendental steps are the bare ex2 / lg2 instructions, and the alphas are
-// stored in log2 units too: the reverse sweep must form a(t,u) + arc with the very same
-// rounding as here, or the occupancies stop being a conserved flow.
-//
-// REBASED alphas.  After 2000 frames an alpha is of magnitude 1e4 and an fp32 ulp there is
-// 1e-3: the reference carries its alphas at that magnitude (transducer_cpu.cpp:30-79) and its
-// gradients are 2e-3..6e-3 of their maximum away from a float64 evaluation for it (measured).
-// Here every block of 16 diagonals stores its alphas relative to an offset of its own: at the
-// start of block k the whole carried state is lowered by delta_k = the floor of its largest
-// entry (an integer, so that the running offset -- needed only for the final cost -- adds up
-// exactly), which keeps every stored number below ~500 in magnitude (ulp 3e-5).  delta_k is
-// written to `deltas` for the reverse sweep, which subtracts it at the same point of the same
-// sum.  The loss and the gradients then sit ~1e-4 from the float64 result.
-// Lane l owns the label positions u = 4l + r, r = 0..3: the value crossing from u-1 is the
-// lane's own for r > 0 and comes from lane l-1 by ONE shuffle per diagonal for r = 0; the four
-// arc pairs and the four alphas of a lane are contiguous (two 16-byte loads, one store).  The
-// pace is set by the dependent chain of a diagonal -- the four ex2 and then the four lg2 queue
-// in the quarter-rate special-function unit -- so the loop holds nothing else: no validity
-// tests, no address arithmetic beyond an increment, the final cost read after the loop.
-// (Cutting the label axis over two or four warps that run a block apart, with one or two
-// positions per lane, was measured and is slower: every node then waits for a shuffle.)
-__global__ void __launch_bounds__(32) alpha_warp_kernel(
-    const float2* __restrict__ arcs, float* __restrict__ costs, float* __restrict__ alphas,
-    float* __restrict__ deltas, int ld, i64 latStride, int nDiag,
-    const int* __restrict__ inLens, const int* __restrict__ labLens, int B, int maxT, int maxU,
-    float* lossSum, unsigned* ticket, int* status) {
-  extern __shared__ __align__(128) uint8_t smemA[];
-  float2* ring = reinterpret_cast<float2*>(smemA);  // [kRing][kDiag * ld]
-  __shared__ uint64_t bar[kRing];
-  __shared__ int abortFlag;
-  const int b = blockIdx.x, lane = threadIdx.x;
-  const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
-  if (T <= 0 || U <= 0) {
-    if (lane == 0) finish_cost_w(costs, b, pos_inf(), B, lossSum, ticket);
-    return;
-  }
-  const float2* ar = arcs + (i64)b * latStride;
-  float* al = alphas + (i64)b * latStride;
-  const int S = T + U - 1;
-  const int nBlocks = (S + kDiag - 1) / kDiag;
-  const int slot = kDiag * ld;  // float2 elements per ring slot
-  // large negative and finite: the identity of the recursion without -inf arithmetic
-  const float kNone = __uint_as_float(kNoArcBits);
-
-  if (lane == 0) {
-    for (int s = 0; s < kRing; ++s) mbar_init(&bar[s], 1);
-    abortFlag = 0;
-    fence_mbar_init();
-  }
-  __syncwarp();
-  int issuedN = 0;  // lane 0: blocks whose copies were issued
-  auto issue = [&](int k) {  // lane 0: rows [16k, 16k+16) of arcs -> ring slot k % kRing
-    if (k < nBlocks) {
-      const int rows = min(kDiag, nDiag - k * kDiag);
-      const uint32_t bytes = (uint32_t)(rows * ld) * 8u;
-      mbar_arrive_expect_tx(&bar[k % kRing], bytes);
-      bulk_load_1d(ring + (size_t)(k % kRing) * slot, ar + (size_t)k * slot, bytes, &bar[k % kRing]);
-      issuedN = k + 1;
-    }
-  };
-  if (lane == 0)
-    for (int k = 0; k < kRing - 1; ++k) issue(k);
-
-  // lanes past the row (ld is a multiple of 4, at most 128) compute on a clamped column: finite
-  // values that are never stored and never reach a lane below them
-  const int u0 = 4 * lane, uc = min(u0, ld - 4);
-  const bool act = u0 < ld;
-  float stayIn[4], stepOut[4];
-#pragma unroll
-  for (int r = 0; r < 4; ++r) stayIn[r] = stepOut[r] = kNone;
-  if (lane == 0) stayIn[0] = 0.0f;  // alpha(0,0) = 0
-  bool ok = true;
-  float up = kNone;  // stepOut[3] of the lane below, one diagonal back
-  float offset = 0.0f;  // sum of the deltas so far: an integer, exact in fp32
-  float* dl = deltas + (i64)b * ((nDiag + kDiag - 1) / kDiag);
-  float nextDelta = 0.0f;  // by how much the state is lowered at the start of the next block
-  for (int k = 0; k < nBlocks; ++k) {
-    if (k > 0) {
-      // rebase (entries of nodes outside the lattice are ~ -6e29 and stay there)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        stayIn[r] -= nextDelta;
-        stepOut[r] -= nextDelta;
-      }
-      up -= nextDelta;
-      offset += nextDelta;
-      if (lane == 0) dl[k] = nextDelta;
-    }
-    // The slot refilled next was read by ALL lanes one block ago: the warp barrier orders those
-    // reads before lane 0's proxy fence and copy issue.
-    __syncwarp();
-    if (lane == 0) {
-      fence_proxy_async_smem();
-      issue(k + kRing - 1);
-    }
-    ok = mbar_wait(&bar[k % kRing], (k / kRing) & 1, &abortFlag, status, kStatusTimeoutTma);
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok) break;
-    const float4* blk = reinterpret_cast<const float4*>(ring + (size_t)(k % kRing) * slot + uc);
-    const int d0 = k * kDiag, nd = min(kDiag, S - d0), ld4 = ld / 2;  // float4 per diagonal
-    float* out = al + (size_t)d0 * ld + u0;
-    // The delta applied at the start of the NEXT block is the floor of the largest entry of
-    // the state now, at the start of this one: the warp-wide maximum then has a whole block to
-    // arrive, off the dependent chain.  (By then the state has sunk by another ~16 arcs; all
-    // that matters is that the stored numbers stay small: below ~1000, ulp 6e-5.)
-    {
-      float m = fmaxf(fmaxf(stayIn[0], stayIn[1]), fmaxf(stayIn[2], stayIn[3]));
-      m = fmaxf(m, fmaxf(fmaxf(stepOut[0], stepOut[1]), fmaxf(stepOut[2], stepOut[3])));
-      nextDelta = (float)__reduce_max_sync(0xffffffffu, __float2int_rd(fmaxf(m, -1.0e9f)));
-    }
-#pragma unroll 4
-    for (int dd = 0; dd < nd; ++dd) {
-      const float4 f01 = blk[dd * ld4], f23 = blk[dd * ld4 + 1];
-      const float fx[4] = {f01.x, f01.z, f23.x, f23.z}, fy[4] = {f01.y, f01.w, f23.y, f23.w};
-      // Position 3 first: its result feeds the shuffle of the next diagonal; position 0 last: it
-      // waits for the shuffle of this one.  (A warp issues in order.)
-      float left[4], m[4], e[4], a[4];
-      left[0] = lane ? up : kNone;
-#pragma unroll
-      for (int r = 1; r < 4; ++r) left[r] = stepOut[r - 1];
-#pragma unroll
-      for (int r = 3; r >= 0; --r) {
-        m[r] = fmaxf(left[r], stayIn[r]);
-        e[r] = ex2_approx(-fabsf(left[r] - stayIn[r]));
-      }
-#pragma unroll
-      for (int r = 3; r >= 0; --r) {
-        a[r] = m[r] + lg2_approx(1.0f + e[r]);
-        stayIn[r] = a[r] + fx[r];
-        stepOut[r] = a[r] + fy[r];
-        if (r == 3) up = __shfl_up_sync(0xffffffffu, stepOut[3], 1);
-      }
-      if (act) *reinterpret_cast<float4*>(out + dd * ld) = make_float4(a[0], a[1], a[2], a[3]);
-    }
-  }
-  if (!ok) {  // a copy never landed: make the failure visible in the result
-    if (lane == 0) {  // give the copies still in flight a bounded time to land
-      for (int j = max(0, issuedN - kRing); j < issuedN; ++j) {
-        const unsigned long long t1 = global_timer_ns();
-        while (!mbar_try_wait(&bar[j % kRing], (j / kRing) & 1) &&
-               global_timer_ns() - t1 < 50000000ull) {
-        }
-      }
-      finish_cost_w(costs, b, __int_as_float(0x7fc00000), B, lossSum, ticket);
-    }
-    return;
-  }
-  // the last diagonal holds only the terminal node (T-1, U-1); its blank arc ends the path
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-    if (u0 + r == U - 1) finish_cost_w(costs, b, -(stayIn[r] + offset) * kLn2F, B, lossSum, ticket);
-}
-
-// ---------------------------------------------------------------------------
-// reverse occupancy sweep
-// ---------------------------------------------------------------------------
-// With g(t,u) the occupancy of node (t,u) (the reference's dalphas, sign dropped):
-//   stay(t,u) = g(t+1,u) * FB(t,u),  FB = 2^((alpha(t,u) + blank arc) - alpha(t+1,u))
-//   step(t,u) = g(t,u+1) * FL(t,u),  FL = 2^((alpha(t,u) + label arc) - alpha(t,u+1))
-//   (alphas and arcs in log2 units; the parenthesised sums are rounded exactly as in the alpha
-//   kernel, so FB and FL of the arcs entering a node add up to 1 to within the error of ex2/lg2.
-//   The stored alphas are relative to a per-block offset, see alpha_warp_kernel: where the
-//   successors' diagonal opens a new block of the alpha kernel, that block's delta is
-//   subtracted from the sum first, exactly as the alpha kernel lowered its carried state.)
-//   g(t,u) = stay + step,            g(T-1,U-1) = 1 (the terminating blank, booked as stay)
-// Warp 0 runs the recursion on (FB, FL) pairs staged in shared memory and hands (stay, step)
-// back the same way.  The helper warps (kHelperGroups groups of four, thread <-> label position
-// u, the diagonals of a block dealt round-robin to the groups) turn the block
-// after the current one into (FB, FL), write the (stay, step) of the block before it to the
-// skewed lattices stayS / stepS, and accumulate per label position sum_t stay -> pBlank[u],
-// sum_t step -> pLabel[u] in a fixed order (per group, the groups' partial sums added in
-// group order at the end).  One thread of a last warp issues the bulk copies of the arc terms
-// and the alphas, kRing-1 blocks ahead (the proxy fence and the copy issue cost ~500 cycles,
-// which no helper warp should carry).
-// Block k holds the diagonals dTop(k) = S-1-16k down to dLo(k) = max(dTop-15, 0).
-constexpr int kHelperGroups = 4;  // helper group j takes the diagonals dd = j (mod 4) of a block
-constexpr int kPerHelper = kDiag / kHelperGroups;  // diagonals of a block per helper thread
-constexpr int kCopyTid = 32 + 128 * kHelperGroups;  // first thread of the copy warp
-constexpr int kGammaThreads = kCopyTid + 32;
-
-__global__ void __launch_bounds__(kGammaThreads) gamma_warp_kernel(
-    const float2* __restrict__ arcs, const float* __restrict__ alphas,
-    const float* __restrict__ deltas, int nDiag, int ld, i64 latStride,
-    const int* __restrict__ inLens, const int* __restrict__ labLens, float* __restrict__ stayS,
-    float* __restrict__ stepS, float* __restrict__ pBlank, float* __restrict__ pLabel, int maxT,
-    int maxU, int* status) {
-  extern __shared__ __align__(128) uint8_t smemG[];
-  // ring slot: arcs of kDiag diagonals, then alphas of kDiag+1 diagonals (+ one spare row)
-  const int arcBytes = kDiag * ld * 8, slotBytes = arcBytes + (kDiag + 2) * ld * 4;
-  float2 (*F)[kDiag][128] = reinterpret_cast<float2 (*)[kDiag][128]>(smemG + kRing * slotBytes);
-  float2 (*G)[kDiag][128] = F + 2;
-  __shared__ uint64_t bar[kRing];
-  __shared__ int abortFlag;
-  __shared__ float sAcc[kHelperGroups][2][128];
-  const int b = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
-  const bool empty = (T <= 0 || U <= 0);
-  // padded tails of the per-position outputs are defined (zero)
-  for (int u = (empty ? 0 : U) + tid; u < maxU; u += kGammaThreads) {
-    pBlank[(i64)b * maxU + u] = 0.0f;
-    pLabel[(i64)b * maxU + u] = 0.0f;
-  }
-  if (empty) return;
-  const float2* ar = arcs + (i64)b * latStride;
-  const float* al = alphas + (i64)b * latStride;
-  float* sS = stayS + (i64)b * latStride;
-  float* pS = stepS + (i64)b * latStride;
-  const int S = T + U - 1;
-  const int nBlocks = (S + kDiag - 1) / kDiag;
-
-  if (tid == 0) {
-    for (int s = 0; s < kRing; ++s) mbar_init(&bar[s], 1);
-    abortFlag = 0;
-    fence_mbar_init();
-  }
-  // the alpha kernel's per-block deltas of this utterance, staged once (after the F/G buffers)
-  float* dl = reinterpret_cast<float*>(G + 2);
-  {
-    const float* src = deltas + (i64)b * ((nDiag + kDiag - 1) / kDiag);
-    for (int k = 1 + tid; k < nBlocks; k += kGammaThreads) dl[k] = src[k];
-  }
-  __syncthreads();
-  auto issue = [&](int k) {  // one thread
-    if (k < nBlocks) {
-      const int dTop = S - 1 - k * kDiag, dLo = max(dTop - (kDiag - 1), 0), nd = dTop - dLo + 1;
-      uint8_t* dst = smemG + (size_t)(k % kRing) * slotBytes;
-      const uint32_t b1 = (uint32_t)(nd * ld) * 8u, b2 = (uint32_t)((nd + 1) * ld) * 4u;
-      mbar_arrive_expect_tx(&bar[k % kRing], b1 + b2);
-      bulk_load_1d(dst, ar + (size_t)dLo * ld, b1, &bar[k % kRing]);
-      bulk_load_1d(dst + arcBytes, al + (size_t)dLo * ld, b2, &bar[k % kRing]);
-    }
-  };
-  const int hu = (tid - 32) & 127;   // helper threads: label position
-  const int hg = (tid - 32) >> 7;    //                 group
-  float accB = 0.0f, accL = 0.0f;
-  auto stage = [&](int k) -> bool {  // helpers: (FB, FL) of block k -> F[k & 1]
-    bool ok = mbar_wait(&bar[k % kRing], (k / kRing) & 1, &abortFlag, status, kStatusTimeoutTma);
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok) return ok;
-    const int dTop = S - 1 - k * kDiag, dLo = max(dTop - (kDiag - 1), 0), nd = dTop - dLo + 1;
-    if (hu >= ld) {  // beyond the row: no node
-      for (int dd = hg; dd < nd; dd += kHelperGroups) F[k & 1][dd][hu] = make_float2(0.0f, 0.0f);
-      return ok;
-    }
-    const uint8_t* src = smemG + (size_t)(k % kRing) * slotBytes;
-    const float2* tb = reinterpret_cast<const float2*>(src);
-    const float* aa = reinterpret_cast<const float*>(src + arcBytes);
-    // all operands of the thread's diagonals first (clamped, unconditional), then the arithmetic:
-    // the shared-memory latency is paid once per block, not once per diagonal
-    float2 arc[kPerHelper];
-    float a[kPerHelper], adn[kPerHelper], art[kPerHelper];
-    // Exactly one diagonal of the block, ddB, has its successors on a diagonal that opens a block
-    // of the alpha kernel (dNext = dTop - ddB + 1 a multiple of 16): there the carried sums were
-    // lowered by that block's delta before they entered it.
-    const int ddB = (dTop + 1) & (kDiag - 1);
-    const int dNextB = dTop - ddB + 1;
-    const float deltaB = (dNextB >= kDiag && dNextB < S) ? dl[dNextB / kDiag] : 0.0f;
-#pragma unroll
-    for (int j = 0; j < kPerHelper; ++j) {
-      const int row = dTop - min(hg + j * kHelperGroups, nd - 1) - dLo;
-      arc[j] = tb[row * ld + hu];
-      a[j] = aa[row * ld + hu];
-      adn[j] = aa[(row + 1) * ld + hu];
-      art[j] = aa[(row + 1) * ld + hu + 1];
-    }
-#pragma unroll
-    for (int j = 0; j < kPerHelper; ++j) {
-      const int dd = hg + j * kHelperGroups, t = dTop - dd - hu;
-      const bool valid = hu < U && t >= 0 && t < T;
-      const float dlt = (dd == ddB) ? deltaB : 0.0f;
-      float2 f;
-      f.x = (valid && t < T - 1) ? ex2_approx(((a[j] + arc[j].x) - dlt) - adn[j]) : 0.0f;
-      if (t == T - 1 && hu == U - 1) f.x = 1.0f;  // terminating blank, fed by g(T,U-1) := 1
-      f.y = (valid && hu < U - 1) ? ex2_approx(((a[j] + arc[j].y) - dlt) - art[j]) : 0.0f;
-      if (dd < nd) F[k & 1][dd][hu] = f;
-    }
-    return ok;
-  };
-  auto post = [&](int k) {  // helpers: (stay, step) of block k -> global, running sums
-    if (hu >= U) return;
-    const int dTop = S - 1 - k * kDiag, nd = min(kDiag, dTop + 1);
-    float2 g[kPerHelper];
-#pragma unroll
-    for (int j = 0; j < kPerHelper; ++j) g[j] = G[k & 1][min(hg + j * kHelperGroups, nd - 1)][hu];
-#pragma unroll
-    for (int j = 0; j < kPerHelper; ++j) {
-      const int dd = hg + j * kHelperGroups, d = dTop - dd, t = d - hu;
-      if (dd < nd && t >= 0 && t < T) {
-        sS[d * ld + hu] = g[j].x;
-        pS[d * ld + hu] = g[j].y;
-        accB += g[j].x;
-        accL += g[j].y;
-      }
-    }
-  };
-
-  const bool helper = tid >= 32 && tid < kCopyTid;
-  int issuedN = 0;  // copy thread: blocks whose copies were issued
-  if (tid == kCopyTid)
-    for (; issuedN < kRing - 1; ++issuedN) issue(issuedN);
-  if (helper) stage(0);
-  __syncthreads();
-
-  // recursion warp: lane l owns u = 4l + r; the value crossing from u+1 is the lane's own
-  // for r < 3 and comes from lane l+1 by one shuffle per diagonal for r = 3
-  const int u0 = 4 * lane;
-  float g[4];
-#pragma unroll
-  for (int r = 0; r < 4; ++r) g[r] = (u0 + r == U - 1) ? 1.0f : 0.0f;
-
-  bool ok = true;
-  for (int k = 0; k < nBlocks && ok; ++k) {
-    if (helper) {
-      if (k > 0) post(k - 1);
-      if (k + 1 < nBlocks) stage(k + 1);
-    } else if (tid == kCopyTid) {
-      fence_proxy_async_smem();  // the slot refilled next was read two blocks ago
-      issue(issuedN++);
-    } else if (warp == 0) {
-      const int nd = min(kDiag, S - k * kDiag);
-#pragma unroll 4
-      for (int dd = 0; dd < nd; ++dd) {
-        const float4* src = reinterpret_cast<const float4*>(&F[k & 1][dd][u0]);
-        const float4 f01 = src[0], f23 = src[1];
-        // (lane 31 gets its own g[0] back: harmless, the label arc of position 127 never
-        // exists, its factor f23.w is 0)
-        const float right3 = __shfl_down_sync(0xffffffffu, g[0], 1);
-        float4 o01, o23;
-        o01.x = g[0] * f01.x;  o01.y = g[1] * f01.y;       // u0:   stay, step
-        o01.z = g[1] * f01.z;  o01.w = g[2] * f01.w;       // u0+1
-        o23.x = g[2] * f23.x;  o23.y = g[3] * f23.y;       // u0+2
-        o23.z = g[3] * f23.z;  o23.w = right3 * f23.w;     // u0+3
-        g[0] = o01.x + o01.y;
-        g[1] = o01.z + o01.w;
-        g[2] = o23.x + o23.y;
-        g[3] = o23.z + o23.w;
-        float4* dst = reinterpret_cast<float4*>(&G[k & 1][dd][u0]);
-        dst[0] = o01;
-        dst[1] = o23;
-      }
-    }
-    __syncthreads();
-    ok = (*(volatile int*)&abortFlag) == 0;
-  }
-  if (helper) {
-    if (ok) post(nBlocks - 1);
-    sAcc[hg][0][hu] = accB;
-    sAcc[hg][1][hu] = accL;
-  }
-  __syncthreads();
-  if (helper && hg == 0 && hu < U) {
-    float sb = 0.0f, sl = 0.0f;
-#pragma unroll
-    for (int j = 0; j < kHelperGroups; ++j) {
-      sb += sAcc[j][0][hu];
-      sl += sAcc[j][1][hu];
-    }
-    const float bad = __int_as_float(0x7fc00000);  // a copy never landed: visible in the result
-    pBlank[(i64)b * maxU + hu] = ok ? sb : bad;
-    pLabel[(i64)b * maxU + hu] = ok ? ((hu < U - 1) ? sl : 0.0f) : bad;
-  }
-  if (!ok && tid == kCopyTid) {  // give the copies still in flight a bounded time to land
-    for (int j = max(0, min(issuedN, nBlocks) - kRing); j < min(issuedN, nBlocks); ++j) {
-      const unsigned long long t1 = global_timer_ns();
-      while (!mbar_try_wait(&bar[j % kRing], (j / kRing) & 1) &&
-             global_timer_ns() - t1 < 50000000ull) {
-      }
-    }
-  }
-}
 
 // ---------------------------------------------------------------------------
 // Viterbi: max-plus sweep in one warp, bit-packed decisions, backtrack, label argmax
@@ -700,42 +290,6 @@ void allow_dyn_smem(K kernel, int bytes) {
 }
 
 }  // namespace
-
-bool lattice_warp_supported(Dims d) { return d.maxU >= 1 && d.maxU <= 128; }
-
-size_t lattice_warp_delta_floats(Dims d) {
-  const SkewGeom g = skew_geom(d);
-  return (size_t)d.B * (size_t)((g.nDiag + kDiag - 1) / kDiag);
-}
-
-void launch_alpha_warp(const float2* arcs, float* costs, float* alphasS, float* deltas, SkewGeom g,
-                       const int* inLens, const int* labLens, Dims d, float* lossSum,
-                       unsigned* ticket, int* status, cudaStream_t stream) {
-  if (d.B <= 0) return;
-  const int smem = kRing * kDiag * g.ld * 8;
-  ScopedKernel sk("alpha_warp", stream);
-  allow_dyn_smem(alpha_warp_kernel, smem);
-  alpha_warp_kernel<<<d.B, 32, smem, stream>>>(arcs, costs, alphasS, deltas, g.ld, g.stride, g.nDiag,
-                                               inLens, labLens, d.B, d.maxT, d.maxU, lossSum,
-                                               ticket, status);
-  TB200_CHECK_LAUNCH();
-}
-
-void launch_gamma_warp(const float2* arcs, const float* alphasS, const float* deltas, SkewGeom g,
-                       const int* inLens, const int* labLens, float* stayS, float* stepS, float* pBlank,
-                       float* pLabel, Dims d, int* status, cudaStream_t stream) {
-  if (d.B <= 0) return;
-  const int slotBytes = kDiag * g.ld * 8 + (kDiag + 2) * g.ld * 4;
-  const int smem = kRing * slotBytes + 4 * kDiag * 128 * (int)sizeof(float2) +
-                   (int)sizeof(float) * ((g.nDiag + kDiag - 1) / kDiag + 1);
-  if (smem > 225 * 1024) throw std::invalid_argument("input too long for the single-warp reverse sweep");
-  ScopedKernel sk("gamma_warp", stream);
-  allow_dyn_smem(gamma_warp_kernel, smem);
-  gamma_warp_kernel<<<d.B, kGammaThreads, smem, stream>>>(arcs, alphasS, deltas, g.nDiag, g.ld, g.stride, inLens,
-                                                          labLens, stayS, stepS, pBlank, pLabel,
-                                                          d.maxT, d.maxU, status);
-  TB200_CHECK_LAUNCH();
-}
 
 bool viterbi_warp_supported(Dims d) { return d.maxU >= 1 && d.maxU <= 256; }
 
