@@ -34,6 +34,7 @@ SIGNATURES = {
     "tb200_profile_reset": (_i, []),
     "tb200_profile_report": (_z, [ctypes.c_char_p, _z]),
     "tb200_check_status": (_i, []),
+    "tb200_call_summary": (_i, [_p, _p, _i, _i, _p, ctypes.POINTER(_i)]),
     "tb200_status_name": (ctypes.c_char_p, [_i]),
     "tb200_selftest_wait_timeout": (_i, [ctypes.c_uint]),
     "tb200_forward": (_i, [_p] * 8 + [_i] * 5),

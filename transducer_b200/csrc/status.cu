@@ -12,6 +12,7 @@
 // to allocate or carry it; host code obtains its device address once per device with
 // cudaGetSymbolAddress.  tb200_check_status() synchronises the calling thread's stream, reads
 // the word, clears it and reports.
+#include <climits>
 #include <mutex>
 #include <string>
 
@@ -47,6 +48,45 @@ __global__ void __launch_bounds__(32) selftest_wait_kernel(int* status, unsigned
                                          sm100::kStatusTimeoutSelfTest, limitNs);
   const bool all = __all_sync(0xffffffffu, ok);
   if (threadIdx.x == 0) *observed = all ? 1 : 0;  // 0: the wait gave up, as it should
+}
+
+// out = {max inLens, max labLens, status code, nodes recomputed}; the last two are taken from the
+// status word, which is cleared, if `word` is not null.
+__global__ void __launch_bounds__(256) call_summary_kernel(const int* __restrict__ inLens,
+                                                           const int* __restrict__ labLens, int B,
+                                                           int* word, int* __restrict__ out) {
+  __shared__ int sT[8], sU[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int t = INT_MIN, u = INT_MIN;
+  for (int b = threadIdx.x; b < B; b += 256) {
+    t = max(t, inLens[b]);
+    u = max(u, labLens[b]);
+  }
+  t = __reduce_max_sync(0xffffffffu, t);
+  u = __reduce_max_sync(0xffffffffu, u);
+  if (lane == 0) {
+    sT[warp] = t;
+    sU[warp] = u;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) {
+      t = max(t, sT[w]);
+      u = max(u, sU[w]);
+    }
+    out[0] = t;
+    out[1] = u;
+    out[2] = word ? atomicExch(word, 0) : 0;
+    out[3] = word ? atomicExch(word + 1, 0) : 0;
+  }
+}
+
+int report_status(int code) {
+  if (code == 0) return kOk;
+  return api_fail(kErrDeviceStatus,
+                  "device status " + std::to_string(code) + ": " + status_name(code) +
+                      " within the time limit; the kernel returned early and its outputs "
+                      "are poisoned (NaN / -1)");
 }
 
 }  // namespace
@@ -99,12 +139,31 @@ int tb200_check_status(void) {
       TB200_CUDA_CHECK(cudaMemsetAsync(word, 0, sizeof(host), s));
       TB200_CUDA_CHECK(cudaStreamSynchronize(s));
     }
-    if (host[0] != 0)
-      return api_fail(kErrDeviceStatus,
-                      "device status " + std::to_string(host[0]) + ": " + status_name(host[0]) +
-                          " within the time limit; the kernel returned early and its outputs "
-                          "are poisoned (NaN / -1)");
-    return kOk;
+    return report_status(host[0]);
+  } catch (const std::exception& e) {
+    return api_fail(kErrCuda, e.what());
+  }
+}
+
+int tb200_call_summary(const int* inLens, const int* labLens, int B, int withStatus, void* scratch,
+                       int* maxLens) {
+  try {
+    if (B <= 0 || !inLens || !labLens || !scratch || !maxLens)
+      return api_fail(kErrInvalidArgument, "tb200_call_summary: null pointer or empty batch");
+    int* out = static_cast<int*>(scratch);
+    int host[4];
+    cudaStream_t s = api_stream();
+    {
+      ScopedKernel sk("call_summary", s);
+      call_summary_kernel<<<1, 256, 0, s>>>(inLens, labLens, B,
+                                            withStatus ? device_status_word() : nullptr, out);
+    }
+    TB200_CHECK_LAUNCH();
+    TB200_CUDA_CHECK(cudaMemcpyAsync(host, out, sizeof(host), cudaMemcpyDeviceToHost, s));
+    TB200_CUDA_CHECK(cudaStreamSynchronize(s));
+    maxLens[0] = host[0];
+    maxLens[1] = host[1];
+    return report_status(host[2]);
   } catch (const std::exception& e) {
     return api_fail(kErrCuda, e.what());
   }

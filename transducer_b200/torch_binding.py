@@ -7,7 +7,8 @@ CUDA tensors only: there is no CPU backend and no PyTorch fallback."""
 import torch
 
 from . import _transducer
-from .errors import DeviceStatusError, raise_for_status  # noqa: F401
+from .errors import (TB200_ERR_DEVICE_STATUS, TB200_OK, DeviceStatusError,  # noqa: F401
+                     raise_for_status)
 
 
 def check_device_status(device=None):
@@ -51,7 +52,7 @@ class Transducer(torch.autograd.Function):
     def forward(ctx, emissions, predictions, labels, input_lengths, label_lengths, blank=0,
                 validate_lengths=True, check_status=False):
         certify_inputs(emissions, predictions, labels, input_lengths, label_lengths,
-                       validate_lengths, allow_bf16=True)
+                       validate_lengths=False, allow_bf16=True)   # (the lengths: finish_call)
         device = emissions.device
         emissions = emissions.contiguous()
         predictions = predictions.contiguous()
@@ -64,7 +65,7 @@ class Transducer(torch.autograd.Function):
             saved_bytes = _transducer.loss_saved_bytes(B, T, U, V)
             saved = _workspace(saved_bytes, device)
             nbytes = _transducer.loss_forward_workspace_bytes(B, T, U, V)
-            ws = _workspace(nbytes, device)
+            ws = _workspace(nbytes + _SUMMARY_BYTES, device)
             fwd = _transducer.loss_forward_bf16 if emissions.dtype is torch.bfloat16 \
                 else _transducer.loss_forward
             fwd(
@@ -72,9 +73,8 @@ class Transducer(torch.autograd.Function):
                 input_lengths.data_ptr(), label_lengths.data_ptr(), costs.data_ptr(),
                 loss_sum.data_ptr(), saved.data_ptr(), saved_bytes, B, T, U, V, blank,
                 ws.data_ptr(), nbytes)
-            if check_status:
-                rc = _transducer.check_status()
-                raise_for_status(rc, _transducer.last_error() if rc else "")
+            finish_call(emissions, predictions, input_lengths, label_lengths, ws, nbytes,
+                        validate_lengths, check_status)
         # `saved` replaces the reference's saved alphas/log_norms/expEs/expPs/expLNs
         # (torch_binding.py:52-55); exp(emissions) is recomputed, never stored
         ctx.save_for_backward(emissions, predictions, saved, labels, input_lengths,
@@ -178,20 +178,43 @@ class TransducerLoss(torch.nn.Module):
         U = predictions.shape[1]
         labels = torch.empty((B, U - 1), device=device, dtype=torch.int32)
         certify_inputs(emissions, predictions, labels, input_lengths, label_lengths,
-                       self.validate_lengths)
+                       validate_lengths=False)   # (the lengths: finish_call)
         emissions = emissions.contiguous()
         predictions = predictions.contiguous()
         with DeviceManager(device):
             nbytes = _transducer.viterbi_decode_workspace_bytes(B, T, U, V)
-            ws = _workspace(nbytes, device)
+            ws = _workspace(nbytes + _SUMMARY_BYTES, device)
             _transducer.viterbi_decode(
                 emissions.data_ptr(), predictions.data_ptr(), input_lengths.data_ptr(),
                 label_lengths.data_ptr(), labels.data_ptr(), B, T, U, V, self.blank,
                 ws.data_ptr(), nbytes)
-            if self.check_status:
-                rc = _transducer.check_status()
-                raise_for_status(rc, _transducer.last_error() if rc else "")
+            finish_call(emissions, predictions, input_lengths, label_lengths, ws, nbytes,
+                        self.validate_lengths, self.check_status)
         return labels
+
+
+_SUMMARY_BYTES = 16   # of device memory behind a call's workspace, for finish_call
+
+
+def finish_call(emissions, predictions, input_lengths, label_lengths, ws, nbytes,
+                validate_lengths, check_status):
+    """The checks of a call that need numbers from the device, after its kernels are enqueued: one
+    small kernel and one synchronisation for the longest lengths (the reference reads them back
+    before its kernels, transducer/torch_binding.py:222-229; here every kernel limits the lengths
+    to the padded shapes, so a call with too long ones may run before it is refused) and the
+    device status.  Replaces two reductions, a stack and two synchronisations: 58 -> 22 us."""
+    batch = emissions.shape[0]
+    if batch > 0 and validate_lengths:
+        rc, max_t, max_u = _transducer.call_summary(
+            input_lengths.data_ptr(), label_lengths.data_ptr(), batch, check_status,
+            ws.data_ptr() + nbytes)
+        if rc in (TB200_OK, TB200_ERR_DEVICE_STATUS):
+            certify_lengths(emissions, predictions, max_t, max_u)
+    elif check_status:
+        rc = _transducer.check_status()
+    else:
+        return
+    raise_for_status(rc, _transducer.last_error() if rc else "")
 
 
 def check_type(var, t, name):
@@ -250,6 +273,10 @@ def certify_inputs(emissions, predictions, labels, input_lengths, label_lengths,
         return
     # one device->host transfer for both maxima (the reference does two, :222-229)
     max_t, max_u = torch.stack((input_lengths.max(), label_lengths.max())).tolist()
+    certify_lengths(emissions, predictions, max_t, max_u)
+
+
+def certify_lengths(emissions, predictions, max_t, max_u):
     if emissions.shape[1] < max_t:
         raise ValueError("Input length mismatch")
     if predictions.shape[1] < max_u + 1:
