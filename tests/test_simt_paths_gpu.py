@@ -1,0 +1,67 @@
+"""GPU tests of the SIMT kernels that serve vocabularies TMA cannot address (not a multiple of 4, or
+below 32) against a float64 evaluation: the factored log-normaliser at the edges of its tiles
+of 32x32 nodes, its steps of 64 words and the clusters that share a tile, and the gradients at the
+edges of their tiles of 64x64 and steps of 32, with labels that share columns."""
+import numpy as np
+import pytest
+import torch
+
+import abi
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def make(B, T, U, V, std=1.0, labels_below=None):
+    g = torch.Generator(device="cuda").manual_seed(B * T + U * V)
+    E = torch.empty((B, T, V), device="cuda").normal_(0, std, generator=g)
+    P = torch.empty((B, U, V), device="cuda").normal_(0, std, generator=g)
+    labels = torch.randint(1, labels_below or V, (B, U - 1), generator=g, device="cuda", dtype=torch.int32)
+    il = torch.randint(max(1, T // 2), T + 1, (B,), generator=g, device="cuda", dtype=torch.int32)
+    ll = torch.randint(0, U, (B,), generator=g, device="cuda", dtype=torch.int32)
+    il[0], ll[0] = T, U - 1
+    return E, P, labels, il, ll
+
+
+@pytest.mark.parametrize("B,T,U,V", [(1, 1, 1, 2), (2, 31, 33, 29), (1, 33, 31, 63), (3, 64, 32, 65),
+                                     (2, 40, 5, 129), (1, 20, 7, 8041), (2, 33, 65, 1025), (16, 200, 40, 257),
+                                     (1, 70, 200, 321)])
+def test_factored_log_normaliser(B, T, U, V):
+    E, P, _, il, ll = make(B, T, U, V, std=2.0)
+    ln, ref, mp = abi.log_norms(E, P, il, ll)
+    d = E.double(), P.double()
+    want = torch.logsumexp(d[0][:, :, None] + d[1][:, None], dim=3)
+    m = torch.as_tensor(abi.valid_mask(il.cpu().numpy(), ll.cpu().numpy(), T, U), device="cuda")
+    # one rounding of the result, one of the logarithm, 2^-22 of an exponential and the sum's own
+    bound = want.abs().max().item() * 2.0 ** -23 + 2.0 ** -20
+    assert (ln.double() - want)[m].abs().max().item() < bound
+    assert torch.equal(ref[0], E[0].max(dim=1)[0]) and torch.equal(mp[0], P[0].max(dim=1)[0])
+
+
+def test_factored_sum_out_of_range_is_recomputed():
+    E, P, _, il, ll = make(2, 50, 9, 77)
+    E[:, 3] -= 1000.0 * (torch.arange(77, device="cuda") != 5)    # E's mass on word 5 ...
+    P[:, 4] -= 1000.0 * (torch.arange(77, device="cuda") == 5)    # ... which P excludes
+    E[0, 7] = float("-inf")
+    ln, _, _ = abi.log_norms(E, P, il, ll)
+    want = torch.logsumexp(E.double()[:, :, None] + P.double()[:, None], dim=3)
+    m = torch.as_tensor(abi.valid_mask(il.cpu().numpy(), ll.cpu().numpy(), 50, 9), device="cuda")
+    ok = m & torch.isfinite(want)
+    assert (ln.double() - want)[ok].abs().max().item() < 2e-7 * 1000.0
+    assert torch.isneginf(ln[0, 7, :int(ll[0]) + 1]).all()
+
+
+@pytest.mark.parametrize("B,T,U,V,below", [(1, 1, 2, 3, None), (2, 63, 64, 65, None), (2, 65, 33, 63, 4),
+                                           (1, 64, 65, 129, None), (2, 33, 128, 30, None), (3, 100, 20, 257, 3)])
+def test_gradients(B, T, U, V, below):
+    E, P, labels, il, ll = make(B, T, U, V, labels_below=below)
+    deltas = torch.linspace(0.5, 1.5, B, device="cuda")
+    fwd = abi.loss_forward(E, P, labels, il, ll)
+    eg, pg = abi.loss_backward(E, P, labels, il, ll, fwd, deltas)
+    n = lambda x: x.cpu().numpy()
+    ref = O.truth64(n(E), n(P), n(labels), n(il), n(ll))
+    s = n(deltas)[:, None, None]
+    # alphas are rounded to 2^-15 at most, T + U of them along a path (4 sigma); 1e-5: fp32 sums
+    tol = 4.0 * np.sqrt(T + U) * 2.0 ** -15 + 1e-5
+    assert abi.rel_to_max(n(eg), ref["egrads"] * s) < tol
+    assert abi.rel_to_max(n(pg), ref["pgrads"] * s) < tol

@@ -215,9 +215,10 @@ bool log_norms_impl(const void* E, const void* P, float* LN, float* rowRef, floa
   }
   const float* Ef = static_cast<const float*>(E);
   const float* Pf = static_cast<const float*>(P);
-  launch_lognorm_exact(Ef, Pf, LN, inLens, labLens, d, g_stream);
-  if (rowRef) launch_row_max(Ef, rowRef, inLens, 0, d.B, d.maxT, d.V, g_stream);
-  if (maxP) launch_row_max(Pf, maxP, labLens, 1, d.B, d.maxU, d.V, g_stream);
+  const bool exact = g_opt.lognorm_path == 1 || rowRef == nullptr;
+  launch_lognorm_simt(Ef, Pf, LN, rowRef, exact ? maxP : (maxP ? maxP : ws.maxPScratch), inLens,
+                      labLens, d, exact, exact ? nullptr : device_status_word(), g_stream);
+  if (!exact && fixup) launch_lognorm_fixup(E, P, LN, inLens, labLens, d, g_stream);
   return false;
 }
 

@@ -84,17 +84,14 @@ void launch_viterbi_lattice(const float* E, const float* P, const float* LN,
                             cudaStream_t stream);
 
 // ---- lognorm_simt.cu ---------------------------------------------------------
-// Exact fp32 logsumexp_v(E[t,v]+P[u,v]) for every valid (t,u); one warp per node.
-void launch_lognorm_exact(const float* E, const float* P, float* LN, const int* inLens,
-                          const int* labLens, Dims d, cudaStream_t stream);
-// The same for a device-resident list of nodes (packed b,t,u triples), count read
-// from *count on the device (at most maxCount entries are processed).
-void launch_lognorm_exact_list(const float* E, const float* P, float* LN,
-                               const int* cells, const int* count, int maxCount,
-                               Dims d, cudaStream_t stream);
-// rowRef[b,t] = max_v E[b,t,v] for t < T_b (0 elsewhere).
-void launch_row_max(const float* X, float* rowMax, const int* lens, int lenOffset,
-                    int B, int maxRows, int V, cudaStream_t stream);
+// fp32 log-normalisers of every valid (t,u) on the SIMT pipes; rowRef[b,t] = max_v E[b,t,v] and
+// maxP[b,u] likewise (0 for padded rows), each unless null.  exact: one logsumexp per node; else the
+// factored sum (rowRef and maxP must not be null), with nodes whose sum left the fp32 range as NaN
+// for the caller to have recomputed (lattice re-layouts, launch_lognorm_fixup) and counted in
+// status[1].
+void launch_lognorm_simt(const float* E, const float* P, float* LN, float* rowRef, float* maxP,
+                         const int* inLens, const int* labLens, Dims d, bool exact, int* status,
+                         cudaStream_t stream);
 // expP[b,u,v] = exp(P[b,u,v]-maxP[b,u]) for u <= labLens[b], 0 for padded rows;
 // also writes maxP[b,u] (0 for padded rows).
 void launch_exp_rows(const float* P, float* expP, float* maxP, const int* labLens,
@@ -112,6 +109,9 @@ size_t lognorm_umma_workspace_floats(Dims d);
 // With labels, EL [B,maxU,maxT] (frames contiguous) and ebl [B,maxT] (all three non-null) and
 // lognorm_umma_gathers(d), the kernel also writes EL[b,u,t] = E[b,t,labels[b,u]] (u < U_b - 1)
 // and ebl[b,t] = E[b,t,blank] for the valid frames, from the chunks it streams anyway.
+// launch_lognorm_fixup: the recomputation, by itself.
+void launch_lognorm_fixup(const void* E, const void* P, float* LN, const int* inLens,
+                          const int* labLens, Dims d, cudaStream_t stream);
 bool lognorm_umma_gathers(Dims d);
 void launch_lognorm_umma(const void* E, const void* P, float* LN, float* rowRef, float* maxP,
                          const int* inLens, const int* labLens, Dims d, float* splitWs,
@@ -212,7 +212,7 @@ void launch_maxplus_pruned(const float* E, const float* P, float* best, const in
 
 // ---- grads_simt.cu -----------------------------------------------------------
 // egrads[b,t,v] = delta_b*(exp(E-rowRef)*sum_u W[t,u]*expP[u,v] - [v==blank]*eBlank[t]),
-// zero for t >= T_b; then the label-arc terms are scattered in.
+// minus the label-arc terms delta_b*em[t,u] at v = label_u; zero for t >= T_b.
 void launch_egrad_simt(const float* E, const float* rowRef, const float* W, int ldW,
                        const float* expP, const float* eBlank, const float* em,
                        const int* labels, const float* deltas, float* egrads,

@@ -867,18 +867,22 @@ void launch_lognorm_umma(const void* E, const void* P, float* LN, float* rowRef,
     }
   }
   TB200_CHECK_LAUNCH();
-  if (fixup) {
-    ScopedKernel sk("lognorm_fixup", stream);
-    const unsigned rows = (unsigned)d.B * (unsigned)d.maxT;
-    if (bf)
-      lognorm_fixup_kernel<bf16><<<(rows + 7) / 8, 256, 0, stream>>>(
-          static_cast<const bf16*>(E), static_cast<const bf16*>(P), LN, inLens, labLens, d.B,
-          d.maxT, d.maxU, d.V);
-    else
-      lognorm_fixup_kernel<float><<<(rows + 7) / 8, 256, 0, stream>>>(
-          static_cast<const float*>(E), static_cast<const float*>(P), LN, inLens, labLens, d.B,
-          d.maxT, d.maxU, d.V);
-  }
+  if (fixup) launch_lognorm_fixup(E, P, LN, inLens, labLens, d, stream);
+}
+
+void launch_lognorm_fixup(const void* E, const void* P, float* LN, const int* inLens,
+                          const int* labLens, Dims d, cudaStream_t stream) {
+  if (d.B <= 0 || d.maxT <= 0 || d.maxU <= 0) return;
+  ScopedKernel sk("lognorm_fixup", stream);
+  const unsigned rows = (unsigned)d.B * (unsigned)d.maxT;
+  if (d.dtype == kDtypeBf16)
+    lognorm_fixup_kernel<bf16><<<(rows + 7) / 8, 256, 0, stream>>>(
+        static_cast<const bf16*>(E), static_cast<const bf16*>(P), LN, inLens, labLens, d.B,
+        d.maxT, d.maxU, d.V);
+  else
+    lognorm_fixup_kernel<float><<<(rows + 7) / 8, 256, 0, stream>>>(
+        static_cast<const float*>(E), static_cast<const float*>(P), LN, inLens, labLens, d.B,
+        d.maxT, d.maxU, d.V);
   TB200_CHECK_LAUNCH();
 }
 
