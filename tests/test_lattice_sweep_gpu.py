@@ -1,6 +1,6 @@
-"""GPU tests of the lattice sweeps (label axes of at most 128 positions) against a float64
+"""GPU tests of the lattice sweeps (label axes of at most 256 positions) against a float64
 evaluation at the edges of what they are cut into: blocks of 16 diagonals, the positions a lane
-owns (1, 2 or 4), tiles of 32 frames, empty and one-node lattices.  The exact SIMT kernels stand
+owns (1, 2, 4, 5..8), tiles of 32 frames, empty and one-node lattices.  The exact SIMT kernels stand
 around the sweeps, so that what is compared is theirs."""
 import numpy as np
 import pytest
@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("T,U", [(1, 1), (1, 2), (15, 1), (16, 1), (17, 16), (16, 17), (31, 2), (32, 33),
-                                 (33, 32), (64, 64), (47, 65), (130, 127), (128, 128), (5, 128), (400, 40)])
+                                 (33, 32), (64, 64), (47, 65), (130, 127), (128, 128), (5, 128), (400, 40),
+                                 (1, 129), (50, 160), (33, 161), (70, 192), (16, 193), (40, 225), (100, 256)])
 def test_edges(T, U):
     B, V = 4, 40
     g = torch.Generator(device="cuda").manual_seed(100 * T + U)
@@ -36,8 +37,9 @@ def test_edges(T, U):
     assert torch.equal(eg, eg2) and torch.equal(pg, pg2)
     n = lambda x: x.cpu().numpy()
     ref = O.truth64(n(E), n(P), n(labels), n(il), n(ll))
-    # A stored alpha is below 1024 in magnitude and rounded to 2^-14, 2^-15 at most, which is what
-    # the T + U factors of a path carry, independently: 4 sigma.  1e-5: the fp32 contractions.
+    # A stored alpha is below 1024 in magnitude (up to 128 positions: relative to its block; beyond:
+    # at T + U <= 356 here) and rounded to 2^-14, 2^-15 at most, which is what the T + U factors of a
+    # path carry, independently: 4 sigma.  1e-5: the fp32 contractions.
     tol = 4.0 * np.sqrt(T + U) * 2.0 ** -15 + 1e-5
     costs = n(fwd["costs"])
     np.testing.assert_allclose(costs[:3], ref["costs"][:3], rtol=1e-6, atol=tol)

@@ -85,14 +85,15 @@ struct LogNormWs {
 
 // What the forward call leaves for the backward call (opaque to the caller).
 struct SavedState {
-  float *rowRef, *maxP, *alphas;
-  float *LN = nullptr, *deltas = nullptr;                 // label axis <= 128
+  float *rowRef, *maxP, *alphas, *ebl;
+  float *LN = nullptr, *deltas = nullptr;                 // label axis <= 256
   float2* arcs = nullptr;
-  float *LNs = nullptr, *ELs = nullptr, *ebl = nullptr;   // longer ones
+  float *LNs = nullptr, *ELs = nullptr;                   // longer ones
   SavedState(Carver& c, const Dims& d) {
     const size_t B = d.B;
     rowRef = c.take<float>(B * d.maxT);
     maxP = c.take<float>(B * d.maxU);
+    ebl = c.take<float>(B * d.maxT);
     if (sweep_supported(d)) {
       const SweepGeom g = sweep_geom(d);
       alphas = c.take<float>(B * g.stride);
@@ -104,25 +105,23 @@ struct SavedState {
       alphas = c.take<float>(B * g.stride);
       LNs = c.take<float>(B * g.stride);
       ELs = c.take<float>(B * g.stride);
-      ebl = c.take<float>(B * d.maxT);
     }
   }
 };
 
 struct ForwardWs {
-  float *EL, *ebl;  // emissions E[t,label_u], E[t,blank] gathered by the log-normaliser pass
-  float* LN;        // row-major log-normalisers before the re-layout (label axis > 128)
+  float* EL;  // label emissions E[t,label_u] gathered by the log-normaliser pass
+  float* LN;        // row-major log-normalisers before the re-layout (label axis > 256)
   ForwardWs(Carver& c, const Dims& d) {
     const size_t cells = (size_t)d.B * d.maxT * d.maxU;
     EL = c.take<float>(lognorm_umma_gathers(d) ? cells : 0);
-    ebl = c.take<float>((size_t)d.B * d.maxT);
     LN = c.take<float>(sweep_supported(d) ? 0 : cells);
   }
 };
 
 struct BackwardWs {
   float *expP, *W, *em, *emT, *nref, *ebl, *eBlank, *pBlank, *pLabel, *maxPScratch;
-  SweepScratch sweep{};                 // label axis <= 128
+  SweepScratch sweep{};                 // label axis <= 256
   float *Ws = nullptr, *EMs = nullptr;  // longer ones
   BackwardWs(Carver& c, const Dims& d) {
     const size_t B = d.B, T = d.maxT, U = d.maxU, V = d.V;
@@ -410,17 +409,16 @@ int loss_forward_any(const void* E, const void* P, const int* labels, const int*
     // the saved state).
     const bool sweep = sweep_supported(d);
     float* LN = sweep ? st.LN : fw.LN;
-    float* ebl = sweep ? fw.ebl : st.ebl;
     // (nodes the tensor-core log-normaliser could not represent are recomputed by the re-layout)
     const bool gathered = log_norms_impl(E, P, LN, st.rowRef, st.maxP, inLens, labLens, d, ws,
-                                         /*fixup=*/false, labels, fw.EL, ebl);
+                                         /*fixup=*/false, labels, fw.EL, st.ebl);
     if (lossSum) {
       TB200_CUDA_CHECK(cudaMemsetAsync(ws.ticket, 0, sizeof(unsigned), g_stream));
       if (B == 0) TB200_CUDA_CHECK(cudaMemsetAsync(lossSum, 0, sizeof(float), g_stream));
     }
     unsigned* ticket = lossSum ? ws.ticket : nullptr;
     if (sweep) {
-      launch_sweep_forward(E, P, LN, gathered ? fw.EL : nullptr, gathered ? ebl : nullptr, st.arcs,
+      launch_sweep_forward(E, P, LN, gathered ? fw.EL : nullptr, st.ebl, st.arcs,
                            st.alphas, st.deltas, costs, lossSum, ticket, labels, inLens, labLens,
                            sweep_geom(d), d, g_stream);
       return;
@@ -428,9 +426,8 @@ int loss_forward_any(const void* E, const void* P, const int* labels, const int*
     const SkewGeom g = skew_geom(d);
     const float* Ef = static_cast<const float*>(E);
     const float* Pf = static_cast<const float*>(P);
-    launch_lattice_prep(Ef, Pf, LN, st.LNs, st.ELs, ebl, labels, inLens, labLens, g, d, g_stream,
-                        gathered ? fw.EL : nullptr);
-    launch_alpha_skew(Pf, costs, st.alphas, st.LNs, st.ELs, ebl, g, labels, inLens, labLens, d,
+    launch_lattice_prep(Ef, Pf, LN, st.LNs, st.ELs, st.ebl, labels, inLens, labLens, g, d, g_stream);
+    launch_alpha_skew(Pf, costs, st.alphas, st.LNs, st.ELs, st.ebl, g, labels, inLens, labLens, d,
                       lossSum, ticket, g_stream);
   });
 }
@@ -499,7 +496,7 @@ int loss_backward_any(const void* E, const void* P, const int* labels, const int
     float* egf = static_cast<float*>(egrads);
     float* pgf = static_cast<float*>(pgrads);
     if (sweep_supported(d)) {
-      launch_sweep_backward(ws.sweep, st.arcs, st.alphas, st.deltas, st.LN, st.rowRef, st.maxP,
+      launch_sweep_backward(ws.sweep, Pf, st.ebl, labels, st.arcs, st.alphas, st.deltas, st.LN, st.rowRef, st.maxP,
                             deltas, ws.W, tensorCore ? ws.emT : ws.em,
                             tensorCore ? ws.nref : nullptr, tensorCore ? ws.ebl : ws.eBlank,
                             ws.pBlank, ws.pLabel, inLens, labLens, sweep_geom(d), d, tensorCore,
@@ -510,9 +507,6 @@ int loss_backward_any(const void* E, const void* P, const int* labels, const int
                         inLens, labLens, ws.Ws, ws.EMs, ws.eBlank, ws.pBlank, ws.pLabel, d,
                         g_stream);
       launch_lattice_unskew(ws.Ws, ws.EMs, ws.W, ldW, ws.em, inLens, labLens, g, d, g_stream);
-      if (tensorCore)
-        launch_tc_operands(ws.W, ws.em, ws.eBlank, st.rowRef, deltas, ws.emT, ws.nref, ws.ebl,
-                           inLens, d, g_stream);
     }
     if (tensorCore) {   // (label axes of 129..256 positions: once per half of the axis)
       launch_grads_umma(E, P, st.maxP, ws.W, ws.emT, ws.nref, ws.ebl, ws.pBlank, ws.pLabel, labels,

@@ -701,51 +701,6 @@ __global__ void __launch_bounds__(256) label_overflow_kernel(
   }
 }
 
-// Operands of the gradient kernel from the outputs of the block-wide reverse sweep (label axes
-// of more than 128 positions): W [B,maxT,ldW] = occupancy * exp(ref + maxP - LN), unrounded,
-// becomes delta_b * W rounded to TF32, in place; the label-arc occupancies em [B,maxT,maxU]
-// become emT [B,maxU,ldT] = delta_b * em, frames contiguous; the blank-arc sums eBlank [B,maxT]
-// become ebl [B,ldT] = delta_b * eBlank; rowRef becomes nref = -rowRef * log2(e); all three zero
-// for frames at or beyond T_b.  One CTA per 32 frames x 32 positions.
-__global__ void __launch_bounds__(256) tc_operands_kernel(
-    float* __restrict__ W, const float* __restrict__ em, const float* __restrict__ eBlank,
-    const float* __restrict__ rowRef, const float* __restrict__ deltas, float* __restrict__ emT,
-    float* __restrict__ nref, float* __restrict__ ebl, const int* __restrict__ inLens, int maxT,
-    int maxU, int ldW, int ldT) {
-  __shared__ float tile[32][33];
-  const int b = blockIdx.z, t0 = blockIdx.x * 32, u0 = blockIdx.y * 32;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int T = min(inLens[b], maxT);
-  const float delta = deltas ? deltas[b] : 1.0f;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int tt = w * 4 + k, t = t0 + tt, u = u0 + lane;
-    float e = 0.0f;
-    if (t < maxT) {
-      if (u < ldW) {
-        float* x = W + ((i64)b * maxT + t) * ldW + u;
-        *x = t < T ? tf32_round(*x * delta) : 0.0f;
-      }
-      if (t < T && u < maxU) e = em[((i64)b * maxT + t) * maxU + u] * delta;
-    }
-    tile[tt][lane] = e;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int uu = u0 + w * 4 + k, t = t0 + lane;
-    if (uu < maxU && t < ldT) emT[((i64)b * maxU + uu) * ldT + t] = tile[lane][w * 4 + k];
-  }
-  if (blockIdx.y == 0 && threadIdx.x < 32) {
-    const int t = t0 + lane;
-    if (t < ldT) {
-      const bool ok = t < T;
-      nref[(i64)b * ldT + t] = ok ? -rowRef[(i64)b * maxT + t] * kLog2e : 0.0f;
-      ebl[(i64)b * ldT + t] = ok ? eBlank[(i64)b * maxT + t] * delta : 0.0f;
-    }
-  }
-}
-
 struct TileCfg {
   int TB, SE, SW, EB, DB;
 };
@@ -820,17 +775,6 @@ bool grads_umma_supported(const void* E, const void* P, const void* egrads,
   const int n = std::min(d.maxU, 128);   // positions of the (first) launch
   return pick_tile((int)round_up64(n, 8), (int)round_up64(n, 32), (int)round_up64(n, 16), passes,
                    kStaticSmemBound, bf).TB > 0;
-}
-
-void launch_tc_operands(float* W, const float* em, const float* eBlank, const float* rowRef,
-                        const float* deltas, float* emT, float* nref, float* ebl,
-                        const int* inLens, Dims d, cudaStream_t stream) {
-  if (d.B <= 0 || d.maxT <= 0 || d.maxU <= 0) return;
-  const int ldW = grads_umma_ld_w(d), ldT = grads_umma_ld_t(d);
-  ScopedKernel sk("lattice_tc_operands", stream);
-  tc_operands_kernel<<<dim3(div_up(ldT, 32), div_up(ldW, 32), d.B), 256, 0, stream>>>(
-      W, em, eBlank, rowRef, deltas, emT, nref, ebl, inLens, d.maxT, d.maxU, ldW, ldT);
-  TB200_CHECK_LAUNCH();
 }
 
 void launch_grads_umma(const void* E, const void* P, const float* maxP, const float* W,

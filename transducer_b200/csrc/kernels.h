@@ -46,14 +46,12 @@ struct SkewGeom {
 };
 SkewGeom skew_geom(Dims d);
 
-// Label axes of more than 128 positions (shorter ones: lattice_sweep.cu).
+// Label axes of more than 256 positions (shorter ones: lattice_sweep.cu).
 // LN (row-major) -> LNs (skewed); ELs[t,u] = E[t,label_u] (skewed); ebl[b,t] = E[t,blank].  NaN
-// entries of LN (nodes the tensor-core log-normaliser marked) are recomputed here with the exact
-// fp32 logsumexp.  If ELrow is not null it holds E[t,label_u] as [B,maxU,maxT] (frames contiguous)
-// and ebl is an INPUT (both written by launch_lognorm_umma): nothing is gathered from E here.
+// entries of LN (nodes a factored log-normaliser marked) are recomputed here exactly.
 void launch_lattice_prep(const float* E, const float* P, const float* LN, float* LNs, float* ELs,
                          float* ebl, const int* labels, const int* inLens, const int* labLens,
-                         SkewGeom g, Dims d, cudaStream_t stream, const float* ELrow);
+                         SkewGeom g, Dims d, cudaStream_t stream);
 
 void launch_alpha_skew(const float* P, float* costs, float* alphasS, const float* LNs,
                        const float* ELs, const float* ebl, SkewGeom g, const int* labels,
@@ -125,13 +123,6 @@ int grads_umma_ld_w(Dims d);  // row length of W: maxU rounded up to 32
 int grads_umma_ld_t(Dims d);  // row length of nref / ebl / emT: maxT rounded up to 4
 bool grads_umma_supported(const void* E, const void* P, const void* egrads,
                           const void* pgrads, Dims d, int passes);
-// Operands of launch_grads_umma from the outputs of the block-wide reverse sweep
-// (launch_gamma_skew + launch_lattice_unskew; label axes of more than 128 positions): W is
-// scaled by deltas[b] and rounded to TF32 in place, em [B,maxT,maxU] becomes emT, eBlank becomes
-// ebl, rowRef becomes nref (layouts as written by launch_sweep_backward with tensorCore = true).
-void launch_tc_operands(float* W, const float* em, const float* eBlank, const float* rowRef,
-                        const float* deltas, float* emT, float* nref, float* ebl,
-                        const int* inLens, Dims d, cudaStream_t stream);
 // E, P, egrads and pgrads are of d.dtype (bf16: passes = 2 only, label axes up to 128; fp32:
 // label axes up to 256 positions, those above 128 as two launches over halves of the axis).
 void launch_grads_umma(const void* E, const void* P, const float* maxP, const float* W,
@@ -141,7 +132,7 @@ void launch_grads_umma(const void* E, const void* P, const float* maxP, const fl
                        int* status, cudaStream_t stream);
 
 // ---- lattice_sweep.cu ------------------------------------------------------------
-// Sweeps for label axes of at most 128 positions (file comment there).  Lattices are skewed:
+// Sweeps for label axes of at most 256 positions (file comment there).  Lattices are skewed:
 // node (t,u) of utterance b at b*stride + (t+u)*ld + u (pairs: permuted within the row).
 bool sweep_supported(Dims d);
 struct SweepGeom {
@@ -156,9 +147,10 @@ SweepGeom sweep_geom(Dims d);
 // are recomputed in place first, exactly), alphas, costs [B] (+inf for an empty utterance) and, if
 // lossSum is not null, their sum in index order.  ELrow [B,maxU,maxT] and ebl [B,maxT]: label and
 // blank emissions as written by launch_lognorm_umma, or both null, and they are gathered from E.
-// E and P are of d.dtype.  For the backward call: arcs and alphas [B,stride], deltas [B,nBlk].
+// E and P are of d.dtype.  For the backward call: arcs and alphas [B,stride], deltas [B,nBlk] and,
+// for axes of more than 128 positions, ebl (written here where it is not an input).
 void launch_sweep_forward(const void* E, const void* P, float* LN, const float* ELrow,
-                          const float* ebl, float2* arcs, float* alphas, float* deltas, float* costs,
+                          float* ebl, float2* arcs, float* alphas, float* deltas, float* costs,
                           float* lossSum, unsigned* ticket, const int* labels, const int* inLens,
                           const int* labLens, SweepGeom g, Dims d, cudaStream_t stream);
 struct SweepScratch {   // of the backward call
@@ -176,7 +168,8 @@ size_t sweep_partial_floats(Dims d);
 //               as emT), eBlank [B,maxT] (passed as ebl); nref and deltas unused.  Operands of the
 //               SIMT gradient kernels.
 //   both:       pBlank / pLabel [B,maxU], sums over t of the two occupancies, unscaled.
-void launch_sweep_backward(const SweepScratch& w, const float2* arcs, const float* alphas,
+void launch_sweep_backward(const SweepScratch& w, const float* P, const float* blankEmissions,
+                           const int* labels, const float2* arcs, const float* alphas,
                            const float* alphaDeltas, const float* LN, const float* rowRef,
                            const float* maxP, const float* deltas, float* W, float* emT, float* nref,
                            float* ebl, float* pBlank, float* pLabel, const int* inLens,

@@ -600,23 +600,19 @@ namespace {
 
 // One CTA per 32x32 (t,u) tile.  Reads LN row-major and gathers E[t,label_u]; writes
 // both skewed.  Column tile 0 also writes ebl[t] = E[t,blank].
-// With ELrow ([B,maxU,maxT], frames contiguous, written by the tensor-core log-normaliser
-// together with ebl) the label and blank emissions are read from there, coalesced, instead of
-// being gathered from E one DRAM sector per node.
 __global__ void __launch_bounds__(256) lattice_prep_kernel(
     const float* __restrict__ E, const float* __restrict__ P, const float* __restrict__ LN,
     float* __restrict__ LNs, float* __restrict__ ELs, float* __restrict__ ebl,
-    const float* __restrict__ ELrow, const int* __restrict__ labels,
-    const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT, int maxU, int V,
-    int blank, int ld, i64 latStride) {
-  __shared__ float tLn[32][33], tEl[32][33];
+    const int* __restrict__ labels, const int* __restrict__ inLens,
+    const int* __restrict__ labLens, int maxT, int maxU, int V, int blank, int ld, i64 latStride) {
+  // (even rows: an anti-diagonal of a tile falls into 32 different banks, with 33 into one)
+  __shared__ float tLn[32][34], tEl[32][34];
   const int b = blockIdx.z, t0 = blockIdx.y * 32, u0 = blockIdx.x * 32;
   const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
   if (t0 >= T || u0 >= U) return;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const float* e = E + (i64)b * maxT * V;
   const float* ln = LN + (i64)b * maxT * maxU;
-  const float* elr = ELrow ? ELrow + (i64)b * maxU * maxT : nullptr;
   const int* lab = labels + (i64)b * (maxU - 1);
   const int u = u0 + lane;
   // all loads first (unconditional, clamped into the lattice): the gathers of the four rows
@@ -629,7 +625,7 @@ __global__ void __launch_bounds__(256) lattice_prep_kernel(
     for (int k = 0; k < 4; ++k) {
       const int tc = min(t0 + w * 4 + k, T - 1);
       va[k] = ln[(i64)tc * maxU + uc];
-      vc[k] = elr ? 0.0f : e[(i64)tc * V + labc];
+      vc[k] = e[(i64)tc * V + labc];
     }
   }
 #pragma unroll
@@ -640,7 +636,7 @@ __global__ void __launch_bounds__(256) lattice_prep_kernel(
       a = va[k];
       c = vc[k];
     }
-    // marked by the tensor-core log-normaliser (its factored sum left the fp32 range):
+    // marked by a factored log-normaliser (its sum left the fp32 range):
     // exact logsumexp by the whole warp
     unsigned todo = __ballot_sync(0xffffffffu, a != a);
     while (todo) {
@@ -658,24 +654,16 @@ __global__ void __launch_bounds__(256) lattice_prep_kernel(
       if (lane == src) a = logf(s) + m;
     }
     tLn[tt][lane] = a;
-    if (!elr) tEl[tt][lane] = c;
+    tEl[tt][lane] = c;
   }
-  if (elr) {  // transposed tile load: lane <-> frame, row <-> label position
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int uu = u0 + w * 4 + k, tl = t0 + lane;
-      const float v = elr[(i64)min(uu, max(U - 2, 0)) * maxT + min(tl, T - 1)];
-      tEl[lane][w * 4 + k] = (uu < U - 1 && tl < T) ? v : 0.0f;
-    }
-  }
-  if (threadIdx.x < 32 && !elr && u0 == 0 && t0 + lane < T)
+  if (threadIdx.x < 32 && u0 == 0 && t0 + lane < T)
     ebl[(i64)b * maxT + t0 + lane] = e[(i64)(t0 + lane) * V + blank];
   __syncthreads();
-  // diagonal s = t + u of this tile: s - (t0+u0) in [0, 62]; lane <-> u
-  for (int ds = w; ds < 63; ds += 8) {
-    const int tt = ds - lane;
-    if (tt >= 0 && tt < 32 && t0 + tt < T && u < U) {
-      const i64 o = (i64)b * latStride + (i64)(t0 + u0 + ds) * ld + u;
+  // lane <-> u
+  for (int k = 0; k < 4; ++k) {   // diagonal i of the tile in the lanes up to i, i + 32 in the others
+    const int tt = (w + 8 * k - lane) & 31;
+    if (t0 + tt < T && u < U) {
+      const i64 o = (i64)b * latStride + (i64)(t0 + tt + u) * ld + u;
       LNs[o] = tLn[tt][lane];
       ELs[o] = tEl[tt][lane];
     }
@@ -689,25 +677,24 @@ __global__ void __launch_bounds__(256) lattice_unskew_kernel(
     const float* __restrict__ Ws, const float* __restrict__ EMs, float* __restrict__ W,
     float* __restrict__ em, const int* __restrict__ inLens, const int* __restrict__ labLens,
     int maxT, int maxU, int ld, i64 latStride, int ldW) {
-  __shared__ float tW[32][33], tE[32][33];
+  // (even rows: an anti-diagonal of a tile falls into 32 different banks, with 33 into one)
+  __shared__ float tW[32][34], tE[32][34];
   const int b = blockIdx.z, t0 = blockIdx.y * 32, u0 = blockIdx.x * 32;
   const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int u = u0 + lane;
   const bool live = t0 < T && u0 < U;
   if (live) {
-    for (int ds = w; ds < 63; ds += 8) {
-      const int tt = ds - lane;
-      if (tt >= 0 && tt < 32) {
-        float a = 0.0f, c = 0.0f;
-        if (t0 + tt < T && u < U) {
-          const i64 o = (i64)b * latStride + (i64)(t0 + u0 + ds) * ld + u;
-          a = Ws[o];
-          c = EMs[o];
-        }
-        tW[tt][lane] = a;
-        tE[tt][lane] = c;
+    for (int k = 0; k < 4; ++k) {   // diagonal i of the tile in the lanes up to i, i + 32 in the others
+      const int tt = (w + 8 * k - lane) & 31;
+      float a = 0.0f, c = 0.0f;
+      if (t0 + tt < T && u < U) {
+        const i64 o = (i64)b * latStride + (i64)(t0 + tt + u) * ld + u;
+        a = Ws[o];
+        c = EMs[o];
       }
+      tW[tt][lane] = a;
+      tE[tt][lane] = c;
     }
   }
   __syncthreads();
@@ -724,11 +711,11 @@ __global__ void __launch_bounds__(256) lattice_unskew_kernel(
 
 void launch_lattice_prep(const float* E, const float* P, const float* LN, float* LNs, float* ELs,
                          float* ebl, const int* labels, const int* inLens, const int* labLens,
-                         SkewGeom g, Dims d, cudaStream_t stream, const float* ELrow) {
+                         SkewGeom g, Dims d, cudaStream_t stream) {
   if (d.B <= 0 || d.maxT <= 0 || d.maxU <= 0) return;
   dim3 grid(div_up(d.maxU, 32), div_up(d.maxT, 32), d.B);
   ScopedKernel sk("lattice_prep", stream);
-  lattice_prep_kernel<<<grid, 256, 0, stream>>>(E, P, LN, LNs, ELs, ebl, ELrow, labels, inLens, labLens,
+  lattice_prep_kernel<<<grid, 256, 0, stream>>>(E, P, LN, LNs, ELs, ebl, labels, inLens, labLens,
                                                 d.maxT, d.maxU, d.V, d.blank, g.ld, g.stride);
   TB200_CHECK_LAUNCH();
 }

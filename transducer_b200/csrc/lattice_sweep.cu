@@ -1,4 +1,4 @@
-// Lattice sweeps for label axes of at most 128 positions: each recursion runs in ONE warp per
+// Lattice sweeps for label axes of at most 256 positions: each recursion runs in ONE warp per
 // utterance, and everything that does not depend on the recursion in kernels of its own that use
 // the whole GPU.
 //
@@ -11,6 +11,10 @@
 //   alpha   transducer/transducer_cpu.cpp:30-79   (transducer_cuda.cu:32-97)
 //   reverse transducer/transducer_cpu.cpp:81-143  (transducer_cuda.cu:99-176)
 //
+// Axes of up to 128 positions run on rebased base-2 logarithms (alpha_sweep_kernel); longer ones
+// (NPL >= 5, "natural" below) on natural logarithms at full magnitude, in the operation order of the
+// block-wide kernels of lattice.cu and bit-identical to them.
+//
 // Diagonal d = t + u of an utterance is one row of ld = 32 NPL numbers; lane l of a sweep owns the
 // NPL adjacent positions u = NPL l + r.  All nodes of a diagonal are independent; the one value
 // per lane that crosses from the neighbouring lane arrives by a warp shuffle.  A sweep is a chain
@@ -18,6 +22,12 @@
 // diagonal takes: operands are brought to shared memory by cp.async, each lane copying just the
 // 8 NPL bytes a row that it reads itself (no barrier, no other warp), several blocks of 16
 // diagonals ahead, and the loop holds nothing but the recursion and its store.
+// Measured (T = 2000, U' = 101, device time, B = 8 / 32): alpha 128 us (140 with bulk copies issued and
+// waited for by the sweeping warp); reverse sweep 10 / 21 us for the factors + 57 us for the recursion
+// (146 us when helper warps of the same CTA prepared the factors and carried away the results).
+// B = 64, T = 750..1500, U' = 151: alpha 213 us, factors 62 + recursion 73 us, operands 125 us, against
+// 381, 511 and (lattices re-laid out twice) 168 us of the block-wide kernels, which take a barrier
+// per diagonal.
 #include <algorithm>
 
 #include "kernels.h"
@@ -30,7 +40,9 @@ namespace {
 using namespace sm100;
 
 constexpr int kDiag = 16;   // diagonals per block
-constexpr int kRing = 4;    // blocks in shared memory
+// blocks in shared memory (three of the wide ones leave room for two CTAs per SM)
+__host__ __device__ constexpr int ring_blocks(int npl) { return npl <= 4 ? 4 : 3; }
+__host__ __device__ constexpr bool natural(int npl) { return npl > 4; }
 constexpr float kLn2F = 0.6931471805599453f;
 constexpr float kLog2e = 1.4426950408889634f;
 // "No such arc": a large negative finite number, the identity of the alpha recursion without -inf
@@ -43,45 +55,53 @@ __device__ __forceinline__ float lg2_approx(float x) {
   return y;
 }
 
-// Place of position u within a row of pairs (arcs, factors): 16-byte pieces of two positions, the
-// pieces of the 32 lanes side by side, so that a warp's 16-byte accesses are contiguous.
+// Place of position u within a row of pairs (operands, factors): 16-byte pieces of two positions,
+// the pieces of the 32 lanes side by side, so that a warp's 16-byte accesses are contiguous; the
+// last position of an odd NPL makes a piece of its own.
 __host__ __device__ constexpr int pair_slot(int u, int npl) {
-  return npl == 1 ? u : (((u % npl) >> 1) * 32 + u / npl) * 2 + (u % npl & 1);
+  const int lane = u / npl, r = u % npl, q = r >> 1;
+  return q < npl / 2 ? (q * 32 + lane) * 2 + (r & 1) : q * 64 + lane;
+}
+// Place of position u within a row of single numbers (alphas, g): as it comes where a lane's
+// positions make one vector access, else one plane of 32 lanes per position of a lane.
+__host__ __device__ constexpr int row_slot(int u, int npl) {
+  return npl <= 4 ? u : (u % npl) * 32 + u / npl;
 }
 
 // Copies blocks of pair rows into this lane's share of a shared-memory ring and reads them back.
 // Lanes without positions of the utterance hold `fill` throughout.
 template <int NPL>
 struct PairRing {
-  static constexpr int ld = 32 * NPL, kRowBytes = ld * 8;
-  static constexpr int kPieces = NPL == 1 ? 1 : NPL / 2, kPiece = NPL == 1 ? 8 : 16;
-  uint8_t* mine;
+  static constexpr int ld = 32 * NPL, kRowBytes = ld * 8, kRing = ring_blocks(NPL);
+  static constexpr int kPieces = NPL / 2, kOdd = kPieces * 512;   // byte offset of the odd position's plane
+  uint8_t* ring;
   const uint8_t* src;
+  int lane;
   bool act;
-  __device__ PairRing(uint8_t* ring, const float2* rows, int lane, int U, unsigned fill)
-      : mine(ring + lane * kPiece), src(reinterpret_cast<const uint8_t*>(rows) + lane * kPiece), act(NPL * lane < U) {
+  __device__ PairRing(uint8_t* ring_, const float2* rows, int lane_, int U, unsigned fillX, unsigned fillY)
+      : ring(ring_), src(reinterpret_cast<const uint8_t*>(rows)), lane(lane_), act(NPL * lane_ < U) {
     if (!act)
-      for (int i = 0; i < kRing * kDiag; ++i)
+      for (int i = 0; i < kRing * kDiag; ++i) {
+        uint8_t* row = ring + i * kRowBytes;
 #pragma unroll
-        for (int q = 0; q < kPieces; ++q) {
-          uint2* z = reinterpret_cast<uint2*>(mine + i * kRowBytes + q * 32 * kPiece);
-          z[0] = make_uint2(fill, fill);
-          if (kPiece == 16) z[1] = make_uint2(fill, fill);
-        }
+        for (int q = 0; q < kPieces; ++q)
+          *reinterpret_cast<uint4*>(row + (q * 32 + lane) * 16) = make_uint4(fillX, fillY, fillX, fillY);
+        if (NPL & 1) *reinterpret_cast<uint2*>(row + kOdd + lane * 8) = make_uint2(fillX, fillY);
+      }
   }
   // rows [row, row + n) -> slot
   __device__ __forceinline__ void issue(int slot, i64 row, int n) {
     if (act) {
-      const uint32_t dst = smem_u32(mine) + (uint32_t)slot * (kDiag * kRowBytes);
-      const uint8_t* from = src + row * kRowBytes;
+      const uint32_t dst = smem_u32(ring) + (uint32_t)slot * (kDiag * kRowBytes) + lane * 16;
+      const uint8_t* from = src + row * kRowBytes + lane * 16;
       auto one = [&](int i) {
 #pragma unroll
-        for (int q = 0; q < kPieces; ++q) {
-          const uint32_t to = dst + i * kRowBytes + q * 32 * kPiece;
-          const uint8_t* f = from + i * kRowBytes + q * 32 * kPiece;
-          if (kPiece == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(f) : "memory");
-          else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to), "l"(f) : "memory");
-        }
+        for (int q = 0; q < kPieces; ++q)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * kRowBytes + q * 512),
+                       "l"(from + i * kRowBytes + q * 512) : "memory");
+        if (NPL & 1)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + i * kRowBytes + kOdd - lane * 8),
+                       "l"(from + i * kRowBytes + kOdd - lane * 8) : "memory");
       };
       if (n == kDiag) {
 #pragma unroll
@@ -97,32 +117,37 @@ struct PairRing {
   __device__ __forceinline__ void wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 1) : "memory"); }
   __device__ __forceinline__ void drain() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
   __device__ __forceinline__ void read(int slot, int i, float (&x)[NPL], float (&y)[NPL]) const {
-    const uint8_t* p = mine + (slot * kDiag + i) * kRowBytes;
-    if constexpr (NPL == 1) {
-      const float2 f = *reinterpret_cast<const float2*>(p);
-      x[0] = f.x;
-      y[0] = f.y;
-    } else {
+    const uint8_t* p = ring + (slot * kDiag + i) * kRowBytes;
 #pragma unroll
-      for (int q = 0; q < kPieces; ++q) {
-        const float4 f = *reinterpret_cast<const float4*>(p + q * 32 * kPiece);
-        x[2 * q] = f.x;
-        y[2 * q] = f.y;
-        x[2 * q + 1] = f.z;
-        y[2 * q + 1] = f.w;
-      }
+    for (int q = 0; q < kPieces; ++q) {
+      const float4 f = *reinterpret_cast<const float4*>(p + (q * 32 + lane) * 16);
+      x[2 * q] = f.x;
+      y[2 * q] = f.y;
+      x[2 * q + 1] = f.z;
+      y[2 * q + 1] = f.w;
+    }
+    if constexpr (NPL & 1) {
+      const float2 f = *reinterpret_cast<const float2*>(p + kOdd + lane * 8);
+      x[NPL - 1] = f.x;
+      y[NPL - 1] = f.y;
     }
   }
 };
 
+// A lane's numbers of a row (row points at its beginning).
 template <int NPL>
-__device__ __forceinline__ void store_row(float* q, const float (&a)[NPL]) {
+__device__ __forceinline__ void store_row(float* row, int lane, const float (&a)[NPL]) {
+  float* q = row + NPL * lane;
   if constexpr (NPL == 4) *reinterpret_cast<float4*>(q) = make_float4(a[0], a[1], a[2], a[3]);
   else if constexpr (NPL == 2) *reinterpret_cast<float2*>(q) = make_float2(a[0], a[1]);
-  else q[0] = a[0];
+  else {
+#pragma unroll
+    for (int r = 0; r < NPL; ++r) row[r * 32 + lane] = a[r];
+  }
 }
 template <int NPL>
-__device__ __forceinline__ void load_row(const float* q, float (&a)[NPL]) {
+__device__ __forceinline__ void load_row(const float* row, int lane, float (&a)[NPL]) {
+  const float* q = row + NPL * lane;
   if constexpr (NPL == 4) {
     const float4 f = *reinterpret_cast<const float4*>(q);
     a[0] = f.x; a[1] = f.y; a[2] = f.z; a[3] = f.w;
@@ -130,7 +155,8 @@ __device__ __forceinline__ void load_row(const float* q, float (&a)[NPL]) {
     const float2 f = *reinterpret_cast<const float2*>(q);
     a[0] = f.x; a[1] = f.y;
   } else {
-    a[0] = q[0];
+#pragma unroll
+    for (int r = 0; r < NPL; ++r) a[r] = row[r * 32 + lane];
   }
 }
 
@@ -185,11 +211,12 @@ __global__ void __launch_bounds__(32) alpha_sweep_kernel(
     return;
   }
   const int S = T + U - 1, nBlocks = (S + kDiag - 1) / kDiag, u0 = NPL * lane;
-  PairRing<NPL> ring(smemA, arcs + (i64)b * stride, lane, U, kNoArcBits);
+  constexpr int kRing = ring_blocks(NPL);
+  PairRing<NPL> ring(smemA, arcs + (i64)b * stride, lane, U, kNoArcBits, kNoArcBits);
   auto issue = [&](int k) { ring.issue(k % kRing, (i64)k * kDiag, k < nBlocks ? min(kDiag, S - k * kDiag) : 0); };
 #pragma unroll
   for (int k = 0; k < kRing - 1; ++k) issue(k);
-  float* al = alphas + (i64)b * stride + u0;
+  float* al = alphas + (i64)b * stride;
   float* dl = deltas + (i64)b * ((nDiag + kDiag - 1) / kDiag);
   const float kNone = __uint_as_float(kNoArcBits);
   float stayIn[NPL], stepOut[NPL];
@@ -245,7 +272,7 @@ __global__ void __launch_bounds__(32) alpha_sweep_kernel(
         stepOut[r] = a[r] + fy[r];
         if (r == NPL - 1) up = __shfl_up_sync(0xffffffffu, stepOut[NPL - 1], 1);
       }
-      if (ring.act) store_row<NPL>(out + i * ld, a);
+      if (ring.act) store_row<NPL>(out + i * ld, lane, a);
     };
     if (nd == kDiag) {
 #pragma unroll
@@ -262,6 +289,104 @@ __global__ void __launch_bounds__(32) alpha_sweep_kernel(
     if (u0 + r == U - 1) finish_cost(costs, b, -(stayIn[r] + offset) * kLn2F, B, lossSum, ticket);
 }
 
+// What the natural sweeps know of an utterance's positions besides the pair rows.
+struct NaturalTerms {
+  const float* P;        // [B,maxU,V]
+  const float* ebl;      // [B,maxT] blank emissions
+  const int* labels;
+  int V, blank;
+};
+
+// log(exp(a)+exp(b)) with the reference's -inf handling and operation order; the correction term
+// is evaluated with the hardware ex2/lg2 units (absolute error ~2e-7, far below one ulp of the
+// alphas it is added to once they exceed a few units in magnitude).
+__device__ __forceinline__ float lse2_fast(float a, float b) {
+  // (one of them -inf: the correction is log(1 + 0) = 0 by itself; branches would cost more than the
+  // sum: 895 instead of ~200 cycles per diagonal)
+  const float m = fmaxf(a, b), v = m + __logf(1.0f + __expf(-fabsf(a - b)));
+  return (m == neg_inf() && a == b) ? m : v;
+}
+
+// Label axes of 129..256 positions: pair rows (LN, E[t,label_u]), (+inf, 0) where there is no node,
+// so that whatever leaves such a node is -inf.  E[t,blank] of a lane's first position is read from
+// shared memory (the first maxStage frames; beyond, from global), the others' follow from it:
+// position r + 1 meets a frame one diagonal after position r.
+template <int NPL>
+__global__ void __launch_bounds__(32) alpha_natural_kernel(
+    const float2* __restrict__ rows, const NaturalTerms n, float* __restrict__ costs,
+    float* __restrict__ alphas, i64 stride, const int* __restrict__ inLens,
+    const int* __restrict__ labLens, int B, int maxT, int maxU, int maxStage, float* lossSum,
+    unsigned* ticket) {
+  constexpr int ld = 32 * NPL, kRing = ring_blocks(NPL);
+  extern __shared__ __align__(128) uint8_t smemA[];
+  const int b = blockIdx.x, lane = threadIdx.x;
+  const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
+  if (T <= 0 || U <= 0) {
+    if (lane == 0) finish_cost(costs, b, pos_inf(), B, lossSum, ticket);
+    return;
+  }
+  const int S = T + U - 1, nBlocks = (S + kDiag - 1) / kDiag, u0 = NPL * lane;
+  PairRing<NPL> ring(smemA, rows + (i64)b * stride, lane, U, 0x7f800000u, 0u);
+  auto issue = [&](int k) { ring.issue(k % kRing, (i64)k * kDiag, k < nBlocks ? min(kDiag, S - k * kDiag) : 0); };
+#pragma unroll
+  for (int k = 0; k < kRing - 1; ++k) issue(k);
+  const float* ebl = n.ebl + (i64)b * maxT;
+  float* sEb = reinterpret_cast<float*>(smemA + kRing * kDiag * ld * 8);
+  for (int t = lane; t < min(T, maxStage); t += 32) sEb[t] = ebl[t];
+  __syncwarp();
+  const float* ebRow = T <= maxStage ? sEb : ebl;
+  auto eblAt = [&](int t) { return ebRow[min(max(t, 0), T - 1)]; };
+  float* al = alphas + (i64)b * stride;
+  float pbl[NPL], plab[NPL], eb[NPL], stay[NPL], step[NPL];
+#pragma unroll
+  for (int r = 0; r < NPL; ++r) {
+    const int u = u0 + r, uc = min(u, U - 1);
+    const float* p = n.P + ((i64)b * maxU + uc) * n.V;
+    pbl[r] = p[n.blank];
+    plab[r] = u < U - 1 ? p[n.labels[(i64)b * (maxU - 1) + u]] : 0.0f;
+    eb[r] = eblAt(-u);
+    stay[r] = step[r] = neg_inf();
+  }
+  if (lane == 0) stay[0] = 0.0f;   // alpha(0,0) = 0
+  float up = neg_inf();
+  for (int k = 0; k < nBlocks; ++k) {
+    issue(k + kRing - 1);
+    ring.wait();
+    const int slot = k % kRing, nd = min(kDiag, S - k * kDiag);
+    float* out = al + (i64)k * kDiag * ld;
+    const int tNext = k * kDiag + 1 - u0;   // frame of position u0 on the diagonal after the block's first
+    auto diag = [&](int i) {
+      float lnv[NPL], el[NPL], a[NPL];
+      ring.read(slot, i, lnv, el);
+      const float ebNext = eblAt(tNext + i), first = lane ? up : neg_inf();
+      // the last position first, whose step leaves by a shuffle; each position still needs the
+      // previous diagonal's step of the one below it
+#pragma unroll
+      for (int r = NPL - 1; r >= 0; --r) {
+        a[r] = lse2_fast(r ? step[(r + NPL - 1) % NPL] : first, stay[r]);
+        stay[r] = ((a[r] + eb[r]) + pbl[r]) - lnv[r];
+        step[r] = ((a[r] + el[r]) + plab[r]) - lnv[r];
+        if (r == NPL - 1) up = __shfl_up_sync(0xffffffffu, step[r], 1);
+      }
+#pragma unroll
+      for (int r = NPL - 1; r > 0; --r) eb[r] = eb[r - 1];
+      eb[0] = ebNext;
+      if (ring.act) store_row<NPL>(out + i * ld, lane, a);
+    };
+    if (nd == kDiag) {
+#pragma unroll
+      for (int i = 0; i < kDiag; ++i) diag(i);
+    } else {
+#pragma unroll 1
+      for (int i = 0; i < nd; ++i) diag(i);
+    }
+  }
+  ring.drain();
+#pragma unroll
+  for (int r = 0; r < NPL; ++r)
+    if (u0 + r == U - 1) finish_cost(costs, b, -stay[r], B, lossSum, ticket);
+}
+
 // ---------------------------------------------------------------------------
 // reverse occupancy sweep
 // ---------------------------------------------------------------------------
@@ -276,15 +401,16 @@ __global__ void __launch_bounds__(32) alpha_sweep_kernel(
 //   g(t,u) = stay + step,            g(T-1,U-1) = 1 (the terminating blank, booked as stay)
 //
 // gamma_factors_kernel: the pairs (FB, FL) of every node of the diagonals below S, zero where there
-// is no arc.  One warp per 4 diagonals.  Bound by memory: 16 bytes read, 8 written per node.
+// is no arc (natural: from the pair rows of alpha_natural_kernel, by the accurate expf).  One warp
+// per 4 diagonals.  Bound by memory: 16 bytes read, 8 written per node.
 constexpr int kFactorRows = 4, kFactorWarps = 8;
 template <int NPL>
 __global__ void __launch_bounds__(32 * kFactorWarps) gamma_factors_kernel(
     const float2* __restrict__ arcs, const float* __restrict__ alphas,
-    const float* __restrict__ deltas, float2* __restrict__ F, unsigned* __restrict__ occTicket,
-    i64 stride, int nDiag, const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT,
+    const float* __restrict__ deltas, const NaturalTerms n, float2* __restrict__ F,
+    unsigned* __restrict__ occTicket, i64 stride, int nDiag, const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT,
     int maxU) {
-  constexpr int ld = 32 * NPL, kPieces = NPL == 1 ? 1 : NPL / 2;
+  constexpr int ld = 32 * NPL, kPieces = NPL / 2;
   const int b = blockIdx.y, lane = threadIdx.x & 31;
   if (blockIdx.x == 0 && threadIdx.x == 0) occTicket[b] = 0u;
   const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU), S = T + U - 1;
@@ -292,51 +418,69 @@ __global__ void __launch_bounds__(32 * kFactorWarps) gamma_factors_kernel(
   if (T <= 0 || U <= 0 || d0 >= S || u0 >= U) return;
   const float* al = alphas + (i64)b * stride;
   const float* dl = deltas + (i64)b * ((nDiag + kDiag - 1) / kDiag);
-  const int uNext = min(u0 + NPL, ld - 1);   // (position 127 has no label arc)
-  float a[kFactorRows + 1][NPL], aN[kFactorRows + 1];
-  float4 f[kFactorRows][kPieces];
+  const int next = row_slot(min(u0 + NPL, ld - 1), NPL);   // (the last position has no label arc)
+  float a[kFactorRows + 1][NPL], aN[kFactorRows + 1], x[kFactorRows][NPL], y[kFactorRows][NPL];
 #pragma unroll
   for (int i = 0; i <= kFactorRows; ++i) {
     const i64 row = (i64)min(d0 + i, S - 1) * ld;
-    load_row<NPL>(al + row + u0, a[i]);
-    aN[i] = al[row + uNext];
+    load_row<NPL>(al + row, lane, a[i]);
+    aN[i] = al[row + next];
     if (i < kFactorRows) {
       const float2* ar = arcs + (i64)b * stride + row;
 #pragma unroll
       for (int q = 0; q < kPieces; ++q) {
-        if constexpr (NPL == 1) {
-          const float2 x = ar[lane];
-          f[i][q] = make_float4(x.x, x.y, 0.0f, 0.0f);
-        } else {
-          f[i][q] = reinterpret_cast<const float4*>(ar)[q * 32 + lane];
-        }
+        const float4 f = reinterpret_cast<const float4*>(ar)[q * 32 + lane];
+        x[i][2 * q] = f.x;
+        y[i][2 * q] = f.y;
+        x[i][2 * q + 1] = f.z;
+        y[i][2 * q + 1] = f.w;
       }
+      if constexpr (NPL & 1) {
+        const float2 f = ar[kPieces * 64 + lane];
+        x[i][NPL - 1] = f.x;
+        y[i][NPL - 1] = f.y;
+      }
+    }
+  }
+  float pbl[NPL], plab[NPL];
+  if constexpr (natural(NPL)) {
+#pragma unroll
+    for (int r = 0; r < NPL; ++r) {
+      const int u = u0 + r;
+      const float* p = n.P + ((i64)b * maxU + min(u, U - 1)) * n.V;
+      pbl[r] = p[n.blank];
+      plab[r] = u < U - 1 ? p[n.labels[(i64)b * (maxU - 1) + u]] : 0.0f;
     }
   }
 #pragma unroll
   for (int i = 0; i < kFactorRows; ++i) {
     const int d = d0 + i;
     if (d >= S) break;
-    // the successors' diagonal opens a block: the carried sums were lowered by its delta
-    const float dlt = ((d + 1) % kDiag == 0 && d + 1 < S) ? dl[(d + 1) / kDiag] : 0.0f;
-    float x[NPL], y[NPL];
+    // (rebased) the successors' diagonal opens a block: the carried sums were lowered by its delta
+    const float dlt = (!natural(NPL) && (d + 1) % kDiag == 0 && d + 1 < S) ? dl[(d + 1) / kDiag] : 0.0f;
 #pragma unroll
     for (int r = 0; r < NPL; ++r) {
       const int u = u0 + r, t = d - u;
       const bool valid = u < U && t >= 0 && t < T;
-      const float4 q = f[i][r / 2];
-      const float ax = r % 2 ? q.z : q.x, ay = r % 2 ? q.w : q.y;
-      x[r] = (valid && t < T - 1) ? ex2_approx(((a[i][r] + ax) - dlt) - a[i + 1][r]) : 0.0f;
-      if (t == T - 1 && u == U - 1) x[r] = 1.0f;   // terminating blank, fed by g(T,U-1) := 1
       const float art = r < NPL - 1 ? a[i + 1][(r + 1) % NPL] : aN[i + 1];
-      y[r] = (valid && u < U - 1) ? ex2_approx(((a[i][r] + ay) - dlt) - art) : 0.0f;
+      float fb, fl;
+      if constexpr (natural(NPL)) {
+        const float eb = n.ebl[(i64)b * maxT + min(max(t, 0), T - 1)], lnv = x[i][r], el = y[i][r];
+        fb = expf((((a[i][r] + eb) + pbl[r]) - lnv) - a[i + 1][r]);
+        fl = expf((((a[i][r] + el) + plab[r]) - lnv) - art);
+      } else {
+        fb = ex2_approx(((a[i][r] + x[i][r]) - dlt) - a[i + 1][r]);
+        fl = ex2_approx(((a[i][r] + y[i][r]) - dlt) - art);
+      }
+      x[i][r] = (valid && t < T - 1) ? fb : 0.0f;
+      if (t == T - 1 && u == U - 1) x[i][r] = 1.0f;   // terminating blank, fed by g(T,U-1) := 1
+      y[i][r] = (valid && u < U - 1) ? fl : 0.0f;
     }
     float2* out = F + (i64)b * stride + (i64)d * ld;
 #pragma unroll
-    for (int q = 0; q < kPieces; ++q) {
-      if constexpr (NPL == 1) out[lane] = make_float2(x[0], y[0]);
-      else reinterpret_cast<float4*>(out)[q * 32 + lane] = make_float4(x[(2 * q) % NPL], y[(2 * q) % NPL], x[(2 * q + 1) % NPL], y[(2 * q + 1) % NPL]);
-    }
+    for (int q = 0; q < kPieces; ++q)
+      reinterpret_cast<float4*>(out)[q * 32 + lane] = make_float4(x[i][2 * q], y[i][2 * q], x[i][2 * q + 1], y[i][2 * q + 1]);
+    if constexpr (NPL & 1) out[kPieces * 64 + lane] = make_float2(x[i][NPL - 1], y[i][NPL - 1]);
   }
 }
 
@@ -352,7 +496,8 @@ __global__ void __launch_bounds__(32) gamma_sweep_kernel(
   const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
   if (T <= 0 || U <= 0) return;
   const int S = T + U - 1, nBlocks = (S + kDiag - 1) / kDiag, u0 = NPL * lane;
-  PairRing<NPL> ring(smemG, F + (i64)b * stride, lane, U, 0u);
+  constexpr int kRing = ring_blocks(NPL);
+  PairRing<NPL> ring(smemG, F + (i64)b * stride, lane, U, 0u, 0u);
   // block k holds the rows [max(S - 16(k+1), 0), S - 16k)
   auto issue = [&](int k) {
     const int lo = max(S - kDiag * (k + 1), 0);
@@ -360,11 +505,11 @@ __global__ void __launch_bounds__(32) gamma_sweep_kernel(
   };
 #pragma unroll
   for (int k = 0; k < kRing - 1; ++k) issue(k);
-  float* out0 = g + (i64)b * stride + u0;
+  float* out0 = g + (i64)b * stride;
   float s[NPL];
 #pragma unroll
   for (int r = 0; r < NPL; ++r) s[r] = (u0 + r == U - 1) ? 1.0f : 0.0f;
-  if (ring.act) store_row<NPL>(out0 + (i64)S * ld, s);
+  if (ring.act) store_row<NPL>(out0 + (i64)S * ld, lane, s);
   // (lane 31 gets its own s[0] back: harmless, the label arc of its last position never exists)
   float right = __shfl_down_sync(0xffffffffu, s[0], 1);
   for (int k = 0; k < nBlocks; ++k) {
@@ -386,7 +531,7 @@ __global__ void __launch_bounds__(32) gamma_sweep_kernel(
       }
 #pragma unroll
       for (int r = 0; r < NPL; ++r) s[r] = n[r];
-      if (ring.act) store_row<NPL>(out + i * ld, s);
+      if (ring.act) store_row<NPL>(out + i * ld, lane, s);
     };
     if (nd == kDiag) {
 #pragma unroll
@@ -407,7 +552,7 @@ struct PrepParams {
   const void* P;
   float* LN;                 // [B,maxT,maxU]; marked nodes are recomputed in place
   const float* ELrow;        // [B,maxU,maxT] label emissions, or null
-  const float* ebl;          // [B,maxT] blank emissions (with ELrow)
+  float* ebl;                // [B,maxT] blank emissions: read with ELrow, else written for the natural sweeps
   float2* arcs;
   const int* labels;
   const int* inLens;
@@ -420,13 +565,20 @@ struct PrepParams {
 // node, written along the diagonals,
 //   (E[t,blank]   + P[u,blank]   - LN[t,u]) * log2(e)
 //   (E[t,label_u] + P[u,label_u] - LN[t,u]) * log2(e),  u < U-1
+// or, for the natural sweeps, (LN[t,u], E[t,label_u]).
 // The tiles beyond both ends of the time axis (`extra` of them on each side) write the "no such
 // arc" of nodes outside the lattice, so that the array needs no fill.  Log-normalisers marked by
 // the tensor-core kernel (NaN) are recomputed exactly first.
 // Bound by memory: reads 8 and writes 8 bytes per node.
+// Row length of a 32x32 tile in shared memory that is written by rows and read along the
+// anti-diagonals (or the other way): element (d - lane, lane) is at d * ld - (ld - 1) * lane, so ld
+// has to be even for 32 different banks -- 33 would put a whole anti-diagonal into one -- and 34
+// keeps columns at a two-way conflict.  (33 -> 34 and two rows per access: sweep_prep 62 -> 38 us at
+// B = 32, T = 2000, U' = 101.)
+constexpr int kTileLd = 34;
 template <typename TIn>
 __global__ void __launch_bounds__(256) sweep_prep_kernel(const PrepParams p) {
-  __shared__ float tLn[32][33], tEl[32][33], tEb[32];
+  __shared__ float tLn[32][kTileLd], tEl[32][kTileLd], tEb[32];
   const int b = blockIdx.z, t0 = ((int)blockIdx.y - p.extra) * 32, u0 = blockIdx.x * 32;
   const int T = min(p.inLens[b], p.maxT), U = min(p.labLens[b] + 1, p.maxU);
   if (T <= 0 || U <= 0) return;
@@ -459,6 +611,7 @@ __global__ void __launch_bounds__(256) sweep_prep_kernel(const PrepParams p) {
     if (threadIdx.x < 32) {
       const int tc = min(t0 + lane, T - 1);
       tEb[lane] = elr ? p.ebl[(i64)b * p.maxT + tc] : to_f32(e[(i64)tc * p.V + p.blank]);
+      if (!elr && natural(p.npl) && u0 == 0) p.ebl[(i64)b * p.maxT + tc] = tEb[lane];
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -488,14 +641,19 @@ __global__ void __launch_bounds__(256) sweep_prep_kernel(const PrepParams p) {
     }
   }
   __syncthreads();
-  for (int ds = w; ds < 63; ds += 8) {
-    const int tt = ds - lane, t = t0 + tt, d = t0 + u0 + ds;
-    if (tt < 0 || tt > 31 || d < 0 || d >= S || u >= Uw) continue;
-    float2 f = make_float2(__uint_as_float(kNoArcBits), __uint_as_float(kNoArcBits));
+  // (lane <-> position; step i takes diagonal i of the tile in the lanes up to i and diagonal
+  // i + 32 in the others: every lane has a node and a warp touches two rows)
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int tt = (w + 8 * k - lane) & 31, t = t0 + tt, d = t + u;
+    if (d < 0 || d >= S || u >= Uw) continue;
+    const bool nat = natural(p.npl);
+    float2 f = nat ? make_float2(pos_inf(), 0.0f)
+                   : make_float2(__uint_as_float(kNoArcBits), __uint_as_float(kNoArcBits));
     if (t >= 0 && t < T && u < U) {
       const float lnv = tLn[tt][lane];
-      f.x = ((tEb[tt] + pbl) - lnv) * kLog2e;
-      if (u < U - 1) f.y = ((tEl[tt][lane] + plab) - lnv) * kLog2e;
+      f.x = nat ? lnv : ((tEb[tt] + pbl) - lnv) * kLog2e;
+      if (u < U - 1) f.y = nat ? tEl[tt][lane] : ((tEl[tt][lane] + plab) - lnv) * kLog2e;
     }
     arcs[(i64)d * p.ld] = f;
   }
@@ -516,8 +674,8 @@ struct OccParams {
   i64 stride;
 };
 
-// One CTA per 32 frames of one utterance, the (up to four) 32x32 lattice tiles of the label axis
-// side by side.  With delta_b the upstream gradient:
+// One CTA per 32 frames of one utterance, the 32x32 lattice tiles of the label axis side by side,
+// kOccWarps warps each.  With delta_b the upstream gradient:
 //   stay(t,u) = g(t+1,u) FB(t,u), step(t,u) = g(t,u+1) FL(t,u)
 //   W [B,maxT,ldW] = delta_b * (stay + step) * exp(ref(t) + maxP(u) - LN(t,u)), rounded to TF32
 //                   (round-to-nearest; the tensor core would otherwise truncate), zero outside
@@ -535,13 +693,21 @@ struct OccParams {
 // [B,maxT,maxU] (through emT), the row sums with row length maxT (through ebl), no nref.
 // Bound by memory: 16 bytes read and 8 written per node.
 constexpr int kOccWarps = 4;              // warps per 32 label positions
-constexpr int kOccThreads = 4 * 32 * kOccWarps;
 constexpr int kOccRows = 32 / kOccWarps;  // frames (diagonals of the tile) per warp
-template <bool TC>
-__global__ void __launch_bounds__(kOccThreads, 2) occupancy_kernel(const OccParams p) {
-  __shared__ float tS[4][32][33], tE[4][32][33];
-  __shared__ float sRow[4][32], sCol[kOccWarps][2][128];
-  __shared__ int sLast;
+// shared memory in floats: two tiles per 32 positions, row sums, column sums per warp, a flag
+__host__ __device__ constexpr int occ_smem_floats(int blocks) {
+  return blocks * (2 * 32 * kTileLd + 32 + 2 * 32 * kOccWarps) + 4;
+}
+template <bool TC, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS <= 640 ? 2 : 1) occupancy_kernel(const OccParams p) {
+  using Tile = float[32][kTileLd];
+  extern __shared__ __align__(16) float smemO[];
+  const int blocks = p.ldW / 32, cols = p.ldW;   // blocks of 32 positions
+  Tile* tS = reinterpret_cast<Tile*>(smemO);
+  Tile* tE = tS + blocks;
+  float* sRow = reinterpret_cast<float*>(tE + blocks);   // [blocks][32]
+  float* sCol = sRow + cols;                             // [kOccWarps][2][cols]
+  int* sLast = reinterpret_cast<int*>(sCol + 2 * kOccWarps * cols);
   const int b = blockIdx.y, t0 = blockIdx.x * 32;
   const int T = min(p.inLens[b], p.maxT), U = min(p.labLens[b] + 1, p.maxU);
   const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) % kOccWarps, ub = threadIdx.x / (32 * kOccWarps);
@@ -550,8 +716,7 @@ __global__ void __launch_bounds__(kOccThreads, 2) occupancy_kernel(const OccPara
   const bool some = T > 0 && U > 0 && t0 < T;
   float* part = p.partial + ((i64)b * gridDim.x + blockIdx.x) * 2 * p.maxU;
   const int u0 = ub * 32, u = u0 + lane;
-  const bool inRange = u0 < p.ldW;
-  const bool live = inRange && some && u0 < U;
+  const bool live = some && u0 < U;
   float shift[kOccRows];   // exp(ref + maxP - LN) of the frames whose row of W this warp writes
   if (live) {
     const int uc = min(u, U - 1);
@@ -563,25 +728,24 @@ __global__ void __launch_bounds__(kOccThreads, 2) occupancy_kernel(const OccPara
     }
     const float2* F = p.F + (i64)b * p.stride + pair_slot(uc, p.npl);
     const float* g = p.g + (i64)b * p.stride;
-    // Lane `lane` of local warp w holds the tile's diagonals ds = w + kOccWarps i with
-    // 0 <= ds - lane < 32: exactly kOccRows of them, taken four at a time with all their loads
-    // issued before the first use (unconditional, clamped into the lattice).
-    const int first = w + (lane > w ? (lane - w + kOccWarps - 1) / kOccWarps * kOccWarps : 0) - lane;
-    const int un = min(u + 1, U - 1);
+    // Step i takes diagonal i of the tile in the lanes up to i and diagonal i + 32 in the others:
+    // every lane has a node and a warp touches two rows.  Four steps at a time with all their
+    // loads issued before the first use (unconditional, clamped into the lattice).
+    const int slot1 = row_slot(uc, p.npl), slot2 = row_slot(min(u + 1, U - 1), p.npl);
 #pragma unroll
     for (int q = 0; q < kOccRows; q += 4) {
       float2 f[4];
       float g1[4], g2[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const i64 row = (i64)(min(t0 + first + kOccWarps * (q + j), T - 1) + uc) * ld;
+        const i64 row = (i64)(min(t0 + ((w + kOccWarps * (q + j) - lane) & 31), T - 1) + uc) * ld;
         f[j] = F[row];
-        g1[j] = g[row + ld + uc];
-        g2[j] = g[row + ld + un];
+        g1[j] = g[row + ld + slot1];
+        g2[j] = g[row + ld + slot2];
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const int tt = first + kOccWarps * (q + j);
+        const int tt = (w + kOccWarps * (q + j) - lane) & 31;
         const bool in = t0 + tt < T && u < U;
         // (arcs that do not exist have factor 0; what they would lead to may never have been
         // written, hence the selects)
@@ -593,40 +757,67 @@ __global__ void __launch_bounds__(kOccThreads, 2) occupancy_kernel(const OccPara
     for (int k = 0; k < kOccRows; ++k) shift[k] = expf(fminf(shift[k], 80.0f));
   }
   __syncthreads();
+  // rows w kOccRows .. of the tile (frames for W, label positions for the transposed emT); beyond
+  // T_b and U_b both occupancies are zero, and so is W
+  const int k0 = w * kOccRows;
+  const int frames = min(kOccRows, p.maxT - (t0 + k0)), positions = min(kOccRows, p.maxU - (u0 + k0));
   float colS = 0.0f, colE = 0.0f;   // sums over the warp's frames
+  if (live) {
+    float* Wp = p.W + ((i64)b * p.maxT + t0 + k0) * p.ldW + u;
 #pragma unroll
-  for (int k = 0; k < kOccRows; ++k) {
-    const int tt = w * kOccRows + k, t = t0 + tt;
-    const float st = live ? tS[ub][tt][lane] : 0.0f, sp = live ? tE[ub][tt][lane] : 0.0f;
-    colS += st;
-    colE += sp;
-    if (inRange) {
-      if (t < p.maxT) {
-        // (beyond T_b and U_b both occupancies are zero, and so is W)
-        float x = 0.0f;
-        if (live && t < T && u < U) x = __fadd_rn(st, sp) * shift[k] * delta;
-        if (TC) x = tf32_round(x);
-        p.W[((i64)b * p.maxT + t) * p.ldW + u] = x;
-      }
-      if (TC) {  // transposed: lane <-> frame, row <-> label position
-        const int uu = u0 + tt, t2 = t0 + lane;
-        if (uu < p.maxU && t2 < p.ldT) p.emT[((i64)b * p.maxU + uu) * p.ldT + t2] = live ? tE[ub][lane][tt] * delta : 0.0f;
-      } else if (t < p.maxT && u < p.maxU) {
-        p.emT[((i64)b * p.maxT + t) * p.maxU + u] = sp;
-      }
+    for (int k = 0; k < kOccRows; ++k) {
+      const float st = tS[ub][k0 + k][lane], sp = tE[ub][k0 + k][lane];
+      colS += st;
+      colE += sp;
+      float x = u < U && t0 + k0 + k < T ? __fadd_rn(st, sp) * shift[k] * delta : 0.0f;
+      if (TC) x = tf32_round(x);
+      if (k < frames) Wp[k * p.ldW] = x;
     }
-    float v = st;
+    if (TC) {  // transposed: lane <-> frame, row <-> label position
+      float* Ep = p.emT + ((i64)b * p.maxU + u0 + k0) * p.ldT + t0 + lane;
+      if (t0 + lane < p.ldT) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) sRow[ub][tt] = v;
+        for (int k = 0; k < kOccRows; ++k)
+          if (k < positions) Ep[k * p.ldT] = tE[ub][lane][k0 + k] * delta;
+      }
+    } else if (u < p.maxU) {
+      float* Ep = p.emT + ((i64)b * p.maxT + t0 + k0) * p.maxU + u;
+#pragma unroll
+      for (int k = 0; k < kOccRows; ++k)
+        if (k < frames) Ep[k * p.maxU] = tE[ub][k0 + k][lane];
+    }
+    if (w == 0) {  // lane <-> frame: sum over the block's positions
+      float v = 0.0f;
+#pragma unroll 8
+      for (int j = 0; j < 32; ++j) v += tS[ub][lane][j];
+      sRow[u0 + lane] = v;
+    }
+  } else {
+    for (int k = 0; k < frames; ++k) {
+      p.W[((i64)b * p.maxT + t0 + k0 + k) * p.ldW + u] = 0.0f;
+      if (!TC && u < p.maxU) p.emT[((i64)b * p.maxT + t0 + k0 + k) * p.maxU + u] = 0.0f;
+    }
+    if (TC && t0 + lane < p.ldT)
+      for (int k = 0; k < positions; ++k) p.emT[((i64)b * p.maxU + u0 + k0 + k) * p.ldT + t0 + lane] = 0.0f;
+    if (w == 0) sRow[u0 + lane] = 0.0f;
   }
-  sCol[w][0][u] = colS;
-  sCol[w][1][u] = colE;
+  sCol[2 * w * cols + u] = colS;
+  sCol[(2 * w + 1) * cols + u] = colE;
   __syncthreads();
+  for (int i = threadIdx.x; some && i < 2 * cols; i += blockDim.x) {
+    const int cw = i >= cols, cu = i - cw * cols;
+    if (cu < p.maxU) {
+      float s = sCol[i];
+#pragma unroll
+      for (int k = 1; k < kOccWarps; ++k) s += sCol[2 * k * cols + i];
+      part[cw * p.maxU + cu] = s;
+    }
+  }
   if (threadIdx.x < 32) {
     const int t = t0 + lane;
     const bool ok = some && t < T;
-    const float rs = ((sRow[0][lane] + sRow[1][lane]) + sRow[2][lane]) + sRow[3][lane];
+    float rs = sRow[lane];
+    for (int j = 1; j < blocks; ++j) rs += sRow[j * 32 + lane];
     if (TC) {
       if (t < p.ldT) {
         p.nref[(i64)b * p.ldT + t] = ok ? -p.rowRef[(i64)b * p.maxT + t] * kLog2e : 0.0f;
@@ -636,37 +827,30 @@ __global__ void __launch_bounds__(kOccThreads, 2) occupancy_kernel(const OccPara
       p.ebl[(i64)b * p.maxT + t] = ok ? rs : 0.0f;
     }
   }
-  const int cw = threadIdx.x >> 7, cu = threadIdx.x & 127;
-  if (some && cw < 2 && cu < p.maxU) {
-    float s = sCol[0][cw][cu];
-#pragma unroll
-    for (int k = 1; k < kOccWarps; ++k) s += sCol[k][cw][cu];
-    part[cw * p.maxU + cu] = s;
-  }
   // the CTA of the utterance that finishes last adds the partial sums
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    sLast = atomicAdd(&p.ticket[b], 1u) == gridDim.x - 1 ? 1 : 0;
+    *sLast = atomicAdd(&p.ticket[b], 1u) == gridDim.x - 1 ? 1 : 0;
   }
   __syncthreads();
-  if (!sLast) return;
+  if (!*sLast) return;
   __threadfence();
   const int tiles = (T > 0 && U > 0) ? (T + 31) / 32 : 0;
-  float* acc = &tS[0][0][0];     // [4][2 * 128] sums of the four quarters of the tiles
+  float* acc = smemO;            // [4][2][cols] sums of the four quarters of the tiles
   const float* all = p.partial + (i64)b * gridDim.x * 2 * p.maxU;
-  for (int i = threadIdx.x; i < 4 * 2 * p.maxU; i += kOccThreads) {
+  for (int i = threadIdx.x; i < 4 * 2 * p.maxU; i += blockDim.x) {
     const int q = i / (2 * p.maxU), c = i - q * 2 * p.maxU;
     const int z0 = tiles * q / 4, z1 = tiles * (q + 1) / 4;
     float s = 0.0f;
 #pragma unroll 8
     for (int z = z0; z < z1; ++z) s += __ldcg(all + (i64)z * 2 * p.maxU + c);
-    acc[q * 256 + c] = s;
+    acc[q * 2 * cols + c] = s;
   }
   __syncthreads();
-  for (int c = threadIdx.x; c < 2 * p.maxU; c += kOccThreads) {
+  for (int c = threadIdx.x; c < 2 * p.maxU; c += blockDim.x) {
     const int cu2 = c < p.maxU ? c : c - p.maxU;
-    const float s = cu2 < U ? ((acc[c] + acc[256 + c]) + acc[512 + c]) + acc[768 + c] : 0.0f;
+    const float s = cu2 < U ? ((acc[c] + acc[2 * cols + c]) + acc[4 * cols + c]) + acc[6 * cols + c] : 0.0f;
     (c < p.maxU ? p.pBlank : p.pLabel)[(i64)b * p.maxU + cu2] = s;
   }
 }
@@ -678,11 +862,11 @@ void allow_dyn_smem(K kernel, int bytes) {
 
 }  // namespace
 
-bool sweep_supported(Dims d) { return d.maxU >= 1 && d.maxU <= 128; }
+bool sweep_supported(Dims d) { return d.maxU >= 1 && d.maxU <= 256; }
 
 SweepGeom sweep_geom(Dims d) {
   SweepGeom g;
-  g.npl = d.maxU <= 32 ? 1 : d.maxU <= 64 ? 2 : 4;
+  g.npl = d.maxU <= 32 ? 1 : d.maxU <= 64 ? 2 : d.maxU <= 128 ? 4 : div_up(d.maxU, 32);
   g.ld = 32 * g.npl;
   g.nDiag = d.maxT + d.maxU;   // one spare row: the node beyond the terminating blank
   g.nBlk = (g.nDiag + kDiag - 1) / kDiag;
@@ -700,12 +884,26 @@ size_t sweep_partial_floats(Dims d) {
     else if ((npl) == 2) { CALL(2); }        \
     else { CALL(4); }                        \
   } while (0)
+#define TB200_BY_NPL_NATURAL(npl, CALL)      \
+  do {                                       \
+    if ((npl) == 5) { CALL(5); }             \
+    else if ((npl) == 6) { CALL(6); }        \
+    else if ((npl) == 7) { CALL(7); }        \
+    else { CALL(8); }                        \
+  } while (0)
+#define TB200_BY_NPL_ANY(npl, CALL)          \
+  do {                                       \
+    if ((npl) <= 4) { TB200_BY_NPL(npl, CALL); } \
+    else { TB200_BY_NPL_NATURAL(npl, CALL); } \
+  } while (0)
 
 void launch_sweep_forward(const void* E, const void* P, float* LN, const float* ELrow,
-                          const float* ebl, float2* arcs, float* alphas, float* deltas, float* costs,
+                          float* ebl, float2* arcs, float* alphas, float* deltas, float* costs,
                           float* lossSum, unsigned* ticket, const int* labels, const int* inLens,
                           const int* labLens, SweepGeom g, Dims d, cudaStream_t stream) {
   if (d.B <= 0) return;
+  if (natural(g.npl) && d.dtype != kDtypeF32)
+    throw std::invalid_argument("bf16 emissions: the label axis must not exceed 128 positions");
   if (d.maxT > 0) {
     PrepParams q{};
     q.E = E; q.P = P; q.LN = LN; q.ELrow = ELrow; q.ebl = ebl; q.arcs = arcs;
@@ -718,8 +916,23 @@ void launch_sweep_forward(const void* E, const void* P, float* LN, const float* 
     else sweep_prep_kernel<float><<<grid, 256, 0, stream>>>(q);
     TB200_CHECK_LAUNCH();
   }
-  const int smem = kRing * kDiag * g.ld * 8;
+  const int ringBytes = ring_blocks(g.npl) * kDiag * g.ld * 8;
   ScopedKernel sk("alpha_sweep", stream);
+  if (natural(g.npl)) {
+    const NaturalTerms n{static_cast<const float*>(P), ebl, labels, d.V, d.blank};
+    // blank emissions in shared memory: as many frames as two CTAs per SM leave room for
+    const int stage = std::min(d.maxT, (112 * 1024 - ringBytes) / 4), smem = ringBytes + stage * 4;
+#define CALL(NPL)                                                                                \
+  allow_dyn_smem(alpha_natural_kernel<NPL>, smem);                                               \
+  alpha_natural_kernel<NPL><<<d.B, 32, smem, stream>>>(arcs, n, costs, alphas, g.stride, inLens, \
+                                                       labLens, d.B, d.maxT, d.maxU, stage,      \
+                                                       lossSum, ticket)
+    TB200_BY_NPL_NATURAL(g.npl, CALL);
+#undef CALL
+    TB200_CHECK_LAUNCH();
+    return;
+  }
+  const int smem = ringBytes;
 #define CALL(NPL)                                                                                \
   allow_dyn_smem(alpha_sweep_kernel<NPL>, smem);                                                 \
   alpha_sweep_kernel<NPL><<<d.B, 32, smem, stream>>>(arcs, costs, alphas, deltas, g.stride,      \
@@ -730,7 +943,8 @@ void launch_sweep_forward(const void* E, const void* P, float* LN, const float* 
   TB200_CHECK_LAUNCH();
 }
 
-void launch_sweep_backward(const SweepScratch& w, const float2* arcs, const float* alphas,
+void launch_sweep_backward(const SweepScratch& w, const float* P, const float* blankEmissions,
+                           const int* labels, const float2* arcs, const float* alphas,
                            const float* alphaDeltas, const float* LN, const float* rowRef,
                            const float* maxP, const float* deltas, float* W, float* emT, float* nref,
                            float* ebl, float* pBlank, float* pLabel, const int* inLens,
@@ -742,18 +956,19 @@ void launch_sweep_backward(const SweepScratch& w, const float2* arcs, const floa
     const dim3 grid(div_up(g.nDiag, kFactorRows * kFactorWarps), d.B);
 #define CALL(NPL)                                                                              \
   gamma_factors_kernel<NPL><<<grid, 32 * kFactorWarps, 0, stream>>>(                           \
-      arcs, alphas, alphaDeltas, w.F, w.ticket, g.stride, g.nDiag, inLens, labLens, d.maxT, d.maxU)
-    TB200_BY_NPL(g.npl, CALL);
+      arcs, alphas, alphaDeltas, n, w.F, w.ticket, g.stride, g.nDiag, inLens, labLens, d.maxT, d.maxU)
+    const NaturalTerms n{P, blankEmissions, labels, d.V, d.blank};
+    TB200_BY_NPL_ANY(g.npl, CALL);
 #undef CALL
     TB200_CHECK_LAUNCH();
   }
   {
-    const int smem = kRing * kDiag * g.ld * 8;
+    const int smem = ring_blocks(g.npl) * kDiag * g.ld * 8;
     ScopedKernel sk("gamma_sweep", stream);
 #define CALL(NPL)                                                                              \
   allow_dyn_smem(gamma_sweep_kernel<NPL>, smem);                                               \
   gamma_sweep_kernel<NPL><<<d.B, 32, smem, stream>>>(w.F, w.g, g.stride, inLens, labLens, d.maxT, d.maxU)
-    TB200_BY_NPL(g.npl, CALL);
+    TB200_BY_NPL_ANY(g.npl, CALL);
 #undef CALL
     TB200_CHECK_LAUNCH();
   }
@@ -765,8 +980,15 @@ void launch_sweep_backward(const SweepScratch& w, const float2* arcs, const floa
   o.ldW = grads_umma_ld_w(d); o.ldT = grads_umma_ld_t(d); o.npl = g.npl; o.stride = g.stride;
   const dim3 grid(div_up(o.ldT, 32), d.B);
   ScopedKernel sk("occupancy", stream);
-  if (tensorCore) occupancy_kernel<true><<<grid, kOccThreads, 0, stream>>>(o);
-  else occupancy_kernel<false><<<grid, kOccThreads, 0, stream>>>(o);
+  const int threads = o.ldW * kOccWarps, smem = occ_smem_floats(o.ldW / 32) * (int)sizeof(float);
+  auto go = [&](auto kernel) {
+    allow_dyn_smem(kernel, smem);
+    kernel<<<grid, threads, smem, stream>>>(o);
+  };
+  // (two CTAs per SM up to 160 positions: registers are limited to that)
+  if (threads <= 512) tensorCore ? go(occupancy_kernel<true, 512>) : go(occupancy_kernel<false, 512>);
+  else if (threads <= 640) tensorCore ? go(occupancy_kernel<true, 640>) : go(occupancy_kernel<false, 640>);
+  else tensorCore ? go(occupancy_kernel<true, 1024>) : go(occupancy_kernel<false, 1024>);
   TB200_CHECK_LAUNCH();
 }
 

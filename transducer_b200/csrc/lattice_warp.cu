@@ -44,7 +44,8 @@ __global__ void __launch_bounds__(256) viterbi_prep_kernel(
     const float* __restrict__ E, const float* __restrict__ LN, const float* __restrict__ best,
     float4* __restrict__ nodes, const int* __restrict__ inLens, const int* __restrict__ labLens,
     int maxT, int maxU, int V, int blank, int ld, i64 latStride) {
-  __shared__ float tLn[32][33], tBs[32][33], tEb[32];
+  // (even rows: an anti-diagonal of a tile falls into 32 different banks, with 33 into one)
+  __shared__ float tLn[32][34], tBs[32][34], tEb[32];
   const int b = blockIdx.z, t0 = blockIdx.y * 32, u0 = blockIdx.x * 32;
   const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
   if (t0 >= T || u0 >= U) return;
@@ -62,10 +63,11 @@ __global__ void __launch_bounds__(256) viterbi_prep_kernel(
   if (threadIdx.x < 32)
     tEb[lane] = E[((i64)b * maxT + min(t0 + lane, T - 1)) * V + blank];
   __syncthreads();
-  for (int ds = w; ds < 63; ds += 8) {
-    const int tt = ds - lane;
-    if (tt >= 0 && tt < 32 && t0 + tt < T && u < U)
-      nodes[(i64)b * latStride + (i64)(t0 + u0 + ds) * ld + u] =
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {   // diagonal i of the tile in the lanes up to i, i + 32 in the others
+    const int tt = (w + 8 * k - lane) & 31;
+    if (t0 + tt < T && u < U)
+      nodes[(i64)b * latStride + (i64)(t0 + tt + u) * ld + u] =
           make_float4(tEb[tt], tLn[tt][lane], tBs[tt][lane], 0.0f);
   }
 }
