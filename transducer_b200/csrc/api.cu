@@ -206,7 +206,13 @@ bool log_norms_impl(const void* E, const void* P, float* LN, float* rowRef, floa
     // the kernel needs somewhere to put the row shifts even if the caller does not want them
     float* mp = maxP ? maxP : ws.maxPScratch;
     if (!rowRef) throw std::invalid_argument("rowRef must not be null");
-    const bool gathers = labels && EL && ebl && lognorm_umma_gathers(d) && g_opt.fused_gather != 0;
+    // Emissions that stay in the L2 (126 MB) until the re-layout are gathered there: handing them out
+    // costs this kernel 5..10 us (the labels are sorted, and a chunk's labels are served one after the
+    // other), a gather from L2 1..3 us.  Forward time of the two kernels, handed out / gathered:
+    // E of 6 MB 60 / 51 us, 65 MB 88 / 84, 256 MB 138 / 144, 640 MB 260 / 270.
+    const size_t bytesE = (size_t)d.B * d.maxT * d.V * (d.dtype == kDtypeBf16 ? 2 : 4);
+    const bool gathers = labels && EL && ebl && lognorm_umma_gathers(d) && g_opt.fused_gather != 0 &&
+                         bytesE > (size_t)96 << 20;
     launch_lognorm_umma(E, P, LN, rowRef, mp, inLens, labLens, d, ws.split,
                         device_status_word(), fixup, g_stream, gathers ? labels : nullptr,
                         gathers ? EL : nullptr, gathers ? ebl : nullptr);
