@@ -685,11 +685,7 @@ def parity_block(w, r, device_case, state):
 NCU_TRAFFIC_BYTES = {
     ("c3", "grads_umma"): 2460688896 + 2661452288,
     ("c3", "lognorm_umma"): 2626279936 + 35040256,
-    ("c3", "alpha_warp"): 60133120 + 2445056,
-    ("c3", "gamma_warp"): 91231744 + 11596032,
-    ("c3", "lattice_prep"): 42460416 + 7390976,
     ("c3", "expp_split"): 146920704 + 230604288,
-    ("c3", "lattice_unskew_round"): 65933568 + 19291904,
 }
 
 
@@ -713,14 +709,18 @@ def kernel_algorithmic_bytes(w, il, ll, elem_bytes=4):
     V = w.V
     return {
         "lognorm_exact": 4.0 * V * (sum_t + sum_u) + 4.0 * sum_tu,
+        "lognorm_factored": 4.0 * V * (sum_t + sum_u) + 4.0 * sum_tu,
         "lognorm_umma": eb * V * (sum_t + sum_u) + 4.0 * sum_tu,
         "maxplus": 4.0 * V * (sum_t + sum_u) + 4.0 * sum_tu,
         "maxplus_pruned": 4.0 * V * sum_t + 4.0 * sum_tu,    # E rows in, scores out
         "maxplus_select_e": 4.0 * V * sum_t,
         "alpha_wavefront": 3 * 4.0 * sum_tu,
         "gamma_wavefront": 5 * 4.0 * sum_tu,
-        "alpha_warp": 3 * 4.0 * sum_tu,    # arc terms (2 floats) in, alpha out
-        "gamma_warp": 5 * 4.0 * sum_tu,    # arc terms + alpha in, stay + step out
+        "sweep_prep": 4 * 4.0 * sum_tu,     # LN and the label emission in, a pair out
+        "alpha_sweep": 3 * 4.0 * sum_tu,    # a pair in, alpha out
+        "gamma_factors": 5 * 4.0 * sum_tu,  # a pair and alpha in, the factors out
+        "gamma_sweep": 3 * 4.0 * sum_tu,    # the factors in, g out
+        "occupancy": 6 * 4.0 * sum_tu,      # factors, g and LN in, W and the label arcs out
         "viterbi_warp": 4 * 4.0 * sum_tu,  # one float4 record per node in
         "egrad_simt": 4.0 * V * sum_t + 4.0 * V * n * w.T + 4.0 * V * sum_u,
         "pgrad_simt": 4.0 * V * sum_t + 4.0 * V * n * (w.U + 1) + 4.0 * V * sum_u,
