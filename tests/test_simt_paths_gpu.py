@@ -51,6 +51,47 @@ def test_factored_sum_out_of_range_is_recomputed():
     assert torch.isneginf(ln[0, 7, :int(ll[0]) + 1]).all()
 
 
+def _spiked(X, height, g, word=None):
+    """One word of every row raised: a word of its own, or the same one throughout."""
+    i = torch.randint(0, X.shape[2], X.shape[:2] + (1,), generator=g, device="cuda")
+    return X.scatter_add(2, i if word is None else torch.full_like(i, word),
+                         torch.full(i.shape, float(height), device="cuda"))
+
+
+@pytest.mark.parametrize("V", [257, 1025])
+@pytest.mark.parametrize("scores", ["plain", "wide", "confident_10", "confident_45", "confident_100", "cancelled_10",
+                                    "cancelled_45", "log_softmax"])
+def test_factored_is_as_close_to_float64_as_exact(scores, V):
+    """Whatever the spread of the scores, the factored kernel may not lose digits against the
+    exact one.  rms over 67584 nodes; 1.1: its scatter (below 1 % per 10^4 nodes) and the two
+    kernels' different last bits."""
+    B, T, U = 8, 256, 33
+    g = torch.Generator(device="cuda").manual_seed(V)
+    E = torch.empty((B, T, V), device="cuda").normal_(generator=g)
+    P = torch.empty((B, U, V), device="cuda").normal_(generator=g)
+    kind, _, h = scores.partition("_")
+    if kind == "wide":
+        E, P = 5 * E, 5 * P
+    elif kind == "confident":
+        E, P = _spiked(E, int(h), g), _spiked(P, int(h), g)
+    elif kind == "cancelled":
+        E, P = _spiked(E, int(h), g, 3), _spiked(P, -int(h), g, 3)
+    elif kind == "log":
+        E, P = torch.log_softmax(5 * E, 2), torch.log_softmax(5 * P, 2)
+    il = torch.full((B,), T, dtype=torch.int32, device="cuda")
+    ll = torch.full((B,), U - 1, dtype=torch.int32, device="cuda")
+    want = torch.stack([torch.logsumexp(E[b].double()[:, None] + P[b].double()[None], dim=2) for b in range(B)])
+    rms = []
+    for path in (0, 1):
+        abi.set_option("lognorm_path", path)
+        try:
+            ln = abi.log_norms(E, P, il, ll)[0]
+        finally:
+            abi.set_option("lognorm_path", 0)
+        rms.append((ln.double() - want).pow(2).mean().sqrt().item())
+    assert rms[0] <= 1.1 * rms[1]
+
+
 @pytest.mark.parametrize("B,T,U,V,below", [(1, 1, 2, 3, None), (2, 63, 64, 65, None), (2, 65, 33, 63, 4),
                                            (1, 64, 65, 129, None), (2, 33, 128, 30, None), (3, 100, 20, 257, 3)])
 def test_gradients(B, T, U, V, below):
