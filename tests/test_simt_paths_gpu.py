@@ -2,6 +2,8 @@
 below 32) against a float64 evaluation: the factored log-normaliser at the edges of its tiles
 of 32x32 nodes, its steps of 64 words and the clusters that share a tile, and the gradients at the
 edges of their tiles of 64x64 and steps of 32, with labels that share columns."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -106,3 +108,55 @@ def test_gradients(B, T, U, V, below):
     tol = 4.0 * np.sqrt(T + U) * 2.0 ** -15 + 1e-5
     assert abi.rel_to_max(n(eg), ref["egrads"] * s) < tol
     assert abi.rel_to_max(n(pg), ref["pgrads"] * s) < tol
+
+
+@pytest.fixture
+def forced():
+    """The factored kernel at any size (small problems go to the exact one by themselves)."""
+    abi.set_option("lognorm_path", 3)
+    yield
+    abi.set_option("lognorm_path", 0)
+
+
+@pytest.mark.parametrize("B,T,U,V", [(1, 1, 1, 2), (2, 31, 33, 29), (1, 33, 31, 63), (3, 64, 32, 65),
+                                     (2, 40, 5, 129), (1, 20, 7, 8041), (2, 33, 65, 1025), (1, 70, 200, 321)])
+def test_factored_tile_edges(forced, B, T, U, V):
+    test_factored_log_normaliser(B, T, U, V)
+
+
+def test_factored_sum_out_of_range_is_recomputed_after_the_kernel(forced):
+    test_factored_sum_out_of_range_is_recomputed()
+
+
+@pytest.mark.parametrize("B,T,U,V", [(1, 1, 2, 3), (2, 63, 64, 65), (1, 64, 65, 129), (2, 33, 128, 30), (1, 40, 200, 77)])
+def test_factored_gradients(forced, B, T, U, V):
+    test_gradients(B, T, U, V, None)
+
+
+def _kernels(fn):
+    """Names of the library's kernels that fn launches."""
+    lib = abi.lib
+    lib.tb200_profile_enable(1)
+    try:
+        lib.tb200_profile_reset()
+        fn()
+        buf = ctypes.create_string_buffer(1 << 14)
+        lib.tb200_profile_report(buf, len(buf))
+    finally:
+        lib.tb200_profile_enable(0)
+    return {line.split()[0] for line in buf.value.decode().splitlines()}
+
+
+@pytest.mark.parametrize("B,T,U,V,kernel", [(8, 400, 1, 1025, "exact"), (8, 400, 4, 1025, "exact"), (64, 1000, 3, 1301, "exact"),
+                                            (1, 40, 30, 29, "exact"), (1, 300, 9, 1025, "exact"),
+                                            (8, 400, 16, 1025, "factored"), (64, 1000, 8, 1301, "factored"),
+                                            (2, 44, 7, 23851, "factored"), (4, 64, 300, 1024, "factored")])
+def test_narrow_label_axes_take_the_exact_kernel(B, T, U, V, kernel):
+    """A tile of the factored kernel is 32 positions wide: below 4 to 9 of them, and for few nodes,
+    the exact kernel's warp per node is the faster one (and both give the same sums)."""
+    E, P, labels, il, ll = make(B, T, U, V)
+    out = {}
+    names = _kernels(lambda: out.update(ln=abi.log_norms(E, P, il, ll)[0]))
+    assert "lognorm_" + kernel in names and len({"lognorm_exact", "lognorm_factored"} & names) == 1
+    want = torch.logsumexp(E[0].double()[:, None] + P[0].double()[None], dim=2)
+    assert (out["ln"][0].double() - want).abs().max().item() < want.abs().max().item() * 2.0 ** -23 + 2.0 ** -20

@@ -194,15 +194,17 @@ bool log_norms_impl(const void* E, const void* P, float* LN, float* rowRef, floa
                     float* ebl = nullptr) {
   if (d.B <= 0 || d.maxT <= 0 || d.maxU <= 0) return false;
   const bool can = lognorm_umma_supported(E, P, d);
-  if (g_opt.lognorm_path == 2 && !can)
+  const int path = g_opt.lognorm_path;
+  const bool tensorCore = can && (path == 0 || path == 2);
+  if (path == 2 && !can)
     throw std::invalid_argument(
         "tensor-core log-normaliser needs alphabetSize % 4 == 0, alphabetSize >= 32, "
         "maxLabelLength <= 256 and 16-byte aligned emissions");
-  if (d.dtype != kDtypeF32 && !(can && g_opt.lognorm_path != 1))
+  if (d.dtype != kDtypeF32 && !tensorCore)
     throw std::invalid_argument(
         "bf16 emissions need the tensor-core log-normaliser: alphabetSize % 8 == 0, "
         "alphabetSize >= 32, 16-byte aligned emissions and predictions");
-  if (can && g_opt.lognorm_path != 1) {
+  if (tensorCore) {
     // the kernel needs somewhere to put the row shifts even if the caller does not want them
     float* mp = maxP ? maxP : ws.maxPScratch;
     if (!rowRef) throw std::invalid_argument("rowRef must not be null");
@@ -220,7 +222,7 @@ bool log_norms_impl(const void* E, const void* P, float* LN, float* rowRef, floa
   }
   const float* Ef = static_cast<const float*>(E);
   const float* Pf = static_cast<const float*>(P);
-  const bool exact = g_opt.lognorm_path == 1 || rowRef == nullptr;
+  const bool exact = path == 1 || rowRef == nullptr || (path != 3 && !lognorm_factored_pays(d));
   launch_lognorm_simt(Ef, Pf, LN, rowRef, exact ? maxP : (maxP ? maxP : ws.maxPScratch), inLens,
                       labLens, d, exact, exact ? nullptr : device_status_word(), g_stream);
   if (!exact && fixup) launch_lognorm_fixup(E, P, LN, inLens, labLens, d, g_stream);
@@ -250,7 +252,7 @@ void* tb200_get_stream(void) { return g_stream; }
 
 int tb200_set_option(const char* key, int value) {
   if (!key) return fail(kErrInvalidArgument, "null option key");
-  if (!strcmp(key, "lognorm_path") && value >= 0 && value <= 2) g_opt.lognorm_path = value;
+  if (!strcmp(key, "lognorm_path") && value >= 0 && value <= 3) g_opt.lognorm_path = value;
   else if (!strcmp(key, "grads_path") && value >= 0 && value <= 2) g_opt.grads_path = value;
   else if (!strcmp(key, "grad_passes") && value >= 1 && value <= 3) g_opt.grad_passes = value;
   else if (!strcmp(key, "fused_gather") && value >= 0 && value <= 1) g_opt.fused_gather = value;

@@ -90,6 +90,8 @@ void launch_viterbi_lattice(const float* E, const float* P, const float* LN,
 void launch_lognorm_simt(const float* E, const float* P, float* LN, float* rowRef, float* maxP,
                          const int* inLens, const int* labLens, Dims d, bool exact, int* status,
                          cudaStream_t stream);
+// Is the factored sum the faster of the two for these sizes?
+bool lognorm_factored_pays(Dims d);
 // expP[b,u,v] = exp(P[b,u,v]-maxP[b,u]) for u <= labLens[b], 0 for padded rows;
 // also writes maxP[b,u] (0 for padded rows).
 void launch_exp_rows(const float* P, float* expP, float* maxP, const int* labLens,

@@ -11,6 +11,7 @@
 // unaligned base pointers): a multiply-add per node and word instead of an exponential.
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "kernels.h"
@@ -269,7 +270,38 @@ __global__ void __launch_bounds__(256) exp_rows_kernel(
   if (threadIdx.x == 0) maxP[(i64)b * maxU + u] = m;
 }
 
+// How lognorm_factored is cut: tiles, and the ranks that share one -- as many as keep the grid within
+// two CTAs per SM (what is resident at once) and leave every rank two steps.  Measured (us, 1 rank /
+// this rule): B=5 T=69 U'=5 V=8042 116 / 17; B=2 T=44 U'=7 V=23850 348 / 54; B=4 T=400 U'=101
+// V=5001 131 / 131.
+constexpr int kFacResident = 2 * 148;
+struct FacGrid {
+  i64 tiles;
+  int steps, ranks;
+};
+FacGrid fac_grid(Dims d) {
+  FacGrid g{(i64)div_up(d.maxU, kFacM) * div_up(d.maxT, kFacM) * d.B, div_up(d.V, kFacK), 1};
+  while (g.ranks < 8 && g.tiles * g.ranks * 2 <= kFacResident && g.ranks * 4 <= g.steps) g.ranks *= 2;
+  return g;
+}
+
 }  // namespace
+
+// Estimates of both kernels' time in us: a warp of lognorm_exact passes over the vocabulary twice,
+// with about 340 words' worth of fixed work; lognorm_factored computes whole tiles whatever the
+// label axis, 2.2 us per step of 64 words with two CTAs on an SM and 1.4 with one.  The line lies at
+// 4 to 9 label positions for many nodes and higher for few.  Measured (us for the call, exact /
+// factored; row maxima and, for the latter, the pass over marked nodes included): B=64 T=1000 V=1301
+// U'=2 220 / 397, 4 343 / 398, 6 472 / 399; B=8 T=400 V=1025 U'=2 18 / 35, 8 30 / 35, 12 42 / 35;
+// B=8 T=400 V=8041 U'=4 150 / 168, 8 201 / 168; B=1 T=300 V=1025 U'=33 19 / 23, 65 27 / 23.
+bool lognorm_factored_pays(Dims d) {
+  const FacGrid g = fac_grid(d);
+  const double ctas = (double)g.tiles * g.ranks, nodes = (double)d.B * d.maxT * d.maxU;
+  const double exact = 4e-3 * d.V + 0.6e-6 * nodes * (d.V + 340.0);
+  const double factored = 6.0 + (ctas <= kFacResident / 2 ? 1.4 : 2.2) * std::max(1.0, ctas / kFacResident) *
+                                    div_up(g.steps, g.ranks);
+  return factored < exact;
+}
 
 void launch_lognorm_simt(const float* E, const float* P, float* LN, float* rowRef, float* maxP,
                          const int* inLens, const int* labLens, Dims d, bool exact, int* status,
@@ -289,13 +321,7 @@ void launch_lognorm_simt(const float* E, const float* P, float* LN, float* rowRe
         E, P, LN, inLens, labLens, d.maxT, d.maxU, d.V);
   } else {
     ScopedKernel sk("lognorm_factored", stream);
-    // Ranks per tile: as many as keep the grid within two CTAs per SM (what is resident at once) and
-    // leave every rank two steps.  Measured (us, 1 rank / this rule / lognorm_exact): B=5 T=69 U'=5
-    // V=8042 116 / 17 / 33; B=2 T=44 U'=7 V=23850 348 / 54 / 94; B=4 T=400 U'=101 V=5001 131 / 131 / 527.
-    const i64 tiles = (i64)div_up(d.maxU, kFacM) * div_up(d.maxT, kFacM) * d.B;
-    const int steps = div_up(d.V, kFacK);
-    int ranks = 1;
-    while (ranks < 8 && tiles * ranks * 2 <= 2 * 148 && ranks * 4 <= steps) ranks *= 2;
+    const int ranks = fac_grid(d).ranks;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(div_up(d.maxU, kFacM) * ranks, div_up(d.maxT, kFacM), d.B);
     cfg.blockDim = dim3(256);
