@@ -2,6 +2,8 @@
 evaluation at the edges of what they are cut into: blocks of 16 diagonals, the positions a lane
 owns (1, 2, 4, 5..8), tiles of 32 frames, empty and one-node lattices.  The exact SIMT kernels stand
 around the sweeps, so that what is compared is theirs."""
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -46,3 +48,30 @@ def test_edges(T, U):
     assert np.isposinf(costs[3])
     assert abi.rel_to_max(n(eg), ref["egrads"]) < tol
     assert abi.rel_to_max(n(pg), ref["pgrads"]) < tol
+
+
+def test_host_threads_with_different_shapes():
+    """Stream and error message are per host thread, a kernel's shared-memory limit is not: a thread's
+    launches may not depend on what another one set for a shorter utterance.  (200 positions: the
+    sweep that stages T blank emissions.)"""
+    def worker(T, failures):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            E, P = torch.randn((1, T, 32), device="cuda"), torch.randn((1, 200, 32), device="cuda")
+            labels = torch.ones((1, 199), dtype=torch.int32, device="cuda")
+            il = torch.tensor([T], dtype=torch.int32, device="cuda")
+            ll = torch.tensor([199], dtype=torch.int32, device="cuda")
+            for _ in range(400):
+                try:
+                    fwd = abi.loss_forward(E, P, labels, il, ll)
+                    abi.loss_backward(E, P, labels, il, ll, fwd)
+                except Exception as e:
+                    failures.append((T, str(e)))
+            torch.cuda.current_stream().synchronize()
+
+    failures = []
+    threads = [threading.Thread(target=worker, args=(T, failures)) for T in (8, 3000, 16, 2000)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures[:3]

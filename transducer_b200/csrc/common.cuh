@@ -32,6 +32,14 @@ inline void cuda_check(cudaError_t err, const char* file, int line) {
   }
 }
 #define TB200_CUDA_CHECK(expr) ::tb200::cuda_check((expr), __FILE__, __LINE__)
+// Raises a kernel's dynamic shared-memory limit to `ceiling`, a constant of the kernel that no launch
+// of it exceeds.  The limit belongs to the function: set to a launch's own size, host threads that
+// call with different shapes overwrite each other's between setting it and launching.
+template <typename K>
+void allow_dyn_smem(K kernel, int ceiling) {
+  cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ceiling), __FILE__,
+             __LINE__);
+}
 #define TB200_CHECK_LAUNCH() ::tb200::cuda_check(cudaGetLastError(), __FILE__, __LINE__)
 
 struct bf16 {

@@ -701,6 +701,8 @@ __global__ void __launch_bounds__(256) label_overflow_kernel(
   }
 }
 
+constexpr int kStaticSmemBound = 3 * 1024;  // barriers + per-position tables of the kernel
+
 struct TileCfg {
   int TB, SE, SW, EB, DB;
 };
@@ -745,14 +747,11 @@ void launch_variant(const GradMaps& tm, GradParams p, TileCfg cfg, Dims d, cudaS
   p.tmemCols = pow2_cols(cols);
   size_t smem = (size_t)cfg.SE * eStage + (size_t)cfg.SW * wStage + 1024;
   if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it may hold all 512 TMEM columns
-  TB200_CUDA_CHECK(cudaFuncSetAttribute(grads_umma_kernel<TB, ESPLIT, PSPLIT, BF>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_dyn_smem(grads_umma_kernel<TB, ESPLIT, PSPLIT, BF>, 227 * 1024 - kStaticSmemBound);
   dim3 grid(div_up(d.V, kVBlock), d.B);
   ScopedKernel sk("grads_umma", stream);
   grads_umma_kernel<TB, ESPLIT, PSPLIT, BF><<<grid, kGradThreads, smem, stream>>>(tm, p);
 }
-
-constexpr int kStaticSmemBound = 3 * 1024;  // barriers + per-position tables of the kernel
 
 }  // namespace
 

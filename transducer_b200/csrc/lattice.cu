@@ -544,9 +544,7 @@ constexpr size_t kMaxDynSmem = 200 * 1024;
 
 template <typename K>
 void allow_smem(K kernel, size_t bytes) {
-  if (bytes > 48 * 1024)
-    TB200_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)bytes));
+  if (bytes > 48 * 1024) allow_dyn_smem(kernel, (int)kMaxDynSmem);
 }
 }  // namespace
 

@@ -855,11 +855,6 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 640 ? 2 : 1) occupancy_ker
   }
 }
 
-template <typename K>
-void allow_dyn_smem(K kernel, int bytes) {
-  TB200_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-}
-
 }  // namespace
 
 bool sweep_supported(Dims d) { return d.maxU >= 1 && d.maxU <= 256; }
@@ -921,9 +916,10 @@ void launch_sweep_forward(const void* E, const void* P, float* LN, const float* 
   if (natural(g.npl)) {
     const NaturalTerms n{static_cast<const float*>(P), ebl, labels, d.V, d.blank};
     // blank emissions in shared memory: as many frames as two CTAs per SM leave room for
-    const int stage = std::min(d.maxT, (112 * 1024 - ringBytes) / 4), smem = ringBytes + stage * 4;
+    constexpr int kCeiling = 112 * 1024;
+    const int stage = std::min(d.maxT, (kCeiling - ringBytes) / 4), smem = ringBytes + stage * 4;
 #define CALL(NPL)                                                                                \
-  allow_dyn_smem(alpha_natural_kernel<NPL>, smem);                                               \
+  allow_dyn_smem(alpha_natural_kernel<NPL>, kCeiling);                                           \
   alpha_natural_kernel<NPL><<<d.B, 32, smem, stream>>>(arcs, n, costs, alphas, g.stride, inLens, \
                                                        labLens, d.B, d.maxT, d.maxU, stage,      \
                                                        lossSum, ticket)
@@ -981,14 +977,14 @@ void launch_sweep_backward(const SweepScratch& w, const float* P, const float* b
   const dim3 grid(div_up(o.ldT, 32), d.B);
   ScopedKernel sk("occupancy", stream);
   const int threads = o.ldW * kOccWarps, smem = occ_smem_floats(o.ldW / 32) * (int)sizeof(float);
-  auto go = [&](auto kernel) {
-    allow_dyn_smem(kernel, smem);
+  auto go = [&](auto kernel, int maxThreads) {
+    allow_dyn_smem(kernel, occ_smem_floats(maxThreads / (32 * kOccWarps)) * (int)sizeof(float));
     kernel<<<grid, threads, smem, stream>>>(o);
   };
   // (two CTAs per SM up to 160 positions: registers are limited to that)
-  if (threads <= 512) tensorCore ? go(occupancy_kernel<true, 512>) : go(occupancy_kernel<false, 512>);
-  else if (threads <= 640) tensorCore ? go(occupancy_kernel<true, 640>) : go(occupancy_kernel<false, 640>);
-  else tensorCore ? go(occupancy_kernel<true, 1024>) : go(occupancy_kernel<false, 1024>);
+  if (threads <= 512) tensorCore ? go(occupancy_kernel<true, 512>, 512) : go(occupancy_kernel<false, 512>, 512);
+  else if (threads <= 640) tensorCore ? go(occupancy_kernel<true, 640>, 640) : go(occupancy_kernel<false, 640>, 640);
+  else tensorCore ? go(occupancy_kernel<true, 1024>, 1024) : go(occupancy_kernel<false, 1024>, 1024);
   TB200_CHECK_LAUNCH();
 }
 

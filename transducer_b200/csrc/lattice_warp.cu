@@ -286,11 +286,6 @@ __global__ void __launch_bounds__(256) viterbi_labels_kernel(
   }
 }
 
-template <typename K>
-void allow_dyn_smem(K kernel, int bytes) {
-  TB200_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-}
-
 }  // namespace
 
 bool viterbi_warp_supported(Dims d) { return d.maxU >= 1 && d.maxU <= 256; }
@@ -324,7 +319,7 @@ void launch_viterbi_warp(const float* E, const float* P, const float* LN, const 
   // of node records), then the ring
   const int slotBytes = kDiag * g.ld * 16;
   const int decBytes = d.maxU * viterbi_words_d(d.maxT, d.maxU) * 4;
-  const int room = 216 * 1024;
+  constexpr int room = 216 * 1024;
   const int decInSmem = decBytes + 3 * slotBytes <= room ? 1 : 0;
   const int ringDepth = std::max(2, std::min(kRing, (room - (decInSmem ? decBytes : 0)) / slotBytes));
   const int smem = ringDepth * slotBytes + (decInSmem ? decBytes : 0);
@@ -334,7 +329,7 @@ void launch_viterbi_warp(const float* E, const float* P, const float* LN, const 
   ScopedKernel sk("viterbi_warp", stream);
 #define CALL(NPL)                                                                              \
   do {                                                                                         \
-    allow_dyn_smem(viterbi_warp_kernel<NPL>, smem);                                            \
+    allow_dyn_smem(viterbi_warp_kernel<NPL>, room);                                            \
     viterbi_warp_kernel<NPL><<<d.B, 32, smem, stream>>>(                                       \
         P, nodes, g.ld, g.stride, g.nDiag, ringDepth, decBits, decInSmem, frames, labels,      \
         inLens, labLens, d.maxT, d.maxU, d.V, d.blank, status);                                \

@@ -841,7 +841,8 @@ void launch_lognorm_umma(const void* E, const void* P, float* LN, float* rowRef,
   // then does every stage have a single consumer of each kind, in program order (with fewer, a
   // fast issuer could mistake an older phase of a stage's barrier for its own).  One CTA per SM.
   const int stages = 4, nAcc = 2;
-  if (stages * stageBytes + 2048 > 220 * 1024 || nAcc * nPart + stages * 64 > 512)
+  constexpr int kCeiling = 220 * 1024;
+  if (stages * stageBytes + 2048 > kCeiling || nAcc * nPart + stages * 64 > 512)
     throw std::invalid_argument("label axis too long for the tensor-core log-normaliser");
   p.stages = stages;
   p.nAcc = nAcc;
@@ -858,11 +859,11 @@ void launch_lognorm_umma(const void* E, const void* P, float* LN, float* rowRef,
     // 8 transform + 8 drain (64 columns each) warps, producer, two MMA issuers
     if (bf) {
       auto k = lognorm_umma_kernel<2, 2, 64, true>;
-      TB200_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      allow_dyn_smem(k, kCeiling);
       k<<<grid, 19 * 32, smem, stream>>>(tmE, tmHi, tmLo, p);
     } else {
       auto k = lognorm_umma_kernel<2, 2, 64>;
-      TB200_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      allow_dyn_smem(k, kCeiling);
       k<<<grid, 19 * 32, smem, stream>>>(tmE, tmHi, tmLo, p);
     }
   }

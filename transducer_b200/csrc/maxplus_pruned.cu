@@ -39,6 +39,7 @@ constexpr int kPRows = kPTop + kBatchP;   // rows of a position list in memory
 // Entries from `count` up to the next multiple of 32 repeat entry 0.
 constexpr int kEWords = 2 * kETop + 4;
 constexpr size_t kSelSmemBytes = 96 * 1024;   // rows staged per CTA of the selection kernels
+constexpr int kPrunedSmemBytes = 227 * 1024 - 80;   // all that maxplus_pruned_kernel's barriers leave
 
 __device__ __forceinline__ int warp_sum_int(int v) { return __reduce_add_sync(0xffffffffu, v); }
 
@@ -600,7 +601,7 @@ void launch_maxplus_pruned(const float* E, const float* P, float* best, const in
     ScopedKernel sk("maxplus_select_p", stream);
     const int wp = (int)std::max<size_t>(1, std::min<size_t>(8, kSelSmemBytes / (rowB + kPTop * sizeof(int2))));
     const size_t smemP = wp * (rowB + kPTop * sizeof(int2));
-    TB200_CUDA_CHECK(cudaFuncSetAttribute(select_p_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemP));
+    allow_dyn_smem(select_p_kernel, (int)kSelSmemBytes);
     select_p_kernel<<<dim3(div_up(d.maxU - 1, wp), d.B), wp * 32, smemP, stream>>>(
         P, s.pList, s.pMeta, labLens, d.maxU, d.V, vp, d.blank, us, wp, status);
   }
@@ -609,7 +610,7 @@ void launch_maxplus_pruned(const float* E, const float* P, float* best, const in
     ScopedKernel sk("maxplus_select_e", stream);
     const int we = (int)std::max<size_t>(1, std::min<size_t>(8, kSelSmemBytes / rowB));
     const size_t smemE = we * rowB;
-    TB200_CUDA_CHECK(cudaFuncSetAttribute(select_e_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemE));
+    allow_dyn_smem(select_e_kernel, (int)kSelSmemBytes);
     select_e_kernel<<<dim3(div_up(d.maxT, we), d.B), we * 32, smemE, stream>>>(
         E, s.eList, inLens, d.maxT, d.V, vp, d.blank, us, we, status);
   }
@@ -632,8 +633,7 @@ void launch_maxplus_pruned(const float* E, const float* P, float* best, const in
   const int threads = 32 * p.warpsPerGroup * p.groups;
   {
     ScopedKernel sk("maxplus_pruned", stream);
-    TB200_CUDA_CHECK(cudaFuncSetAttribute(maxplus_pruned_kernel,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_dyn_smem(maxplus_pruned_kernel, kPrunedSmemBytes);
     maxplus_pruned_kernel<<<dim3(div_up(d.maxT, p.framesPerCta), d.B), threads, smem, stream>>>(p);
   }
   TB200_CHECK_LAUNCH();
