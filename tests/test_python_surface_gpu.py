@@ -225,3 +225,25 @@ def test_wrapper_without_length_validation_gives_the_same_result():
     # the default wrapper still refuses lengths that do not fit (it reads them back)
     with pytest.raises(ValueError):
         TransducerLoss()(E, P, labels, il + 100, ll)
+
+
+def test_length_check_alone_does_not_wait_for_the_kernels():
+    """validate_lengths without check_status synchronises ahead of the kernels, as the reference
+    does, and returns while they run (about 5 ms here: one warp's chain of 20200 diagonals)."""
+    B, T, U, V = 2, 20000, 200, 32
+    E, P = torch.randn((B, T, V), device="cuda"), torch.randn((B, U + 1, V), device="cuda")
+    labels = torch.ones((B, U), dtype=torch.int32, device="cuda")
+    il = torch.full((B,), T, dtype=torch.int32, device="cuda")
+    ll = torch.full((B,), U, dtype=torch.int32, device="cuda")
+    criterion = TransducerLoss(validate_lengths=True, check_status=False)
+    with torch.no_grad():
+        for _ in range(2):   # (the first call also loads the kernels)
+            torch.cuda.synchronize()
+            costs = criterion(E, P, labels, il, ll)
+            running = not torch.cuda.current_stream().query()
+        assert running
+        assert torch.isfinite(costs).all()
+        with pytest.raises(ValueError, match="Input length mismatch"):
+            criterion(E, P, labels, il + 1, ll)
+        with pytest.raises(ValueError, match="Output length mismatch"):
+            criterion.viterbi(E, P, il, ll + 1)

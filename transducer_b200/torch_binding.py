@@ -52,7 +52,7 @@ class Transducer(torch.autograd.Function):
     def forward(ctx, emissions, predictions, labels, input_lengths, label_lengths, blank=0,
                 validate_lengths=True, check_status=False):
         certify_inputs(emissions, predictions, labels, input_lengths, label_lengths,
-                       validate_lengths=False, allow_bf16=True)   # (the lengths: finish_call)
+                       validate_lengths and not check_status, allow_bf16=True)
         device = emissions.device
         emissions = emissions.contiguous()
         predictions = predictions.contiguous()
@@ -120,8 +120,9 @@ class TransducerLoss(torch.nn.Module):
         blank (int, optional): id of the blank label (default 0).
         validate_lengths (bool, optional): compare the largest input / label length with the
             padded shapes, as the reference does (default).  That check reads two numbers back
-            from the device, i.e. it synchronises the host with the stream on every call;
-            pass False to skip it when the lengths are known to fit -- the call then only
+            from the device, i.e. it synchronises the host with the stream on every call: with
+            check_status after the kernels, in one go with the status, else before them, so that
+            the call returns while they run.  Pass False to skip it when the lengths are known to fit -- the call then only
             enqueues work (and can be captured in a CUDA graph).  No counterpart in the
             reference.
         check_status (bool, optional): after the forward and the backward kernels, wait for
@@ -178,7 +179,7 @@ class TransducerLoss(torch.nn.Module):
         U = predictions.shape[1]
         labels = torch.empty((B, U - 1), device=device, dtype=torch.int32)
         certify_inputs(emissions, predictions, labels, input_lengths, label_lengths,
-                       validate_lengths=False)   # (the lengths: finish_call)
+                       self.validate_lengths and not self.check_status)
         emissions = emissions.contiguous()
         predictions = predictions.contiguous()
         with DeviceManager(device):
@@ -198,11 +199,15 @@ _SUMMARY_BYTES = 16   # of device memory behind a call's workspace, for finish_c
 
 def finish_call(emissions, predictions, input_lengths, label_lengths, ws, nbytes,
                 validate_lengths, check_status):
-    """The checks of a call that need numbers from the device, after its kernels are enqueued: one
-    small kernel and one synchronisation for the longest lengths (the reference reads them back
-    before its kernels, transducer/torch_binding.py:222-229; here every kernel limits the lengths
-    to the padded shapes, so a call with too long ones may run before it is refused) and the
-    device status.  Replaces two reductions, a stack and two synchronisations: 58 -> 22 us."""
+    """The device status of a call that waits for its kernels, and with it the lengths: one small
+    kernel and one synchronisation after the kernels are enqueued (the reference reads the
+    longest lengths back before its kernels, transducer/torch_binding.py:222-229; here every kernel
+    limits the lengths to the padded shapes, so a call with too long ones may run before it is
+    refused).  Replaces two reductions, a stack and two synchronisations: 58 -> 22 us.  A call
+    that does not check the status has its lengths checked ahead of its kernels
+    (certify_inputs) and returns without waiting for them."""
+    if not check_status:
+        return
     batch = emissions.shape[0]
     if batch > 0 and validate_lengths:
         rc, max_t, max_u = _transducer.call_summary(
@@ -210,10 +215,8 @@ def finish_call(emissions, predictions, input_lengths, label_lengths, ws, nbytes
             ws.data_ptr() + nbytes)
         if rc in (TB200_OK, TB200_ERR_DEVICE_STATUS):
             certify_lengths(emissions, predictions, max_t, max_u)
-    elif check_status:
-        rc = _transducer.check_status()
     else:
-        return
+        rc = _transducer.check_status()
     raise_for_status(rc, _transducer.last_error() if rc else "")
 
 
