@@ -96,8 +96,9 @@ int tb200_check_status(void);
 /* What a checked call wants to know when it is done, for one kernel and one synchronisation of
  * the calling thread's stream: the largest input and label length (maxLens[2], host memory; the
  * reference's wrapper reads the two maxima before the call, transducer/torch_binding.py:222-229)
- * and, if withStatus is not 0, the status word as tb200_check_status reports it.  scratch: 16 bytes
- * of device memory. */
+ * and, with withStatus = 1, the status word as tb200_check_status reports it; 2: the same, but the
+ * word is left as it is for a later tb200_check_status (a caller that will refuse the lengths has not
+ * reported the status).  scratch: 16 bytes of device memory. */
 int tb200_call_summary(const int* inLens, const int* labLens, int B, int withStatus, void* scratch,
                        int* maxLens);
 const char* tb200_status_name(int code);

@@ -4,6 +4,8 @@ host as TB200_ERR_DEVICE_STATUS / DeviceStatusError, with the CUDA context still
 The failure is produced the only permitted way: a self-test kernel waits, with a limit of a few
 microseconds, on a barrier that nothing ever completes, and returns normally.  Nothing here
 faults, traps or hangs a GPU.  The code -> exception mapping is tested without a GPU."""
+import ctypes
+
 import pytest
 import torch
 
@@ -76,3 +78,33 @@ def test_python_surface_raises_device_status_error():
         TransducerLoss()(E, P, lab, il, ll)
     costs = TransducerLoss()(E, P, lab, il, ll)               # next call is clean
     assert torch.isfinite(costs).all()
+
+
+@pytest.mark.gpu
+def test_a_length_error_does_not_swallow_the_device_status():
+    import abi
+    from transducer_b200 import DeviceStatusError, TransducerLoss, torch_binding
+    E, P = torch.randn((1, 4, 32), device="cuda"), torch.randn((1, 2, 32), device="cuda")
+    lab = torch.ones((1, 1), dtype=torch.int32, device="cuda")
+    il = torch.tensor([4], dtype=torch.int32, device="cuda")
+    ll = torch.tensor([1], dtype=torch.int32, device="cuda")
+    torch_binding.check_device_status()                       # clean to begin with
+    abi.use_torch_stream()
+    abi.check(abi.lib.tb200_selftest_wait_timeout(20))
+    with pytest.raises(ValueError, match="Input length mismatch"):
+        TransducerLoss()(E, P, lab, il + 1, ll)
+    with pytest.raises(ValueError, match="Output length mismatch"):
+        TransducerLoss().viterbi(E, P, il, ll + 1)
+    with pytest.raises(DeviceStatusError, match="self-test"):
+        torch_binding.check_device_status()
+    # a good call still reports it once
+    abi.check(abi.lib.tb200_selftest_wait_timeout(20))
+    with pytest.raises(DeviceStatusError, match="self-test"):
+        TransducerLoss()(E, P, lab, il, ll)
+    assert torch.isfinite(TransducerLoss()(E, P, lab, il, ll)).all()
+    # and a C caller that asks for it with the summary has it reported and cleared
+    abi.check(abi.lib.tb200_selftest_wait_timeout(20))
+    scratch, lens = torch.zeros(4, dtype=torch.int32, device="cuda"), (ctypes.c_int * 2)()
+    summary = lambda: abi.lib.tb200_call_summary(il.data_ptr(), ll.data_ptr(), 1, 1, scratch.data_ptr(), lens)
+    assert summary() == errors.TB200_ERR_DEVICE_STATUS and list(lens) == [4, 1]
+    assert summary() == 0

@@ -170,12 +170,13 @@ PYBIND11_MODULE(_transducer, m) {
   // Returns the code of tb200_check_status (0, or 5 = a kernel gave up) without throwing, so the
   // Python layer can raise its own exception type; the text is in last_error().
   m.def("check_status", []() { return tb200_check_status(); });
-  // (code as check_status, longest input length, longest label length), after one synchronisation
+  // (code as check_status, longest input length, longest label length), after one synchronisation;
+  // the status word is left for check_status to clear
   m.def("call_summary",
         [](addr ilen, addr llen, int B, bool withStatus, addr scratch) {
           int maxLens[2] = {0, 0};
           const int rc = tb200_call_summary(at<const int>(ilen), at<const int>(llen), B,
-                                            withStatus ? 1 : 0, at<void>(scratch), maxLens);
+                                            withStatus ? 2 : 0, at<void>(scratch), maxLens);
           return py::make_tuple(rc, maxLens[0], maxLens[1]);
         },
         "input_lengths"_a, "label_lengths"_a, "batch_size"_a, "with_status"_a, "scratch"_a);

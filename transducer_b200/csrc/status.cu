@@ -50,11 +50,11 @@ __global__ void __launch_bounds__(32) selftest_wait_kernel(int* status, unsigned
   if (threadIdx.x == 0) *observed = all ? 1 : 0;  // 0: the wait gave up, as it should
 }
 
-// out = {max inLens, max labLens, status code, nodes recomputed}; the last two are taken from the
-// status word, which is cleared, if `word` is not null.
+// out = {max inLens, max labLens, status code}; the last from the status word, if `word` is not null,
+// which is cleared or left as it is.
 __global__ void __launch_bounds__(256) call_summary_kernel(const int* __restrict__ inLens,
                                                            const int* __restrict__ labLens, int B,
-                                                           int* word, int* __restrict__ out) {
+                                                           int* word, bool clear, int* __restrict__ out) {
   __shared__ int sT[8], sU[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int t = INT_MIN, u = INT_MIN;
@@ -76,8 +76,8 @@ __global__ void __launch_bounds__(256) call_summary_kernel(const int* __restrict
     }
     out[0] = t;
     out[1] = u;
-    out[2] = word ? atomicExch(word, 0) : 0;
-    out[3] = word ? atomicExch(word + 1, 0) : 0;
+    out[2] = !word ? 0 : clear ? atomicExch(word, 0) : atomicAdd(word, 0);
+    if (word && clear) atomicExch(word + 1, 0);
   }
 }
 
@@ -151,12 +151,13 @@ int tb200_call_summary(const int* inLens, const int* labLens, int B, int withSta
     if (B <= 0 || !inLens || !labLens || !scratch || !maxLens)
       return api_fail(kErrInvalidArgument, "tb200_call_summary: null pointer or empty batch");
     int* out = static_cast<int*>(scratch);
-    int host[4];
+    int host[3];
     cudaStream_t s = api_stream();
     {
       ScopedKernel sk("call_summary", s);
       call_summary_kernel<<<1, 256, 0, s>>>(inLens, labLens, B,
-                                            withStatus ? device_status_word() : nullptr, out);
+                                            withStatus ? device_status_word() : nullptr,
+                                            withStatus == 1, out);
     }
     TB200_CHECK_LAUNCH();
     TB200_CUDA_CHECK(cudaMemcpyAsync(host, out, sizeof(host), cudaMemcpyDeviceToHost, s));

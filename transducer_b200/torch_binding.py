@@ -214,7 +214,10 @@ def finish_call(emissions, predictions, input_lengths, label_lengths, ws, nbytes
             input_lengths.data_ptr(), label_lengths.data_ptr(), batch, check_status,
             ws.data_ptr() + nbytes)
         if rc in (TB200_OK, TB200_ERR_DEVICE_STATUS):
+            # (a length error leaves the status for the next check, as it did not report it)
             certify_lengths(emissions, predictions, max_t, max_u)
+        if rc == TB200_ERR_DEVICE_STATUS:
+            rc = _transducer.check_status()
     else:
         rc = _transducer.check_status()
     raise_for_status(rc, _transducer.last_error() if rc else "")
