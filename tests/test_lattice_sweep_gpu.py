@@ -75,3 +75,30 @@ def test_host_threads_with_different_shapes():
     for t in threads:
         t.join()
     assert not failures, failures[:3]
+
+
+@pytest.mark.parametrize("T,U", [(1, 129), (60, 150), (31, 161), (90, 200), (40, 225), (100, 256), (4200, 256)])
+def test_wide_axes_against_the_row_major_kernel(T, U):
+    """Axes of 129..256 positions (natural logarithms at full magnitude) against the kernel behind
+    tb200_forward on the same log-normalisers; more frames than the sweep stages (4096 at 256
+    positions) included."""
+    B, V = 3, 36
+    g = torch.Generator(device="cuda").manual_seed(T + U)
+    E = torch.empty((B, T, V), device="cuda").normal_(0, 3, generator=g)
+    P = torch.empty((B, U, V), device="cuda").normal_(0, 3, generator=g)
+    E[1, :, 1:].masked_fill_(torch.rand((T, V - 1), generator=g, device="cuda") < 0.2, float("-inf"))
+    labels = torch.randint(1, V, (B, U - 1), generator=g, device="cuda", dtype=torch.int32)
+    il = torch.tensor([T, T, max(1, T // 2)], dtype=torch.int32, device="cuda")
+    ll = torch.tensor([U - 1, U - 2, U // 2], dtype=torch.int32, device="cuda")
+    abi.set_option("lognorm_path", 1)
+    try:
+        ln = abi.log_norms(E, P, il, ll)[0]
+        costs = abi.loss_forward(E, P, labels, il, ll)["costs"]
+    finally:
+        abi.set_option("lognorm_path", 0)
+    want = abi.forward(E, P, ln, labels, il, ll)[0]
+    # per node of a path of T + U: 2^-22 of the hardware logaddexp, three roundings of an alpha (4 sigma)
+    finite = torch.isfinite(want)
+    tol = (T + U) * 2.0 ** -22 + 4.0 * (3 * (T + U)) ** 0.5 * 2.0 ** -24 * want[finite].max().item()
+    assert finite[0] and finite[2]   # (the masked utterance of one frame has no path)
+    assert (costs - want)[finite].abs().max().item() < tol and torch.equal(costs[~finite], want[~finite])

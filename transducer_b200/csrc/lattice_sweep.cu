@@ -300,16 +300,19 @@ struct NaturalTerms {
 // log(exp(a)+exp(b)) with the reference's -inf handling and operation order; the correction term
 // is evaluated with the hardware ex2/lg2 units (absolute error ~2e-7, far below one ulp of the
 // alphas it is added to once they exceed a few units in magnitude).
+// What counts is the number of instructions (895 instead of ~200 cycles per diagonal with branches for
+// -inf).  One of them -inf: the correction is log(1 + 0) by itself.  Both: the minimum with 0 turns
+// the NaN of their difference into a finite correction.  The .ftz forms have the same results: an
+// exponential that would be subnormal adds nothing to 1.
 __device__ __forceinline__ float lse2_fast(float a, float b) {
-  // (one of them -inf: the correction is log(1 + 0) = 0 by itself; branches would cost more than the
-  // sum: 895 instead of ~200 cycles per diagonal)
-  const float m = fmaxf(a, b), v = m + __logf(1.0f + __expf(-fabsf(a - b)));
-  return (m == neg_inf() && a == b) ? m : v;
+  float m;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));   // (NaN if one of them is)
+  return m + lg2_approx(1.0f + ex2_approx(fminf(-fabsf(a - b), 0.0f) * kLog2e)) * kLn2F;
 }
 
 // Label axes of 129..256 positions: pair rows (LN, E[t,label_u]), (+inf, 0) where there is no node,
 // so that whatever leaves such a node is -inf.  E[t,blank] of a lane's first position is read from
-// shared memory (the first maxStage frames; beyond, from global), the others' follow from it:
+// shared memory (an utterance of more than maxStage frames: from global), the others' follow from it:
 // position r + 1 meets a frame one diagonal after position r.
 template <int NPL>
 __global__ void __launch_bounds__(32) alpha_natural_kernel(
@@ -332,9 +335,10 @@ __global__ void __launch_bounds__(32) alpha_natural_kernel(
   for (int k = 0; k < kRing - 1; ++k) issue(k);
   const float* ebl = n.ebl + (i64)b * maxT;
   float* sEb = reinterpret_cast<float*>(smemA + kRing * kDiag * ld * 8);
-  for (int t = lane; t < min(T, maxStage); t += 32) sEb[t] = ebl[t];
+  const bool staged = T <= maxStage;
+  for (int t = lane; staged && t < T; t += 32) sEb[t] = ebl[t];
   __syncwarp();
-  const float* ebRow = T <= maxStage ? sEb : ebl;
+  const float* ebRow = staged ? sEb : ebl;
   auto eblAt = [&](int t) { return ebRow[min(max(t, 0), T - 1)]; };
   float* al = alphas + (i64)b * stride;
   float pbl[NPL], plab[NPL], eb[NPL], stay[NPL], step[NPL];
