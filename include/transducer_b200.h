@@ -58,8 +58,9 @@ void* tb200_get_stream(void);
  *                   weights are always rounded once to TF32.  1: exp(E), exp(P) rounded
  *                   once too; 2 (default): exp(E) split hi+lo (exact products for
  *                   pgrads); 3: exp(P) split as well (smaller tiles, slower)
- *   "fused_gather"  1 (default): the tensor-core log-normaliser also hands out E[t,label_u] and
- *                   E[t,blank] from the rows it streams; 0: a separate gather pass fetches them
+ *   "fused_gather"  2: the tensor-core log-normaliser also hands out E[t,label_u] and E[t,blank] from
+ *                   the rows it streams; 0: the lattice re-layout fetches them; 1 (default): the
+ *                   former for emissions of more than 96 MB, which have left the L2 by then
  *   "maxplus_path"  label-arc scores of the Viterbi pass (tb200_label_arc_scores): 0 auto,
  *                   1 the full loop over the alphabet, 2 candidate lists with an exact bound
  * Unknown keys return TB200_ERR_INVALID_ARGUMENT.  No counterpart in the reference. */

@@ -213,8 +213,9 @@ bool log_norms_impl(const void* E, const void* P, float* LN, float* rowRef, floa
     // other), a gather from L2 1..3 us.  Forward time of the two kernels, handed out / gathered:
     // E of 6 MB 60 / 51 us, 65 MB 88 / 84, 256 MB 138 / 144, 640 MB 260 / 270.
     const size_t bytesE = (size_t)d.B * d.maxT * d.V * (d.dtype == kDtypeBf16 ? 2 : 4);
-    const bool gathers = labels && EL && ebl && lognorm_umma_gathers(d) && g_opt.fused_gather != 0 &&
-                         bytesE > (size_t)96 << 20;
+    const int handOut = g_opt.fused_gather;
+    const bool gathers = labels && EL && ebl && lognorm_umma_gathers(d) &&
+                         (handOut == 2 || (handOut == 1 && bytesE > (size_t)96 << 20));
     launch_lognorm_umma(E, P, LN, rowRef, mp, inLens, labLens, d, ws.split,
                         device_status_word(), fixup, g_stream, gathers ? labels : nullptr,
                         gathers ? EL : nullptr, gathers ? ebl : nullptr);
@@ -255,7 +256,7 @@ int tb200_set_option(const char* key, int value) {
   if (!strcmp(key, "lognorm_path") && value >= 0 && value <= 3) g_opt.lognorm_path = value;
   else if (!strcmp(key, "grads_path") && value >= 0 && value <= 2) g_opt.grads_path = value;
   else if (!strcmp(key, "grad_passes") && value >= 1 && value <= 3) g_opt.grad_passes = value;
-  else if (!strcmp(key, "fused_gather") && value >= 0 && value <= 1) g_opt.fused_gather = value;
+  else if (!strcmp(key, "fused_gather") && value >= 0 && value <= 2) g_opt.fused_gather = value;
   else if (!strcmp(key, "maxplus_path") && value >= 0 && value <= 2) g_opt.maxplus_path = value;
   else return fail(kErrInvalidArgument, std::string("unknown option or bad value: ") + key);
   return kOk;
