@@ -39,9 +39,10 @@ def test_edges(T, U):
     assert torch.equal(eg, eg2) and torch.equal(pg, pg2)
     n = lambda x: x.cpu().numpy()
     ref = O.truth64(n(E), n(P), n(labels), n(il), n(ll))
-    # A stored alpha is below 1024 in magnitude (up to 128 positions: relative to its block; beyond:
-    # at T + U <= 356 here) and rounded to 2^-14, 2^-15 at most, which is what the T + U factors of a
-    # path carry, independently: 4 sigma.  1e-5: the fp32 contractions.
+    # A stored alpha is below 1024 in magnitude for these scores (up to 128 positions: at most two blocks
+    # of 16 arcs of up to 20 below its block's offset; beyond: at T + U <= 356) and rounded to 2^-14,
+    # 2^-15 at most, which is what the T + U factors of a path carry, independently: 4 sigma.
+    # 1e-5: the fp32 contractions.
     tol = 4.0 * np.sqrt(T + U) * 2.0 ** -15 + 1e-5
     costs = n(fwd["costs"])
     np.testing.assert_allclose(costs[:3], ref["costs"][:3], rtol=1e-6, atol=tol)
@@ -75,6 +76,50 @@ def test_host_threads_with_different_shapes():
     for t in threads:
         t.join()
     assert not failures, failures[:3]
+
+
+@pytest.mark.parametrize("T,U,std,bias,masked", [(130, 100, 15.0, 0.0, False), (200, 30, 3.0, 25.0, False),
+                                                 (90, 160, 15.0, 0.0, False), (60, 60, 1.0, 0.0, True),
+                                                 (60, 170, 1.0, 0.0, True)])
+def test_large_and_masked_scores(T, U, std, bias, masked):
+    """Arcs far larger than N(0,1) scores give, and words masked by -inf (from the second frame on, so
+    that every node stays reachable).  How large a stored alpha gets depends on the arcs, and
+    so does what its rounding costs."""
+    B, V, blank = 3, 40, 0
+    g = torch.Generator(device="cuda").manual_seed(T * U)
+    E = torch.empty((B, T, V), device="cuda").normal_(0, std, generator=g)
+    P = torch.empty((B, U, V), device="cuda").normal_(0, std, generator=g)
+    E[:, :, blank] += bias
+    labels = torch.randint(1, V, (B, U - 1), generator=g, device="cuda", dtype=torch.int32)
+    il = torch.tensor([T, T - 1, T // 2], dtype=torch.int32, device="cuda")
+    ll = torch.tensor([U - 1, U // 2, U - 2], dtype=torch.int32, device="cuda")
+    E_ref = E.clone()
+    if masked:
+        hide = torch.rand((B, T - 1, V - 1), generator=g, device="cuda") < 0.2
+        E[:, 1:, 1:].masked_fill_(hide, float("-inf"))
+        E_ref[:, 1:, 1:].masked_fill_(hide, -1e4)   # (the oracle's lattice wants finite scores)
+    abi.set_option("lognorm_path", 1)
+    abi.set_option("grads_path", 1)
+    try:
+        fwd = abi.loss_forward(E, P, labels, il, ll)
+        eg, pg = abi.loss_backward(E, P, labels, il, ll, fwd)
+    finally:
+        abi.set_option("lognorm_path", 0)
+        abi.set_option("grads_path", 0)
+    n = lambda x: x.cpu().numpy()
+    ref = O.truth64(n(E_ref), n(P), n(labels), n(il), n(ll))
+    # largest arc a path takes, in nats: among the best of each node, as an upper bound the blank's
+    lse = torch.logsumexp(E.double()[:, :, None] + P.double()[:, None], dim=3)
+    arc = (lse - E[:, :, None, blank] - P[:, None, :, blank]).max().item()
+    # a stored alpha: up to 128 positions at most 32 arcs below its offset, in log2 units; beyond, the
+    # whole path.  Rounded to half an ulp, T + U of them along a path, independently: 4 sigma, and
+    # twice that for the three roundings of an arc's sum.
+    size = 32 * arc * 1.4427 if U <= 128 else float(np.max(ref["costs"])) + 32 * arc
+    tol = 8.0 * np.sqrt(T + U) * 2.0 ** -25 * size + 1e-5
+    assert tol < 0.05
+    np.testing.assert_allclose(n(fwd["costs"]), ref["costs"], rtol=1e-6, atol=tol)
+    assert abi.rel_to_max(n(eg), ref["egrads"]) < tol
+    assert abi.rel_to_max(n(pg), ref["pgrads"]) < tol
 
 
 @pytest.mark.parametrize("T,U", [(1, 129), (60, 150), (31, 161), (90, 200), (40, 225), (100, 256), (4200, 256)])

@@ -247,3 +247,36 @@ def test_length_check_alone_does_not_wait_for_the_kernels():
             criterion(E, P, labels, il + 1, ll)
         with pytest.raises(ValueError, match="Output length mismatch"):
             criterion.viterbi(E, P, il, ll + 1)
+
+
+def test_too_long_lengths_are_refused_after_the_kernels():
+    """The default call fetches the lengths together with the status after its kernels, which limit
+    them to the padded shapes; the offender sits behind the first 256 utterances, a block of the
+    kernel that looks for it.  The call after the refusal is right."""
+    B, T, U, V = 300, 6, 3, 32
+    g = torch.Generator(device="cuda").manual_seed(5)
+    E = torch.empty((B, T, V), device="cuda").normal_(generator=g)
+    P = torch.empty((B, U + 1, V), device="cuda").normal_(generator=g)
+    labels = torch.randint(1, V, (B, U), generator=g, device="cuda", dtype=torch.int32)
+    il = torch.randint(1, T, (B,), generator=g, device="cuda", dtype=torch.int32)
+    ll = torch.randint(0, U, (B,), generator=g, device="cuda", dtype=torch.int32)
+    criterion = TransducerLoss()
+    want = criterion(E, P, labels, il, ll)
+    best = criterion.viterbi(E, P, il, ll)
+    for at in (0, 255, 256, 299):
+        il2, ll2 = il.clone(), ll.clone()
+        il2[at], ll2[at] = T + 1, U + 1
+        with pytest.raises(ValueError, match="Input length mismatch"):
+            criterion(E, P, labels, il2, ll)
+        with pytest.raises(ValueError, match="Output length mismatch"):
+            criterion(E, P, labels, il, ll2)
+        with pytest.raises(ValueError, match="Input length mismatch"):
+            criterion.viterbi(E, P, il2, ll)
+        with pytest.raises(ValueError, match="Output length mismatch"):
+            criterion.viterbi(E, P, il, ll2)
+    il2, ll2 = il.clone(), ll.clone()
+    il2[299], ll2[299] = T, U          # as long as the padding: fine
+    assert torch.isfinite(criterion(E, P, labels, il2, ll2)).all()
+    assert torch.equal(criterion(E, P, labels, il, ll), want)
+    valid = torch.arange(U, device="cuda")[None] < ll[:, None]
+    assert torch.equal(criterion.viterbi(E, P, il, ll)[valid], best[valid])
