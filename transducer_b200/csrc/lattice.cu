@@ -488,13 +488,18 @@ void check_lattice_fits_int(Dims d) {
 
 }  // namespace
 
-#define TB200_DISPATCH_STRIPS(cfg, CALL)                  \
+// (the skewed kernels serve label axes of more than 256 positions only)
+#define TB200_DISPATCH_WIDE_STRIPS(cfg, CALL)             \
   do {                                                    \
-    if ((cfg).R == 1 && (cfg).threads <= 256) { CALL(1, 8, 256); } \
-    else if ((cfg).R == 1) { CALL(1, 4, 1024); }          \
+    if ((cfg).R == 1) { CALL(1, 4, 1024); }               \
     else if ((cfg).R == 2) { CALL(2, 2, 1024); }          \
     else if ((cfg).R == 4) { CALL(4, 1, 1024); }          \
     else { CALL(8, 1, 1024); }                            \
+  } while (0)
+#define TB200_DISPATCH_STRIPS(cfg, CALL)                  \
+  do {                                                    \
+    if ((cfg).R == 1 && (cfg).threads <= 256) { CALL(1, 8, 256); } \
+    else { TB200_DISPATCH_WIDE_STRIPS(cfg, CALL); }       \
   } while (0)
 
 void launch_alpha(const float* E, const float* P, float* costs, float* alphas,
@@ -534,7 +539,7 @@ void launch_alpha_skew(const float* P, float* costs, float* alphasS, const float
   alpha_kernel<R, PF, NT, true><<<d.B, cfg.threads, 0, stream>>>(                    \
       nullptr, P, costs, alphasS, LNs, ELs, ebl, g.ld, g.stride, labels, inLens,    \
       labLens, d.B, d.maxT, d.maxU, d.V, d.blank, lossSum, ticket)
-  TB200_DISPATCH_STRIPS(cfg, CALL);
+  TB200_DISPATCH_WIDE_STRIPS(cfg, CALL);
 #undef CALL
   TB200_CHECK_LAUNCH();
 }
@@ -586,7 +591,7 @@ void launch_gamma_skew(const float* P, const float* alphasS, const float* LNs,
       nullptr, P, alphasS, LNs, ELs, ebl, g.ld, g.stride, rowRef, maxP, labels,       \
       inLens, labLens, nullptr, nullptr, nullptr, Ws, g.ld, EMs, eBlank, pBlank,      \
       pLabel, d.maxT, d.maxU, d.V, d.blank)
-  TB200_DISPATCH_STRIPS(cfg, CALL);
+  TB200_DISPATCH_WIDE_STRIPS(cfg, CALL);
 #undef CALL
   TB200_CHECK_LAUNCH();
 }
