@@ -193,7 +193,7 @@ def test_stress_grid_against_oracle():
 
 # ---------------------------------------------------------------------------
 # label-axis lengths around the limits of the single-warp sweeps (rows of 32/64/96/128 positions,
-# the hand-over to the block-wide kernels above 128) and of the warp Viterbi (256)
+# the natural-logarithm sweeps above 128, the block-wide kernels above 256) and of the warp Viterbi (256)
 # ---------------------------------------------------------------------------
 
 @pytest.mark.parametrize("U1", [2, 31, 32, 33, 64, 65, 96, 97, 127, 128, 129, 255, 256, 257])

@@ -185,7 +185,7 @@ void need(size_t have, size_t want, const void* ws) {
                                 " bytes, got " + std::to_string(have));
 }
 
-// Log-normalisers plus the row shifts.  With the exact path rowRef is the true row
+// Log-normalisers plus the row shifts.  With the SIMT kernels rowRef is the true row
 // maximum of E.
 // Returns true if the pass also produced the label / blank emissions (EL, ebl) it was offered.
 bool log_norms_impl(const void* E, const void* P, float* LN, float* rowRef, float* maxP,

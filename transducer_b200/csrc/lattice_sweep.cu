@@ -13,7 +13,8 @@
 //
 // Axes of up to 128 positions run on rebased base-2 logarithms (alpha_sweep_kernel); longer ones
 // (NPL >= 5, "natural" below) on natural logarithms at full magnitude, in the operation order of the
-// block-wide kernels of lattice.cu and bit-identical to them.
+// block-wide kernels of lattice.cu (costs bit-identical to theirs: 18 shapes, T = 77..5000,
+// U' = 129..256).
 //
 // Diagonal d = t + u of an utterance is one row of ld = 32 NPL numbers; lane l of a sweep owns the
 // NPL adjacent positions u = NPL l + r.  All nodes of a diagonal are independent; the one value
@@ -22,12 +23,12 @@
 // diagonal takes: operands are brought to shared memory by cp.async, each lane copying just the
 // 8 NPL bytes a row that it reads itself (no barrier, no other warp), several blocks of 16
 // diagonals ahead, and the loop holds nothing but the recursion and its store.
-// Measured (T = 2000, U' = 101, device time, B = 8 / 32): alpha 128 us (140 with bulk copies issued and
-// waited for by the sweeping warp); reverse sweep 10 / 21 us for the factors + 57 us for the recursion
-// (146 us when helper warps of the same CTA prepared the factors and carried away the results).
-// B = 64, T = 750..1500, U' = 151: alpha 213 us, factors 62 + recursion 73 us, operands 125 us, against
-// 381, 511 and (lattices re-laid out twice) 168 us of the block-wide kernels, which take a barrier
-// per diagonal.
+// Measured (T = 2000, U' = 101, device time, B = 8 / 32): alpha 132 us (147 with bulk copies issued and
+// waited for by the sweeping warp); reverse sweep 12 / 27 us for the factors + 60 us for the recursion
+// (152 us when helper warps of the same CTA prepared the factors and carried away the results).
+// B = 64, T = 750..1500, U' = 151: alpha 195 us, factors 65 + recursion 76 us, operands 105 us, against
+// 384, 512 and (lattices re-laid out twice) 168 us of the block-wide kernels, which take a barrier
+// per diagonal.  B = 8, T = 4000, U' = 251: alpha 855 us, block-wide 954.
 #include <algorithm>
 
 #include "kernels.h"
@@ -190,9 +191,11 @@ __device__ __forceinline__ void finish_cost(float* costs, int b, float cost, int
 // Here every block of 16 diagonals stores its alphas relative to an offset of its own: at the
 // start of block k the whole carried state is lowered by delta_k = the floor of its largest
 // entry (an integer, so that the running offset -- needed only for the final cost -- adds up
-// exactly), which keeps every stored number below ~500 in magnitude (ulp 3e-5).  delta_k is
-// written to `deltas` for the reverse sweep, which subtracts it at the same point of the same
-// sum.  The loss and the gradients then sit ~1e-4 from the float64 result.
+// exactly).  As delta_k is taken one block early, a stored number that matters lies at most 32
+// arcs below its offset: a few hundred for N(0,1..2) scores (ulp 3e-5), 4600 for arcs of
+// 100 nats; nothing else bounds it.  delta_k is written to `deltas` for the reverse sweep, which
+// subtracts it at the same point of the same sum.  The loss and the gradients then sit ~1e-4 from
+// the float64 result.
 //
 // The pace is set by the special-function unit: NPL ex2 and NPL lg2 per diagonal, 8 issue cycles
 // each, in a chain.  (Cutting the label axis over two or four warps that run a block apart was
@@ -241,8 +244,7 @@ __global__ void __launch_bounds__(32) alpha_sweep_kernel(
     }
     // The delta applied at the start of the NEXT block is the floor of the largest entry of
     // the state now, at the start of this one: the warp-wide maximum then has a whole block to
-    // arrive, off the dependent chain.  (By then the state has sunk by another ~16 arcs; all
-    // that matters is that the stored numbers stay small: below ~1000, ulp 6e-5.)
+    // arrive, off the dependent chain.  (By then the state has sunk by another 16 arcs.)
     {
       float m = kNone;
 #pragma unroll
@@ -406,7 +408,7 @@ __global__ void __launch_bounds__(32) alpha_natural_kernel(
 //
 // gamma_factors_kernel: the pairs (FB, FL) of every node of the diagonals below S, zero where there
 // is no arc (natural: from the pair rows of alpha_natural_kernel, by the accurate expf).  One warp
-// per 4 diagonals.  Bound by memory: 16 bytes read, 8 written per node.
+// per 4 diagonals.  Bound by memory: a pair and an alpha (12 bytes) read, 8 written per node.
 constexpr int kFactorRows = 4, kFactorWarps = 8;
 template <int NPL>
 __global__ void __launch_bounds__(32 * kFactorWarps) gamma_factors_kernel(

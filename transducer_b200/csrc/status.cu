@@ -1,7 +1,8 @@
 // Device status word: how a bounded wait that ran out inside a kernel reaches the host.
 //
-// Every wait of the tensor-core and single-warp sweep kernels (on an mbarrier that a TMA copy,
-// an MMA commit or another role completes) gives up after sm100::kWaitLimitNs.  The kernel then
+// Every wait on an mbarrier that a copy, an MMA commit or another role completes (the tensor-core
+// kernels, the Viterbi sweep, the candidate lists; the loss's sweeps wait for nothing but their own
+// cp.async groups) gives up after sm100::kWaitLimitNs.  The kernel then
 // records WHICH wait in this word (first failure wins, the word is sticky), drains its roles,
 // frees its tensor memory, poisons its outputs (NaN costs / log-normalisers / gradients, -1
 // labels) and returns normally -- the context stays usable.  The reference has no device-side
