@@ -57,25 +57,31 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) lognorm_exact_kernel(
 // the split is what fills the chip.  exp(E - rowMax) and exp(P - maxP) of a step are formed once
 // per CTA and stored transposed (lanes = 8 words x 4 rows: the stores of a warp fall into 32
 // different banks), while the next step's entries are already on their way into registers.
-// Precision: an exponential keeps what the subtraction of the row's maximum rounded off, sums have
-// three levels (16 words, 16 steps, the rest), and the logarithm is taken and the references added in
-// fp64, so that the result is no further from float64 than lognorm_exact's.  Measured, V = 29..8041,
+// Precision: the exponentials are exact to the hardware's ex2 whatever the row's maximum (below), sums
+// have three levels (16 words, 16 steps, the rest), and the logarithm is taken and the references added
+// in fp64, so that the result is no further from float64 than lognorm_exact's.  Measured, V = 29..8041,
 // rms over the nodes relative to lognorm_exact's own (1e-7..1.5e-6, mostly the rounding of the
-// result): N(0,1..5) scores 0.74..0.99, confident words 5..45 above the rest 0.75..1.01, such words
-// cancelled by P 0.77..0.99, log-softmax rows 0.71..1.0; above 1 only where one word of a V = 29
-// alphabet carries a small logarithm (1.12, 1.4e-7).  (With ex2 of the rounded difference and logf:
-// up to 8.5 times.)
-// The references lie kFacShift below the rows' maxima: a factor is at most e^32, a sum at most
-// V e^64 = 6e27 V, and what factors lose as subnormal numbers, V 2^-150 e^32, is below 2^-26 of a
-// sum of V 2^-124 e^32 or more, i.e. down to sums 110 below the two maxima.
+// result): N(0,1..5) scores 0.74..0.91, confident words 5..45 above the rest 0.61..0.92, such words
+// cancelled by P 0.77..0.92, crossing 0.40..1.02, log-softmax rows 0.65..0.99.  (With ex2 of the
+// rounded difference and logf: up to 8.5.)
+// The references lie 2^46 below the rows' maxima: a factor is at most 2^47, a sum V 2^94, and what
+// factors below 2^-126 lose, V 2^-126 2^47, is below 2^-26 of a sum of V 2^-53 or more, i.e. down
+// to sums e^-94 (V = 1025) of the two maxima's product.
 // A batch of few tiles would leave most of the chip idle through a long vocabulary: a cluster of up
 // to 8 CTAs then shares a tile, each with its part of the steps, and the first adds the others'
 // sums, read from their shared memory, in rank order.
 // Nodes with a smaller sum, or one that is not finite, become NaN, as from the tensor-core kernel:
 // the caller has them recomputed exactly.
-// Bound by fp32 issue: per word and thread 16 FFMA, two 16-byte shared loads and, by the thirty-
-// second part each, an exponential, a load and a store.
-constexpr float kFacShift = 32.0f;
+// Bound by fp32 issue: per word and thread 16 FFMA, two 16-byte shared loads and one exponential with
+// its load and store, about ten instructions more.  (B=16 T=600 U'=81 V=1025: 134 us; 158 with expf of
+// the difference and the remainder of a 2Sum, 115 with the bare ex2 of it.)
+constexpr float kFacShift = 46.0f;
+__device__ __forceinline__ float ex2_ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float fac_ref(float rowMax) { return rintf(rowMax * 1.4426950408889634f) - kFacShift; }
 constexpr int kFacM = 32, kFacK = 64, kFacLd = kFacM + 4;
 __global__ void __launch_bounds__(256) lognorm_factored_kernel(
     const float* __restrict__ E, const float* __restrict__ P, const float* __restrict__ rowMax,
@@ -99,7 +105,7 @@ __global__ void __launch_bounds__(256) lognorm_factored_kernel(
   const int kk = lane & 7, row = 4 * w + (lane >> 3);
   const i64 tRow = (i64)b * maxT + min(t0 + row, T - 1), uRow = (i64)b * maxU + min(u0 + row, U - 1);
   const float *er = E + tRow * V + vBegin + kk, *pr = P + uRow * V + vBegin + kk;   // advanced step by step
-  const float eRef = rowMax[tRow] - kFacShift, pRef = maxP[uRow] - kFacShift;
+  const float eRef = fac_ref(rowMax[tRow]), pRef = fac_ref(maxP[uRow]);
   float xe[2][8], xp[2][8];   // entries of the next two steps
   int left = vEnd - vBegin - kk;   // words from the next step's first one on
   auto load = [&](float (&ye)[8], float (&yp)[8]) {
@@ -120,11 +126,13 @@ __global__ void __launch_bounds__(256) lognorm_factored_kernel(
     pr += kFacK;
     left -= kFacK;
   };
-  // exp(x - ref), the subtraction's rounding error (2Sum) put back to first order, so that a word far
-  // below its row's maximum keeps its last bits.  (Its remainder is NaN where the word is masked.)
+  // exp(x) 2^-ref = 2^f 2^(n - ref), n = rint(x log2(e)) and |f| <= 1/2 by Cody and Waite's reduction with
+  // log2(e) in two parts: the reference is an integer in the exponent, so that nothing is rounded
+  // off a word however far below its row's maximum it lies.  (f is not finite where it is masked.)
   auto ex = [](float x, float ref) {
-    const float d = x - ref, c = d - x, r = (x - (d - c)) - (ref + c), y = expf(d);
-    return d < -200.0f ? 0.0f : fmaf(y, r, y);
+    constexpr float kLog2e = 1.4426950408889634f, kLog2eLo = 1.9259629911e-8f;
+    const float n = rintf(x * kLog2e), f = fmaf(x, kLog2eLo, fmaf(x, kLog2e, -n)), k = n - ref;
+    return k < -200.0f ? 0.0f : ex2_ftz(f) * ex2_ftz(k);
   };
   auto put = [&](int s, const float (&ye)[8], const float (&yp)[8]) {
 #pragma unroll
@@ -195,7 +203,7 @@ __global__ void __launch_bounds__(256) lognorm_factored_kernel(
     }
     cluster.sync();
   }
-  const float smallest = (float)V * 4e-24f;   // V 2^-124 e^shift
+  const float smallest = (float)V * 0x1p-53f;
   int flagged = 0;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -208,8 +216,8 @@ __global__ void __launch_bounds__(256) lognorm_factored_kernel(
         x = red[i];
         for (int r = 1; r < ranks; ++r) x += cluster.map_shared_rank(red, r)[i];
       }
-      const double ref = (double)(rowMax[(i64)b * maxT + t] - kFacShift) + (double)(maxP[(i64)b * maxU + u] - kFacShift);
-      float ln = (float)(ref + log((double)x));
+      const double ref = (double)fac_ref(rowMax[(i64)b * maxT + t]) + (double)fac_ref(maxP[(i64)b * maxU + u]);
+      float ln = (float)(ref * 0.6931471805599453 + log((double)x));
       if (!(x >= smallest && x < pos_inf())) {
         ln = __int_as_float(0x7fc00000);
         ++flagged;
@@ -289,16 +297,16 @@ FacGrid fac_grid(Dims d) {
 
 // Estimates of both kernels' time in us: a warp of lognorm_exact passes over the vocabulary twice,
 // with about 340 words' worth of fixed work; lognorm_factored computes whole tiles whatever the
-// label axis, 2.2 us per step of 64 words with two CTAs on an SM and 1.4 with one.  The line lies at
+// label axis, 1.8 us per step of 64 words with two CTAs on an SM and 1.2 with one.  The line lies at
 // 4 to 9 label positions for many nodes and higher for few.  Measured (us for the call, exact /
 // factored; row maxima and, for the latter, the pass over marked nodes included): B=64 T=1000 V=1301
-// U'=2 220 / 397, 4 343 / 398, 6 472 / 399; B=8 T=400 V=1025 U'=2 18 / 35, 8 30 / 35, 12 42 / 35;
-// B=8 T=400 V=8041 U'=4 150 / 168, 8 201 / 168; B=1 T=300 V=1025 U'=33 19 / 23, 65 27 / 23.
+// U'=2 220 / 347, 4 343 / 348, 6 472 / 348; B=8 T=400 V=1025 U'=2 19 / 33, 8 29 / 33, 12 42 / 34;
+// B=8 T=400 V=8041 U'=4 136 / 150, 8 202 / 151; B=1 T=300 V=1025 U'=33 19 / 23, 65 27 / 23.
 bool lognorm_factored_pays(Dims d) {
   const FacGrid g = fac_grid(d);
   const double ctas = (double)g.tiles * g.ranks, nodes = (double)d.B * d.maxT * d.maxU;
   const double exact = 4e-3 * d.V + 0.6e-6 * nodes * (d.V + 340.0);
-  const double factored = 6.0 + (ctas <= kFacResident / 2 ? 1.4 : 2.2) * std::max(1.0, ctas / kFacResident) *
+  const double factored = 9.0 + (ctas <= kFacResident / 2 ? 1.2 : 1.8) * std::max(1.0, ctas / kFacResident) *
                                     div_up(g.steps, g.ranks);
   return factored < exact;
 }
