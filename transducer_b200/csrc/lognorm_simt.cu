@@ -72,9 +72,11 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) lognorm_exact_kernel(
 // sums, read from their shared memory, in rank order.
 // Nodes with a smaller sum, or one that is not finite, become NaN, as from the tensor-core kernel:
 // the caller has them recomputed exactly.
-// Bound by fp32 issue: per word and thread 16 FFMA, two 16-byte shared loads and one exponential with
-// its load and store, about ten instructions more.  (B=16 T=600 U'=81 V=1025: 134 us; 158 with expf of
-// the difference and the remainder of a 2Sum, 115 with the bare ex2 of it.)
+// Per word and thread 16 FFMA, two 16-byte shared loads and one exponential with its load and store, about
+// ten instructions more; bound by the shared-memory and special-function queue (44 % of the issue
+// slots used, stalls: short scoreboard 1.9, queue full 1.5 per instruction), so that two products per
+// instruction (fma.rn.f32x2) gained 1 % and were not kept.  (B=16 T=600 U'=81 V=1025: 130 us; 135 with
+// rint, 158 with expf of the difference and the remainder of a 2Sum, 115 with the bare ex2 of it.)
 constexpr float kFacShift = 46.0f;
 __device__ __forceinline__ float ex2_ftz(float x) {
   float y;
@@ -131,7 +133,8 @@ __global__ void __launch_bounds__(256) lognorm_factored_kernel(
   // off a word however far below its row's maximum it lies.  (f is not finite where it is masked.)
   auto ex = [](float x, float ref) {
     constexpr float kLog2e = 1.4426950408889634f, kLog2eLo = 1.9259629911e-8f;
-    const float n = rintf(x * kLog2e), f = fmaf(x, kLog2eLo, fmaf(x, kLog2e, -n)), k = n - ref;
+    constexpr float kRound = 12582912.0f;   // 1.5 2^23: adding it rounds to an integer
+    const float n = (x * kLog2e + kRound) - kRound, f = fmaf(x, kLog2eLo, fmaf(x, kLog2e, -n)), k = n - ref;
     return k < -200.0f ? 0.0f : ex2_ftz(f) * ex2_ftz(k);
   };
   auto put = [&](int s, const float (&ye)[8], const float (&yp)[8]) {
