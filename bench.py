@@ -683,9 +683,14 @@ def parity_block(w, r, device_case, state):
 # dram__bytes_read.sum + dram__bytes_write.sum per launch from one ncu capture of the named
 # kernel on this workload (1-pass captures at the bench size).  Keyed by (workload, kernel).
 NCU_TRAFFIC_BYTES = {
-    ("c3", "grads_umma"): 2460688896 + 2661452288,
-    ("c3", "lognorm_umma"): 2626279936 + 35040256,
-    ("c3", "expp_split"): 146920704 + 230604288,
+    ("c3", "grads_umma"): 2439271168 + 2632888832,
+    ("c3", "lognorm_umma"): 2625769216 + 32078080,
+    ("c3", "expp_split"): 133476352 + 146547968,
+    ("c3", "sweep_prep"): 41429504 + 2235136,
+    ("c3", "alpha_sweep"): 45159168 + 161024,
+    ("c3", "gamma_factors"): 69312000 + 6980096,
+    ("c3", "gamma_sweep"): 45132032 + 167168,
+    ("c3", "occupancy"): 87623680 + 24183552,
 }
 
 
