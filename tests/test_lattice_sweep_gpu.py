@@ -51,6 +51,59 @@ def test_edges(T, U):
     assert abi.rel_to_max(n(pg), ref["pgrads"]) < tol
 
 
+@pytest.mark.parametrize("S", [30, 31, 32, 33, 47, 48, 49, 63, 64, 65, 96])
+def test_around_the_middle_diagonal(S):
+    """The two halves of a sweep meet at a multiple of 16 diagonals: lattices of S diagonals, short and long
+    label axes (every number of positions per lane), utterances whose middle lies elsewhere beside them."""
+    for U in (1, 2, 9, 33, 40, 65, 129, 161, 193, 225):
+        T = S + 1 - U
+        if T < 1:
+            T, U = S // 3 + 1, S - S // 3   # (the axes swapped: more positions than frames)
+        B, V = 3, 36
+        g = torch.Generator(device="cuda").manual_seed(1000 * S + U)
+        E = torch.empty((B, T, V), device="cuda").normal_(generator=g)
+        P = torch.empty((B, U, V), device="cuda").normal_(generator=g)
+        labels = torch.randint(1, V, (B, U - 1), generator=g, device="cuda", dtype=torch.int32)
+        il = torch.tensor([T, max(1, T // 2), T], dtype=torch.int32, device="cuda")
+        ll = torch.tensor([U - 1, U - 1, (U - 1) // 2], dtype=torch.int32, device="cuda")
+        abi.set_option("lognorm_path", 1)
+        abi.set_option("grads_path", 1)
+        try:
+            fwd = abi.loss_forward(E, P, labels, il, ll)
+            eg, pg = abi.loss_backward(E, P, labels, il, ll, fwd)
+        finally:
+            abi.set_option("lognorm_path", 0)
+            abi.set_option("grads_path", 0)
+        n = lambda x: x.cpu().numpy()
+        ref = O.truth64(n(E), n(P), n(labels), n(il), n(ll))
+        tol = 4.0 * np.sqrt(T + U) * 2.0 ** -15 + 1e-5   # (as test_edges)
+        np.testing.assert_allclose(n(fwd["costs"]), ref["costs"], rtol=1e-6, atol=tol)
+        np.testing.assert_allclose(fwd["loss_sum"].item(), ref["costs"].sum(), rtol=1e-6, atol=3 * tol)
+        assert abi.rel_to_max(n(eg), ref["egrads"]) < tol, (T, U)
+        assert abi.rel_to_max(n(pg), ref["pgrads"]) < tol, (T, U)
+
+
+@pytest.mark.parametrize("U", [5, 40, 100, 150])
+def test_an_utterance_without_a_path(U):
+    """Every label of utterance 1 masked by -inf: its cost is +inf, and the others do not notice."""
+    B, T, V = 3, 50, 40
+    g = torch.Generator(device="cuda").manual_seed(U)
+    E = torch.empty((B, T, V), device="cuda").normal_(generator=g)
+    P = torch.empty((B, U, V), device="cuda").normal_(generator=g)
+    labels = torch.randint(1, V, (B, U - 1), generator=g, device="cuda", dtype=torch.int32)
+    il = torch.full((B,), T, dtype=torch.int32, device="cuda")
+    ll = torch.full((B,), U - 1, dtype=torch.int32, device="cuda")
+    whole = abi.loss_forward(E, P, labels, il, ll)
+    eg0, pg0 = abi.loss_backward(E, P, labels, il, ll, whole)
+    E[1, :, 1:] = float("-inf")
+    fwd = abi.loss_forward(E, P, labels, il, ll)
+    eg, pg = abi.loss_backward(E, P, labels, il, ll, fwd)
+    assert torch.isposinf(fwd["costs"][1])
+    for b in (0, 2):
+        assert torch.equal(fwd["costs"][b], whole["costs"][b])
+        assert torch.equal(eg[b], eg0[b]) and torch.equal(pg[b], pg0[b])
+
+
 def test_host_threads_with_different_shapes():
     """Stream and error message are per host thread, a kernel's shared-memory limit is not: a thread's
     launches may not depend on what another one set for a shorter utterance.  (200 positions: the

@@ -73,11 +73,11 @@ struct Carver {
 int ld_w(const Dims& d) { return (int)round_up64(d.maxU > 0 ? d.maxU : 1, 32); }
 
 struct LogNormWs {
-  unsigned* ticket;  // alpha kernel's completion counter
+  unsigned* ticket;  // alpha kernel's completion counters: of the batch, then of the utterances
   float* split;      // exp(P) hi/lo operand of the tensor-core path
   float* maxPScratch;
   LogNormWs(Carver& c, const Dims& d) {
-    ticket = c.take<unsigned>(16);
+    ticket = c.take<unsigned>(16 + (size_t)d.B);
     maxPScratch = c.take<float>((size_t)d.B * d.maxU);
     split = c.take<float>(lognorm_umma_workspace_floats(d));
   }
@@ -421,15 +421,13 @@ int loss_forward_any(const void* E, const void* P, const int* labels, const int*
     // (nodes the tensor-core log-normaliser could not represent are recomputed by the re-layout)
     const bool gathered = log_norms_impl(E, P, LN, st.rowRef, st.maxP, inLens, labLens, d, ws,
                                          /*fixup=*/false, labels, fw.EL, st.ebl);
-    if (lossSum) {
-      TB200_CUDA_CHECK(cudaMemsetAsync(ws.ticket, 0, sizeof(unsigned), g_stream));
-      if (B == 0) TB200_CUDA_CHECK(cudaMemsetAsync(lossSum, 0, sizeof(float), g_stream));
-    }
+    TB200_CUDA_CHECK(cudaMemsetAsync(ws.ticket, 0, sizeof(unsigned) * (16 + (size_t)B), g_stream));
+    if (lossSum && B == 0) TB200_CUDA_CHECK(cudaMemsetAsync(lossSum, 0, sizeof(float), g_stream));
     unsigned* ticket = lossSum ? ws.ticket : nullptr;
     if (sweep) {
       launch_sweep_forward(E, P, LN, gathered ? fw.EL : nullptr, st.ebl, st.arcs,
-                           st.alphas, st.deltas, costs, lossSum, ticket, labels, inLens, labLens,
-                           sweep_geom(d), d, g_stream);
+                           st.alphas, st.deltas, costs, lossSum, ticket, ws.ticket + 16, labels, inLens,
+                           labLens, sweep_geom(d), d, /*score=*/false, g_stream);
       return;
     }
     const SkewGeom g = skew_geom(d);

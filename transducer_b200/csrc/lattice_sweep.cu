@@ -3,32 +3,44 @@
 // the whole GPU.
 //
 //   sweep_prep       arc log-probabilities of every node (log2 units), skewed
-//   alpha_sweep      alpha recursion                                          (forward call)
-//   gamma_factors    2^(alpha + arc - alpha') of every arc                    (backward call)
-//   gamma_sweep      occupancy recursion: two products and a sum per node
+//   alpha_sweep      alpha and beta recursions up to the middle               (forward call)
+//   gamma_factors    2^(alpha + arc - alpha'), 2^(arc + beta' - beta)         (backward call)
+//   gamma_sweep      occupancy recursions from the middle: two products and a sum per node
 //   occupancy        the operands of the gradient kernels
 //
 //   alpha   transducer/transducer_cpu.cpp:30-79   (transducer_cuda.cu:32-97)
 //   reverse transducer/transducer_cpu.cpp:81-143  (transducer_cuda.cu:99-176)
 //
-// Axes of up to 128 positions run on rebased base-2 logarithms (alpha_sweep_kernel); longer ones
-// (NPL >= 5, "natural" below) on natural logarithms at full magnitude, in the operation order of the
-// block-wide kernels of lattice.cu (costs bit-identical to theirs: 18 shapes, T = 77..5000,
-// U' = 129..256).
-//
 // Diagonal d = t + u of an utterance is one row of ld = 32 NPL numbers; lane l of a sweep owns the
 // NPL adjacent positions u = NPL l + r.  All nodes of a diagonal are independent; the one value
 // per lane that crosses from the neighbouring lane arrives by a warp shuffle.  A sweep is a chain
-// of T + U - 1 dependent diagonals whatever the batch, so what counts is how few instructions a
-// diagonal takes: operands are brought to shared memory by cp.async, each lane copying just the
+// of dependent diagonals whatever the batch, so what counts is how many they are and how few
+// instructions each takes.
+//
+// FROM BOTH ENDS.  Every path crosses each of the S = T + U - 1 diagonals once, so with alpha (all paths
+// to a node) up to the middle diagonal M and beta (all paths from a node) down to it, the total is
+// the sum over M of alpha beta, and the occupancy of a node of M is its share of that sum.  From there
+// the occupancies spread to both ends: towards the start by the share of each node's inflow that came
+// over an arc (from the alphas, as the reference does all the way), towards the end by the share of its
+// outflow that leaves over an arc (from the betas).  The shares of a node add up to one to within a
+// rounding either way, so neither half drifts.  The two halves are two warps that know nothing of each
+// other, and both chains are half as long as from one end.
+//
+// Operands are brought to shared memory by cp.async, each lane copying just the
 // 8 NPL bytes a row that it reads itself (no barrier, no other warp), several blocks of 16
 // diagonals ahead, and the loop holds nothing but the recursion and its store.
-// Measured (T = 2000, U' = 101, device time, B = 8 / 32): alpha 132 us (147 with bulk copies issued and
-// waited for by the sweeping warp); reverse sweep 12 / 27 us for the factors + 60 us for the recursion
-// (152 us when helper warps of the same CTA prepared the factors and carried away the results).
-// B = 64, T = 750..1500, U' = 151: alpha 195 us, factors 65 + recursion 76 us, operands 105 us, against
-// 384, 512 and (lattices re-laid out twice) 168 us of the block-wide kernels, which take a barrier
-// per diagonal.  B = 8, T = 4000, U' = 251: alpha 855 us, block-wide 954.
+//
+// Measured (T = 2000, U' = 101, B = 8 and 32 alike): alpha sweep 132 -> 76 us, reverse sweep 60 -> 37 us
+// against one warp from one end.
+//
+// Axes of up to 128 positions run like that, on rebased base-2 logarithms; longer ones (NPL >= 5) too where
+// only the costs are wanted (scoring, B = 64, T = 500..1000, U' = 101..201: 242 -> 71 us).  With gradients
+// to follow they keep to the reference's form ("natural" below): one warp from one end, natural logarithms
+// at full magnitude, in the operation order of the block-wide kernels of lattice.cu (costs bit-identical to
+// theirs: 18 shapes, T = 77..5000, U' = 129..256).  At a magnitude of 1e4 the rounding of an alpha is
+// 1e-3, and the gradients carry it: any other order of these operations moves them by as much (rel
+// 1.3e-3 between this form and the sweeps from both ends, which are the ones closer to float64), more than
+// this path's results are to move.
 #include <algorithm>
 
 #include "kernels.h"
@@ -43,12 +55,22 @@ using namespace sm100;
 constexpr int kDiag = 16;   // diagonals per block
 // blocks in shared memory (three of the wide ones leave room for two CTAs per SM)
 __host__ __device__ constexpr int ring_blocks(int npl) { return npl <= 4 ? 4 : 3; }
-__host__ __device__ constexpr bool natural(int npl) { return npl > 4; }
+__host__ __device__ constexpr bool natural(int npl) { return npl > 4; }   // (where gradients are to follow)
+// The diagonal at which the halves of an utterance of S >= 1 diagonals meet: a whole number of blocks, so
+// that the blocks of the first half are full.
+__device__ __forceinline__ int middle(int S) { return (S / 2) & ~(kDiag - 1); }
 constexpr float kLn2F = 0.6931471805599453f;
 constexpr float kLog2e = 1.4426950408889634f;
 // "No such arc": a large negative finite number, the identity of the alpha recursion without -inf
 // arithmetic, so that the sweeps need no validity logic.
 constexpr unsigned kNoArcBits = 0xF0F0F0F0u;
+
+// A log-probability as an arc term: a word masked by -inf makes no arc (NaN stays NaN).
+__device__ __forceinline__ float arc_term(float x) {
+  float y;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(x), "f"(__uint_as_float(kNoArcBits)));
+  return y;
+}
 
 __device__ __forceinline__ float lg2_approx(float x) {
   float y;
@@ -197,30 +219,33 @@ __device__ __forceinline__ void finish_cost(float* costs, int b, float cost, int
 // subtracts it at the same point of the same sum.  The loss and the gradients then sit ~1e-4 from
 // the float64 result.
 //
+// The betas are rebased likewise, in blocks of 16 from the end; beta of diagonal d is stored in row d + 1,
+// behind the alphas (row M holds alpha, row M + 1 beta of the middle diagonal).  deltas of an utterance:
+// [0] the alphas' offset at M, [k] of the alphas' block k, [nBlk - 1 - k] of the betas' block k,
+// [nBlk - 1] the betas' offset at M.
+//
 // The pace is set by the special-function unit: NPL ex2 and NPL lg2 per diagonal, 8 issue cycles
 // each, in a chain.  (Cutting the label axis over two or four warps that run a block apart was
 // measured and is slower: every node then waits for a shuffle.)
+__device__ __forceinline__ float lse2_log2(float a, float b) {
+  return fmaxf(a, b) + lg2_approx(1.0f + ex2_approx(-fabsf(a - b)));
+}
+
+// floor of the largest of a lane's numbers over the warp, at least -1e9: the next delta
+__device__ __forceinline__ float next_delta(float m) {
+  return (float)__reduce_max_sync(0xffffffffu, __float2int_rd(fmaxf(m, -1.0e9f)));
+}
+
+// alpha of the diagonals 0..M; returns the offset of M
 template <int NPL>
-__global__ void __launch_bounds__(32) alpha_sweep_kernel(
-    const float2* __restrict__ arcs, float* __restrict__ costs, float* __restrict__ alphas,
-    float* __restrict__ deltas, i64 stride, int nDiag, const int* __restrict__ inLens,
-    const int* __restrict__ labLens, int B, int maxT, int maxU, float* lossSum, unsigned* ticket) {
-  constexpr int ld = 32 * NPL;
-  extern __shared__ __align__(128) uint8_t smemA[];
-  const int b = blockIdx.x, lane = threadIdx.x;
-  const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
-  if (T <= 0 || U <= 0) {
-    if (lane == 0) finish_cost(costs, b, pos_inf(), B, lossSum, ticket);
-    return;
-  }
-  const int S = T + U - 1, nBlocks = (S + kDiag - 1) / kDiag, u0 = NPL * lane;
-  constexpr int kRing = ring_blocks(NPL);
-  PairRing<NPL> ring(smemA, arcs + (i64)b * stride, lane, U, kNoArcBits, kNoArcBits);
-  auto issue = [&](int k) { ring.issue(k % kRing, (i64)k * kDiag, k < nBlocks ? min(kDiag, S - k * kDiag) : 0); };
+__device__ __forceinline__ float alpha_half(uint8_t* smem, const float2* arcs, float* al, float* dl,
+                                            int lane, int U, int M) {
+  constexpr int ld = 32 * NPL, kRing = ring_blocks(NPL);
+  const int nBlocks = M / kDiag;
+  PairRing<NPL> ring(smem, arcs, lane, U, kNoArcBits, kNoArcBits);
+  auto issue = [&](int k) { ring.issue(k % kRing, (i64)k * kDiag, k < nBlocks ? kDiag : 0); };
 #pragma unroll
   for (int k = 0; k < kRing - 1; ++k) issue(k);
-  float* al = alphas + (i64)b * stride;
-  float* dl = deltas + (i64)b * ((nDiag + kDiag - 1) / kDiag);
   const float kNone = __uint_as_float(kNoArcBits);
   float stayIn[NPL], stepOut[NPL];
 #pragma unroll
@@ -229,7 +254,7 @@ __global__ void __launch_bounds__(32) alpha_sweep_kernel(
   float up = kNone;        // stepOut of the lane below's last position, one diagonal back
   float offset = 0.0f;     // sum of the deltas so far: an integer, exact in fp32
   float nextDelta = 0.0f;  // by how much the state is lowered at the start of the next block
-  for (int k = 0; k < nBlocks; ++k) {
+  for (int k = 0; k <= nBlocks; ++k) {
     issue(k + kRing - 1);
     if (k > 0) {
       // rebase (entries of nodes outside the lattice are ~ -6e29 and stay there)
@@ -242,6 +267,14 @@ __global__ void __launch_bounds__(32) alpha_sweep_kernel(
       offset += nextDelta;
       if (lane == 0) dl[k] = nextDelta;
     }
+    float* out = al + (i64)k * kDiag * ld;
+    if (k == nBlocks) {   // the middle diagonal: nothing leaves it here
+      float a[NPL];
+#pragma unroll
+      for (int r = 0; r < NPL; ++r) a[r] = lse2_log2(r ? stepOut[(r + NPL - 1) % NPL] : lane ? up : kNone, stayIn[r]);
+      if (ring.act) store_row<NPL>(out, lane, a);
+      break;
+    }
     // The delta applied at the start of the NEXT block is the floor of the largest entry of
     // the state now, at the start of this one: the warp-wide maximum then has a whole block to
     // arrive, off the dependent chain.  (By then the state has sunk by another 16 arcs.)
@@ -249,12 +282,12 @@ __global__ void __launch_bounds__(32) alpha_sweep_kernel(
       float m = kNone;
 #pragma unroll
       for (int r = 0; r < NPL; ++r) m = fmaxf(m, fmaxf(stayIn[r], stepOut[r]));
-      nextDelta = (float)__reduce_max_sync(0xffffffffu, __float2int_rd(fmaxf(m, -1.0e9f)));
+      nextDelta = next_delta(m);
     }
     ring.wait();
-    const int slot = k % kRing, nd = min(kDiag, S - k * kDiag);
-    float* out = al + (i64)k * kDiag * ld;
-    auto diag = [&](int i) {
+    const int slot = k % kRing;
+#pragma unroll
+    for (int i = 0; i < kDiag; ++i) {
       float fx[NPL], fy[NPL], left[NPL], m[NPL], e[NPL], a[NPL];
       ring.read(slot, i, fx, fy);
       // The last position first: its result feeds the shuffle of the next diagonal; position 0
@@ -275,20 +308,137 @@ __global__ void __launch_bounds__(32) alpha_sweep_kernel(
         if (r == NPL - 1) up = __shfl_up_sync(0xffffffffu, stepOut[NPL - 1], 1);
       }
       if (ring.act) store_row<NPL>(out + i * ld, lane, a);
-    };
-    if (nd == kDiag) {
-#pragma unroll
-      for (int i = 0; i < kDiag; ++i) diag(i);
-    } else {
-#pragma unroll 1
-      for (int i = 0; i < nd; ++i) diag(i);
     }
   }
   ring.drain();
-  // the last diagonal holds only the terminal node (T-1, U-1); its blank arc ends the path
+  return offset;
+}
+
+// beta of the diagonals S-1 down to M, that of d in row d + 1; returns the offset of M
+template <int NPL>
+__device__ __forceinline__ float beta_half(uint8_t* smem, const float2* arcs, float* al, float* dlEnd,
+                                           int lane, int U, int S, int M) {
+  constexpr int ld = 32 * NPL, kRing = ring_blocks(NPL);
+  const int nBlocks = (S - M + kDiag - 1) / kDiag, u0 = NPL * lane;
+  PairRing<NPL> ring(smem, arcs, lane, U, kNoArcBits, kNoArcBits);
+  // block k holds the rows [max(S - 16(k+1), M), S - 16k)
+  auto issue = [&](int k) {
+    const int lo = max(S - kDiag * (k + 1), M);
+    ring.issue(k % kRing, lo, k < nBlocks ? S - kDiag * k - lo : 0);
+  };
 #pragma unroll
-  for (int r = 0; r < NPL; ++r)
-    if (u0 + r == U - 1) finish_cost(costs, b, -(stayIn[r] + offset) * kLn2F, B, lossSum, ticket);
+  for (int k = 0; k < kRing - 1; ++k) issue(k);
+  const float kNone = __uint_as_float(kNoArcBits);
+  float bt[NPL];   // of the diagonal above; at first of the node beyond the terminating blank
+#pragma unroll
+  for (int r = 0; r < NPL; ++r) bt[r] = u0 + r == U - 1 ? 0.0f : kNone;
+  // (lane 31 gets its own back: harmless, the label arc of its last position never exists)
+  float right = __shfl_down_sync(0xffffffffu, bt[0], 1);
+  float offset = 0.0f, nextDelta = 0.0f;
+  for (int k = 0; k < nBlocks; ++k) {
+    issue(k + kRing - 1);
+    if (k > 0) {
+#pragma unroll
+      for (int r = 0; r < NPL; ++r) bt[r] -= nextDelta;
+      right -= nextDelta;
+      offset += nextDelta;
+      if (lane == 0) dlEnd[-k] = nextDelta;
+    }
+    {
+      float m = kNone;
+#pragma unroll
+      for (int r = 0; r < NPL; ++r) m = fmaxf(m, bt[r]);
+      nextDelta = next_delta(m);
+    }
+    ring.wait();
+    const int slot = k % kRing, lo = max(S - kDiag * (k + 1), M), nd = S - kDiag * k - lo;
+    float* out = al + (i64)(lo + 1) * ld;
+    auto diag = [&](int i) {
+      float x[NPL], y[NPL], m[NPL], e[NPL];
+      ring.read(slot, i, x, y);
+      // position 0 first, whose result leaves by the shuffle; the last one waits for it
+#pragma unroll
+      for (int r = 0; r < NPL; ++r) {
+        const float p = bt[r] + x[r], q = (r < NPL - 1 ? bt[(r + 1) % NPL] : right) + y[r];
+        m[r] = fmaxf(p, q);
+        e[r] = ex2_approx(-fabsf(p - q));
+      }
+#pragma unroll
+      for (int r = 0; r < NPL; ++r) {
+        bt[r] = m[r] + lg2_approx(1.0f + e[r]);
+        if (r == 0) right = __shfl_down_sync(0xffffffffu, bt[0], 1);
+      }
+      if (ring.act) store_row<NPL>(out + i * ld, lane, bt);
+    };
+    if (nd == kDiag) {
+#pragma unroll
+      for (int i = kDiag - 1; i >= 0; --i) diag(i);
+    } else {
+#pragma unroll 1
+      for (int i = nd - 1; i >= 0; --i) diag(i);
+    }
+  }
+  ring.drain();
+  return offset;
+}
+
+// Of a lane's nodes of the middle diagonal: 2^(alpha + beta - m), m the largest exponent of the warp, into
+// w; returns m, and the warp's sum of w in `total`.  No path at all (m ~ -6e29): total = 0, w = 0.
+template <int NPL>
+__device__ __forceinline__ float meet(const float* al, int lane, int U, int M, float (&w)[NPL], float& total) {
+  constexpr int ld = 32 * NPL;
+  float m = -INFINITY;
+#pragma unroll
+  for (int r = 0; r < NPL; ++r) {
+    const int u = NPL * lane + r, at = row_slot(min(u, U - 1), NPL);
+    const float a = __ldcg(al + (i64)M * ld + at), bt = __ldcg(al + (i64)(M + 1) * ld + at);
+    w[r] = u < U ? a + bt : -INFINITY;
+    m = fmaxf(m, w[r]);
+  }
+  m = warp_max(m);
+  float s = 0.0f;
+#pragma unroll
+  for (int r = 0; r < NPL; ++r) {
+    const bool nan = w[r] != w[r];
+    w[r] = m > -1.0e28f || nan ? exp2f(w[r] - m) : 0.0f;
+    s += w[r];
+  }
+  total = warp_sum(s);
+  return m;
+}
+
+// One warp per half of an utterance (blockIdx.y); the half that finishes last adds up the cost.
+template <int NPL>
+__global__ void __launch_bounds__(32) alpha_sweep_kernel(
+    const float2* __restrict__ arcs, float* __restrict__ costs, float* alphas, float* deltas, i64 stride,
+    int nBlk, const int* __restrict__ inLens, const int* __restrict__ labLens, int B, int maxT, int maxU,
+    float* lossSum, unsigned* ticket, unsigned* halves) {
+  extern __shared__ __align__(128) uint8_t smemA[];
+  const int b = blockIdx.x, lane = threadIdx.x;
+  const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
+  if (T <= 0 || U <= 0) {
+    if (lane == 0 && blockIdx.y == 0) finish_cost(costs, b, pos_inf(), B, lossSum, ticket);
+    return;
+  }
+  const int S = T + U - 1, M = middle(S);
+  float* al = alphas + (i64)b * stride;
+  float* dl = deltas + (i64)b * nBlk;
+  const float offset = blockIdx.y == 0
+      ? alpha_half<NPL>(smemA, arcs + (i64)b * stride, al, dl, lane, U, M)
+      : beta_half<NPL>(smemA, arcs + (i64)b * stride, al, dl + nBlk - 1, lane, U, S, M);
+  if (lane == 0) dl[blockIdx.y == 0 ? 0 : nBlk - 1] = offset;
+  __threadfence();
+  __syncwarp();
+  unsigned before = 0;
+  if (lane == 0) before = atomicAdd(&halves[b], 1u);
+  if (__shfl_sync(0xffffffffu, before, 0) == 0u) return;
+  __threadfence();
+  float w[NPL], total;
+  const float m = meet<NPL>(al, lane, U, M, w, total);
+  if (lane == 0) {
+    const double log2p = (double)__ldcg(dl) + (double)__ldcg(dl + nBlk - 1) + (double)(m + log2f(total));
+    finish_cost(costs, b, total == 0.0f ? pos_inf() : (float)(-log2p * 0.69314718055994530942), B, lossSum, ticket);
+  }
 }
 
 // What the natural sweeps know of an utterance's positions besides the pair rows.
@@ -396,25 +546,32 @@ __global__ void __launch_bounds__(32) alpha_natural_kernel(
 // ---------------------------------------------------------------------------
 // reverse occupancy sweep
 // ---------------------------------------------------------------------------
-// With g(t,u) the occupancy of node (t,u) (the reference's dalphas, sign dropped):
+// With g(t,u) the occupancy of node (t,u) (the reference's dalphas, sign dropped), alphas, betas and arcs in
+// log2 units: below the middle diagonal
 //   stay(t,u) = g(t+1,u) * FB(t,u),  FB = 2^((alpha(t,u) + blank arc) - alpha(t+1,u))
 //   step(t,u) = g(t,u+1) * FL(t,u),  FL = 2^((alpha(t,u) + label arc) - alpha(t,u+1))
-//   (alphas and arcs in log2 units; the parenthesised sums are rounded exactly as in the alpha
-//   kernel, so FB and FL of the arcs entering a node add up to 1 to within the error of ex2/lg2.
-//   The stored alphas are relative to a per-block offset, see alpha_sweep_kernel: where the
-//   successors' diagonal opens a new block, that block's delta is subtracted from the sum first,
-//   exactly as the alpha kernel lowered its carried state.)
-//   g(t,u) = stay + step,            g(T-1,U-1) = 1 (the terminating blank, booked as stay)
+//   g(t,u) = stay + step
+// and from it on
+//   stay(t,u) = g(t,u) * FB(t,u),    FB = 2^((blank arc + beta(t+1,u)) - beta(t,u))
+//   step(t,u) = g(t,u) * FL(t,u),    FL = 2^((label arc + beta(t,u+1)) - beta(t,u))
+//   g(t,u) = stay(t-1,u) + step(t,u-1),   the terminating blank being the stay of (T-1,U-1)
+// The parenthesised sums are rounded exactly as in the sweeps, so FB and FL of the arcs entering
+// (leaving) a node add up to 1 to within the error of ex2/lg2.  The stored numbers are relative to
+// a per-block offset: where the neighbouring diagonal opens a block or closes one, that block's delta
+// is subtracted where the sweep lowered its state.
+//
+// (natural: the first form all the way, g(T-1,U-1) = 1 fed by a node beyond the terminating blank.)
 //
 // gamma_factors_kernel: the pairs (FB, FL) of every node of the diagonals below S, zero where there
 // is no arc (natural: from the pair rows of alpha_natural_kernel, by the accurate expf).  One warp
-// per 4 diagonals.  Bound by memory: a pair and an alpha (12 bytes) read, 8 written per node.
+// per 4 diagonals.  Bound by memory: a pair and an alpha (12 bytes) read, 8
+// written per node.
 constexpr int kFactorRows = 4, kFactorWarps = 8;
 template <int NPL>
 __global__ void __launch_bounds__(32 * kFactorWarps) gamma_factors_kernel(
     const float2* __restrict__ arcs, const float* __restrict__ alphas,
     const float* __restrict__ deltas, const NaturalTerms n, float2* __restrict__ F,
-    unsigned* __restrict__ occTicket, i64 stride, int nDiag, const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT,
+    unsigned* __restrict__ occTicket, i64 stride, int nBlk, const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT,
     int maxU) {
   constexpr int ld = 32 * NPL, kPieces = NPL / 2;
   const int b = blockIdx.y, lane = threadIdx.x & 31;
@@ -422,8 +579,10 @@ __global__ void __launch_bounds__(32 * kFactorWarps) gamma_factors_kernel(
   const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU), S = T + U - 1;
   const int d0 = (blockIdx.x * kFactorWarps + (threadIdx.x >> 5)) * kFactorRows, u0 = NPL * lane;
   if (T <= 0 || U <= 0 || d0 >= S || u0 >= U) return;
-  const float* al = alphas + (i64)b * stride;
-  const float* dl = deltas + (i64)b * ((nDiag + kDiag - 1) / kDiag);
+  // (the middle is a multiple of kFactorRows: the warp's rows lie on one side of it)
+  const bool fwd = natural(NPL) || d0 < middle(S);
+  const float* al = alphas + (i64)b * stride + (fwd ? 0 : ld);   // (beta of d is in row d + 1)
+  const float* dl = deltas + (i64)b * nBlk;
   const int next = row_slot(min(u0 + NPL, ld - 1), NPL);   // (the last position has no label arc)
   float a[kFactorRows + 1][NPL], aN[kFactorRows + 1], x[kFactorRows][NPL], y[kFactorRows][NPL];
 #pragma unroll
@@ -462,24 +621,25 @@ __global__ void __launch_bounds__(32 * kFactorWarps) gamma_factors_kernel(
   for (int i = 0; i < kFactorRows; ++i) {
     const int d = d0 + i;
     if (d >= S) break;
-    // (rebased) the successors' diagonal opens a block: the carried sums were lowered by its delta
-    const float dlt = (!natural(NPL) && (d + 1) % kDiag == 0 && d + 1 < S) ? dl[(d + 1) / kDiag] : 0.0f;
+    float dlt = 0.0f;   // of the block that diagonal d + 1 opens, or (betas) that d opens
+    if (!natural(NPL) && fwd && (d + 1) % kDiag == 0) dlt = dl[(d + 1) / kDiag];
+    if (!natural(NPL) && !fwd && (S - 1 - d) % kDiag == 0 && d < S - 1) dlt = dl[nBlk - 1 - (S - 1 - d) / kDiag];
 #pragma unroll
     for (int r = 0; r < NPL; ++r) {
       const int u = u0 + r, t = d - u;
       const bool valid = u < U && t >= 0 && t < T;
-      const float art = r < NPL - 1 ? a[i + 1][(r + 1) % NPL] : aN[i + 1];
+      const float above = a[i + 1][r], aboveN = r < NPL - 1 ? a[i + 1][(r + 1) % NPL] : aN[i + 1];
       float fb, fl;
       if constexpr (natural(NPL)) {
         const float eb = n.ebl[(i64)b * maxT + min(max(t, 0), T - 1)], lnv = x[i][r], el = y[i][r];
-        fb = expf((((a[i][r] + eb) + pbl[r]) - lnv) - a[i + 1][r]);
-        fl = expf((((a[i][r] + el) + plab[r]) - lnv) - art);
+        fb = expf((((a[i][r] + eb) + pbl[r]) - lnv) - above);
+        fl = expf((((a[i][r] + el) + plab[r]) - lnv) - aboveN);
       } else {
-        fb = ex2_approx(((a[i][r] + x[i][r]) - dlt) - a[i + 1][r]);
-        fl = ex2_approx(((a[i][r] + y[i][r]) - dlt) - art);
+        fb = ex2_approx(fwd ? ((a[i][r] + x[i][r]) - dlt) - above : ((above - dlt) + x[i][r]) - a[i][r]);
+        fl = ex2_approx(fwd ? ((a[i][r] + y[i][r]) - dlt) - aboveN : ((aboveN - dlt) + y[i][r]) - a[i][r]);
       }
       x[i][r] = (valid && t < T - 1) ? fb : 0.0f;
-      if (t == T - 1 && u == U - 1) x[i][r] = 1.0f;   // terminating blank, fed by g(T,U-1) := 1
+      if (t == T - 1 && u == U - 1) x[i][r] = 1.0f;   // the terminating blank
       y[i][r] = (valid && u < U - 1) ? fl : 0.0f;
     }
     float2* out = F + (i64)b * stride + (i64)d * ld;
@@ -490,10 +650,96 @@ __global__ void __launch_bounds__(32 * kFactorWarps) gamma_factors_kernel(
   }
 }
 
-// The recursion on the prepared factors: g of the diagonals S (the node beyond the terminating
-// blank) down to 0.
+// The recursions on the prepared factors, one warp per half (blockIdx.y): g of the diagonals M down to
+// 0, and of M + 1 up to S - 1.
 template <int NPL>
 __global__ void __launch_bounds__(32) gamma_sweep_kernel(
+    const float2* __restrict__ F, const float* __restrict__ alphas, float* __restrict__ g, i64 stride,
+    const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT, int maxU) {
+  constexpr int ld = 32 * NPL, kRing = ring_blocks(NPL);
+  extern __shared__ __align__(128) uint8_t smemG[];
+  const int b = blockIdx.x, lane = threadIdx.x;
+  const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
+  if (T <= 0 || U <= 0) return;
+  const int S = T + U - 1, M = middle(S);
+  PairRing<NPL> ring(smemG, F + (i64)b * stride, lane, U, 0u, 0u);
+  float* out0 = g + (i64)b * stride;
+  const bool down = blockIdx.y == 0;
+  // downwards block k holds the rows [M - 16(k+1), M - 16k); upwards the rows from M + 16k on, the last
+  // of which is S - 2
+  const int nBlocks = down ? M / kDiag : (S - 1 - M + kDiag - 1) / kDiag;
+  auto issue = [&](int k) {
+    if (down) ring.issue(k % kRing, M - kDiag * (k + 1), k < nBlocks ? kDiag : 0);
+    else ring.issue(k % kRing, M + kDiag * k, k < nBlocks ? min(kDiag, S - 1 - M - kDiag * k) : 0);
+  };
+#pragma unroll
+  for (int k = 0; k < kRing - 1; ++k) issue(k);
+  float s[NPL], total;
+  meet<NPL>(alphas + (i64)b * stride, lane, U, M, s, total);
+  const float share = total != 0.0f ? 1.0f / total : 0.0f;
+#pragma unroll
+  for (int r = 0; r < NPL; ++r) s[r] *= share;
+  if (down) {
+    if (ring.act) store_row<NPL>(out0 + (i64)M * ld, lane, s);
+    // (lane 31 gets its own s[0] back: harmless, the label arc of its last position never exists)
+    float right = __shfl_down_sync(0xffffffffu, s[0], 1);
+    for (int k = 0; k < nBlocks; ++k) {
+      issue(k + kRing - 1);
+      ring.wait();
+      const int slot = k % kRing;
+      float* out = out0 + (i64)(M - kDiag * (k + 1)) * ld;
+#pragma unroll
+      for (int i = kDiag - 1; i >= 0; --i) {
+        float x[NPL], y[NPL], n[NPL];
+        ring.read(slot, i, x, y);
+        // position 0 first: its result is shuffled for the next diagonal; the last position, which
+        // waits for the shuffle, at the end
+        const float in = right;
+#pragma unroll
+        for (int r = 0; r < NPL; ++r) {
+          const float nb = r < NPL - 1 ? s[(r + 1) % NPL] : in;
+          n[r] = __fadd_rn(__fmul_rn(s[r], x[r]), __fmul_rn(nb, y[r]));
+          if (r == 0) right = __shfl_down_sync(0xffffffffu, n[0], 1);
+        }
+#pragma unroll
+        for (int r = 0; r < NPL; ++r) s[r] = n[r];
+        if (ring.act) store_row<NPL>(out + i * ld, lane, s);
+      }
+    }
+  } else {
+    for (int k = 0; k < nBlocks; ++k) {
+      issue(k + kRing - 1);
+      ring.wait();
+      const int slot = k % kRing, nd = min(kDiag, S - 1 - M - kDiag * k);
+      float* out = out0 + (i64)(M + kDiag * k + 1) * ld;
+      auto diag = [&](int i) {
+        float x[NPL], y[NPL];
+        ring.read(slot, i, x, y);
+        // the last position's step leaves by the shuffle
+#pragma unroll
+        for (int r = 0; r < NPL; ++r) y[r] = __fmul_rn(s[r], y[r]);
+        const float left = __shfl_up_sync(0xffffffffu, y[NPL - 1], 1);
+#pragma unroll
+        for (int r = NPL - 1; r >= 0; --r)
+          s[r] = __fadd_rn(__fmul_rn(s[r], x[r]), r ? y[(r + NPL - 1) % NPL] : lane ? left : 0.0f);
+        if (ring.act) store_row<NPL>(out + i * ld, lane, s);
+      };
+      if (nd == kDiag) {
+#pragma unroll
+        for (int i = 0; i < kDiag; ++i) diag(i);
+      } else {
+#pragma unroll 1
+        for (int i = 0; i < nd; ++i) diag(i);
+      }
+    }
+  }
+  ring.drain();
+}
+
+// natural: one warp per utterance, g of the diagonals S (the node beyond the terminating
+// blank) down to 0.
+template <int NPL>
+__global__ void __launch_bounds__(32) gamma_sweep_natural_kernel(
     const float2* __restrict__ F, float* __restrict__ g, i64 stride, const int* __restrict__ inLens,
     const int* __restrict__ labLens, int maxT, int maxU) {
   constexpr int ld = 32 * NPL;
@@ -564,6 +810,7 @@ struct PrepParams {
   const int* inLens;
   const int* labLens;
   int maxT, maxU, V, blank, npl, ld, extra;
+  bool nat;                  // for the natural sweeps
   i64 stride;
 };
 
@@ -617,7 +864,7 @@ __global__ void __launch_bounds__(256) sweep_prep_kernel(const PrepParams p) {
     if (threadIdx.x < 32) {
       const int tc = min(t0 + lane, T - 1);
       tEb[lane] = elr ? p.ebl[(i64)b * p.maxT + tc] : to_f32(e[(i64)tc * p.V + p.blank]);
-      if (!elr && natural(p.npl) && u0 == 0) p.ebl[(i64)b * p.maxT + tc] = tEb[lane];
+      if (!elr && p.nat && u0 == 0) p.ebl[(i64)b * p.maxT + tc] = tEb[lane];
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -653,13 +900,12 @@ __global__ void __launch_bounds__(256) sweep_prep_kernel(const PrepParams p) {
   for (int k = 0; k < 4; ++k) {
     const int tt = (w + 8 * k - lane) & 31, t = t0 + tt, d = t + u;
     if (d < 0 || d >= S || u >= Uw) continue;
-    const bool nat = natural(p.npl);
-    float2 f = nat ? make_float2(pos_inf(), 0.0f)
-                   : make_float2(__uint_as_float(kNoArcBits), __uint_as_float(kNoArcBits));
+    float2 f = p.nat ? make_float2(pos_inf(), 0.0f)
+                     : make_float2(__uint_as_float(kNoArcBits), __uint_as_float(kNoArcBits));
     if (t >= 0 && t < T && u < U) {
       const float lnv = tLn[tt][lane];
-      f.x = nat ? lnv : ((tEb[tt] + pbl) - lnv) * kLog2e;
-      if (u < U - 1) f.y = nat ? tEl[tt][lane] : ((tEl[tt][lane] + plab) - lnv) * kLog2e;
+      f.x = p.nat ? lnv : arc_term(((tEb[tt] + pbl) - lnv) * kLog2e);
+      if (u < U - 1) f.y = p.nat ? tEl[tt][lane] : arc_term(((tEl[tt][lane] + plab) - lnv) * kLog2e);
     }
     arcs[(i64)d * p.ld] = f;
   }
@@ -682,7 +928,7 @@ struct OccParams {
 
 // One CTA per 32 frames of one utterance, the 32x32 lattice tiles of the label axis side by side,
 // kOccWarps warps each.  With delta_b the upstream gradient:
-//   stay(t,u) = g(t+1,u) FB(t,u), step(t,u) = g(t,u+1) FL(t,u)
+//   stay and step as above (g of the successors below the middle diagonal, of the node from it on)
 //   W [B,maxT,ldW] = delta_b * (stay + step) * exp(ref(t) + maxP(u) - LN(t,u)), rounded to TF32
 //                   (round-to-nearest; the tensor core would otherwise truncate), zero outside
 //                   the valid lattice.  (The exponent is clamped at 80: it only gets there where
@@ -737,6 +983,7 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 640 ? 2 : 1) occupancy_ker
     // Step i takes diagonal i of the tile in the lanes up to i and diagonal i + 32 in the others:
     // every lane has a node and a warp touches two rows.  Four steps at a time with all their
     // loads issued before the first use (unconditional, clamped into the lattice).
+    const int M = natural(p.npl) ? T + U : middle(T + U - 1);
     const int slot1 = row_slot(uc, p.npl), slot2 = row_slot(min(u + 1, U - 1), p.npl);
 #pragma unroll
     for (int q = 0; q < kOccRows; q += 4) {
@@ -744,10 +991,11 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 640 ? 2 : 1) occupancy_ker
       float g1[4], g2[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const i64 row = (i64)(min(t0 + ((w + kOccWarps * (q + j) - lane) & 31), T - 1) + uc) * ld;
+        const int d = min(t0 + ((w + kOccWarps * (q + j) - lane) & 31), T - 1) + uc;
+        const i64 row = (i64)d * ld, rowG = d < M ? row + ld : row;
         f[j] = F[row];
-        g1[j] = g[row + ld + slot1];
-        g2[j] = g[row + ld + slot2];
+        g1[j] = g[rowG + slot1];
+        g2[j] = g[rowG + (d < M ? slot2 : slot1)];
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -870,7 +1118,7 @@ SweepGeom sweep_geom(Dims d) {
   g.npl = d.maxU <= 32 ? 1 : d.maxU <= 64 ? 2 : d.maxU <= 128 ? 4 : div_up(d.maxU, 32);
   g.ld = 32 * g.npl;
   g.nDiag = d.maxT + d.maxU;   // one spare row: the node beyond the terminating blank
-  g.nBlk = (g.nDiag + kDiag - 1) / kDiag;
+  g.nBlk = (g.nDiag + kDiag - 1) / kDiag + 1;
   g.stride = (i64)g.ld * g.nDiag;
   return g;
 }
@@ -883,7 +1131,11 @@ size_t sweep_partial_floats(Dims d) {
   do {                                       \
     if ((npl) == 1) { CALL(1); }             \
     else if ((npl) == 2) { CALL(2); }        \
-    else { CALL(4); }                        \
+    else if ((npl) <= 4) { CALL(4); }        \
+    else if ((npl) == 5) { CALL(5); }        \
+    else if ((npl) == 6) { CALL(6); }        \
+    else if ((npl) == 7) { CALL(7); }        \
+    else { CALL(8); }                        \
   } while (0)
 #define TB200_BY_NPL_NATURAL(npl, CALL)      \
   do {                                       \
@@ -892,25 +1144,21 @@ size_t sweep_partial_floats(Dims d) {
     else if ((npl) == 7) { CALL(7); }        \
     else { CALL(8); }                        \
   } while (0)
-#define TB200_BY_NPL_ANY(npl, CALL)          \
-  do {                                       \
-    if ((npl) <= 4) { TB200_BY_NPL(npl, CALL); } \
-    else { TB200_BY_NPL_NATURAL(npl, CALL); } \
-  } while (0)
-
 void launch_sweep_forward(const void* E, const void* P, float* LN, const float* ELrow,
                           float* ebl, float2* arcs, float* alphas, float* deltas, float* costs,
-                          float* lossSum, unsigned* ticket, const int* labels, const int* inLens,
-                          const int* labLens, SweepGeom g, Dims d, cudaStream_t stream) {
+                          float* lossSum, unsigned* ticket, unsigned* halves, const int* labels,
+                          const int* inLens, const int* labLens, SweepGeom g, Dims d, bool score,
+                          cudaStream_t stream) {
   if (d.B <= 0) return;
-  if (natural(g.npl) && d.dtype != kDtypeF32)
+  const bool nat = natural(g.npl) && !score;
+  if (nat && d.dtype != kDtypeF32)
     throw std::invalid_argument("bf16 emissions: the label axis must not exceed 128 positions");
   if (d.maxT > 0) {
     PrepParams q{};
     q.E = E; q.P = P; q.LN = LN; q.ELrow = ELrow; q.ebl = ebl; q.arcs = arcs;
     q.labels = labels; q.inLens = inLens; q.labLens = labLens;
     q.maxT = d.maxT; q.maxU = d.maxU; q.V = d.V; q.blank = d.blank; q.npl = g.npl; q.ld = g.ld;
-    q.extra = div_up(d.maxU, 32); q.stride = g.stride;
+    q.extra = div_up(d.maxU, 32); q.nat = nat; q.stride = g.stride;
     const dim3 grid(div_up(d.maxU, 32), div_up(d.maxT, 32) + 2 * q.extra, d.B);
     ScopedKernel sk("sweep_prep", stream);
     if (d.dtype == kDtypeBf16) sweep_prep_kernel<bf16><<<grid, 256, 0, stream>>>(q);
@@ -919,7 +1167,7 @@ void launch_sweep_forward(const void* E, const void* P, float* LN, const float* 
   }
   const int ringBytes = ring_blocks(g.npl) * kDiag * g.ld * 8;
   ScopedKernel sk("alpha_sweep", stream);
-  if (natural(g.npl)) {
+  if (nat) {
     const NaturalTerms n{static_cast<const float*>(P), ebl, labels, d.V, d.blank};
     // blank emissions in shared memory: as many frames as two CTAs per SM leave room for
     constexpr int kCeiling = 112 * 1024;
@@ -935,11 +1183,11 @@ void launch_sweep_forward(const void* E, const void* P, float* LN, const float* 
     return;
   }
   const int smem = ringBytes;
-#define CALL(NPL)                                                                                \
-  allow_dyn_smem(alpha_sweep_kernel<NPL>, smem);                                                 \
-  alpha_sweep_kernel<NPL><<<d.B, 32, smem, stream>>>(arcs, costs, alphas, deltas, g.stride,      \
-                                                     g.nDiag, inLens, labLens, d.B, d.maxT,      \
-                                                     d.maxU, lossSum, ticket)
+#define CALL(NPL)                                                                                 \
+  allow_dyn_smem(alpha_sweep_kernel<NPL>, smem);                                                  \
+  alpha_sweep_kernel<NPL><<<dim3(d.B, 2), 32, smem, stream>>>(arcs, costs, alphas, deltas, g.stride, \
+                                                              g.nBlk, inLens, labLens, d.B, d.maxT, \
+                                                              d.maxU, lossSum, ticket, halves)
   TB200_BY_NPL(g.npl, CALL);
 #undef CALL
   TB200_CHECK_LAUNCH();
@@ -958,9 +1206,9 @@ void launch_sweep_backward(const SweepScratch& w, const float* P, const float* b
     const dim3 grid(div_up(g.nDiag, kFactorRows * kFactorWarps), d.B);
 #define CALL(NPL)                                                                              \
   gamma_factors_kernel<NPL><<<grid, 32 * kFactorWarps, 0, stream>>>(                           \
-      arcs, alphas, alphaDeltas, n, w.F, w.ticket, g.stride, g.nDiag, inLens, labLens, d.maxT, d.maxU)
+      arcs, alphas, alphaDeltas, n, w.F, w.ticket, g.stride, g.nBlk, inLens, labLens, d.maxT, d.maxU)
     const NaturalTerms n{P, blankEmissions, labels, d.V, d.blank};
-    TB200_BY_NPL_ANY(g.npl, CALL);
+    TB200_BY_NPL(g.npl, CALL);
 #undef CALL
     TB200_CHECK_LAUNCH();
   }
@@ -969,8 +1217,14 @@ void launch_sweep_backward(const SweepScratch& w, const float* P, const float* b
     ScopedKernel sk("gamma_sweep", stream);
 #define CALL(NPL)                                                                              \
   allow_dyn_smem(gamma_sweep_kernel<NPL>, smem);                                               \
-  gamma_sweep_kernel<NPL><<<d.B, 32, smem, stream>>>(w.F, w.g, g.stride, inLens, labLens, d.maxT, d.maxU)
-    TB200_BY_NPL_ANY(g.npl, CALL);
+  gamma_sweep_kernel<NPL><<<dim3(d.B, 2), 32, smem, stream>>>(w.F, alphas, w.g, g.stride, inLens, labLens, d.maxT, d.maxU)
+    if (g.npl <= 2) { if (g.npl == 1) { CALL(1); } else { CALL(2); } }
+    else if (g.npl <= 4) { CALL(4); }
+#undef CALL
+#define CALL(NPL)                                                                              \
+  allow_dyn_smem(gamma_sweep_natural_kernel<NPL>, smem);                                       \
+  gamma_sweep_natural_kernel<NPL><<<d.B, 32, smem, stream>>>(w.F, w.g, g.stride, inLens, labLens, d.maxT, d.maxU)
+    else { TB200_BY_NPL_NATURAL(g.npl, CALL); }
 #undef CALL
     TB200_CHECK_LAUNCH();
   }
