@@ -194,6 +194,20 @@ int tb200_loss_forward(const float* emissions, const float* predictions,
                        int maxInputLength, int maxLabelLength, int alphabetSize,
                        int blank, void* workspace, size_t workspaceBytes);
 
+/* The costs alone, where no backward call will follow (torch_binding.py:25-58 under no_grad): nothing is
+ * saved, and label axes of more than 128 positions need not keep to the rounding that their gradients
+ * depend on.  workspace: tb200_loss_score_workspace_bytes().  _bf16: see tb200_loss_forward_bf16. */
+size_t tb200_loss_score_workspace_bytes(int batchSize, int maxInputLength, int maxLabelLength,
+                                        int alphabetSize);
+int tb200_loss_score(const float* emissions, const float* predictions, const int* labels,
+                     const int* inputLengths, const int* labelLengths, float* costs,
+                     float* lossSum, int batchSize, int maxInputLength, int maxLabelLength,
+                     int alphabetSize, int blank, void* workspace, size_t workspaceBytes);
+int tb200_loss_score_bf16(const void* emissions, const void* predictions, const int* labels,
+                          const int* inputLengths, const int* labelLengths, float* costs,
+                          float* lossSum, int batchSize, int maxInputLength, int maxLabelLength,
+                          int alphabetSize, int blank, void* workspace, size_t workspaceBytes);
+
 /* transducer/torch_binding.py:60-90 (Transducer.backward): reverse sweep + dense
  * gradient contractions + deltas scaling, from the same inputs and the `saved`
  * buffer of the forward call.  Every element of egrads [B,maxT,V] and pgrads

@@ -10,6 +10,7 @@ import torch
 
 import abi
 from oracle import oracle as O
+from transducer_b200 import TransducerLoss
 
 pytestmark = pytest.mark.gpu
 
@@ -200,3 +201,50 @@ def test_wide_axes_against_the_row_major_kernel(T, U):
     tol = (T + U) * 2.0 ** -22 + 4.0 * (3 * (T + U)) ** 0.5 * 2.0 ** -24 * want[finite].max().item()
     assert finite[0] and finite[2]   # (the masked utterance of one frame has no path)
     assert (costs - want)[finite].abs().max().item() < tol and torch.equal(costs[~finite], want[~finite])
+
+
+@pytest.mark.parametrize("T,U", [(1, 1), (40, 9), (33, 65), (100, 128), (1, 129), (60, 150), (33, 161), (90, 200),
+                                 (40, 225), (700, 256), (20, 257)])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_costs_alone(T, U, dtype):
+    """The call without a backward call to follow against float64, through the module as well (which takes it
+    under no_grad and where no input requires a gradient); beyond 128 positions it has sweeps of its own."""
+    B, V = 3, 40
+    if dtype == "bf16" and U > 128:
+        pytest.skip("bf16: label axes of at most 128 positions")
+    g = torch.Generator(device="cuda").manual_seed(10 * T + U)
+    E = torch.empty((B, T, V), device="cuda").normal_(generator=g)
+    P = torch.empty((B, U, V), device="cuda").normal_(generator=g)
+    if dtype == "bf16":
+        E, P = E.bfloat16(), P.bfloat16()
+    labels = torch.randint(1, V, (B, U - 1), generator=g, device="cuda", dtype=torch.int32)
+    il = torch.tensor([T, max(1, T // 2), 0], dtype=torch.int32, device="cuda")
+    ll = torch.tensor([U - 1, U // 2 if U > 1 else 0, U - 1], dtype=torch.int32, device="cuda")
+    lib = abi.lib
+    costs, total = torch.zeros((B,), device="cuda"), torch.zeros((1,), device="cuda")
+    n = lib.tb200_loss_score_workspace_bytes(B, T, U, V)
+    ws = abi.workspace(n)
+    abi.use_torch_stream()
+    fn = lib.tb200_loss_score_bf16 if dtype == "bf16" else lib.tb200_loss_score
+    args = [abi.ptr(t) for t in (E, P, labels, il, ll, costs, total)] + [B, T, U, V, 0, abi.ptr(ws)]
+    assert fn(*args, n - 256) == 1   # (too small a workspace is refused)
+    abi.check(fn(*args, n))
+    h = lambda x: x.float().cpu().numpy()
+    ref = O.truth64(h(E), h(P), labels.cpu().numpy(), il.cpu().numpy(), ll.cpu().numpy())["costs"]
+    # as test_edges, and 2^-19 a node for the log-normalisers (tensor cores)
+    tol = 4.0 * np.sqrt(T + U) * 2.0 ** -15 + 1e-5 + (T + U) * 2.0 ** -19
+    np.testing.assert_allclose(h(costs)[:2], ref[:2], rtol=1e-6, atol=tol)
+    assert np.isposinf(h(costs)[2])
+    crit = TransducerLoss()
+    with torch.no_grad():
+        quiet = crit(E, P, labels, il, ll)
+    plain = crit(E, P, labels, il, ll)
+    E.requires_grad_(True)
+    graded = crit(E, P, labels, il, ll)
+    assert torch.equal(quiet, costs) and torch.equal(plain, costs) and not quiet.requires_grad
+    assert graded.requires_grad
+    # with gradients to follow, axes beyond 128 positions carry alphas at full magnitude: three roundings of
+    # them a node (4 sigma), and 2^-22 of the hardware logaddexp
+    if U > 128:
+        tol += (T + U) * 2.0 ** -22 + 4.0 * (3 * (T + U)) ** 0.5 * 2.0 ** -24 * float(np.max(ref[:2]))
+    np.testing.assert_allclose(h(graded.detach())[:2], h(costs)[:2], rtol=1e-6, atol=2 * tol)

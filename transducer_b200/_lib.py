@@ -48,6 +48,9 @@ SIGNATURES = {
     "tb200_loss_saved_bytes": (_z, [_i] * 4),
     "tb200_loss_forward": (_i, [_p] * 8 + [_z] + [_i] * 5 + [_p, _z]),
     "tb200_loss_forward_bf16": (_i, [_p] * 8 + [_z] + [_i] * 5 + [_p, _z]),
+    "tb200_loss_score_workspace_bytes": (_z, [_i] * 4),
+    "tb200_loss_score": (_i, [_p] * 7 + [_i] * 5 + [_p, _z]),
+    "tb200_loss_score_bf16": (_i, [_p] * 7 + [_i] * 5 + [_p, _z]),
     "tb200_loss_backward_bf16": (_i, [_p] * 6 + [_z] + [_p] * 3 + [_i] * 5 + [_p, _z]),
     "tb200_loss_backward_workspace_bytes": (_z, [_i] * 4),
     "tb200_loss_backward": (_i, [_p] * 6 + [_z] + [_p] * 3 + [_i] * 5 + [_p, _z]),

@@ -110,6 +110,22 @@ PYBIND11_MODULE(_transducer, m) {
         "max_input_length"_a, "max_label_length"_a, "alphabet_size"_a, "blank"_a, "workspace"_a,
         "workspace_bytes"_a);
 
+  m.def("loss_score_workspace_bytes", &tb200_loss_score_workspace_bytes);
+
+  m.def("loss_score",
+        [](addr e, addr p, addr labels, addr ilen, addr llen, addr costs, addr loss_sum, int B, int T,
+           int U, int V, int blank, addr ws, size_t wsBytes, bool bf16) {
+          check(bf16 ? tb200_loss_score_bf16(at<const void>(e), at<const void>(p), at<const int>(labels),
+                                             at<const int>(ilen), at<const int>(llen), at<float>(costs),
+                                             at<float>(loss_sum), B, T, U, V, blank, at<void>(ws), wsBytes)
+                     : tb200_loss_score(at<const float>(e), at<const float>(p), at<const int>(labels),
+                                        at<const int>(ilen), at<const int>(llen), at<float>(costs),
+                                        at<float>(loss_sum), B, T, U, V, blank, at<void>(ws), wsBytes));
+        },
+        "emissions"_a, "predictions"_a, "labels"_a, "input_lengths"_a, "label_lengths"_a,
+        "costs"_a, "loss_sum"_a, "batch_size"_a, "max_input_length"_a, "max_label_length"_a,
+        "alphabet_size"_a, "blank"_a, "workspace"_a, "workspace_bytes"_a, "bf16"_a);
+
   m.def("loss_forward_bf16",
         [](addr e, addr p, addr labels, addr ilen, addr llen, addr costs, addr loss_sum,
            addr saved, size_t savedBytes, int B, int T, int U, int V, int blank, addr ws,

@@ -398,24 +398,27 @@ size_t tb200_loss_forward_workspace_bytes(int B, int maxT, int maxU, int V) {
 
 namespace {
 
+// score: no backward call will read what is left in `saved`, which may then sit behind the workspace.
 int loss_forward_any(const void* E, const void* P, const int* labels, const int* inLens,
                      const int* labLens, float* costs, float* lossSum, void* saved,
                      size_t savedBytes, int B, int maxT, int maxU, int V, int blank,
-                     void* workspace, size_t workspaceBytes, int dtype) {
+                     void* workspace, size_t workspaceBytes, int dtype, bool score = false) {
   return guarded([&] {
     Dims d{B, maxT, maxU, V, blank, dtype};
     check_dims(d);
     if (dtype != kDtypeF32 && maxU > 128)
       throw std::invalid_argument("bf16 emissions: the label axis must not exceed 128 positions");
-    need(workspaceBytes, tb200_loss_forward_workspace_bytes(B, maxT, maxU, V), workspace);
-    need(savedBytes, tb200_loss_saved_bytes(B, maxT, maxU, V), saved);
+    const size_t forwardBytes = tb200_loss_forward_workspace_bytes(B, maxT, maxU, V);
+    need(workspaceBytes, score ? tb200_loss_score_workspace_bytes(B, maxT, maxU, V) : forwardBytes, workspace);
+    if (score) saved = static_cast<char*>(workspace) + forwardBytes;
+    else need(savedBytes, tb200_loss_saved_bytes(B, maxT, maxU, V), saved);
     Carver cs(saved);
     SavedState st(cs, d);
     Carver c(workspace);
     ForwardWs fw(c, d);
     LogNormWs ws(c, d);
-    // The shape alone decides which sweeps run (the backward call must pick the ones that match
-    // the saved state).
+    // The shape (and whether a backward call may follow) alone decides which sweeps run: the backward call
+    // must pick the ones that match the saved state.
     const bool sweep = sweep_supported(d);
     float* LN = sweep ? st.LN : fw.LN;
     // (nodes the tensor-core log-normaliser could not represent are recomputed by the re-layout)
@@ -427,7 +430,7 @@ int loss_forward_any(const void* E, const void* P, const int* labels, const int*
     if (sweep) {
       launch_sweep_forward(E, P, LN, gathered ? fw.EL : nullptr, st.ebl, st.arcs,
                            st.alphas, st.deltas, costs, lossSum, ticket, ws.ticket + 16, labels, inLens,
-                           labLens, sweep_geom(d), d, /*score=*/false, g_stream);
+                           labLens, sweep_geom(d), d, score, g_stream);
       return;
     }
     const SkewGeom g = skew_geom(d);
@@ -455,6 +458,24 @@ int tb200_loss_forward_bf16(const void* E, const void* P, const int* labels, con
                             void* workspace, size_t workspaceBytes) {
   return loss_forward_any(E, P, labels, inLens, labLens, costs, lossSum, saved, savedBytes, B, maxT,
                           maxU, V, blank, workspace, workspaceBytes, kDtypeBf16);
+}
+
+size_t tb200_loss_score_workspace_bytes(int B, int maxT, int maxU, int V) {
+  return tb200_loss_forward_workspace_bytes(B, maxT, maxU, V) + tb200_loss_saved_bytes(B, maxT, maxU, V);
+}
+
+int tb200_loss_score(const float* E, const float* P, const int* labels, const int* inLens,
+                     const int* labLens, float* costs, float* lossSum, int B, int maxT, int maxU, int V,
+                     int blank, void* workspace, size_t workspaceBytes) {
+  return loss_forward_any(E, P, labels, inLens, labLens, costs, lossSum, nullptr, 0, B, maxT, maxU, V, blank,
+                          workspace, workspaceBytes, kDtypeF32, /*score=*/true);
+}
+
+int tb200_loss_score_bf16(const void* E, const void* P, const int* labels, const int* inLens,
+                          const int* labLens, float* costs, float* lossSum, int B, int maxT, int maxU, int V,
+                          int blank, void* workspace, size_t workspaceBytes) {
+  return loss_forward_any(E, P, labels, inLens, labLens, costs, lossSum, nullptr, 0, B, maxT, maxU, V, blank,
+                          workspace, workspaceBytes, kDtypeBf16, /*score=*/true);
 }
 
 size_t tb200_loss_backward_workspace_bytes(int B, int maxT, int maxU, int V) {

@@ -50,7 +50,8 @@ class Transducer(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, emissions, predictions, labels, input_lengths, label_lengths, blank=0,
-                validate_lengths=True, check_status=False):
+                validate_lengths=True, check_status=False, score=False):
+        # (score: the costs alone are wanted, no backward call can follow)
         certify_inputs(emissions, predictions, labels, input_lengths, label_lengths,
                        validate_lengths and not check_status, allow_bf16=True)
         device = emissions.device
@@ -61,6 +62,19 @@ class Transducer(torch.autograd.Function):
         f32 = dict(device=device, dtype=torch.float32)
         costs = torch.empty((B,), **f32)
         loss_sum = torch.empty((1,), **f32)
+        if score:
+            with DeviceManager(device):
+                nbytes = _transducer.loss_score_workspace_bytes(B, T, U, V)
+                ws = _workspace(nbytes + _SUMMARY_BYTES, device)
+                _transducer.loss_score(
+                    emissions.data_ptr(), predictions.data_ptr(), labels.data_ptr(),
+                    input_lengths.data_ptr(), label_lengths.data_ptr(), costs.data_ptr(),
+                    loss_sum.data_ptr(), B, T, U, V, blank, ws.data_ptr(), nbytes,
+                    emissions.dtype is torch.bfloat16)
+                finish_call(emissions, predictions, input_lengths, label_lengths, ws, nbytes,
+                            validate_lengths, check_status)
+            ctx.mark_non_differentiable(loss_sum)
+            return costs, loss_sum
         with DeviceManager(device):
             saved_bytes = _transducer.loss_saved_bytes(B, T, U, V)
             saved = _workspace(saved_bytes, device)
@@ -106,7 +120,7 @@ class Transducer(torch.autograd.Function):
             if ctx.check_status:
                 rc = _transducer.check_status()
                 raise_for_status(rc, _transducer.last_error() if rc else "")
-        return egrads, pgrads, None, None, None, None, None, None
+        return egrads, pgrads, None, None, None, None, None, None, None
 
 
 class TransducerLoss(torch.nn.Module):
@@ -161,7 +175,8 @@ class TransducerLoss(torch.nn.Module):
         """
         costs, loss_sum = Transducer.apply(
             emissions, predictions, labels, input_lengths, label_lengths, self.blank,
-            self.validate_lengths, self.check_status)
+            self.validate_lengths, self.check_status,
+            not (torch.is_grad_enabled() and (emissions.requires_grad or predictions.requires_grad)))
         self.last_loss_sum = loss_sum
         if self.reduction == "sum":
             return costs.sum()
