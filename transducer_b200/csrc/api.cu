@@ -152,7 +152,7 @@ struct BackwardWs {
 struct ViterbiWs {
   float *LN, *rowRef, *maxP, *best;
   uint32_t* decBits;
-  float4* nodes;  // skewed per-node operands of the single-warp sweep (label axis <= 256)
+  float* nodes;   // skewed operands of the single-warp sweep (label axis <= 256)
   char* prune;    // candidate lists of the pruned max-plus (null where it does not apply)
   ViterbiWs(Carver& c, const Dims& d) {
     const size_t B = d.B, T = d.maxT, U = d.maxU;
@@ -161,7 +161,7 @@ struct ViterbiWs {
     maxP = c.take<float>(B * U);
     best = c.take<float>(B * T * U);
     decBits = c.take<uint32_t>(std::max(viterbi_decbits_words(d), viterbi_warp_decbits_words(d)));
-    nodes = c.take<float4>(viterbi_warp_nodes(d));
+    nodes = c.take<float>(viterbi_warp_scratch_floats(d));
     prune = c.take<char>(maxplus_pruned_scratch_bytes(d));
   }
 };
@@ -334,7 +334,7 @@ int tb200_viterbi(const float* E, const float* P, const float* LN, int* labels,
     struct Temporaries {
       float* best = nullptr;
       uint32_t* dec = nullptr;
-      float4* nodes = nullptr;
+      float* nodes = nullptr;
       void* prune = nullptr;
       cudaStream_t stream;
       ~Temporaries() {
@@ -348,14 +348,14 @@ int tb200_viterbi(const float* E, const float* P, const float* LN, int* labels,
     TB200_CUDA_CHECK(cudaMallocAsync((void**)&tmp.best, sizeof(float) * cells, g_stream));
     TB200_CUDA_CHECK(cudaMallocAsync((void**)&tmp.dec, sizeof(uint32_t) * decWords, g_stream));
     if (warp)
-      TB200_CUDA_CHECK(cudaMallocAsync((void**)&tmp.nodes, sizeof(float4) * viterbi_warp_nodes(d),
+      TB200_CUDA_CHECK(cudaMallocAsync((void**)&tmp.nodes, sizeof(float) * viterbi_warp_scratch_floats(d),
                                        g_stream));
     if (maxplus_pruned_supported(d) && g_opt.maxplus_path != 1)
       TB200_CUDA_CHECK(cudaMallocAsync(&tmp.prune, maxplus_pruned_scratch_bytes(d), g_stream));
     best_label_scores(E, P, tmp.best, inLens, labLens, d, tmp.prune);
     if (warp)
-      launch_viterbi_warp(E, P, LN, tmp.best, tmp.nodes, tmp.dec, labels, inLens, labLens, d,
-                          device_status_word(), g_stream);
+      launch_viterbi_warp(E, P, const_cast<float*>(LN), /*fix=*/false, tmp.best, tmp.nodes, tmp.dec, labels,
+                          inLens, labLens, d, g_stream);
     else
       launch_viterbi_lattice(E, P, LN, tmp.best, tmp.dec, labels, inLens, labLens, d, g_stream);
   });
@@ -605,11 +605,13 @@ int tb200_viterbi_decode(const float* E, const float* P, const int* inLens,
     Carver c(workspace);
     ViterbiWs ws(c, d);
     LogNormWs lw(c, d);
-    log_norms_impl(E, P, ws.LN, ws.rowRef, ws.maxP, inLens, labLens, d, lw);
+    // (nodes the log-normaliser could not represent are recomputed by the re-layout)
+    const bool warp = viterbi_warp_supported(d);
+    log_norms_impl(E, P, ws.LN, ws.rowRef, ws.maxP, inLens, labLens, d, lw, /*fixup=*/!warp);
     best_label_scores(E, P, ws.best, inLens, labLens, d, ws.prune);
-    if (viterbi_warp_supported(d))
-      launch_viterbi_warp(E, P, ws.LN, ws.best, ws.nodes, ws.decBits, labels, inLens, labLens, d,
-                          device_status_word(), g_stream);
+    if (warp)
+      launch_viterbi_warp(E, P, ws.LN, /*fix=*/true, ws.best, ws.nodes, ws.decBits, labels, inLens,
+                          labLens, d, g_stream);
     else
       launch_viterbi_lattice(E, P, ws.LN, ws.best, ws.decBits, labels, inLens, labLens, d,
                              g_stream);

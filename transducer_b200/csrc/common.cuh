@@ -89,6 +89,18 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+
+// log sum_v exp(e[v] + p[v]) by one warp, every lane has the result.
+template <typename TIn>
+__device__ __forceinline__ float warp_logsumexp(const TIn* e, const TIn* p, int V, int lane) {
+  float m = neg_inf();
+  for (int v = lane; v < V; v += 32) m = fmaxf(m, to_f32(e[v]) + to_f32(p[v]));
+  m = warp_max(m);
+  float s = 0.0f;
+  if (m != neg_inf() && m != pos_inf())
+    for (int v = lane; v < V; v += 32) s += expf((to_f32(e[v]) + to_f32(p[v])) - m);
+  return logf(warp_sum(s)) + m;
+}
 #endif
 
 }  // namespace tb200

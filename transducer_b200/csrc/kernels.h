@@ -182,14 +182,15 @@ void launch_sweep_backward(const SweepScratch& w, const float* P, const float* b
 
 // ---- lattice_warp.cu -------------------------------------------------------------
 // Viterbi sweep in one warp per utterance (label axis <= 256): same results as
-// launch_viterbi_lattice.  `nodes` is scratch of viterbi_warp_nodes(d) float4, decBits of
-// viterbi_warp_decbits_words(d) words.
+// launch_viterbi_lattice.  scratch: viterbi_warp_scratch_floats(d) floats (8-byte aligned), decBits:
+// viterbi_warp_decbits_words(d) words.  fix: NaN entries of LN are recomputed in place first (else LN is
+// only read).
 bool viterbi_warp_supported(Dims d);
-size_t viterbi_warp_nodes(Dims d);
+size_t viterbi_warp_scratch_floats(Dims d);
 size_t viterbi_warp_decbits_words(Dims d);  // its decision bits are packed along t+u
-void launch_viterbi_warp(const float* E, const float* P, const float* LN, const float* best,
-                         float4* nodes, uint32_t* decBits, int* labels, const int* inLens,
-                         const int* labLens, Dims d, int* status, cudaStream_t stream);
+void launch_viterbi_warp(const float* E, const float* P, float* LN, bool fix, const float* best,
+                         float* scratch, uint32_t* decBits, int* labels, const int* inLens,
+                         const int* labLens, Dims d, cudaStream_t stream);
 
 // ---- maxplus.cu --------------------------------------------------------------
 // best[b,t,u] = max over v != blank of E[b,t,v] + P[b,u,v] for t < T_b, u < U_b - 1.  With

@@ -1,14 +1,13 @@
 // Viterbi sweep for label axes of at most 256 positions: the recursion runs in ONE warp.
 //
-// The wavefront kernels of lattice.cu spend a block barrier and a shared-memory exchange on
-// every anti-diagonal.  Here lane l of a single warp owns adjacent label positions; all nodes of
-// a diagonal are independent, the one value per lane that crosses from the neighbouring lane
-// arrives by a warp shuffle, and a block of 16 diagonals of the skewed operand array (node (t,u)
-// at (t+u)*ld + u) is one contiguous range of memory, fetched by one bulk asynchronous copy into
-// a shared-memory ring several blocks ahead of its use.
+// Lane l of the warp owns adjacent label positions; all nodes of a diagonal d = t + u are
+// independent, the one value per lane that crosses from the neighbouring lane arrives by a warp
+// shuffle, and the operands of a node, a pair, come by cp.async through the ring of pair_ring.cuh.
+// (Not from both ends, as the loss's sweeps: the scores are added in the reference's order.)
 #include <algorithm>
 
 #include "kernels.h"
+#include "pair_ring.cuh"
 #include "profile.h"
 #include "sm100.cuh"
 
@@ -16,59 +15,87 @@ namespace tb200 {
 namespace {
 
 using namespace sm100;
-
-constexpr int kDiag = 16;   // diagonals per block
-constexpr int kRing = 4;    // blocks in flight
+using namespace sweep;
 
 // ---------------------------------------------------------------------------
 // Viterbi: max-plus sweep in one warp, bit-packed decisions, backtrack, label argmax
 // ---------------------------------------------------------------------------
-// Per node the sweep needs E[t,blank], LN[t,u] and best[t,u] (the max-plus label score of
-// maxplus.cu); viterbi_prep_kernel lays them out skewed as one float4 per node, so that a block
-// of diagonals is one bulk copy.  The scores are formed in the reference's operation order,
-// ((score + E[t,blank]) + P[u,blank]) - LN and (score + best) - LN, so every comparison, and
-// with it the path, is bit-identical to transducer_cpu.cpp:145-222.
-// Nodes outside the lattice hold the record (-1e30, 0, -1e30): whatever enters them leaves as
-// about -1e30, which loses every comparison against a real score.  With that the sweep needs
-// no case distinctions at all: the blank arc into frame 0 and the label arc into position 0
-// come from such nodes (or from the -inf fed to lane 0) and lose by themselves.
+// Per node the sweep needs LN[t,u], best[t,u] (the max-plus label score of maxplus.cu) and E[t,blank].  The
+// first two are a pair of the skewed rows written by viterbi_prep_kernel; the blank emissions are in shared
+// memory, and a lane reads one of them per diagonal: position r + 1 meets a frame one diagonal after
+// position r.  The scores are formed in the reference's operation order, ((score + E[t,blank]) +
+// P[u,blank]) - LN and (score + best) - LN, so every comparison, and with it the path, is bit-identical
+// to transducer_cpu.cpp:145-222.  Nodes outside the lattice hold the pair (1e30, 0): whatever
+// enters them leaves as about -1e30, which loses every comparison against a real score, as does the
+// label arc of the last position, whose best is -1e30.  With that the sweep needs no case distinctions
+// at all: the blank arc into frame 0 and the label arc into position 0 come from such nodes
+// (or from the -inf fed to lane 0) and lose by themselves.
 constexpr float kNoNode = -1.0e30f;
 
-__global__ void __launch_bounds__(256) viterbi_fill_kernel(float4* __restrict__ nodes, i64 n) {
-  const float4 none = make_float4(kNoNode, 0.0f, kNoNode, 0.0f);
-  for (i64 k = (i64)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (i64)gridDim.x * blockDim.x)
-    nodes[k] = none;
-}
+struct VitPrepParams {
+  const float* E;
+  const float* P;
+  float* LN;               // [B,maxT,maxU]
+  bool fix;                // recompute its marked (NaN) nodes, in place
+  const float* best;
+  float2* nodes;
+  float* ebl;              // [B,maxT]
+  const int* inLens;
+  const int* labLens;
+  int maxT, maxU, V, blank, npl, extra;
+  i64 stride;
+};
 
-__global__ void __launch_bounds__(256) viterbi_prep_kernel(
-    const float* __restrict__ E, const float* __restrict__ LN, const float* __restrict__ best,
-    float4* __restrict__ nodes, const int* __restrict__ inLens, const int* __restrict__ labLens,
-    int maxT, int maxU, int V, int blank, int ld, i64 latStride) {
-  // (even rows: an anti-diagonal of a tile falls into 32 different banks, with 33 into one)
-  __shared__ float tLn[32][34], tBs[32][34], tEb[32];
-  const int b = blockIdx.z, t0 = blockIdx.y * 32, u0 = blockIdx.x * 32;
-  const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
-  if (t0 >= T || u0 >= U) return;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const float* ln = LN + (i64)b * maxT * maxU;
-  const float* bs = best + (i64)b * maxT * maxU;
-  const int u = u0 + lane, uc = min(u, U - 1), ub = min(u, max(U - 2, 0));
+// One CTA per 32x32 (t,u) tile; the tiles beyond both ends of the time axis (`extra` of them on each side)
+// write the pairs of nodes outside the lattice, so that the array needs no fill.  Bound by memory: 8
+// bytes read and 8 written per node.  (Records of 16 bytes, a fill of the array and a pass over LN for
+// marked nodes before it took 126 us at B = 64, T = 750..1500, U' = 76..151, this takes 48; the sweep
+// on those records 232 us, on pairs 166.)
+__global__ void __launch_bounds__(256) viterbi_prep_kernel(const VitPrepParams p) {
+  __shared__ float tLn[32][kTileLd], tBs[32][kTileLd];
+  const int b = blockIdx.z, t0 = ((int)blockIdx.y - p.extra) * 32, u0 = blockIdx.x * 32;
+  const int T = min(p.inLens[b], p.maxT), U = min(p.labLens[b] + 1, p.maxU);
+  if (T <= 0 || U <= 0) return;
+  const int Uw = (U + p.npl - 1) / p.npl * p.npl, S = T + U - 1;
+  if (u0 >= Uw || t0 + u0 + 62 < 0 || t0 + u0 >= S) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, u = u0 + lane;
+  if (t0 + 31 >= 0 && t0 < T && u0 < U) {   // does the tile hold any node?
+    const float* e = p.E + (i64)b * p.maxT * p.V;
+    const float* pr = p.P + (i64)b * p.maxU * p.V;
+    float* ln = p.LN + (i64)b * p.maxT * p.maxU;
+    const float* bs = p.best + (i64)b * p.maxT * p.maxU;
+    const int uc = min(u, U - 1), ub = min(u, max(U - 2, 0));
+    float va[4], vb[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int tt = w * 4 + k, tc = min(t0 + tt, T - 1);
-    tLn[tt][lane] = ln[(i64)tc * maxU + uc];
-    // the label arc of the last position does not exist
-    tBs[tt][lane] = (u < U - 1) ? bs[(i64)tc * maxU + ub] : kNoNode;
+    for (int k = 0; k < 4; ++k) {
+      const i64 at = (i64)min(t0 + w * 4 + k, T - 1) * p.maxU;
+      va[k] = ln[at + uc];
+      vb[k] = bs[at + ub];
+    }
+    if (u0 == 0 && threadIdx.x < 32 && t0 + lane < T)
+      p.ebl[(i64)b * p.maxT + t0 + lane] = e[(i64)(t0 + lane) * p.V + p.blank];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int tt = w * 4 + k, t = t0 + tt;
+      unsigned todo = __ballot_sync(0xffffffffu, p.fix && t < T && u < U && va[k] != va[k]);
+      while (todo) {
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const float exact = warp_logsumexp(e + (i64)t * p.V, pr + (i64)(u0 + src) * p.V, p.V, lane);
+        if (lane == src) ln[(i64)t * p.maxU + u] = va[k] = exact;
+      }
+      tLn[tt][lane] = va[k];
+      tBs[tt][lane] = u < U - 1 ? vb[k] : kNoNode;   // the label arc of the last position does not exist
+    }
   }
-  if (threadIdx.x < 32)
-    tEb[lane] = E[((i64)b * maxT + min(t0 + lane, T - 1)) * V + blank];
   __syncthreads();
+  float2* nodes = p.nodes + (i64)b * p.stride + pair_slot(u, p.npl);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {   // diagonal i of the tile in the lanes up to i, i + 32 in the others
-    const int tt = (w + 8 * k - lane) & 31;
-    if (t0 + tt < T && u < U)
-      nodes[(i64)b * latStride + (i64)(t0 + tt + u) * ld + u] =
-          make_float4(tEb[tt], tLn[tt][lane], tBs[tt][lane], 0.0f);
+    const int tt = (w + 8 * k - lane) & 31, t = t0 + tt, d = t + u;
+    if (d < 0 || d >= S || u >= Uw) continue;
+    nodes[(i64)d * (32 * p.npl)] =
+        t >= 0 && t < T && u < U ? make_float2(tLn[tt][lane], tBs[tt][lane]) : make_float2(-kNoNode, 0.0f);
   }
 }
 
@@ -84,15 +111,14 @@ __host__ __device__ inline int viterbi_words_d(int maxT, int maxU) { return (max
 // decBits scratch otherwise: the backtrack is a chain of dependent reads of them.
 template <int NPL>
 __global__ void __launch_bounds__(32) viterbi_warp_kernel(
-    const float* __restrict__ P, const float4* __restrict__ nodes,
-    int ld, i64 latStride, int nDiag, int ringDepth, uint32_t* __restrict__ decBits, int decInSmem,
-    int* __restrict__ frames, int* __restrict__ labelsOut, const int* __restrict__ inLens,
-    const int* __restrict__ labLens, int maxT, int maxU, int V, int blank, int* status) {
+    const float* __restrict__ P, const float2* __restrict__ nodes, const float* __restrict__ ebl,
+    i64 stride, int maxStage, uint32_t* __restrict__ decBits, int decInSmem,
+    int* __restrict__ frames, const int* __restrict__ inLens,
+    const int* __restrict__ labLens, int maxT, int maxU, int V, int blank) {
+  constexpr int ld = 32 * NPL, kRing = ring_blocks(NPL);
   extern __shared__ __align__(128) uint8_t smemV[];
-  __shared__ uint64_t bar[kRing];
-  __shared__ int abortFlag;
   __shared__ int sFrame[256];  // frame at which label u-1 was emitted (U <= 256 here)
-  const int b = blockIdx.x, i = threadIdx.x, lane = i & 31, warp = i >> 5;
+  const int b = blockIdx.x, i = threadIdx.x, lane = i;
   const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
   int* fr = frames + (i64)b * maxU;
   if (T <= 0 || U <= 0) {
@@ -100,109 +126,82 @@ __global__ void __launch_bounds__(32) viterbi_warp_kernel(
     return;
   }
   const float* p = P + (i64)b * maxU * V;
-  const float4* nd = nodes + (i64)b * latStride;
   const int wordsD = viterbi_words_d(maxT, maxU);
-  uint32_t* dec = decInSmem
-                      ? reinterpret_cast<uint32_t*>(smemV + (size_t)ringDepth * kDiag * ld * 16)
-                      : decBits + (i64)b * maxU * wordsD;
+  // shared memory: ring, blank emissions (of utterances of up to maxStage frames), decision bits
+  float* sEb = reinterpret_cast<float*>(smemV + kRing * kDiag * ld * 8);
+  uint32_t* dec = decInSmem ? reinterpret_cast<uint32_t*>(sEb + maxStage)
+                            : decBits + (i64)b * maxU * wordsD;
   for (int u = i; u < 256; u += 32) sFrame[u] = -1;
-  if (i == 0) {
-    for (int s = 0; s < kRing; ++s) mbar_init(&bar[s], 1);
-    abortFlag = 0;
-    fence_mbar_init();
+  const int S = T + U - 1, nBlocks = (S + kDiag - 1) / kDiag, u0 = NPL * lane;
+  PairRing<NPL> ring(smemV, nodes + (i64)b * stride, lane, U, 0x7149f2cau /* 1e30 */, 0u);
+  auto issue = [&](int k) { ring.issue(k % kRing, (i64)k * kDiag, k < nBlocks ? min(kDiag, S - k * kDiag) : 0); };
+#pragma unroll
+  for (int k = 0; k < kRing - 1; ++k) issue(k);
+  const float* eb0 = ebl + (i64)b * maxT;
+  const bool staged = T <= maxStage;
+  if (staged) {
+#pragma unroll 8
+    for (int t = lane; t < T; t += 32) sEb[t] = eb0[t];
   }
-  __syncthreads();
-
-  if (warp == 0) {
-    float4* ring = reinterpret_cast<float4*>(smemV);  // [ringDepth][kDiag * ld]
-    const int S = T + U - 1;
-    const int nBlocks = (S + kDiag - 1) / kDiag;
-    const int slot = kDiag * ld;
-    auto issue = [&](int k) {  // lane 0
-      if (k < nBlocks) {
-        const int rows = min(kDiag, nDiag - k * kDiag);
-        const uint32_t bytes = (uint32_t)(rows * ld) * 16u;
-        mbar_arrive_expect_tx(&bar[k % ringDepth], bytes);
-        bulk_load_1d(ring + (size_t)(k % ringDepth) * slot, nd + (size_t)k * slot, bytes,
-                     &bar[k % ringDepth]);
+  __syncwarp();
+  const float* ebRow = staged ? sEb : eb0;
+  auto eblAt = [&](int t) { return ebRow[min(max(t, 0), T - 1)]; };
+  float pbl[NPL], eb[NPL], stay[NPL], stepOut[NPL];
+  uint32_t bits[NPL];
+#pragma unroll
+  for (int r = 0; r < NPL; ++r) {
+    pbl[r] = (u0 + r < U) ? p[(i64)(u0 + r) * V + blank] : 0.0f;
+    eb[r] = eblAt(-(u0 + r));
+    stay[r] = stepOut[r] = kNoNode;
+    bits[r] = 0u;
+  }
+  if (lane == 0) stay[0] = 0.0f;  // score 0 enters the origin (as if by its blank arc)
+  float up = neg_inf();
+  for (int k = 0; k < nBlocks; ++k) {
+    issue(k + kRing - 1);
+    ring.wait();
+    const int slot = k % kRing, nd = min(kDiag, S - k * kDiag);
+    const int tNext = k * kDiag + 1 - u0;   // frame of position u0 on the diagonal after the block's first
+    const uint32_t bit0 = 1u << (kDiag * (k & 1));
+    auto diag = [&](int dd) {
+      float ln[NPL], bs[NPL];
+      ring.read(slot, dd, ln, bs);
+      const float ebNext = eblAt(tNext + dd), first = lane ? up : neg_inf();
+      // the last position first, whose step leaves by a shuffle; each position still needs the
+      // previous diagonal's step of the one below it
+#pragma unroll
+      for (int r = NPL - 1; r >= 0; --r) {
+        const float left = r ? stepOut[(r + NPL - 1) % NPL] : first;
+        // the larger of the two arcs, the blank arc on ties (strict '>', as the reference)
+        const bool takeStep = left > stay[r];
+        const float sc = takeStep ? left : stay[r];
+        if (takeStep) bits[r] |= bit0 << dd;
+        stay[r] = ((sc + eb[r]) + pbl[r]) - ln[r];
+        stepOut[r] = (sc + bs[r]) - ln[r];
+        if (r == NPL - 1) up = __shfl_up_sync(0xffffffffu, stepOut[r], 1);
       }
+#pragma unroll
+      for (int r = NPL - 1; r > 0; --r) eb[r] = eb[r - 1];
+      eb[0] = ebNext;
     };
-    if (lane == 0)
-      for (int k = 0; k < ringDepth - 1; ++k) issue(k);
-    const int u0 = NPL * lane;
-    float pbl[NPL], stay[NPL], stepOut[NPL];
-    uint32_t bits[NPL];
-    uint32_t* decU[NPL];
+    if (nd == kDiag) {
 #pragma unroll
-    for (int r = 0; r < NPL; ++r) {
-      pbl[r] = (u0 + r < U) ? p[(i64)(u0 + r) * V + blank] : 0.0f;
-      stay[r] = stepOut[r] = kNoNode;
-      bits[r] = 0u;
-      decU[r] = dec + (i64)min(u0 + r, maxU - 1) * wordsD;
+      for (int dd = 0; dd < kDiag; ++dd) diag(dd);
+    } else {
+#pragma unroll 1
+      for (int dd = 0; dd < nd; ++dd) diag(dd);
     }
-    if (lane == 0) stay[0] = 0.0f;  // score 0 enters the origin (as if by its blank arc)
-    bool ok = true;
-    int kFail = 0;
-    for (int k = 0; k < nBlocks; ++k) {
-      __syncwarp();  // all lanes have read the slot that is refilled next
-      if (lane == 0) {
-        fence_proxy_async_smem();
-        issue(k + ringDepth - 1);
-      }
-      ok = mbar_wait(&bar[k % ringDepth], (k / ringDepth) & 1, &abortFlag, status, kStatusTimeoutTma);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) {
-        kFail = k;
-        break;
-      }
-      const float4* blk = ring + (size_t)(k % ringDepth) * slot;
-      const int ndg = min(kDiag, S - k * kDiag);
-#pragma unroll 2
-      for (int dd = 0; dd < ndg; ++dd) {
-        const int d = k * kDiag + dd;
-        float4 nv[NPL];
+    if ((k & 1) || k == nBlocks - 1) {   // a word of 32 diagonals is complete
 #pragma unroll
-        for (int r = 0; r < NPL; ++r) nv[r] = blk[dd * ld + min(u0 + r, ld - 1)];
-        const float up = __shfl_up_sync(0xffffffffu, stepOut[NPL - 1], 1);
-        const uint32_t bit = 1u << (d & 31);
-        float left[NPL];
-        left[0] = lane ? up : neg_inf();
-#pragma unroll
-        for (int r = 1; r < NPL; ++r) left[r] = stepOut[r - 1];
-#pragma unroll
-        for (int r = 0; r < NPL; ++r) {
-          // the larger of the two arcs, the blank arc on ties (strict '>', as the reference)
-          const bool takeStep = left[r] > stay[r];
-          const float sc = takeStep ? left[r] : stay[r];
-          bits[r] |= takeStep ? bit : 0u;
-          stay[r] = ((sc + nv[r].x) + pbl[r]) - nv[r].y;   // E[t,blank], LN[t,u]
-          stepOut[r] = (sc + nv[r].z) - nv[r].y;           // best[t,u]
-        }
-        if ((d & 31) == 31 || d == S - 1) {
-#pragma unroll
-          for (int r = 0; r < NPL; ++r) {
-            if (u0 + r < U) decU[r][d >> 5] = bits[r];
-            bits[r] = 0u;
-          }
-        }
+      for (int r = 0; r < NPL; ++r) {
+        if (u0 + r < U) dec[(i64)(u0 + r) * wordsD + (k >> 1)] = bits[r];
+        bits[r] = 0u;
       }
     }
-    if (!ok && lane == 0) {  // give the copies still in flight a bounded time to land
-      for (int j = kFail; j < min(kFail + ringDepth, nBlocks); ++j) {
-        const unsigned long long t1 = global_timer_ns();
-        while (!mbar_try_wait(&bar[j % ringDepth], (j / ringDepth) & 1) &&
-               global_timer_ns() - t1 < 50000000ull) {
-        }
-      }
-    }
-    __threadfence_block();
   }
+  ring.drain();
+  __threadfence_block();
   __syncthreads();
-  if (abortFlag) {  // a copy never landed (recorded in the status word): no path, labels = -1
-    for (int u = i; u < U - 1; u += 32) labelsOut[(i64)b * (maxU - 1) + u] = -1;
-    for (int u = i; u < maxU; u += 32) fr[u] = -1;
-    return;
-  }
 
   // Backtrack from (T-1,U-1) along row u in diagonal coordinates d = t + u.  Each iteration
   // consumes either one label or one 32-diagonal word of blanks, so it ends within
@@ -297,32 +296,40 @@ size_t viterbi_warp_decbits_words(Dims d) {
              : 0;
 }
 
-size_t viterbi_warp_nodes(Dims d) {
-  const SkewGeom g = skew_geom(d);
-  return viterbi_warp_supported(d) ? (size_t)d.B * (size_t)g.stride : 0;
+// Rows of pairs: positions per lane (up to 8) and length of an utterance.
+static int viterbi_npl(Dims d) { return div_up(std::max(d.maxU, 1), 32); }
+static i64 viterbi_stride(Dims d) { return (i64)32 * viterbi_npl(d) * (d.maxT + d.maxU); }
+
+size_t viterbi_warp_scratch_floats(Dims d) {
+  return viterbi_warp_supported(d) ? (size_t)d.B * (2 * (size_t)viterbi_stride(d) + (size_t)d.maxT) : 0;
 }
 
-void launch_viterbi_warp(const float* E, const float* P, const float* LN, const float* best,
-                         float4* nodes, uint32_t* decBits, int* labels, const int* inLens,
-                         const int* labLens, Dims d, int* status, cudaStream_t stream) {
+void launch_viterbi_warp(const float* E, const float* P, float* LN, bool fix, const float* best,
+                         float* scratch, uint32_t* decBits, int* labels, const int* inLens,
+                         const int* labLens, Dims d, cudaStream_t stream) {
   if (d.B <= 0 || d.maxT <= 0 || d.maxU <= 0) return;
-  const SkewGeom g = skew_geom(d);
+  const int npl = viterbi_npl(d), ld = 32 * npl;
+  const i64 stride = viterbi_stride(d);
+  float2* nodes = reinterpret_cast<float2*>(scratch);
+  float* ebl = scratch + 2 * (size_t)d.B * stride;
   {
-    dim3 grid(div_up(d.maxU, 32), div_up(d.maxT, 32), d.B);
+    VitPrepParams q{};
+    q.E = E; q.P = P; q.LN = LN; q.fix = fix; q.best = best; q.nodes = nodes; q.ebl = ebl;
+    q.inLens = inLens; q.labLens = labLens;
+    q.maxT = d.maxT; q.maxU = d.maxU; q.V = d.V; q.blank = d.blank; q.npl = npl;
+    q.extra = div_up(d.maxU, 32); q.stride = stride;
+    dim3 grid(div_up(d.maxU, 32), div_up(d.maxT, 32) + 2 * q.extra, d.B);
     ScopedKernel sk("viterbi_prep", stream);
-    viterbi_fill_kernel<<<148 * 8, 256, 0, stream>>>(nodes, (i64)d.B * g.stride);
-    viterbi_prep_kernel<<<grid, 256, 0, stream>>>(E, LN, best, nodes, inLens, labLens, d.maxT,
-                                                  d.maxU, d.V, d.blank, g.ld, g.stride);
+    viterbi_prep_kernel<<<grid, 256, 0, stream>>>(q);
     TB200_CHECK_LAUNCH();
   }
-  // shared memory: the decision bits (if they leave room for a ring of at least three blocks
-  // of node records), then the ring
-  const int slotBytes = kDiag * g.ld * 16;
-  const int decBytes = d.maxU * viterbi_words_d(d.maxT, d.maxU) * 4;
+  // shared memory: the ring, the blank emissions and the decision bits where they fit
   constexpr int room = 216 * 1024;
-  const int decInSmem = decBytes + 3 * slotBytes <= room ? 1 : 0;
-  const int ringDepth = std::max(2, std::min(kRing, (room - (decInSmem ? decBytes : 0)) / slotBytes));
-  const int smem = ringDepth * slotBytes + (decInSmem ? decBytes : 0);
+  const int ringBytes = ring_blocks(npl) * kDiag * ld * 8;
+  const int stage = std::min(d.maxT, (room - ringBytes) / 4);
+  const i64 decBytes = (i64)d.maxU * viterbi_words_d(d.maxT, d.maxU) * 4;
+  const int decInSmem = ringBytes + stage * 4 + decBytes <= room ? 1 : 0;
+  const int smem = ringBytes + stage * 4 + (decInSmem ? (int)decBytes : 0);
   int* frames = reinterpret_cast<int*>(decBits) +
                 (size_t)d.B * d.maxU * viterbi_words_d(d.maxT, d.maxU);
   {
@@ -331,10 +338,10 @@ void launch_viterbi_warp(const float* E, const float* P, const float* LN, const 
   do {                                                                                         \
     allow_dyn_smem(viterbi_warp_kernel<NPL>, room);                                            \
     viterbi_warp_kernel<NPL><<<d.B, 32, smem, stream>>>(                                       \
-        P, nodes, g.ld, g.stride, g.nDiag, ringDepth, decBits, decInSmem, frames, labels,      \
-        inLens, labLens, d.maxT, d.maxU, d.V, d.blank, status);                                \
+        P, nodes, ebl, stride, stage, decBits, decInSmem, frames, inLens, labLens, d.maxT,     \
+        d.maxU, d.V, d.blank);                                                                 \
   } while (0)
-  switch (g.ld / 32) {
+  switch (npl) {
     case 1: CALL(1); break;
     case 2: CALL(2); break;
     case 3: CALL(3); break;

@@ -739,15 +739,8 @@ __global__ void __launch_bounds__(256) lognorm_fixup_kernel(
     while (todo) {
       const int src = __ffs(todo) - 1;
       todo &= todo - 1;
-      const TIn* pr = P + ((i64)b * maxU + u0 + src) * V;
-      float m = neg_inf();
-      for (int v = lane; v < V; v += 32) m = fmaxf(m, to_f32(er[v]) + to_f32(pr[v]));
-      m = warp_max(m);
-      float s = 0.0f;
-      if (m != neg_inf() && m != pos_inf())
-        for (int v = lane; v < V; v += 32) s += expf((to_f32(er[v]) + to_f32(pr[v])) - m);
-      s = warp_sum(s);
-      if (lane == 0) ln[u0 + src] = logf(s) + m;
+      const float exact = warp_logsumexp(er, P + ((i64)b * maxU + u0 + src) * V, V, lane);
+      if (lane == 0) ln[u0 + src] = exact;
     }
   }
 }
