@@ -130,3 +130,32 @@ def test_viterbi_labels_do_not_depend_on_the_path():
     finally:
         abi.set_option("maxplus_path", 0)
     assert torch.equal(got[1], got[2])
+
+
+@pytest.mark.parametrize("U", [2, 3, 33, 34, 65, 66, 97, 129, 193, 257, 300])
+@pytest.mark.parametrize("V", [1024, 2049])
+def test_pairs_of_positions(U, V):
+    """A lane evaluates two adjacent positions: label axes around multiples of 32, 64 and 256, with few frames
+    (fewer than the groups of a CTA) and lists whose walk goes beyond the head."""
+    gen = torch.Generator().manual_seed(U * V)
+    B, T = 2, 19
+    E = torch.randn(B, T, V, generator=gen).cuda()
+    P = torch.randn(B, U, V, generator=gen)
+    P[:, ::3] *= 0.01      # nearly flat positions: the whole list is walked
+    P = P.cuda()
+    il, ll = lengths(B, T, U, gen)
+    full, lists = both_paths(E, P, il, ll, 0)
+    assert_identical(full, lists, il, ll)
+
+
+def test_label_axes_too_long_for_the_lists():
+    """Where the heads of the lists do not fit a CTA's shared memory the full loop runs (and no scratch is asked)."""
+    B, T, U, V = 1, 3, 1400, 1024
+    assert abi.lib.tb200_label_arc_scores_workspace_bytes(B, T, U, V) == 0
+    gen = torch.Generator().manual_seed(1)
+    E, P = torch.randn(B, T, V, generator=gen).cuda(), torch.randn(B, U, V, generator=gen).cuda()
+    il, ll = lengths(B, T, U, gen)
+    got = abi.label_arc_scores(E, P, il, ll)
+    want = numpy_scores(E.cpu().numpy(), P.cpu().numpy(), 0)
+    n = int(ll[0])
+    assert np.array_equal(got.cpu().numpy()[0, :T, :n], want[0, :, :n])

@@ -32,14 +32,24 @@ using namespace sm100;
 
 constexpr int kETop = 128;    // entries listed per frame
 constexpr int kPTop = 128;    // entries listed per label position
-constexpr int kBatchP = 8;    // list entries fetched at a time beyond the head
 constexpr int kPre = 32;      // entries of every position's list kept in shared memory
-constexpr int kPRows = kPTop + kBatchP;   // rows of a position list in memory
+constexpr int kHead = 8;      // of them walked by every lane for its own positions
+constexpr int kPRows = kPTop + 1;   // rows of a position list in memory
+constexpr int kMaxGroups = 15;      // groups of a CTA of the evaluation kernel (one named barrier each)
 // A frame's list in memory: offsets v*us (int) [kETop], values [kETop], bound, count, padding.
 // Entries from `count` up to the next multiple of 32 repeat entry 0.
 constexpr int kEWords = 2 * kETop + 4;
 constexpr size_t kSelSmemBytes = 96 * 1024;   // rows staged per CTA of the selection kernels
-constexpr int kPrunedSmemBytes = 227 * 1024 - 80;   // all that maxplus_pruned_kernel's barriers leave
+constexpr size_t kPrunedSmemBytes = 227 * 1024 - 256;   // all that maxplus_pruned_kernel's barriers leave
+
+// Both sums at once (add.rn.f32x2: each rounded as by itself).
+__device__ __forceinline__ float2 add_pair(float2 a, float2 b) {
+  float2 s;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "add.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(s.x), "=f"(s.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return s;
+}
 
 __device__ __forceinline__ int warp_sum_int(int v) { return __reduce_add_sync(0xffffffffu, v); }
 
@@ -349,14 +359,26 @@ struct PrunedParams {
   int maxT, maxU, V, us, groups, warpsPerGroup, framesPerCta, fbCap;
 };
 
+// Row strides of the list heads in shared memory: a lane's two positions make one access, and the 32
+// entries of one position fall into 16 banks.
+__host__ __device__ constexpr int head_val_stride(int us) { return us + 2; }   // floats
+__host__ __device__ constexpr int head_idx_stride(int us) { return us + 4; }   // 16-bit numbers
+
 // CTA = `groups` groups of `warpsPerGroup` warps over a chunk of frames of one utterance.  A
-// group takes every groups-th frame: its row of E and its list arrive by bulk copy, one frame
-// ahead, in the group's own pair of buffers; inside a group, warp w evaluates the label
-// positions 32w .. 32w+31 (+ 32*warpsPerGroup ...) of the frame.  The heads of the positions'
+// group takes every groups-th frame: its row of E and its list arrive by bulk copy in the group's
+// buffer, while other groups work; inside a group, warp w evaluates the label positions 64w .. 64w+63
+// (+ 64*warpsPerGroup ...) of the frame, two adjacent ones a lane.  The heads of the positions'
 // lists (kPre entries, 16-bit indices) sit in shared memory for the whole CTA.
-__global__ void __launch_bounds__(512) maxplus_pruned_kernel(const PrunedParams p) {
+//
+// Bound by instruction issue: one entry of the frame's list costs a load of the transposed P, its
+// address, half a packed addition and half a three-way maximum per position.  Two positions a lane
+// halve the loads and addresses; walking a position's list to its end lane by lane made a warp wait for
+// the longest of 32 walks (~35 entries, 6 on average), so beyond kHead entries the whole warp takes one
+// position at a time, 32 entries at once.  Measured (B = 64, T = 750..1500, U' = 76..151, V = 4096, N(0,1)):
+// 1219 -> 811 us.  (Shorter lists of the frames, kETop 96 / 64: 924 / 1197 us, the walks get longer.)
+__global__ void __launch_bounds__(1024) maxplus_pruned_kernel(const PrunedParams p) {
   extern __shared__ __align__(16) uint8_t stagedBytes[];
-  __shared__ uint64_t bar[4][2];
+  __shared__ uint64_t bar[kMaxGroups];
   __shared__ int abortFlag;
   const int b = blockIdx.y;
   const int T = min(p.inLens[b], p.maxT), nLab = min(p.labLens[b] + 1, p.maxU) - 1;
@@ -366,132 +388,147 @@ __global__ void __launch_bounds__(512) maxplus_pruned_kernel(const PrunedParams 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grp = warp / p.warpsPerGroup, wInG = warp - grp * p.warpsPerGroup;
   const bool leader = wInG == 0 && lane == 0;
-  const int nUB = (nLab + 31) >> 5;
+  const int nUB = (nLab + 63) >> 6;
   const float* e = p.E + (i64)b * p.maxT * p.V;
   const bool bulk = (p.V & 3) == 0 && (reinterpret_cast<uintptr_t>(e) & 15) == 0;
   // (rows are kept a multiple of 16 bytes apart, so that the lists behind them stay aligned)
   const int rowStride = (p.V + 3) & ~3;
   const size_t rowBytes = (size_t)rowStride * 4, listBytes = (size_t)kEWords * 4;
-  const size_t bufBytes = rowBytes + listBytes;
-  uint8_t* myBufs = stagedBytes + (size_t)grp * 2 * bufBytes;
-  float* sPreVal = reinterpret_cast<float*>(stagedBytes + (size_t)p.groups * 2 * bufBytes);  // [kPre][us]
-  float* sThP = sPreVal + (size_t)kPre * p.us;                                                // [us]
-  unsigned short* sPreIdx = reinterpret_cast<unsigned short*>(sThP + p.us);                   // [kPre][us]
+  const int valStride = head_val_stride(p.us), idxStride = head_idx_stride(p.us);
+  float* row = reinterpret_cast<float*>(stagedBytes + (size_t)grp * (rowBytes + listBytes));
+  int* el = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(row) + rowBytes);
+  float* sPreVal = reinterpret_cast<float*>(stagedBytes + (size_t)p.groups * (rowBytes + listBytes));  // [kPre][valStride]
+  float* sThP = sPreVal + (size_t)kPre * valStride;                                                     // [us]
+  unsigned short* sPreIdx = reinterpret_cast<unsigned short*>(sThP + p.us);                             // [kPre][idxStride]
   if (threadIdx.x == 0) {
-    for (int g = 0; g < 4; ++g) {
-      mbar_init(&bar[g][0], 1);
-      mbar_init(&bar[g][1], 1);
-    }
+    for (int g = 0; g < p.groups; ++g) mbar_init(&bar[g], 1);
     abortFlag = 0;
     fence_mbar_init();
   }
-  {  // the heads of the lists and the positions' bounds
-    const int2* pl0 = p.pList + (i64)b * kPRows * p.us;
-    for (int i = threadIdx.x; i < kPre * p.us; i += blockDim.x) {
-      const int2 c = __ldg(pl0 + i);
-      sPreVal[i] = __int_as_float(c.y);
-      sPreIdx[i] = (unsigned short)c.x;
+  for (int u = threadIdx.x; u < p.us; u += blockDim.x) {  // the heads of the lists and the positions' bounds
+    const bool mine = u < nLab;
+    const int2 meta = mine ? __ldg(p.pMeta + (i64)b * p.us + u) : make_int2(0, 0);
+    const int2* pl = p.pList + (i64)b * kPRows * p.us + u;
+    sThP[u] = mine ? __int_as_float(meta.x) : neg_inf();
+#pragma unroll 8
+    for (int k = 0; k < kPre; ++k) {
+      // (an entry behind the list must never win)
+      const int2 c = k < meta.y ? __ldg(pl + (i64)k * p.us) : make_int2(0, __float_as_int(neg_inf()));
+      sPreVal[k * valStride + u] = __int_as_float(c.y);
+      sPreIdx[k * idxStride + u] = (unsigned short)c.x;
     }
-    for (int i = threadIdx.x; i < p.us; i += blockDim.x)
-      sThP[i] = i < nLab ? __int_as_float(__ldg(p.pMeta + (i64)b * p.us + i).x) : neg_inf();
   }
   __syncthreads();
   const int first = tBeg + grp;                       // my group's frames: first, first + groups, ...
   const int nMine = first < tEnd ? (tEnd - first + p.groups - 1) / p.groups : 0;
   const int groupThreads = p.warpsPerGroup * 32;
   auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(groupThreads) : "memory"); };
-  auto fetch = [&](int i) {   // my group's i-th frame -> buffer i & 1
-    const int t = first + i * p.groups, buf = i & 1;
-    float* rows = reinterpret_cast<float*>(myBufs + buf * bufBytes);
-    int* ls = reinterpret_cast<int*>(myBufs + buf * bufBytes + rowBytes);
-    const int* el = p.eList + ((i64)b * p.maxT + t) * kEWords;
-    if (bulk) {
-      if (leader) {
-        mbar_arrive_expect_tx(&bar[grp][buf], (uint32_t)(rowBytes + listBytes));
-        bulk_load_1d(rows, e + (i64)t * p.V, (uint32_t)rowBytes, &bar[grp][buf]);
-        bulk_load_1d(ls, el, (uint32_t)listBytes, &bar[grp][buf]);
-      }
-    } else {
-      const int tid = wInG * 32 + lane;
-      for (int v = tid; v < p.V; v += groupThreads) rows[v] = __ldg(e + (i64)t * p.V + v);
-      for (int k = tid; k < kEWords; k += groupThreads) ls[k] = __ldg(el + k);
-    }
-  };
-  if (nMine > 0) fetch(0);
   bool ok = true;
   for (int i = 0; i < nMine; ++i) {
-    const int t = first + i * p.groups, buf = i & 1;
-    group_sync();   // every warp of the group has left frame i-1, whose buffer the next copy takes
-    if (i + 1 < nMine) fetch(i + 1);
+    const int t = first + i * p.groups;
+    const int* elMem = p.eList + ((i64)b * p.maxT + t) * kEWords;
+    group_sync();   // every warp of the group has left frame i-1, whose buffer the copy takes
     if (bulk) {
-      ok = mbar_wait(&bar[grp][buf], (i >> 1) & 1, &abortFlag, p.status, kStatusTimeoutTma);
+      if (leader) {
+        mbar_arrive_expect_tx(&bar[grp], (uint32_t)(rowBytes + listBytes));
+        bulk_load_1d(row, e + (i64)t * p.V, (uint32_t)rowBytes, &bar[grp]);
+        bulk_load_1d(el, elMem, (uint32_t)listBytes, &bar[grp]);
+        if (i + 1 < nMine) bulk_prefetch_l2(e + (i64)(t + p.groups) * p.V, (uint32_t)rowBytes);
+      }
+      ok = mbar_wait(&bar[grp], i & 1, &abortFlag, p.status, kStatusTimeoutTma);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
     } else {
+      const int tid = wInG * 32 + lane;
+      for (int v = tid; v < p.V; v += groupThreads) row[v] = __ldg(e + (i64)t * p.V + v);
+      for (int k = tid; k < kEWords; k += groupThreads) el[k] = __ldg(elMem + k);
       group_sync();
     }
-    const float* row = reinterpret_cast<const float*>(myBufs + buf * bufBytes);
-    const int* el = reinterpret_cast<const int*>(myBufs + buf * bufBytes + rowBytes);
     const int4* off4 = reinterpret_cast<const int4*>(el);
     const float4* val4 = reinterpret_cast<const float4*>(el + kETop);
     const float thE = __int_as_float(el[2 * kETop]);
     const int nE = el[2 * kETop + 1];
     for (int ub = wInG; ub < nUB; ub += p.warpsPerGroup) {
-      const int u = ub * 32 + lane;
-      const bool mine = u < nLab;
-      float L = neg_inf();
-      // 1. the frame's own candidates against this position, 16 loads in flight
-      const float* pt = p.PT + (i64)b * p.V * p.us + u;   // (u < us: the stride is a multiple of 32)
+      const int u = ub * 64 + 2 * lane;      // my positions u, u + 1
+      const int uc = min(u, p.us - 2);       // (the row stride is a multiple of 32, not of 64)
+      float L[2] = {neg_inf(), neg_inf()};
+      // 1. the frame's own candidates against these positions, 16 loads in flight
+      const float* pt = p.PT + (i64)b * p.V * p.us + uc;
       for (int j4 = 0; 4 * j4 < nE; j4 += 4) {
-        float x[16];
+        float2 x[16];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int4 o = off4[j4 + q];
-          x[4 * q] = __ldg(pt + o.x); x[4 * q + 1] = __ldg(pt + o.y);
-          x[4 * q + 2] = __ldg(pt + o.z); x[4 * q + 3] = __ldg(pt + o.w);
+          x[4 * q] = __ldg(reinterpret_cast<const float2*>(pt + o.x));
+          x[4 * q + 1] = __ldg(reinterpret_cast<const float2*>(pt + o.y));
+          x[4 * q + 2] = __ldg(reinterpret_cast<const float2*>(pt + o.z));
+          x[4 * q + 3] = __ldg(reinterpret_cast<const float2*>(pt + o.w));
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const float4 ev = val4[j4 + q];
-          L = fmaxf(fmaxf(L, ev.x + x[4 * q]), ev.y + x[4 * q + 1]);
-          L = fmaxf(fmaxf(L, ev.z + x[4 * q + 2]), ev.w + x[4 * q + 3]);
+          const float evs[4] = {ev.x, ev.y, ev.z, ev.w};
+          float2 s[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) s[k] = add_pair(make_float2(evs[k], evs[k]), x[4 * q + k]);
+          L[0] = fmaxf(fmaxf(L[0], s[0].x), s[1].x);
+          L[1] = fmaxf(fmaxf(L[1], s[0].y), s[1].y);
+          L[0] = fmaxf(fmaxf(L[0], s[2].x), s[3].x);
+          L[1] = fmaxf(fmaxf(L[1], s[2].y), s[3].y);
         }
       }
-      // 2. the position's candidates, best first, while one of them could still win: the
-      //    head of the list from shared memory, the rest kBatchP entries at a time (a lane
-      //    that has stopped ignores what was fetched for it; the entry behind a list is -inf)
-      bool live = mine;
-      for (int k0 = 0; k0 < kPre && __any_sync(0xffffffffu, live); k0 += 4) {
+      // 2. the positions' candidates, best first, while one of them could still win: the head of
+      //    each list by the lane that owns the position ...
+      bool live[2] = {u < nLab, u + 1 < nLab};
+      for (int k0 = 0; k0 < kHead && __any_sync(0xffffffffu, live[0] || live[1]); k0 += 4) {
 #pragma unroll
         for (int k = k0; k < k0 + 4; ++k) {
-          const float pv = sPreVal[k * p.us + u];
-          const int v = sPreIdx[k * p.us + u];
-          live = live && (pv + thE > L);
-          if (live) L = fmaxf(L, row[v] + pv);
+          const float2 pv = *reinterpret_cast<const float2*>(sPreVal + k * valStride + uc);
+          const ushort2 v = *reinterpret_cast<const ushort2*>(sPreIdx + k * idxStride + uc);
+          live[0] = live[0] && (pv.x + thE > L[0]);
+          live[1] = live[1] && (pv.y + thE > L[1]);
+          if (live[0]) L[0] = fmaxf(L[0], row[v.x] + pv.x);
+          if (live[1]) L[1] = fmaxf(L[1], row[v.y] + pv.y);
         }
       }
-      const int2* pl = p.pList + (i64)b * kPRows * p.us + u;
-      for (int j0 = kPre; __any_sync(0xffffffffu, live); j0 += kBatchP) {
-        int2 c[kBatchP];
+      //    ... and the rest by the whole warp, one position after the other, 32 entries at a time
+      //    (an entry that can no longer win is a sum like any other)
 #pragma unroll
-        for (int k = 0; k < kBatchP; ++k) c[k] = __ldg(pl + (i64)(j0 + k) * p.us);
-#pragma unroll
-        for (int k = 0; k < kBatchP; ++k) {
-          const float pv = __int_as_float(c[k].y);
-          live = live && (pv + thE > L);
-          if (live) L = fmaxf(L, row[c[k].x] + pv);
+      for (int h = 0; h < 2; ++h) {
+        for (unsigned todo = __ballot_sync(0xffffffffu, live[h]); todo; todo &= todo - 1) {
+          const int src = __ffs(todo) - 1, us1 = ub * 64 + 2 * src + h;
+          float best = __shfl_sync(0xffffffffu, L[h], src);
+          float pv = sPreVal[lane * valStride + us1];
+          int v = sPreIdx[lane * idxStride + us1];
+          int n = kPTop;
+          for (int j0 = 0;;) {
+            float c = best;
+            if (pv + thE > best) c = fmaxf(c, row[v] + pv);
+            best = warp_max(c);
+            j0 += kPre;
+            // could the entries behind these still win?
+            if (j0 >= n || !(__shfl_sync(0xffffffffu, pv, 31) + thE > best)) break;
+            if (j0 == kPre) n = __ldg(p.pMeta + (i64)b * p.us + us1).y;
+            const int2 e2 = j0 + lane < n ? __ldg(p.pList + ((i64)b * kPRows + j0 + lane) * p.us + us1)
+                                          : make_int2(0, __float_as_int(neg_inf()));
+            v = e2.x;
+            pv = __int_as_float(e2.y);
+          }
+          if (lane == src) L[h] = best;
         }
       }
       // 3. settled?
-      if (mine) {
-        const i64 node = ((i64)b * p.maxT + t) * p.maxU + u;
-        if (sThP[u] + thE > L) {
-          const int at = atomicAdd(p.fbCount, 1);
-          if (at < p.fbCap) p.fbList[at] = (unsigned long long)node;
-        } else {
-          p.best[node] = L;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (u + h < nLab) {
+          const i64 node = ((i64)b * p.maxT + t) * p.maxU + u + h;
+          if (sThP[u + h] + thE > L[h]) {
+            const int at = atomicAdd(p.fbCount, 1);
+            if (at < p.fbCap) p.fbList[at] = (unsigned long long)node;
+          } else {
+            p.best[node] = L[h];
+          }
         }
-      }
     }
   }
   if (!ok) {
@@ -499,11 +536,9 @@ __global__ void __launch_bounds__(512) maxplus_pruned_kernel(const PrunedParams 
     // the full evaluation redoes every node, and give the group's copies a bounded time.
     if (leader) {
       atomicAdd(p.fbCount, p.fbCap + 1);
-      for (int k = 0; k < 2; ++k) {
-        const unsigned long long t1 = global_timer_ns();
-        while (!mbar_try_wait(&bar[grp][k], 0) && !mbar_try_wait(&bar[grp][k], 1) &&
-               global_timer_ns() - t1 < 50000000ull) {
-        }
+      const unsigned long long t1 = global_timer_ns();
+      while (!mbar_try_wait(&bar[grp], 0) && !mbar_try_wait(&bar[grp], 1) &&
+             global_timer_ns() - t1 < 50000000ull) {
       }
     }
     group_sync();
@@ -535,6 +570,9 @@ __global__ void __launch_bounds__(256) maxplus_listed_kernel(
 }
 
 int label_stride(Dims d) { return (int)round_up64(d.maxU > 1 ? d.maxU - 1 : 1, 32); }
+size_t heads_bytes(int us) {
+  return kPre * (head_val_stride(us) * sizeof(float) + head_idx_stride(us) * sizeof(unsigned short)) + us * sizeof(float);
+}
 int fallback_capacity(Dims d) {
   const i64 nodes = (i64)d.B * d.maxT * (d.maxU - 1);
   return (int)std::min<i64>(1 << 22, std::max<i64>(4096, nodes / 64));
@@ -574,7 +612,9 @@ struct Scratch {
 bool maxplus_pruned_supported(Dims d) {
   // below ~1000 words the lists are most of the row
   return d.B > 0 && d.B <= 65535 && d.maxT > 0 && d.maxU > 1 && d.V >= 1024 && d.V <= kMaxWords &&
-         (i64)d.V * label_stride(d) < (i64(1) << 31);
+         (i64)d.V * label_stride(d) < (i64(1) << 31) &&
+         // (one row and the heads of all lists fit the evaluation kernel)
+         heads_bytes(label_stride(d)) + ((size_t)d.V + 3 + kEWords) * sizeof(float) <= kPrunedSmemBytes;
 }
 
 size_t maxplus_pruned_scratch_bytes(Dims d) {
@@ -620,20 +660,19 @@ void launch_maxplus_pruned(const float* E, const float* P, float* best, const in
   p.inLens = inLens; p.labLens = labLens; p.fbList = s.fbList; p.fbCount = s.fbCount;
   p.maxT = d.maxT; p.maxU = d.maxU; p.V = d.V; p.us = us;
   p.status = status;
-  // warps of a group: one per 32 label positions (at most 8); groups: as many as keep the CTA
-  // near ten warps and its buffers within ~100 KB
-  p.warpsPerGroup = std::min(8, div_up(d.maxU - 1, 32));
-  const size_t perGroup = 2 * (rowB + kEWords * sizeof(int));
-  p.groups = (int)std::max<size_t>(1, std::min<size_t>(std::min(4, 10 / p.warpsPerGroup),
-                                                       (100 * 1024) / perGroup));
-  p.framesPerCta = 16 * p.groups;
+  // warps of a group: one per 64 label positions (at most 4); groups: as many as the threads of a CTA and
+  // its shared memory allow
+  p.warpsPerGroup = std::min(4, div_up(d.maxU - 1, 64));
+  const size_t perGroup = rowB + kEWords * sizeof(int), heads = heads_bytes(us);
+  p.groups = (int)std::max<size_t>(1, std::min<size_t>(std::min(kMaxGroups, 32 / p.warpsPerGroup),
+                                                       (kPrunedSmemBytes - heads) / perGroup));
+  p.framesPerCta = 8 * p.groups;
   p.fbCap = fallback_capacity(d);
-  const size_t smem = p.groups * perGroup +
-                      (size_t)us * (kPre * (sizeof(float) + sizeof(unsigned short)) + sizeof(float));
+  const size_t smem = p.groups * perGroup + heads;
   const int threads = 32 * p.warpsPerGroup * p.groups;
   {
     ScopedKernel sk("maxplus_pruned", stream);
-    allow_dyn_smem(maxplus_pruned_kernel, kPrunedSmemBytes);
+    allow_dyn_smem(maxplus_pruned_kernel, (int)kPrunedSmemBytes);
     maxplus_pruned_kernel<<<dim3(div_up(d.maxT, p.framesPerCta), d.B), threads, smem, stream>>>(p);
   }
   TB200_CHECK_LAUNCH();
