@@ -113,3 +113,37 @@ def test_unsupported_shape_is_refused_when_forced():
     case = make(1, 40, 5, 30, seed=1)
     with pytest.raises(ValueError, match="tensor-core gradients"):
         grads(*case, path=2)
+
+
+# (utterances x blocks of 128 columns) that one CTA per item would leave most SMs to: their frames are cut
+# into parts; with short and empty utterances that have fewer tiles than there are parts
+@pytest.mark.parametrize("B,T,U,V", [(1, 96, 5, 128), (1, 97, 5, 128), (3, 700, 20, 100), (2, 2000, 101, 64),
+                                     (37, 200, 9, 520), (5, 300, 70, 4000), (150, 100, 5, 128), (2, 500, 151, 256)])
+def test_frames_cut_into_parts(B, T, U, V):
+    E, P, labels, il, ll, deltas = make(B, T, U, V, seed=B + T, repeat_labels=V == 64)
+    if B > 2:
+        il[1], il[2] = 1, 0
+    case = (E, P, labels, il, ll, deltas)
+    _, eg_s, pg_s = grads(*case, path=1)
+    fwd, eg_t, pg_t = grads(*case, path=2)
+    eg_2, pg_2 = abi.loss_backward(E, P, labels, il, ll, fwd, deltas)   # (the counters are zero again)
+    assert torch.equal(eg_t, eg_2) and torch.equal(pg_t, pg_2)
+    assert (eg_t - eg_s).abs().max().item() <= 1e-3 * eg_s.abs().max().item()
+    assert (pg_t - pg_s).abs().max().item() <= 1e-3 * pg_s.abs().max().item()
+    for b in range(B):
+        assert not eg_t[b, int(il[b]):].any() and not pg_t[b, int(ll[b]) + 1:].any()
+
+
+@pytest.mark.parametrize("T,U,V,hi", [(70, 100, 100, 100), (33, 128, 130, 4), (95, 40, 64, 64), (64, 18, 128, 128),
+                                      (40, 151, 36, 36), (50, 201, 128, 3), (40, 60, 2048, 20)])
+def test_labels_that_are_not_staged(T, U, V, hi):
+    """More labels in a block of columns than the gradient kernel stages, distinct and repeated."""
+    B = 3
+    E, P, labels, il, ll, deltas = make(B, T, U, V, seed=T + U)
+    g = torch.Generator(device="cuda").manual_seed(U)
+    labels = torch.randint(1, hi, (B, U - 1), generator=g, device="cuda", dtype=torch.int32)
+    ll[1] = min(17, U - 1)
+    case = (E, P, labels, il, ll, deltas)
+    _, eg_s, _ = grads(*case, path=1)
+    _, eg_t, _ = grads(*case, path=2)
+    assert (eg_t - eg_s).abs().max().item() <= 1e-3 * eg_s.abs().max().item()

@@ -122,6 +122,7 @@ struct ForwardWs {
 struct BackwardWs {
   float *expP, *W, *em, *emT, *nref, *ebl, *eBlank, *pBlank, *pLabel, *maxPScratch;
   SweepScratch sweep{};                 // label axis <= 256
+  float* gradPartial = nullptr;
   float *Ws = nullptr, *EMs = nullptr;  // longer ones
   BackwardWs(Carver& c, const Dims& d) {
     const size_t B = d.B, T = d.maxT, U = d.maxU, V = d.V;
@@ -131,6 +132,8 @@ struct BackwardWs {
       sweep.F = c.take<float2>(B * g.stride);
       sweep.g = c.take<float>(B * g.stride);
       sweep.ticket = c.take<unsigned>(B);
+      sweep.gradTickets = c.take<unsigned>(kGradTickets);
+      gradPartial = c.take<float>(grads_umma_partial_floats(d));
       sweep.partial = c.take<float>(sweep_partial_floats(d));
     } else {
       const SkewGeom g = skew_geom(d);
@@ -538,8 +541,8 @@ int loss_backward_any(const void* E, const void* P, const int* labels, const int
     }
     if (tensorCore) {   // (label axes of 129..256 positions: once per half of the axis)
       launch_grads_umma(E, P, st.maxP, ws.W, ws.emT, ws.nref, ws.ebl, ws.pBlank, ws.pLabel, labels,
-                        deltas, egrads, pgrads, inLens, labLens, d, passes, device_status_word(),
-                        g_stream);
+                        deltas, egrads, pgrads, inLens, labLens, d, passes, ws.gradPartial,
+                        ws.sweep.gradTickets, device_status_word(), g_stream);
       return;
     }
     launch_exp_rows(Pf, ws.expP, ws.maxPScratch, labLens, B, maxU, V, g_stream);

@@ -40,6 +40,9 @@
 // takes GEMM2 -> next exponentials and gradient reads -> next GEMM1 off the critical path.
 // D2 stays in TMEM across all tiles and becomes pgrads[:, v-block] at the end.
 //
+// The last, partly filled round of CTAs (all of them, where an utterance batch and vocabulary make
+// fewer than half as many blocks as the chip has SMs) is cut along the frames: see grad_split.
+//
 // Operand precision (`passes`): the lattice weights W are always rounded once to TF32
 // (round-to-nearest, 2^-12 relative, unbiased).  passes = 1: exp(E) and exp(P) likewise.
 // passes = 2 (default): exp(E) is split hi + lo with hi exactly representable in TF32, two
@@ -69,6 +72,15 @@ constexpr int kGradThreads = 20 * 32;
 constexpr int kStageRows = 2 + kMaxStagedLabels;  // row shifts, blank-arc sums, staged label rows
 constexpr int kMaxRing = 4;
 
+constexpr int kTileFrames = 48;   // frames of a tile, roughly (the tile height depends on the label axis)
+constexpr int kMaxPos = 128;      // label positions of a launch
+
+struct GradSplit {
+  i64 whole;
+  int cut, parts;   // items, CTAs of each of them
+  i64 ctas() const { return whole + (i64)cut * parts; }
+};
+
 struct GradParams {
   const void* P;         // [B,maxU,V] fp32 or bf16, as are egrads and pgrads
   const float* maxP;     // [B,maxU]
@@ -97,7 +109,29 @@ struct GradParams {
   int eBufs;    // copies of the expE^T operand in tensor memory (2 if the columns allow)
   int dBufs;    // copies of the D1 accumulator (likewise)
   int tmemCols;
+  int blocksV;  // blocks of 128 vocabulary columns
+  int whole;    // items (utterance, block) that one CTA processes alone
+  int parts;    // CTAs of each of the others
+  float* partial;     // [items cut, parts, kMaxPos positions, 128 columns] their sums over their frames
+  unsigned* tickets;  // [items cut] parts done: zero on entry, zero again on exit
 };
+
+// One CTA per item (utterance, block of 128 columns) and one CTA per SM: n items take
+// ceil(n / SMs) rounds, and the last one may leave most SMs idle.  Its rem = n mod SMs items are
+// cut along the frames into SMs / rem parts (a part is worth at least two tiles: the operand expP^T
+// and the sums over the frames cost a CTA about as much as one), numbered behind the whole items so
+// that they start last.  Every part leaves its sums over the frames in `partial`, and the one that
+// finishes last adds them in frame order.  Measured, whole / cut: 8 items of 2000 frames (V = 100)
+// 88 / 31 us, 64 items 89 / 58, 632 items (V = 10000, 40 in the last round) 335 / 311.
+GradSplit grad_split(Dims d) {
+  constexpr int kSMs = kGradTickets, kMaxParts = 16;
+  const i64 n = (i64)div_up(d.V, kVBlock) * d.B;
+  const int rem = (int)(n % kSMs);
+  int parts = rem > 0 ? std::min(kMaxParts, kSMs / rem) : 1;
+  parts = std::min(parts, div_up(d.maxT, 2 * kTileFrames));
+  if (parts < 2) return GradSplit{n, 0, 1};
+  return GradSplit{n - rem, rem, parts};
+}
 
 struct GradMaps {
   CUtensorMap E, G, Wk, Wmn, nref, ebl, emT;
@@ -125,7 +159,14 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
   using TIO = typename std::conditional<BF, bf16, float>::type;
   constexpr int TBH = TB / 2;  // frames per owner half
   static_assert(TBH % 8 == 0, "tile halves move through TMEM in 8-column pieces");
-  const int b = blockIdx.y, v0 = blockIdx.x * kVBlock;
+  int item = blockIdx.x, part = 0, parts = 1;
+  const int cutItem = item < p.whole ? 0 : (item - p.whole) / p.parts;
+  if (item >= p.whole) {
+    part = item - p.whole - cutItem * p.parts;
+    parts = p.parts;
+    item = p.whole + cutItem;
+  }
+  const int b = item / p.blocksV, v0 = (item - b * p.blocksV) * kVBlock;
   const int T = min(p.inLens[b], p.maxT), Utot = min(p.labLens[b] + 1, p.maxU);
   // my range of label positions: local u <-> position uOff + u; U of them belong to the utterance
   const int U = max(0, min(Utot - p.uOff, 128));
@@ -141,11 +182,17 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
     const int v = v0 + threadIdx.x;
     if (threadIdx.x < kVBlock && v < p.V) {
       if (!p.accumulate)
-        for (int t = 0; t < p.maxT; ++t) from_f32(eg[(i64)t * p.V + v], 0.0f);
-      for (int u = 0; u < rowsMine; ++u) from_f32(pg[(i64)u * p.V + v], 0.0f);
+        for (int t = part; t < p.maxT; t += parts) from_f32(eg[(i64)t * p.V + v], 0.0f);
+      for (int u = part; u < rowsMine; u += parts) from_f32(pg[(i64)u * p.V + v], 0.0f);
     }
     return;
   }
+  // my tiles: [tile0, tile0 + nTiles) of the utterance
+  const int tilesAll = (T + TB - 1) / TB;
+  parts = min(parts, tilesAll);
+  if (part >= parts) return;
+  const int tile0 = (int)((i64)tilesAll * part / parts);
+  const int nTiles = (int)((i64)tilesAll * (part + 1) / parts) - tile0;
 
   extern __shared__ uint8_t smemRaw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) &
@@ -173,12 +220,15 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
   __shared__ short sListU[128], sListV[128];
   __shared__ int sLab[128];
   __shared__ float sPb[128], sPl[128];
+  __shared__ int sLastPart, sSplit[3];   // (the split: not kept in registers through the loops)
 
-  const int nTiles = (T + TB - 1) / TB;
   // (the blank-arc terms go with the launch that writes egrads)
   const bool blankHere = !p.accumulate && p.blank >= v0 && p.blank < v0 + kVBlock;
 
   if (threadIdx.x == 0) {
+    sSplit[0] = cutItem;
+    sSplit[1] = part;
+    sSplit[2] = parts;
     for (int s = 0; s < SE; ++s) {
       mbar_init(&barEFull[s], 1);
       mbar_init(&barStore[s], kGroupWarps);   // gradient tile complete in shared memory
@@ -275,7 +325,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
     }
     int fs = 0;  // stage of the next fill
     auto fill = [&](int i) {
-      const int t0 = i * TB;
+      const int t0 = (tile0 + i) * TB;
       uint8_t* st = smem + (size_t)fs * kEStage;
       if (lane == 0) mbar_arrive_expect_tx(&barEFull[fs], bytes);
       __syncwarp();
@@ -294,9 +344,9 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
       // wait until the store engine has read their box before the stage is refilled
       if (lane < kBoxes && v0 + kBoxCols * lane < p.V) {
         if (p.accumulate)
-          tma_reduce_add_3d(&tm.G, smem + (size_t)ss * kEStage + lane * kBoxBytes, v0 + kBoxCols * lane, i * TB, b);
+          tma_reduce_add_3d(&tm.G, smem + (size_t)ss * kEStage + lane * kBoxBytes, v0 + kBoxCols * lane, (tile0 + i) * TB, b);
         else
-          tma_store_3d(&tm.G, smem + (size_t)ss * kEStage + lane * kBoxBytes, v0 + kBoxCols * lane, i * TB, b);
+          tma_store_3d(&tm.G, smem + (size_t)ss * kEStage + lane * kBoxBytes, v0 + kBoxCols * lane, (tile0 + i) * TB, b);
         tma_store_commit();
         if (issued < nTiles) tma_store_wait_read();
       }
@@ -332,7 +382,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
       if (i >= SW) ok = mbar_wait(&barWFree[s], wph, abortp, p.status, kStatusTimeoutStageFree);
       if (!__all_sync(0xffffffffu, ok)) break;
       uint8_t* st = smemW + (size_t)s * wStage;
-      const int t0 = i * TB;
+      const int t0 = (tile0 + i) * TB;
       if (lane == 0) mbar_arrive_expect_tx(&barWFull[s], (uint32_t)(2 * wBytes));
       __syncwarp();
       const int j = lane >> 1;
@@ -424,7 +474,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
     // gradient arithmetic.  Within a group the halves h = 0,1 split the frames of a tile; all
     // 16 warps split the label positions of the prologue and the epilogue.
     const int grp = warp >> 3, q = warp & 3, h = (warp >> 2) & 1;
-    const int part = grp * 2 + h;  // 0..3: share of the prologue / epilogue
+    const int share = grp * 2 + h;  // 0..3: of the prologue / epilogue
     const int vl = q * 32 + lane;
     const int v = v0 + vl;
     const bool vOk = v < p.V;
@@ -436,7 +486,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
       const TIO* pp = static_cast<const TIO*>(p.P) + ((i64)b * p.maxU + p.uOff) * p.V;
       const float* mp = p.maxP + (i64)b * p.maxU + p.uOff;
       const int vc = min(v, p.V - 1);
-      for (int u0 = 8 * part; u0 < p.Ku; u0 += 32) {
+      for (int u0 = 8 * share; u0 < p.Ku; u0 += 32) {
         // unconditional loads from clamped addresses: all eight are in flight together
         float raw[8], sh[8];
 #pragma unroll
@@ -475,7 +525,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
       int se = 0, eb = 0;          // E stage and expE^T copy of tile i
       uint32_t sph = 0, eph = 0;   // and their phases
       for (int i = 0; i < nTiles && ok; ++i) {
-        const int t0 = i * TB;
+        const int t0 = (tile0 + i) * TB;
         // live frames in my half (may be <= 0); none for a column beyond the vocabulary
         const int tValid = vOk ? min(TB, T - t0) - h * TBH : 0;
         ok = mbar_wait(&barEFull[se], sph, abortp, p.status, kStatusTimeoutTma);
@@ -535,7 +585,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
       int se = 0, eb = 0, db = 0;            // E stage, expE^T copy and D1 copy of tile i
       uint32_t sph = 0, eph = 0, dph = 0;    // and their phases
       for (int i = 0; i < nTiles && ok; ++i) {
-        const int t0 = i * TB;
+        const int t0 = (tile0 + i) * TB;
         const int tValid = vOk ? min(TB, T - t0) - h * TBH : 0;
         ok = mbar_wait(&barEFull[se], sph, abortp, p.status, kStatusTimeoutTma) &&
              mbar_wait(&barD1Full[db], dph, abortp, p.status, kStatusTimeoutMma) &&
@@ -593,21 +643,69 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
       }
     }
 
+    const int cut = ((volatile int*)sSplit)[0], myPart = ((volatile int*)sSplit)[1], nParts = ((volatile int*)sSplit)[2];
     // padded frames beyond the last tile: exact zeros
     if (vOk && !p.accumulate)
-      for (int t = nTiles * TB + part; t < p.maxT; t += 4) from_f32(eg[(i64)t * p.V + v], 0.0f);
+      for (int t = (T + TB - 1) / TB * TB + share + 4 * myPart; t < p.maxT; t += 4 * nParts)
+        from_f32(eg[(i64)t * p.V + v], 0.0f);
 
     // pgrads[u, v] = delta * (expP[u,v] * D2[v,u] - sparse)
     if (ok) ok = mbar_wait(&barD2Done, 0, abortp, p.status, kStatusTimeoutMma);
     ok = __all_sync(0xffffffffu, ok);
-    if (ok) {
-      tc_fence_after();
-      for (int u0 = 8 * part; u0 < p.Ku; u0 += 32) {
-        uint32_t d2[8], xh[8], xl[8];
+    bool writer = ok;
+    const float* partials = p.partial + (size_t)cut * p.parts * (kMaxPos * kVBlock) + vl;
+    if (nParts > 1) {
+      // my sums over my frames (NaN if they never came); the part that finishes last goes on
+      float* mine = p.partial + ((size_t)cut * p.parts + myPart) * (kMaxPos * kVBlock) + vl;
+      if (ok) tc_fence_after();
+      for (int u0 = 8 * share; u0 < p.Ku; u0 += 32) {
+        uint32_t d2[8];
         tmem_ld8(tBase + laneAddr + cD2 + u0, d2);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          mine[(u0 + j) * kVBlock] = ok ? __uint_as_float(d2[j]) : __int_as_float(0x7fc00000);
+      }
+      __threadfence();
+      asm volatile("bar.sync 1, %0;" ::"n"(2 * kGroupWarps * 32) : "memory");
+      if (threadIdx.x == 0) {
+        const unsigned done = atomicAdd(&p.tickets[cut], 1u);
+        sLastPart = done == (unsigned)(nParts - 1) ? 1 : 0;
+        if (sLastPart) p.tickets[cut] = 0u;   // ready for the next launch
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(2 * kGroupWarps * 32) : "memory");
+      writer = sLastPart != 0;
+      __threadfence();
+    }
+    if (writer) {
+      tc_fence_after();
+      for (int u0 = 8 * share; u0 < p.Ku; u0 += 32) {
+        uint32_t d2[8], xh[8], xl[8];
+        if (nParts == 1) tmem_ld8(tBase + laneAddr + cD2 + u0, d2);
         tmem_ld8(tBase + laneAddr + cPhi + u0, xh);
         if (PSPLIT) tmem_ld8(tBase + laneAddr + cPlo + u0, xl);
         tmem_wait_ld();
+        if (nParts > 1) {
+          float sum[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) sum[j] = 0.0f;
+          for (int z0 = 0; z0 < nParts; z0 += 4) {   // (32 loads in flight)
+            float x[4][8];
+#pragma unroll
+            for (int z = 0; z < 4; ++z)
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                x[z][j] = __ldcg(partials + (size_t)min(z0 + z, nParts - 1) * (kMaxPos * kVBlock) + (u0 + j) * kVBlock);
+#pragma unroll
+            for (int z = 0; z < 4; ++z)
+              if (z0 + z < nParts) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) sum[j] += x[z][j];
+              }
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) d2[j] = __float_as_uint(sum[j]);
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int u = u0 + j;
@@ -652,52 +750,83 @@ int pow2_cols(int x) {
 // columns it subtracts the occupancies of the first kMaxStagedLabels label positions (in
 // position order) whose label falls into the block; with a vocabulary of ten thousand entries a
 // block sees one or two labels, but a vocabulary of 100 puts all of an utterance's labels into
-// one block.  The remaining positions are applied here, one CTA per (block, utterance,
-// framesPerCta frames), in position order (so that repeated labels are combined in a fixed order):
+// one block.  The remaining positions are applied here, one CTA per (block, utterance, group of
+// frames), in position order (so that repeated labels are combined in a fixed order):
 //   egrads[b, t, label_u] -= emT[b, u, t]        (emT already carries delta_b)
-// The CTA rebuilds the block's list exactly as the gradient kernel does and returns at once if
-// it is short enough, which is the normal case.
+// A CTA lists the block's labels as the gradient kernel does and returns at once if they are few
+// enough, which is the normal case.  Else it brings 32 frames of the positions' rows to shared memory at a
+// time and a thread per column walks its positions, so that both sides are read along memory.
+// Measured (B = 8, T = 2000, U = 100, V = 100): 27 us, 35 with a thread per frame.  (Walking the unstaged
+// positions inside the gradient kernel's loop costs that kernel 7 % whether it has any or not.)
+constexpr int kOvfFrames = 32;
 template <typename TIO>
-__global__ void __launch_bounds__(256) label_overflow_kernel(
+__global__ void __launch_bounds__(128) label_overflow_kernel(
     const int* __restrict__ labels, const float* __restrict__ emT, TIO* __restrict__ egrads,
     const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT, int maxU, int V,
-    int ldT, int uOff, int framesPerCta) {
-  __shared__ short sU[128];
-  __shared__ short sV[128];
-  __shared__ int sCount;
-  const int b = blockIdx.y, v0 = blockIdx.x * kVBlock;
-  const int T = min(inLens[b], maxT), Utot = min(labLens[b] + 1, maxU);
-  // the labelled positions of this launch's range: uOff + u, u < U - 1 in the code below
-  const int U = min(Utot - uOff, 129);
-  if (T <= 0 || U <= 1) return;
-  __shared__ int sLab[128];
-  int mine = -1;
-  if ((int)threadIdx.x < U - 1 && threadIdx.x < 128) mine = labels[(i64)b * (maxU - 1) + uOff + threadIdx.x];
-  if (threadIdx.x < 128) sLab[threadIdx.x] = mine;
-  // the normal case, decided by all threads at once: the block holds no more labels than are staged
-  if (__syncthreads_count(mine >= v0 && mine < v0 + kVBlock) <= kMaxStagedLabels) return;
-  if (threadIdx.x == 0) {
-    int n = 0;
-    for (int u = 0; u < U - 1 && u < 128; ++u) {
-      const int lab = sLab[u];
-      if (lab >= v0 && lab < v0 + kVBlock) {
-        if (n >= kMaxStagedLabels) {
-          sU[n - kMaxStagedLabels] = (short)u;
-          sV[n - kMaxStagedLabels] = (short)(lab - v0);
-        }
-        ++n;
-      }
+    int ldT, int uOff, int span, int framesPerCta) {
+  constexpr int kWords = (kMaxPos + 31) / 32;
+  __shared__ unsigned sMask[kWords];
+  __shared__ short sU[kMaxPos], sV[kMaxPos], sNext[kMaxPos];
+  __shared__ float sEm[kMaxPos][kOvfFrames + 1];
+  const int b = blockIdx.y, v0 = blockIdx.x * kVBlock, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int T = min(inLens[b], maxT), tBeg = blockIdx.z * framesPerCta, tEnd = min(T, tBeg + framesPerCta);
+  // the labelled positions of the launch's range: uOff + u, u < n
+  const int n = min(min(labLens[b] + 1, maxU) - 1 - uOff, span);
+  if (tBeg >= tEnd || n <= kMaxStagedLabels) return;
+  int any = 0;
+  for (int u = tid; u < 32 * kWords; u += 128) {
+    const int lab = u < n ? labels[(i64)b * (maxU - 1) + uOff + u] - v0 : -1;
+    const unsigned m = __ballot_sync(0xffffffffu, lab >= 0 && lab < kVBlock);
+    if (lane == 0) sMask[u >> 5] = m;
+    any += __popc(m);
+  }
+  if (__syncthreads_or(any) == 0) return;   // (most blocks of a large vocabulary: without a look at the masks)
+  int count = -kMaxStagedLabels;
+  for (int w = 0; w < kWords; ++w) count += __popc(sMask[w]);
+  if (count <= 0) return;
+  // the unstaged positions in position order
+  for (int u = tid; u < 32 * kWords; u += 128) {
+    if (!((sMask[u >> 5] >> (u & 31)) & 1u)) continue;
+    int rank = __popc(sMask[u >> 5] & ((1u << (u & 31)) - 1)) - kMaxStagedLabels;
+    for (int w = 0; w < (u >> 5); ++w) rank += __popc(sMask[w]);
+    if (rank >= 0) {
+      sU[rank] = (short)u;
+      sV[rank] = (short)(labels[(i64)b * (maxU - 1) + uOff + u] - v0);
     }
-    sCount = max(0, n - kMaxStagedLabels);
   }
   __syncthreads();
-  // a thread owns frames t = blockIdx.z * framesPerCta + thread + 256 j and applies the positions one
-  // after the other, so repeated labels are combined in position order
-  const int n = sCount;
-  for (int t = blockIdx.z * framesPerCta + threadIdx.x; t < min(T, (int)(blockIdx.z + 1) * framesPerCta); t += 256) {
-    TIO* row = egrads + ((i64)b * maxT + t) * V + v0;
-    for (int k = 0; k < n; ++k)
-      from_f32(row[sV[k]], to_f32(row[sV[k]]) - emT[((i64)b * maxU + uOff + sU[k]) * ldT + t]);
+  // those of my column, chained
+  int first = -1, last = -1;
+#pragma unroll 8
+  for (int k = 0; k < count; ++k)
+    if (sV[k] == tid) {
+      if (last < 0) first = k;
+      else sNext[last] = (short)k;
+      last = k;
+    }
+  if (last >= 0) sNext[last] = -1;
+  for (int t0 = tBeg; t0 < tEnd; t0 += kOvfFrames) {
+    const int frames = min(kOvfFrames, tEnd - t0);
+    float x[kOvfFrames];
+    TIO* col = egrads + ((i64)b * maxT + t0) * V + v0 + tid;
+    if (first >= 0) {
+#pragma unroll
+      for (int j = 0; j < kOvfFrames; ++j) x[j] = to_f32(col[(i64)min(j, frames - 1) * V]);
+    }
+#pragma unroll 8
+    for (int k = warp; k < count; k += 4)   // (frames beyond the last are not used)
+      sEm[k][lane] = emT[((i64)b * maxU + uOff + sU[k]) * ldT + min(t0 + lane, T - 1)];
+    __syncthreads();
+    if (first >= 0) {
+      for (int k = first; k >= 0; k = sNext[k]) {
+#pragma unroll
+        for (int j = 0; j < kOvfFrames; ++j) x[j] -= sEm[k][j];
+      }
+#pragma unroll
+      for (int j = 0; j < kOvfFrames; ++j)
+        if (j < frames) from_f32(col[(i64)j * V], x[j]);
+    }
+    __syncthreads();
   }
 }
 
@@ -736,7 +865,7 @@ TileCfg pick_tile(int Ku, int ldW, int N2, int passes, int staticSmem, bool bf =
 }
 
 template <int TB, bool ESPLIT, bool PSPLIT, bool BF = false>
-void launch_variant(const GradMaps& tm, GradParams p, TileCfg cfg, Dims d, cudaStream_t stream) {
+void launch_variant(const GradMaps& tm, GradParams p, TileCfg cfg, unsigned ctas, cudaStream_t stream) {
   const int eStage = e_stage_bytes(TB, BF);
   const int wStage = 2 * (p.ldW / 32) * TB * 128;
   p.stagesE = cfg.SE;
@@ -748,22 +877,27 @@ void launch_variant(const GradMaps& tm, GradParams p, TileCfg cfg, Dims d, cudaS
   size_t smem = (size_t)cfg.SE * eStage + (size_t)cfg.SW * wStage + 1024;
   if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it may hold all 512 TMEM columns
   allow_dyn_smem(grads_umma_kernel<TB, ESPLIT, PSPLIT, BF>, 227 * 1024 - kStaticSmemBound);
-  dim3 grid(div_up(d.V, kVBlock), d.B);
   ScopedKernel sk("grads_umma", stream);
-  grads_umma_kernel<TB, ESPLIT, PSPLIT, BF><<<grid, kGradThreads, smem, stream>>>(tm, p);
+  grads_umma_kernel<TB, ESPLIT, PSPLIT, BF><<<ctas, kGradThreads, smem, stream>>>(tm, p);
 }
 
 }  // namespace
 
 int grads_umma_ld_w(Dims d) { return (int)round_up64(d.maxU > 0 ? d.maxU : 1, 32); }
 int grads_umma_ld_t(Dims d) { return (int)round_up64(d.maxT > 0 ? d.maxT : 1, 4); }
+size_t grads_umma_partial_floats(Dims d) {
+  if (d.B <= 0 || d.maxT <= 0 || d.V <= 0) return 0;
+  const GradSplit s = grad_split(d);
+  return (size_t)s.cut * (s.parts > 1 ? s.parts : 0) * kMaxPos * kVBlock;
+}
 
 bool grads_umma_supported(const void* E, const void* P, const void* egrads,
                           const void* pgrads, Dims d, int passes) {
   const bool bf = d.dtype == kDtypeBf16;
   // (label axes of 129..256 positions: two launches, the second adding to egrads -- fp32 only,
   // a bf16 sum would be rounded twice)
-  if (d.V % (bf ? 8 : 4) != 0 || d.V < 32 || d.maxU < 1 || d.maxU > (bf ? 128 : 256) || d.B > 65535)
+  if (d.V % (bf ? 8 : 4) != 0 || d.V < 32 || d.maxU < 1 || d.maxU > (bf ? 128 : 256) || d.B > 65535 ||
+      grad_split(d).ctas() > 0x7fffffff)
     return false;
   if (bf && passes != 2) return false;   // one operand precision is built for bf16 storage
   // E and egrads are TMA operands (16-byte base); the column owners read P and write pgrads
@@ -780,7 +914,7 @@ void launch_grads_umma(const void* E, const void* P, const float* maxP, const fl
                        const float* emT, const float* nref, const float* ebl, const float* pBlank,
                        const float* pLabel, const int* labels, const float* deltas, void* egrads,
                        void* pgrads, const int* inLens, const int* labLens, Dims d, int passes,
-                       int* status, cudaStream_t stream) {
+                       float* partial, unsigned* tickets, int* status, cudaStream_t stream) {
   if (d.B <= 0 || d.V <= 0) return;
   const bool bf = d.dtype == kDtypeBf16;
   if (bf && passes != 2) throw std::invalid_argument("bf16 gradients are built for grad_passes = 2 only");
@@ -790,6 +924,10 @@ void launch_grads_umma(const void* E, const void* P, const float* maxP, const fl
   p.status = status;
   p.maxT = d.maxT; p.maxU = d.maxU; p.V = d.V; p.blank = d.blank;
   p.ldT = grads_umma_ld_t(d);
+  const GradSplit split = grad_split(d);
+  p.blocksV = div_up(d.V, kVBlock);
+  p.whole = (int)split.whole; p.parts = split.parts;
+  p.partial = partial; p.tickets = tickets;
   const uint64_t V = d.V, T = d.maxT, B = d.B, ldWall = grads_umma_ld_w(d), ldT = p.ldT, U = d.maxU;
   // one launch per range of 128 label positions (see GradParams::uOff)
   for (int uOff = 0; uOff < d.maxU; uOff += 128) {
@@ -816,13 +954,13 @@ void launch_grads_umma(const void* E, const void* P, const float* maxP, const fl
     tm.nref = make_tmap_f32_rows(nref, ldT, B, 1, ldT * 4, B * ldT * 4, TB);
     tm.ebl = make_tmap_f32_rows(ebl, ldT, B, 1, ldT * 4, B * ldT * 4, TB);
     tm.emT = make_tmap_f32_rows(emT, ldT, U, B, ldT * 4, U * ldT * 4, TB);
-#define GO(TBV, EV, PV) launch_variant<TBV, EV, PV>(tm, p, cfg, d, stream)
+#define GO(TBV, EV, PV) launch_variant<TBV, EV, PV>(tm, p, cfg, (unsigned)split.ctas(), stream)
 #define GO_TB(EV, PV) \
   do { if (TB == 64) GO(64, EV, PV); else if (TB == 48) GO(48, EV, PV); else GO(32, EV, PV); } while (0)
     if (bf) {
-      if (TB == 64) launch_variant<64, true, false, true>(tm, p, cfg, d, stream);
-      else if (TB == 48) launch_variant<48, true, false, true>(tm, p, cfg, d, stream);
-      else launch_variant<32, true, false, true>(tm, p, cfg, d, stream);
+      if (TB == 64) launch_variant<64, true, false, true>(tm, p, cfg, (unsigned)split.ctas(), stream);
+      else if (TB == 48) launch_variant<48, true, false, true>(tm, p, cfg, (unsigned)split.ctas(), stream);
+      else launch_variant<32, true, false, true>(tm, p, cfg, (unsigned)split.ctas(), stream);
     } else if (passes == 3) GO_TB(true, true);
     else if (passes == 2) GO_TB(true, false);
     else GO_TB(false, false);
@@ -834,14 +972,14 @@ void launch_grads_umma(const void* E, const void* P, const float* maxP, const fl
       ScopedKernel sk("label_overflow", stream);
       // (few vocabulary blocks: the kernel will have work -- spread the frames over more CTAs;
       // many blocks: almost every CTA returns at once -- keep them few)
-      const int framesPerCta = d.V <= 1024 ? 256 : 1024;
+      const int framesPerCta = d.V <= 1024 ? 2 * kOvfFrames : 1024;
       const dim3 grid(div_up(d.V, kVBlock), d.B, div_up(d.maxT, framesPerCta));
       if (bf)
-        label_overflow_kernel<bf16><<<grid, 256, 0, stream>>>(
-            labels, emT, static_cast<bf16*>(egrads), inLens, labLens, d.maxT, d.maxU, d.V, p.ldT, uOff, framesPerCta);
+        label_overflow_kernel<bf16><<<grid, kVBlock, 0, stream>>>(
+            labels, emT, static_cast<bf16*>(egrads), inLens, labLens, d.maxT, d.maxU, d.V, p.ldT, uOff, n, framesPerCta);
       else
-        label_overflow_kernel<float><<<grid, 256, 0, stream>>>(
-            labels, emT, static_cast<float*>(egrads), inLens, labLens, d.maxT, d.maxU, d.V, p.ldT, uOff, framesPerCta);
+        label_overflow_kernel<float><<<grid, kVBlock, 0, stream>>>(
+            labels, emT, static_cast<float*>(egrads), inLens, labLens, d.maxT, d.maxU, d.V, p.ldT, uOff, n, framesPerCta);
       TB200_CHECK_LAUNCH();
     }
   }

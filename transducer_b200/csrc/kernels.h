@@ -127,11 +127,14 @@ bool grads_umma_supported(const void* E, const void* P, const void* egrads,
                           const void* pgrads, Dims d, int passes);
 // E, P, egrads and pgrads are of d.dtype (bf16: passes = 2 only, label axes up to 128; fp32:
 // label axes up to 256 positions, those above 128 as two launches over halves of the axis).
+// partial: scratch of grads_umma_partial_floats(d) floats; tickets: kGradTickets zeros, left zero.
+constexpr int kGradTickets = 148;   // one per SM
+size_t grads_umma_partial_floats(Dims d);
 void launch_grads_umma(const void* E, const void* P, const float* maxP, const float* W,
                        const float* emT, const float* nref, const float* ebl, const float* pBlank,
                        const float* pLabel, const int* labels, const float* deltas, void* egrads,
                        void* pgrads, const int* inLens, const int* labLens, Dims d, int passes,
-                       int* status, cudaStream_t stream);
+                       float* partial, unsigned* tickets, int* status, cudaStream_t stream);
 
 // ---- lattice_sweep.cu ------------------------------------------------------------
 // Sweeps for label axes of at most 256 positions (file comment there).  Lattices are skewed:
@@ -161,6 +164,7 @@ struct SweepScratch {   // of the backward call
   float2* F;         // [B,stride]
   float* g;          // [B,stride]
   unsigned* ticket;  // [B]
+  unsigned* gradTickets;  // [kGradTickets], zeroed for launch_grads_umma
   float* partial;    // sweep_partial_floats(d)
 };
 size_t sweep_partial_floats(Dims d);

@@ -486,15 +486,19 @@ __global__ void __launch_bounds__(32) alpha_natural_kernel(
 // per 4 diagonals.  Bound by memory: a pair and an alpha (12 bytes) read, 8
 // written per node.
 constexpr int kFactorRows = 4, kFactorWarps = 8;
+static_assert(kGradTickets <= 32 * kFactorWarps, "one thread per ticket");
 template <int NPL>
 __global__ void __launch_bounds__(32 * kFactorWarps) gamma_factors_kernel(
     const float2* __restrict__ arcs, const float* __restrict__ alphas,
     const float* __restrict__ deltas, const NaturalTerms n, float2* __restrict__ F,
-    unsigned* __restrict__ occTicket, i64 stride, int nBlk, const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT,
+    unsigned* __restrict__ occTicket, unsigned* __restrict__ gradTickets, i64 stride, int nBlk, const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT,
     int maxU) {
   constexpr int ld = 32 * NPL, kPieces = NPL / 2;
   const int b = blockIdx.y, lane = threadIdx.x & 31;
-  if (blockIdx.x == 0 && threadIdx.x == 0) occTicket[b] = 0u;
+  if (blockIdx.x == 0) {   // the counters of the kernels behind this one
+    if (threadIdx.x == 0) occTicket[b] = 0u;
+    if (b == 0 && threadIdx.x < kGradTickets) gradTickets[threadIdx.x] = 0u;
+  }
   const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU), S = T + U - 1;
   const int d0 = (blockIdx.x * kFactorWarps + (threadIdx.x >> 5)) * kFactorRows, u0 = NPL * lane;
   if (T <= 0 || U <= 0 || d0 >= S || u0 >= U) return;
@@ -1111,7 +1115,7 @@ void launch_sweep_backward(const SweepScratch& w, const float* P, const float* b
     const dim3 grid(div_up(g.nDiag, kFactorRows * kFactorWarps), d.B);
 #define CALL(NPL)                                                                              \
   gamma_factors_kernel<NPL><<<grid, 32 * kFactorWarps, 0, stream>>>(                           \
-      arcs, alphas, alphaDeltas, n, w.F, w.ticket, g.stride, g.nBlk, inLens, labLens, d.maxT, d.maxU)
+      arcs, alphas, alphaDeltas, n, w.F, w.ticket, w.gradTickets, g.stride, g.nBlk, inLens, labLens, d.maxT, d.maxU)
     const NaturalTerms n{P, blankEmissions, labels, d.V, d.blank};
     TB200_BY_NPL(g.npl, CALL);
 #undef CALL
