@@ -31,7 +31,7 @@
 //           The stage also carries the tile's sparse-term rows (blank-arc sums, label-arc
 //           occupancies of the labels that fall into this column block).
 //   W ring  the two copies of the W tile; released by the two GEMMs alone.
-// Roles (20 warps): 8 column-owner warps of the exp group (TMEM lane quarter x frame half;
+// Roles (20 warps): 8 column-owner warps of the exp group (TMEM lane quarter x even / odd tiles;
 // raw E -> exp(E - ref) in TMEM), 8 column-owner warps of the gradient group (D1 x exponentials
 // from TMEM - sparse terms -> the gradient, into the E stage), a mover warp (fills E stages,
 // stores finished tiles and refills the stage at once), a W loader warp, and one MMA-issuing
@@ -206,6 +206,11 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
   constexpr int kRowBytes = TB * 4;            // one row of per-frame scalars
   constexpr int kRowStride = row_stride_bytes(TB);  // TMA destinations are 128-byte aligned
   constexpr int kEStage = e_stage_bytes(TB, BF);   // E tile + kStageRows rows of scalars
+  // Do the two halves of a group of column owners take alternate tiles, or halves of every tile?
+  // Alternate where the ring and both pairs of tensor-memory operands make every tile of a half find
+  // its own ring slots and copies (all even); operand precision 3 leaves less.
+  const bool alt = SE == 4 && p.eBufs == 2 && p.dBufs == 2;
+  const int owners = alt ? kGroupWarps / 2 : kGroupWarps;   // warps of a group per tile
   const int wBytes = nUB * kBoxBytes;
   const int wStage = 2 * wBytes;               // K-major copy, MN-major copy
   uint8_t* smemW = smem + (size_t)SE * kEStage;
@@ -231,17 +236,17 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
     sSplit[2] = parts;
     for (int s = 0; s < SE; ++s) {
       mbar_init(&barEFull[s], 1);
-      mbar_init(&barStore[s], kGroupWarps);   // gradient tile complete in shared memory
+      mbar_init(&barStore[s], owners);        // gradient tile complete in shared memory
     }
     for (int s = 0; s < SW; ++s) {
       mbar_init(&barWFull[s], 1);
       mbar_init(&barWFree[s], 2);             // both MMA issuers done with it
     }
     for (int s = 0; s < 2; ++s) {
-      mbar_init(&barEReady[s], kGroupWarps);
-      mbar_init(&barE2Free[s], 1 + kGroupWarps);  // GEMM2 done with it + gradient warps have read it
+      mbar_init(&barEReady[s], owners);
+      mbar_init(&barE2Free[s], 1 + owners);   // GEMM2 done with it + gradient warps have read it
       mbar_init(&barD1Full[s], 1);
-      mbar_init(&barD1Free[s], kGroupWarps);
+      mbar_init(&barD1Free[s], owners);
     }
     mbar_init(&barPReady, 2 * kGroupWarps);
     mbar_init(&barD2Done, 1);
@@ -471,8 +476,12 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
     // Thread (q, lane) owns vocabulary column v0 + q*32 + lane = TMEM lane q*32 + lane.  Two
     // groups of 8 warps: group 0 turns raw E into exp(E - ref) (shared memory in place + TMEM),
     // group 1 turns that into the gradient, so tile i+1's exponentials overlap tile i's
-    // gradient arithmetic.  Within a group the halves h = 0,1 split the frames of a tile; all
-    // 16 warps split the label positions of the prologue and the epilogue.
+    // gradient arithmetic.  Within a group the halves h = 0,1 take alternate tiles (or, see `alt`, split
+    // the frames of a tile): half of what a tile costs a warp are round trips to barriers and to
+    // tensor memory, ~1200 cycles whatever the frames (cycle stamps; without any copy to or from memory
+    // and without most of the MMAs the kernel was as slow).  Measured: B = 32, T = 1500..2000, U' = 61..101,
+    // V = 10000 1086 -> 1082 us, bf16 996 -> 972, B = 64, U' = 76..151, V = 4096 958 -> 947.  All 16 warps split the label positions
+    // of the prologue and the epilogue.
     const int grp = warp >> 3, q = warp & 3, h = (warp >> 2) & 1;
     const int share = grp * 2 + h;  // 0..3: of the prologue / epilogue
     const int vl = q * 32 + lane;
@@ -520,14 +529,13 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
       return reinterpret_cast<TIO*>(col + t * 128 + ((chunk ^ (t & 7)) << 4));
     };
 
+    const int first = alt ? h : 0, step = alt ? 2 : 1;                 // my tiles
+    const int hBeg = alt ? 0 : h, hEnd = alt ? 2 : h + 1;              // my halves of their frames
     if (grp == 0) {
       // ---- exp group: raw E -> exp(E - ref), in place, and into TMEM as GEMM2's A operand ----
-      int se = 0, eb = 0;          // E stage and expE^T copy of tile i
+      int se = first, eb = first;  // E stage and expE^T copy of tile i
       uint32_t sph = 0, eph = 0;   // and their phases
-      for (int i = 0; i < nTiles && ok; ++i) {
-        const int t0 = (tile0 + i) * TB;
-        // live frames in my half (may be <= 0); none for a column beyond the vocabulary
-        const int tValid = vOk ? min(TB, T - t0) - h * TBH : 0;
+      for (int i = first; i < nTiles && ok; i += step) {
         ok = mbar_wait(&barEFull[se], sph, abortp, p.status, kStatusTimeoutTma);
         if (ok && i >= EB)  // this copy of expE^T must have been consumed by GEMM2
           ok = mbar_wait(&barE2Free[eb], eph ^ 1u, abortp, p.status, kStatusTimeoutMma);
@@ -536,43 +544,46 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
         tc_fence_after();
         uint8_t* stE = smem + (size_t)se * kEStage;
         uint8_t* col = stE + colOff;
-        const float* nr = reinterpret_cast<const float*>(stE + kEBytes) + h * TBH;
-        const uint32_t cEhi = cE + eb * kECols + h * TBH, cElo = cEhi + TB;
-        float xs[TBH];
+#pragma unroll 1
+        for (int hh = hBeg; hh < hEnd; ++hh) {
+          // live frames in this half (may be <= 0); none for a column beyond the vocabulary
+          const int tValid = vOk ? min(TB, T - (tile0 + i) * TB) - hh * TBH : 0;
+          const float* nr = reinterpret_cast<const float*>(stE + kEBytes) + hh * TBH;
+          const uint32_t cEhi = cE + eb * kECols + hh * TBH, cElo = cEhi + TB;
+          float xs[TBH];
 #pragma unroll
-        for (int j = 0; j < TBH; j += 4) {
-          const float4 sh = *reinterpret_cast<const float4*>(nr + j);
-          const float shj[4] = {sh.x, sh.y, sh.z, sh.w};
+          for (int j = 0; j < TBH; j += 4) {
+            const float4 sh = *reinterpret_cast<const float4*>(nr + j);
+            const float shj[4] = {sh.x, sh.y, sh.z, sh.w};
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int t = h * TBH + j + k;
-            xs[j + k] = fmaf(to_f32(*elemAt(col, t)), kLog2e, shj[k]);
+            for (int k = 0; k < 4; ++k)
+              xs[j + k] = fmaf(to_f32(*elemAt(col, hh * TBH + j + k)), kLog2e, shj[k]);
           }
-        }
-        if (tValid < TBH) {  // last tile of the utterance (or a column beyond the vocabulary):
-#pragma unroll             // frames at or beyond T_b contribute nothing, exp2(-inf) = 0
-          for (int j = 0; j < TBH; ++j)
-            if (j >= tValid) xs[j] = -INFINITY;
-        }
-#pragma unroll
-        for (int c = 0; c < TBH; c += 8) {
-          uint32_t hi[8], lo[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float x = ex2_approx(xs[c + j]);
-            if (ESPLIT) split_tf32(x, hi[j], lo[j]);
-            else hi[j] = __float_as_uint(tf32_round(x));
+          if (tValid < TBH) {  // last tile of the utterance (or a column beyond the vocabulary):
+#pragma unroll               // frames at or beyond T_b contribute nothing, exp2(-inf) = 0
+            for (int j = 0; j < TBH; ++j)
+              if (j >= tValid) xs[j] = -INFINITY;
           }
-          tmem_st8(tBase + laneAddr + cEhi + c, hi);
-          if (ESPLIT) tmem_st8(tBase + laneAddr + cElo + c, lo);
+#pragma unroll
+          for (int c = 0; c < TBH; c += 8) {
+            uint32_t hi[8], lo[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const float x = ex2_approx(xs[c + j]);
+              if (ESPLIT) split_tf32(x, hi[j], lo[j]);
+              else hi[j] = __float_as_uint(tf32_round(x));
+            }
+            tmem_st8(tBase + laneAddr + cEhi + c, hi);
+            if (ESPLIT) tmem_st8(tBase + laneAddr + cElo + c, lo);
+          }
         }
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
         // exp(E - ref) of the tile is in TMEM and the raw tile in shared memory is dead
         if (lane == 0) mbar_arrive(&barEReady[eb]);
-        if (++se == SE) { se = 0; sph ^= 1u; }
-        if (++eb == EB) { eb = 0; eph ^= 1u; }
+        if ((se += step) >= SE) { se -= SE; sph ^= 1u; }
+        if ((eb += step) >= EB) { eb -= EB; eph ^= 1u; }
       }
     } else {
       // ---- gradient group: egrads tile = expE * D1 - sparse (delta_b is inside W and the rows) ----
@@ -582,64 +593,64 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
       unsigned stagedMine = 0;
       for (int k = 0; k < nStaged; ++k)
         if (sListV[k] == vl) stagedMine |= 1u << k;
-      int se = 0, eb = 0, db = 0;            // E stage, expE^T copy and D1 copy of tile i
-      uint32_t sph = 0, eph = 0, dph = 0;    // and their phases
-      for (int i = 0; i < nTiles && ok; ++i) {
-        const int t0 = (tile0 + i) * TB;
-        const int tValid = vOk ? min(TB, T - t0) - h * TBH : 0;
+      int se = first, eb = first, db = first;  // E stage, expE^T copy and D1 copy of tile i
+      uint32_t sph = 0, eph = 0, dph = 0;      // and their phases
+      for (int i = first; i < nTiles && ok; i += step) {
         ok = mbar_wait(&barEFull[se], sph, abortp, p.status, kStatusTimeoutTma) &&
              mbar_wait(&barD1Full[db], dph, abortp, p.status, kStatusTimeoutMma) &&
              mbar_wait(&barEReady[eb], eph, abortp, p.status, kStatusTimeoutOperand);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        // expE * D1, both from tensor memory (expE = hi + lo exactly)
-        const uint32_t cEhi = cE + eb * kECols + h * TBH, cElo = cEhi + TB;
-        float d1[TBH];
-#pragma unroll
-        for (int c = 0; c < TBH; c += 8) {
-          uint32_t r[8], xh[8], xl[8];
-          tmem_ld8(tBase + laneAddr + cD1 + db * TB + h * TBH + c, r);
-          tmem_ld8(tBase + laneAddr + cEhi + c, xh);
-          if (ESPLIT) tmem_ld8(tBase + laneAddr + cElo + c, xl);
-          tmem_wait_ld();
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            float x = __uint_as_float(xh[j]);
-            if (ESPLIT) x += __uint_as_float(xl[j]);
-            d1[c + j] = x * __uint_as_float(r[j]);
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(&barD1Free[db]);
-          mbar_arrive(&barE2Free[eb]);
-        }
         uint8_t* stE = smem + (size_t)se * kEStage;
         uint8_t* col = stE + colOff;
-        const float* rows = reinterpret_cast<const float*>(stE + kEBytes + kRowStride) + h * TBH;
-        if (v == p.blank && !p.accumulate) {
+#pragma unroll 1
+        for (int hh = hBeg; hh < hEnd; ++hh) {
+          // expE * D1, both from tensor memory (expE = hi + lo exactly)
+          const uint32_t cEhi = cE + eb * kECols + hh * TBH, cElo = cEhi + TB;
+          float d1[TBH];
 #pragma unroll
-          for (int j = 0; j < TBH; ++j) d1[j] -= rows[j];
-        }
-        for (unsigned m0 = stagedMine; m0; m0 &= m0 - 1) {
-          const float* m = rows + (1 + (__ffs(m0) - 1)) * (kRowStride / 4);
+          for (int c = 0; c < TBH; c += 8) {
+            uint32_t r[8], xh[8], xl[8];
+            tmem_ld8(tBase + laneAddr + cD1 + db * TB + hh * TBH + c, r);
+            tmem_ld8(tBase + laneAddr + cEhi + c, xh);
+            if (ESPLIT) tmem_ld8(tBase + laneAddr + cElo + c, xl);
+            tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < TBH; ++j) d1[j] -= m[j];
-        }
+            for (int j = 0; j < 8; ++j) {
+              float x = __uint_as_float(xh[j]);
+              if (ESPLIT) x += __uint_as_float(xl[j]);
+              d1[c + j] = x * __uint_as_float(r[j]);
+            }
+          }
+          if (hh == hEnd - 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+              mbar_arrive(&barD1Free[db]);
+              mbar_arrive(&barE2Free[eb]);
+            }
+          }
+          const float* rows = reinterpret_cast<const float*>(stE + kEBytes + kRowStride) + hh * TBH;
+          if (v == p.blank && !p.accumulate) {
 #pragma unroll
-        for (int j = 0; j < TBH; ++j) {
-          const int t = h * TBH + j;
+            for (int j = 0; j < TBH; ++j) d1[j] -= rows[j];
+          }
+          for (unsigned m0 = stagedMine; m0; m0 &= m0 - 1) {
+            const float* m = rows + (1 + (__ffs(m0) - 1)) * (kRowStride / 4);
+#pragma unroll
+            for (int j = 0; j < TBH; ++j) d1[j] -= m[j];
+          }
           // (frames at or beyond T_b: expE and the rows of W are zero there, so is d1)
-          from_f32(*elemAt(col, t), d1[j]);
+#pragma unroll
+          for (int j = 0; j < TBH; ++j) from_f32(*elemAt(col, hh * TBH + j), d1[j]);
         }
         fence_proxy_async_smem();  // the tile is read next by TMA stores
         __syncwarp();
         if (lane == 0) mbar_arrive(&barStore[se]);  // my part of the gradient tile is in place
-        if (++se == SE) { se = 0; sph ^= 1u; }
-        if (++eb == EB) { eb = 0; eph ^= 1u; }
-        if (++db == DB) { db = 0; dph ^= 1u; }
+        if ((se += step) >= SE) { se -= SE; sph ^= 1u; }
+        if ((eb += step) >= EB) { eb -= EB; eph ^= 1u; }
+        if ((db += step) >= DB) { db -= DB; dph ^= 1u; }
       }
     }
 
