@@ -99,7 +99,7 @@ struct SavedState {
       alphas = c.take<float>(B * g.stride);
       arcs = c.take<float2>(B * g.stride);
       LN = c.take<float>(B * d.maxT * d.maxU);
-      deltas = c.take<float>(B * g.nBlk);
+      deltas = c.take<float>(B * std::max(g.nBlk, 2));   // (costs alone: an offset per half)
     } else {
       const SkewGeom g = skew_geom(d);
       alphas = c.take<float>(B * g.stride);

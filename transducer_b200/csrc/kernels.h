@@ -144,7 +144,7 @@ struct SweepGeom {
   int npl;      // adjacent label positions per lane of a sweep
   int ld;       // positions per anti-diagonal row, 32 * npl
   int nDiag;    // rows per utterance
-  int nBlk;     // blocks of 16 rows and one: entries of `deltas` per utterance
+  int nBlk;     // blocks of 16 rows: entries of `deltas` per utterance
   i64 stride;   // ld * nDiag
 };
 SweepGeom sweep_geom(Dims d);
@@ -152,9 +152,9 @@ SweepGeom sweep_geom(Dims d);
 // are recomputed in place first, exactly), alphas, costs [B] (+inf for an empty utterance) and, if
 // lossSum is not null, their sum in index order.  ELrow [B,maxU,maxT] and ebl [B,maxT]: label and
 // blank emissions as written by launch_lognorm_umma, or both null, and they are gathered from E.
-// E and P are of d.dtype.  ticket (with lossSum) and halves [B]: zeros.  score: no backward call will
-// follow.  For the backward call: arcs and alphas [B,stride], deltas [B,nBlk] and,
-// for axes of more than 128 positions, ebl (written here where it is not an input).
+// E and P are of d.dtype.  ticket (with lossSum) and halves [B]: zeros.  For the backward call: arcs and
+// alphas [B,stride], deltas [B,nBlk] and, for axes of more than 128 positions, ebl (written here where
+// it is not an input).  score: no backward call will follow; alphas and deltas are scratch then.
 void launch_sweep_forward(const void* E, const void* P, float* LN, const float* ELrow,
                           float* ebl, float2* arcs, float* alphas, float* deltas, float* costs,
                           float* lossSum, unsigned* ticket, unsigned* halves, const int* labels,

@@ -3,44 +3,46 @@
 // the whole GPU.
 //
 //   sweep_prep       arc log-probabilities of every node (log2 units), skewed
-//   alpha_sweep      alpha and beta recursions up to the middle               (forward call)
-//   gamma_factors    2^(alpha + arc - alpha'), 2^(arc + beta' - beta)         (backward call)
-//   gamma_sweep      occupancy recursions from the middle: two products and a sum per node
+//   alpha_sweep      alpha recursion                                          (forward call)
+//   score_sweep      costs alone: alpha and beta recursions up to the middle  (score call)
+//   gamma_factors    2^(alpha + arc - alpha') of every arc                    (backward call)
+//   gamma_sweep      occupancy recursion: two products and a sum per node
 //   occupancy        the operands of the gradient kernels
 //
 //   alpha   transducer/transducer_cpu.cpp:30-79   (transducer_cuda.cu:32-97)
 //   reverse transducer/transducer_cpu.cpp:81-143  (transducer_cuda.cu:99-176)
 //
+// Axes of up to 128 positions run on rebased base-2 logarithms (alpha_sweep_kernel); longer ones
+// (NPL >= 5, "natural" below) on natural logarithms at full magnitude, in the operation order of the
+// block-wide kernels of lattice.cu (costs bit-identical to theirs: 18 shapes, T = 77..5000,
+// U' = 129..256).
+//
 // Diagonal d = t + u of an utterance is one row of ld = 32 NPL numbers; lane l of a sweep owns the
 // NPL adjacent positions u = NPL l + r.  All nodes of a diagonal are independent; the one value
 // per lane that crosses from the neighbouring lane arrives by a warp shuffle.  A sweep is a chain
-// of dependent diagonals whatever the batch, so what counts is how many they are and how few
-// instructions each takes.
-//
-// FROM BOTH ENDS.  Every path crosses each of the S = T + U - 1 diagonals once, so with alpha (all paths
-// to a node) up to the middle diagonal M and beta (all paths from a node) down to it, the total is
-// the sum over M of alpha beta, and the occupancy of a node of M is its share of that sum.  From there
-// the occupancies spread to both ends: towards the start by the share of each node's inflow that came
-// over an arc (from the alphas, as the reference does all the way), towards the end by the share of its
-// outflow that leaves over an arc (from the betas).  The shares of a node add up to one to within a
-// rounding either way, so neither half drifts.  The two halves are two warps that know nothing of each
-// other, and both chains are half as long as from one end.
-//
-// Operands are brought to shared memory by cp.async, each lane copying just the
+// of T + U - 1 dependent diagonals whatever the batch, so what counts is how few instructions a
+// diagonal takes: operands are brought to shared memory by cp.async, each lane copying just the
 // 8 NPL bytes a row that it reads itself (no barrier, no other warp), several blocks of 16
 // diagonals ahead, and the loop holds nothing but the recursion and its store.
+// Measured (T = 2000, U' = 101, device time, B = 8 / 32): alpha 132 us (147 with bulk copies issued and
+// waited for by the sweeping warp); reverse sweep 12 / 27 us for the factors + 60 us for the recursion
+// (152 us when helper warps of the same CTA prepared the factors and carried away the results).
+// B = 64, T = 750..1500, U' = 151: alpha 195 us, factors 65 + recursion 76 us, operands 105 us, against
+// 384, 512 and (lattices re-laid out twice) 168 us of the block-wide kernels, which take a barrier
+// per diagonal.  B = 8, T = 4000, U' = 251: alpha 855 us, block-wide 954.
 //
-// Measured (T = 2000, U' = 101, B = 8 and 32 alike): alpha sweep 132 -> 76 us, reverse sweep 60 -> 37 us
-// against one warp from one end.
-//
-// Axes of up to 128 positions run like that, on rebased base-2 logarithms; longer ones (NPL >= 5) too where
-// only the costs are wanted (scoring, B = 64, T = 500..1000, U' = 101..201: 242 -> 71 us).  With gradients
-// to follow they keep to the reference's form ("natural" below): one warp from one end, natural logarithms
-// at full magnitude, in the operation order of the block-wide kernels of lattice.cu (costs bit-identical to
-// theirs: 18 shapes, T = 77..5000, U' = 129..256).  At a magnitude of 1e4 the rounding of an alpha is
-// 1e-3, and the gradients carry it: any other order of these operations moves them by as much (rel
-// 1.3e-3 between this form and the sweeps from both ends, which are the ones closer to float64), more than
-// this path's results are to move.
+// COSTS ALONE.  Every path crosses each of the S = T + U - 1 diagonals once, so with alpha (all paths to a
+// node) up to the middle diagonal M and beta (all paths from a node) down to it, the total is the sum
+// over M of alpha beta.  The two halves are two warps that know nothing of each other, both chains are
+// half as long, nothing but their ends is stored, and every label axis runs on rebased logarithms.  B = 64,
+// T = 500..1000, U' = 101..201: 242 -> 71 us.
+// With gradients to follow each recursion keeps to one warp from one end.  The weights W of the gradient
+// products are rounded to TF32 behind the sweeps, and any other order of operations in front of that
+// rounding flips some of them by one step, 2^-10 of a weight near one.  Where a blank is nearly certain
+// its gradient is the small difference of two occupancies, and the flip shows: blank emissions raised by 4,
+// entries differed by up to 3.3e-2 of the larger of themselves and the rms (4.74e-5 at B = 20, where
+// 2^-10 / B is 4.88e-5), while the whole gradient differed by 3e-5 to 1e-4.  (Both sweeps took 113 us
+// instead of 192 us so, at T = 2000, U' = 101.)
 #include <algorithm>
 
 #include "kernels.h"
@@ -138,14 +140,104 @@ __device__ __forceinline__ void finish_cost(float* costs, int b, float cost, int
 // subtracts it at the same point of the same sum.  The loss and the gradients then sit ~1e-4 from
 // the float64 result.
 //
-// The betas are rebased likewise, in blocks of 16 from the end; beta of diagonal d is stored in row d + 1,
-// behind the alphas (row M holds alpha, row M + 1 beta of the middle diagonal).  deltas of an utterance:
-// [0] the alphas' offset at M, [k] of the alphas' block k, [nBlk - 1 - k] of the betas' block k,
-// [nBlk - 1] the betas' offset at M.
-//
 // The pace is set by the special-function unit: NPL ex2 and NPL lg2 per diagonal, 8 issue cycles
 // each, in a chain.  (Cutting the label axis over two or four warps that run a block apart was
 // measured and is slower: every node then waits for a shuffle.)
+template <int NPL>
+__global__ void __launch_bounds__(32) alpha_sweep_kernel(
+    const float2* __restrict__ arcs, float* __restrict__ costs, float* __restrict__ alphas,
+    float* __restrict__ deltas, i64 stride, int nDiag, const int* __restrict__ inLens,
+    const int* __restrict__ labLens, int B, int maxT, int maxU, float* lossSum, unsigned* ticket) {
+  constexpr int ld = 32 * NPL;
+  extern __shared__ __align__(128) uint8_t smemA[];
+  const int b = blockIdx.x, lane = threadIdx.x;
+  const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
+  if (T <= 0 || U <= 0) {
+    if (lane == 0) finish_cost(costs, b, pos_inf(), B, lossSum, ticket);
+    return;
+  }
+  const int S = T + U - 1, nBlocks = (S + kDiag - 1) / kDiag, u0 = NPL * lane;
+  constexpr int kRing = ring_blocks(NPL);
+  PairRing<NPL> ring(smemA, arcs + (i64)b * stride, lane, U, kNoArcBits, kNoArcBits);
+  auto issue = [&](int k) { ring.issue(k % kRing, (i64)k * kDiag, k < nBlocks ? min(kDiag, S - k * kDiag) : 0); };
+#pragma unroll
+  for (int k = 0; k < kRing - 1; ++k) issue(k);
+  float* al = alphas + (i64)b * stride;
+  float* dl = deltas + (i64)b * ((nDiag + kDiag - 1) / kDiag);
+  const float kNone = __uint_as_float(kNoArcBits);
+  float stayIn[NPL], stepOut[NPL];
+#pragma unroll
+  for (int r = 0; r < NPL; ++r) stayIn[r] = stepOut[r] = kNone;
+  if (lane == 0) stayIn[0] = 0.0f;  // alpha(0,0) = 0
+  float up = kNone;        // stepOut of the lane below's last position, one diagonal back
+  float offset = 0.0f;     // sum of the deltas so far: an integer, exact in fp32
+  float nextDelta = 0.0f;  // by how much the state is lowered at the start of the next block
+  for (int k = 0; k < nBlocks; ++k) {
+    issue(k + kRing - 1);
+    if (k > 0) {
+      // rebase (entries of nodes outside the lattice are ~ -6e29 and stay there)
+#pragma unroll
+      for (int r = 0; r < NPL; ++r) {
+        stayIn[r] -= nextDelta;
+        stepOut[r] -= nextDelta;
+      }
+      up -= nextDelta;
+      offset += nextDelta;
+      if (lane == 0) dl[k] = nextDelta;
+    }
+    // The delta applied at the start of the NEXT block is the floor of the largest entry of
+    // the state now, at the start of this one: the warp-wide maximum then has a whole block to
+    // arrive, off the dependent chain.  (By then the state has sunk by another 16 arcs.)
+    {
+      float m = kNone;
+#pragma unroll
+      for (int r = 0; r < NPL; ++r) m = fmaxf(m, fmaxf(stayIn[r], stepOut[r]));
+      nextDelta = (float)__reduce_max_sync(0xffffffffu, __float2int_rd(fmaxf(m, -1.0e9f)));
+    }
+    ring.wait();
+    const int slot = k % kRing, nd = min(kDiag, S - k * kDiag);
+    float* out = al + (i64)k * kDiag * ld;
+    auto diag = [&](int i) {
+      float fx[NPL], fy[NPL], left[NPL], m[NPL], e[NPL], a[NPL];
+      ring.read(slot, i, fx, fy);
+      // The last position first: its result feeds the shuffle of the next diagonal; position 0
+      // last: it waits for the shuffle of this one.  (A warp issues in order.)
+      left[0] = lane ? up : kNone;
+#pragma unroll
+      for (int r = 1; r < NPL; ++r) left[r] = stepOut[r - 1];
+#pragma unroll
+      for (int r = NPL - 1; r >= 0; --r) {
+        m[r] = fmaxf(left[r], stayIn[r]);
+        e[r] = ex2_approx(-fabsf(left[r] - stayIn[r]));
+      }
+#pragma unroll
+      for (int r = NPL - 1; r >= 0; --r) {
+        a[r] = m[r] + lg2_approx(1.0f + e[r]);
+        stayIn[r] = a[r] + fx[r];
+        stepOut[r] = a[r] + fy[r];
+        if (r == NPL - 1) up = __shfl_up_sync(0xffffffffu, stepOut[NPL - 1], 1);
+      }
+      if (ring.act) store_row<NPL>(out + i * ld, lane, a);
+    };
+    if (nd == kDiag) {
+#pragma unroll
+      for (int i = 0; i < kDiag; ++i) diag(i);
+    } else {
+#pragma unroll 1
+      for (int i = 0; i < nd; ++i) diag(i);
+    }
+  }
+  ring.drain();
+  // the last diagonal holds only the terminal node (T-1, U-1); its blank arc ends the path
+#pragma unroll
+  for (int r = 0; r < NPL; ++r)
+    if (u0 + r == U - 1) finish_cost(costs, b, -(stayIn[r] + offset) * kLn2F, B, lossSum, ticket);
+}
+
+// ---------------------------------------------------------------------------
+// costs alone
+// ---------------------------------------------------------------------------
+// (rebased like alpha_sweep_kernel; the betas in blocks of 16 from the end)
 __device__ __forceinline__ float lse2_log2(float a, float b) {
   return fmaxf(a, b) + lg2_approx(1.0f + ex2_approx(-fabsf(a - b)));
 }
@@ -155,11 +247,10 @@ __device__ __forceinline__ float next_delta(float m) {
   return (float)__reduce_max_sync(0xffffffffu, __float2int_rd(fmaxf(m, -1.0e9f)));
 }
 
-// alpha of the diagonals 0..M; returns the offset of M
+// alpha of the middle diagonal M into `row`; returns its offset
 template <int NPL>
-__device__ __forceinline__ float alpha_half(uint8_t* smem, const float2* arcs, float* al, float* dl,
-                                            int lane, int U, int M) {
-  constexpr int ld = 32 * NPL, kRing = ring_blocks(NPL);
+__device__ __forceinline__ float alpha_half(uint8_t* smem, const float2* arcs, float* row, int lane, int U, int M) {
+  constexpr int kRing = ring_blocks(NPL);
   const int nBlocks = M / kDiag;
   PairRing<NPL> ring(smem, arcs, lane, U, kNoArcBits, kNoArcBits);
   auto issue = [&](int k) { ring.issue(k % kRing, (i64)k * kDiag, k < nBlocks ? kDiag : 0); };
@@ -184,14 +275,12 @@ __device__ __forceinline__ float alpha_half(uint8_t* smem, const float2* arcs, f
       }
       up -= nextDelta;
       offset += nextDelta;
-      if (lane == 0) dl[k] = nextDelta;
     }
-    float* out = al + (i64)k * kDiag * ld;
     if (k == nBlocks) {   // the middle diagonal: nothing leaves it here
       float a[NPL];
 #pragma unroll
       for (int r = 0; r < NPL; ++r) a[r] = lse2_log2(r ? stepOut[(r + NPL - 1) % NPL] : lane ? up : kNone, stayIn[r]);
-      if (ring.act) store_row<NPL>(out, lane, a);
+      if (ring.act) store_row<NPL>(row, lane, a);
       break;
     }
     // The delta applied at the start of the NEXT block is the floor of the largest entry of
@@ -226,18 +315,17 @@ __device__ __forceinline__ float alpha_half(uint8_t* smem, const float2* arcs, f
         stepOut[r] = a[r] + fy[r];
         if (r == NPL - 1) up = __shfl_up_sync(0xffffffffu, stepOut[NPL - 1], 1);
       }
-      if (ring.act) store_row<NPL>(out + i * ld, lane, a);
     }
   }
   ring.drain();
   return offset;
 }
 
-// beta of the diagonals S-1 down to M, that of d in row d + 1; returns the offset of M
+// beta of the middle diagonal into `row`, from the end; returns its offset
 template <int NPL>
-__device__ __forceinline__ float beta_half(uint8_t* smem, const float2* arcs, float* al, float* dlEnd,
-                                           int lane, int U, int S, int M) {
-  constexpr int ld = 32 * NPL, kRing = ring_blocks(NPL);
+__device__ __forceinline__ float beta_half(uint8_t* smem, const float2* arcs, float* row, int lane, int U, int S,
+                                           int M) {
+  constexpr int kRing = ring_blocks(NPL);
   const int nBlocks = (S - M + kDiag - 1) / kDiag, u0 = NPL * lane;
   PairRing<NPL> ring(smem, arcs, lane, U, kNoArcBits, kNoArcBits);
   // block k holds the rows [max(S - 16(k+1), M), S - 16k)
@@ -261,7 +349,6 @@ __device__ __forceinline__ float beta_half(uint8_t* smem, const float2* arcs, fl
       for (int r = 0; r < NPL; ++r) bt[r] -= nextDelta;
       right -= nextDelta;
       offset += nextDelta;
-      if (lane == 0) dlEnd[-k] = nextDelta;
     }
     {
       float m = kNone;
@@ -271,7 +358,6 @@ __device__ __forceinline__ float beta_half(uint8_t* smem, const float2* arcs, fl
     }
     ring.wait();
     const int slot = k % kRing, lo = max(S - kDiag * (k + 1), M), nd = S - kDiag * k - lo;
-    float* out = al + (i64)(lo + 1) * ld;
     auto diag = [&](int i) {
       float x[NPL], y[NPL], m[NPL], e[NPL];
       ring.read(slot, i, x, y);
@@ -287,7 +373,6 @@ __device__ __forceinline__ float beta_half(uint8_t* smem, const float2* arcs, fl
         bt[r] = m[r] + lg2_approx(1.0f + e[r]);
         if (r == 0) right = __shfl_down_sync(0xffffffffu, bt[0], 1);
       }
-      if (ring.act) store_row<NPL>(out + i * ld, lane, bt);
     };
     if (nd == kDiag) {
 #pragma unroll
@@ -298,20 +383,19 @@ __device__ __forceinline__ float beta_half(uint8_t* smem, const float2* arcs, fl
     }
   }
   ring.drain();
+  if (ring.act) store_row<NPL>(row, lane, bt);
   return offset;
 }
 
 // Of a lane's nodes of the middle diagonal: 2^(alpha + beta - m), m the largest exponent of the warp, into
 // w; returns m, and the warp's sum of w in `total`.  No path at all (m ~ -6e29): total = 0, w = 0.
 template <int NPL>
-__device__ __forceinline__ float meet(const float* al, int lane, int U, int M, float (&w)[NPL], float& total) {
-  constexpr int ld = 32 * NPL;
+__device__ __forceinline__ float meet(const float* al, const float* be, int lane, int U, float (&w)[NPL], float& total) {
   float m = -INFINITY;
 #pragma unroll
   for (int r = 0; r < NPL; ++r) {
     const int u = NPL * lane + r, at = row_slot(min(u, U - 1), NPL);
-    const float a = __ldcg(al + (i64)M * ld + at), bt = __ldcg(al + (i64)(M + 1) * ld + at);
-    w[r] = u < U ? a + bt : -INFINITY;
+    w[r] = u < U ? __ldcg(al + at) + __ldcg(be + at) : -INFINITY;
     m = fmaxf(m, w[r]);
   }
   m = warp_max(m);
@@ -327,10 +411,11 @@ __device__ __forceinline__ float meet(const float* al, int lane, int U, int M, f
 }
 
 // One warp per half of an utterance (blockIdx.y); the half that finishes last adds up the cost.
+// ends [B, 2, 32 NPL] and offsets [B, 2]: scratch; halves [B]: zeros.
 template <int NPL>
-__global__ void __launch_bounds__(32) alpha_sweep_kernel(
-    const float2* __restrict__ arcs, float* __restrict__ costs, float* alphas, float* deltas, i64 stride,
-    int nBlk, const int* __restrict__ inLens, const int* __restrict__ labLens, int B, int maxT, int maxU,
+__global__ void __launch_bounds__(32) score_sweep_kernel(
+    const float2* __restrict__ arcs, float* __restrict__ costs, float* ends, float* offsets, i64 stride,
+    const int* __restrict__ inLens, const int* __restrict__ labLens, int B, int maxT, int maxU,
     float* lossSum, unsigned* ticket, unsigned* halves) {
   extern __shared__ __align__(128) uint8_t smemA[];
   const int b = blockIdx.x, lane = threadIdx.x;
@@ -340,12 +425,11 @@ __global__ void __launch_bounds__(32) alpha_sweep_kernel(
     return;
   }
   const int S = T + U - 1, M = middle(S);
-  float* al = alphas + (i64)b * stride;
-  float* dl = deltas + (i64)b * nBlk;
-  const float offset = blockIdx.y == 0
-      ? alpha_half<NPL>(smemA, arcs + (i64)b * stride, al, dl, lane, U, M)
-      : beta_half<NPL>(smemA, arcs + (i64)b * stride, al, dl + nBlk - 1, lane, U, S, M);
-  if (lane == 0) dl[blockIdx.y == 0 ? 0 : nBlk - 1] = offset;
+  float* al = ends + (i64)b * 64 * NPL;
+  float* be = al + 32 * NPL;
+  const float offset = blockIdx.y == 0 ? alpha_half<NPL>(smemA, arcs + (i64)b * stride, al, lane, U, M)
+                                       : beta_half<NPL>(smemA, arcs + (i64)b * stride, be, lane, U, S, M);
+  if (lane == 0) offsets[2 * b + blockIdx.y] = offset;
   __threadfence();
   __syncwarp();
   unsigned before = 0;
@@ -353,9 +437,9 @@ __global__ void __launch_bounds__(32) alpha_sweep_kernel(
   if (__shfl_sync(0xffffffffu, before, 0) == 0u) return;
   __threadfence();
   float w[NPL], total;
-  const float m = meet<NPL>(al, lane, U, M, w, total);
+  const float m = meet<NPL>(al, be, lane, U, w, total);
   if (lane == 0) {
-    const double log2p = (double)__ldcg(dl) + (double)__ldcg(dl + nBlk - 1) + (double)(m + log2f(total));
+    const double log2p = (double)__ldcg(offsets + 2 * b) + (double)__ldcg(offsets + 2 * b + 1) + (double)(m + log2f(total));
     finish_cost(costs, b, total == 0.0f ? pos_inf() : (float)(-log2p * 0.69314718055994530942), B, lossSum, ticket);
   }
 }
@@ -465,33 +549,26 @@ __global__ void __launch_bounds__(32) alpha_natural_kernel(
 // ---------------------------------------------------------------------------
 // reverse occupancy sweep
 // ---------------------------------------------------------------------------
-// With g(t,u) the occupancy of node (t,u) (the reference's dalphas, sign dropped), alphas, betas and arcs in
-// log2 units: below the middle diagonal
+// With g(t,u) the occupancy of node (t,u) (the reference's dalphas, sign dropped):
 //   stay(t,u) = g(t+1,u) * FB(t,u),  FB = 2^((alpha(t,u) + blank arc) - alpha(t+1,u))
 //   step(t,u) = g(t,u+1) * FL(t,u),  FL = 2^((alpha(t,u) + label arc) - alpha(t,u+1))
-//   g(t,u) = stay + step
-// and from it on
-//   stay(t,u) = g(t,u) * FB(t,u),    FB = 2^((blank arc + beta(t+1,u)) - beta(t,u))
-//   step(t,u) = g(t,u) * FL(t,u),    FL = 2^((label arc + beta(t,u+1)) - beta(t,u))
-//   g(t,u) = stay(t-1,u) + step(t,u-1),   the terminating blank being the stay of (T-1,U-1)
-// The parenthesised sums are rounded exactly as in the sweeps, so FB and FL of the arcs entering
-// (leaving) a node add up to 1 to within the error of ex2/lg2.  The stored numbers are relative to
-// a per-block offset: where the neighbouring diagonal opens a block or closes one, that block's delta
-// is subtracted where the sweep lowered its state.
-//
-// (natural: the first form all the way, g(T-1,U-1) = 1 fed by a node beyond the terminating blank.)
+//   (alphas and arcs in log2 units; the parenthesised sums are rounded exactly as in the alpha
+//   kernel, so FB and FL of the arcs entering a node add up to 1 to within the error of ex2/lg2.
+//   The stored alphas are relative to a per-block offset, see alpha_sweep_kernel: where the
+//   successors' diagonal opens a new block, that block's delta is subtracted from the sum first,
+//   exactly as the alpha kernel lowered its carried state.)
+//   g(t,u) = stay + step,            g(T-1,U-1) = 1 (the terminating blank, booked as stay)
 //
 // gamma_factors_kernel: the pairs (FB, FL) of every node of the diagonals below S, zero where there
 // is no arc (natural: from the pair rows of alpha_natural_kernel, by the accurate expf).  One warp
-// per 4 diagonals.  Bound by memory: a pair and an alpha (12 bytes) read, 8
-// written per node.
+// per 4 diagonals.  Bound by memory: a pair and an alpha (12 bytes) read, 8 written per node.
 constexpr int kFactorRows = 4, kFactorWarps = 8;
 static_assert(kGradTickets <= 32 * kFactorWarps, "one thread per ticket");
 template <int NPL>
 __global__ void __launch_bounds__(32 * kFactorWarps) gamma_factors_kernel(
     const float2* __restrict__ arcs, const float* __restrict__ alphas,
     const float* __restrict__ deltas, const NaturalTerms n, float2* __restrict__ F,
-    unsigned* __restrict__ occTicket, unsigned* __restrict__ gradTickets, i64 stride, int nBlk, const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT,
+    unsigned* __restrict__ occTicket, unsigned* __restrict__ gradTickets, i64 stride, int nDiag, const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT,
     int maxU) {
   constexpr int ld = 32 * NPL, kPieces = NPL / 2;
   const int b = blockIdx.y, lane = threadIdx.x & 31;
@@ -502,10 +579,8 @@ __global__ void __launch_bounds__(32 * kFactorWarps) gamma_factors_kernel(
   const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU), S = T + U - 1;
   const int d0 = (blockIdx.x * kFactorWarps + (threadIdx.x >> 5)) * kFactorRows, u0 = NPL * lane;
   if (T <= 0 || U <= 0 || d0 >= S || u0 >= U) return;
-  // (the middle is a multiple of kFactorRows: the warp's rows lie on one side of it)
-  const bool fwd = natural(NPL) || d0 < middle(S);
-  const float* al = alphas + (i64)b * stride + (fwd ? 0 : ld);   // (beta of d is in row d + 1)
-  const float* dl = deltas + (i64)b * nBlk;
+  const float* al = alphas + (i64)b * stride;
+  const float* dl = deltas + (i64)b * ((nDiag + kDiag - 1) / kDiag);
   const int next = row_slot(min(u0 + NPL, ld - 1), NPL);   // (the last position has no label arc)
   float a[kFactorRows + 1][NPL], aN[kFactorRows + 1], x[kFactorRows][NPL], y[kFactorRows][NPL];
 #pragma unroll
@@ -544,25 +619,24 @@ __global__ void __launch_bounds__(32 * kFactorWarps) gamma_factors_kernel(
   for (int i = 0; i < kFactorRows; ++i) {
     const int d = d0 + i;
     if (d >= S) break;
-    float dlt = 0.0f;   // of the block that diagonal d + 1 opens, or (betas) that d opens
-    if (!natural(NPL) && fwd && (d + 1) % kDiag == 0) dlt = dl[(d + 1) / kDiag];
-    if (!natural(NPL) && !fwd && (S - 1 - d) % kDiag == 0 && d < S - 1) dlt = dl[nBlk - 1 - (S - 1 - d) / kDiag];
+    // (rebased) the successors' diagonal opens a block: the carried sums were lowered by its delta
+    const float dlt = (!natural(NPL) && (d + 1) % kDiag == 0 && d + 1 < S) ? dl[(d + 1) / kDiag] : 0.0f;
 #pragma unroll
     for (int r = 0; r < NPL; ++r) {
       const int u = u0 + r, t = d - u;
       const bool valid = u < U && t >= 0 && t < T;
-      const float above = a[i + 1][r], aboveN = r < NPL - 1 ? a[i + 1][(r + 1) % NPL] : aN[i + 1];
+      const float art = r < NPL - 1 ? a[i + 1][(r + 1) % NPL] : aN[i + 1];
       float fb, fl;
       if constexpr (natural(NPL)) {
         const float eb = n.ebl[(i64)b * maxT + min(max(t, 0), T - 1)], lnv = x[i][r], el = y[i][r];
-        fb = expf((((a[i][r] + eb) + pbl[r]) - lnv) - above);
-        fl = expf((((a[i][r] + el) + plab[r]) - lnv) - aboveN);
+        fb = expf((((a[i][r] + eb) + pbl[r]) - lnv) - a[i + 1][r]);
+        fl = expf((((a[i][r] + el) + plab[r]) - lnv) - art);
       } else {
-        fb = ex2_approx(fwd ? ((a[i][r] + x[i][r]) - dlt) - above : ((above - dlt) + x[i][r]) - a[i][r]);
-        fl = ex2_approx(fwd ? ((a[i][r] + y[i][r]) - dlt) - aboveN : ((aboveN - dlt) + y[i][r]) - a[i][r]);
+        fb = ex2_approx(((a[i][r] + x[i][r]) - dlt) - a[i + 1][r]);
+        fl = ex2_approx(((a[i][r] + y[i][r]) - dlt) - art);
       }
       x[i][r] = (valid && t < T - 1) ? fb : 0.0f;
-      if (t == T - 1 && u == U - 1) x[i][r] = 1.0f;   // the terminating blank
+      if (t == T - 1 && u == U - 1) x[i][r] = 1.0f;   // terminating blank, fed by g(T,U-1) := 1
       y[i][r] = (valid && u < U - 1) ? fl : 0.0f;
     }
     float2* out = F + (i64)b * stride + (i64)d * ld;
@@ -573,96 +647,10 @@ __global__ void __launch_bounds__(32 * kFactorWarps) gamma_factors_kernel(
   }
 }
 
-// The recursions on the prepared factors, one warp per half (blockIdx.y): g of the diagonals M down to
-// 0, and of M + 1 up to S - 1.
-template <int NPL>
-__global__ void __launch_bounds__(32) gamma_sweep_kernel(
-    const float2* __restrict__ F, const float* __restrict__ alphas, float* __restrict__ g, i64 stride,
-    const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT, int maxU) {
-  constexpr int ld = 32 * NPL, kRing = ring_blocks(NPL);
-  extern __shared__ __align__(128) uint8_t smemG[];
-  const int b = blockIdx.x, lane = threadIdx.x;
-  const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
-  if (T <= 0 || U <= 0) return;
-  const int S = T + U - 1, M = middle(S);
-  PairRing<NPL> ring(smemG, F + (i64)b * stride, lane, U, 0u, 0u);
-  float* out0 = g + (i64)b * stride;
-  const bool down = blockIdx.y == 0;
-  // downwards block k holds the rows [M - 16(k+1), M - 16k); upwards the rows from M + 16k on, the last
-  // of which is S - 2
-  const int nBlocks = down ? M / kDiag : (S - 1 - M + kDiag - 1) / kDiag;
-  auto issue = [&](int k) {
-    if (down) ring.issue(k % kRing, M - kDiag * (k + 1), k < nBlocks ? kDiag : 0);
-    else ring.issue(k % kRing, M + kDiag * k, k < nBlocks ? min(kDiag, S - 1 - M - kDiag * k) : 0);
-  };
-#pragma unroll
-  for (int k = 0; k < kRing - 1; ++k) issue(k);
-  float s[NPL], total;
-  meet<NPL>(alphas + (i64)b * stride, lane, U, M, s, total);
-  const float share = total != 0.0f ? 1.0f / total : 0.0f;
-#pragma unroll
-  for (int r = 0; r < NPL; ++r) s[r] *= share;
-  if (down) {
-    if (ring.act) store_row<NPL>(out0 + (i64)M * ld, lane, s);
-    // (lane 31 gets its own s[0] back: harmless, the label arc of its last position never exists)
-    float right = __shfl_down_sync(0xffffffffu, s[0], 1);
-    for (int k = 0; k < nBlocks; ++k) {
-      issue(k + kRing - 1);
-      ring.wait();
-      const int slot = k % kRing;
-      float* out = out0 + (i64)(M - kDiag * (k + 1)) * ld;
-#pragma unroll
-      for (int i = kDiag - 1; i >= 0; --i) {
-        float x[NPL], y[NPL], n[NPL];
-        ring.read(slot, i, x, y);
-        // position 0 first: its result is shuffled for the next diagonal; the last position, which
-        // waits for the shuffle, at the end
-        const float in = right;
-#pragma unroll
-        for (int r = 0; r < NPL; ++r) {
-          const float nb = r < NPL - 1 ? s[(r + 1) % NPL] : in;
-          n[r] = __fadd_rn(__fmul_rn(s[r], x[r]), __fmul_rn(nb, y[r]));
-          if (r == 0) right = __shfl_down_sync(0xffffffffu, n[0], 1);
-        }
-#pragma unroll
-        for (int r = 0; r < NPL; ++r) s[r] = n[r];
-        if (ring.act) store_row<NPL>(out + i * ld, lane, s);
-      }
-    }
-  } else {
-    for (int k = 0; k < nBlocks; ++k) {
-      issue(k + kRing - 1);
-      ring.wait();
-      const int slot = k % kRing, nd = min(kDiag, S - 1 - M - kDiag * k);
-      float* out = out0 + (i64)(M + kDiag * k + 1) * ld;
-      auto diag = [&](int i) {
-        float x[NPL], y[NPL];
-        ring.read(slot, i, x, y);
-        // the last position's step leaves by the shuffle
-#pragma unroll
-        for (int r = 0; r < NPL; ++r) y[r] = __fmul_rn(s[r], y[r]);
-        const float left = __shfl_up_sync(0xffffffffu, y[NPL - 1], 1);
-#pragma unroll
-        for (int r = NPL - 1; r >= 0; --r)
-          s[r] = __fadd_rn(__fmul_rn(s[r], x[r]), r ? y[(r + NPL - 1) % NPL] : lane ? left : 0.0f);
-        if (ring.act) store_row<NPL>(out + i * ld, lane, s);
-      };
-      if (nd == kDiag) {
-#pragma unroll
-        for (int i = 0; i < kDiag; ++i) diag(i);
-      } else {
-#pragma unroll 1
-        for (int i = 0; i < nd; ++i) diag(i);
-      }
-    }
-  }
-  ring.drain();
-}
-
-// natural: one warp per utterance, g of the diagonals S (the node beyond the terminating
+// The recursion on the prepared factors: g of the diagonals S (the node beyond the terminating
 // blank) down to 0.
 template <int NPL>
-__global__ void __launch_bounds__(32) gamma_sweep_natural_kernel(
+__global__ void __launch_bounds__(32) gamma_sweep_kernel(
     const float2* __restrict__ F, float* __restrict__ g, i64 stride, const int* __restrict__ inLens,
     const int* __restrict__ labLens, int maxT, int maxU) {
   constexpr int ld = 32 * NPL;
@@ -734,6 +722,7 @@ struct PrepParams {
   const int* labLens;
   int maxT, maxU, V, blank, npl, ld, extra;
   bool nat;                  // for the natural sweeps
+  bool score;                // for score_sweep_kernel: words masked by -inf make no arc
   i64 stride;
 };
 
@@ -813,8 +802,9 @@ __global__ void __launch_bounds__(256) sweep_prep_kernel(const PrepParams p) {
                      : make_float2(__uint_as_float(kNoArcBits), __uint_as_float(kNoArcBits));
     if (t >= 0 && t < T && u < U) {
       const float lnv = tLn[tt][lane];
-      f.x = p.nat ? lnv : arc_term(((tEb[tt] + pbl) - lnv) * kLog2e);
-      if (u < U - 1) f.y = p.nat ? tEl[tt][lane] : arc_term(((tEl[tt][lane] + plab) - lnv) * kLog2e);
+      f.x = p.nat ? lnv : ((tEb[tt] + pbl) - lnv) * kLog2e;
+      if (u < U - 1) f.y = p.nat ? tEl[tt][lane] : ((tEl[tt][lane] + plab) - lnv) * kLog2e;
+      if (p.score) f = make_float2(arc_term(f.x), arc_term(f.y));
     }
     arcs[(i64)d * p.ld] = f;
   }
@@ -837,7 +827,7 @@ struct OccParams {
 
 // One CTA per 32 frames of one utterance, the 32x32 lattice tiles of the label axis side by side,
 // kOccWarps warps each.  With delta_b the upstream gradient:
-//   stay and step as above (g of the successors below the middle diagonal, of the node from it on)
+//   stay(t,u) = g(t+1,u) FB(t,u), step(t,u) = g(t,u+1) FL(t,u)
 //   W [B,maxT,ldW] = delta_b * (stay + step) * exp(ref(t) + maxP(u) - LN(t,u)), rounded to TF32
 //                   (round-to-nearest; the tensor core would otherwise truncate), zero outside
 //                   the valid lattice.  (The exponent is clamped at 80: it only gets there where
@@ -892,7 +882,6 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 640 ? 2 : 1) occupancy_ker
     // Step i takes diagonal i of the tile in the lanes up to i and diagonal i + 32 in the others:
     // every lane has a node and a warp touches two rows.  Four steps at a time with all their
     // loads issued before the first use (unconditional, clamped into the lattice).
-    const int M = natural(p.npl) ? T + U : middle(T + U - 1);
     const int slot1 = row_slot(uc, p.npl), slot2 = row_slot(min(u + 1, U - 1), p.npl);
 #pragma unroll
     for (int q = 0; q < kOccRows; q += 4) {
@@ -900,11 +889,10 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 640 ? 2 : 1) occupancy_ker
       float g1[4], g2[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const int d = min(t0 + ((w + kOccWarps * (q + j) - lane) & 31), T - 1) + uc;
-        const i64 row = (i64)d * ld, rowG = d < M ? row + ld : row;
+        const i64 row = (i64)(min(t0 + ((w + kOccWarps * (q + j) - lane) & 31), T - 1) + uc) * ld;
         f[j] = F[row];
-        g1[j] = g[rowG + slot1];
-        g2[j] = g[rowG + (d < M ? slot2 : slot1)];
+        g1[j] = g[row + ld + slot1];
+        g2[j] = g[row + ld + slot2];
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -1027,7 +1015,7 @@ SweepGeom sweep_geom(Dims d) {
   g.npl = d.maxU <= 32 ? 1 : d.maxU <= 64 ? 2 : d.maxU <= 128 ? 4 : div_up(d.maxU, 32);
   g.ld = 32 * g.npl;
   g.nDiag = d.maxT + d.maxU;   // one spare row: the node beyond the terminating blank
-  g.nBlk = (g.nDiag + kDiag - 1) / kDiag + 1;
+  g.nBlk = (g.nDiag + kDiag - 1) / kDiag;
   g.stride = (i64)g.ld * g.nDiag;
   return g;
 }
@@ -1040,11 +1028,7 @@ size_t sweep_partial_floats(Dims d) {
   do {                                       \
     if ((npl) == 1) { CALL(1); }             \
     else if ((npl) == 2) { CALL(2); }        \
-    else if ((npl) <= 4) { CALL(4); }        \
-    else if ((npl) == 5) { CALL(5); }        \
-    else if ((npl) == 6) { CALL(6); }        \
-    else if ((npl) == 7) { CALL(7); }        \
-    else { CALL(8); }                        \
+    else { CALL(4); }                        \
   } while (0)
 #define TB200_BY_NPL_NATURAL(npl, CALL)      \
   do {                                       \
@@ -1053,6 +1037,12 @@ size_t sweep_partial_floats(Dims d) {
     else if ((npl) == 7) { CALL(7); }        \
     else { CALL(8); }                        \
   } while (0)
+#define TB200_BY_NPL_ANY(npl, CALL)          \
+  do {                                       \
+    if ((npl) <= 4) { TB200_BY_NPL(npl, CALL); } \
+    else { TB200_BY_NPL_NATURAL(npl, CALL); } \
+  } while (0)
+
 void launch_sweep_forward(const void* E, const void* P, float* LN, const float* ELrow,
                           float* ebl, float2* arcs, float* alphas, float* deltas, float* costs,
                           float* lossSum, unsigned* ticket, unsigned* halves, const int* labels,
@@ -1067,7 +1057,7 @@ void launch_sweep_forward(const void* E, const void* P, float* LN, const float* 
     q.E = E; q.P = P; q.LN = LN; q.ELrow = ELrow; q.ebl = ebl; q.arcs = arcs;
     q.labels = labels; q.inLens = inLens; q.labLens = labLens;
     q.maxT = d.maxT; q.maxU = d.maxU; q.V = d.V; q.blank = d.blank; q.npl = g.npl; q.ld = g.ld;
-    q.extra = div_up(d.maxU, 32); q.nat = nat; q.stride = g.stride;
+    q.extra = div_up(d.maxU, 32); q.nat = nat; q.score = score; q.stride = g.stride;
     const dim3 grid(div_up(d.maxU, 32), div_up(d.maxT, 32) + 2 * q.extra, d.B);
     ScopedKernel sk("sweep_prep", stream);
     if (d.dtype == kDtypeBf16) sweep_prep_kernel<bf16><<<grid, 256, 0, stream>>>(q);
@@ -1075,6 +1065,18 @@ void launch_sweep_forward(const void* E, const void* P, float* LN, const float* 
     TB200_CHECK_LAUNCH();
   }
   const int ringBytes = ring_blocks(g.npl) * kDiag * g.ld * 8;
+  if (score) {
+    ScopedKernel sk("score_sweep", stream);
+#define CALL(NPL)                                                                                \
+  allow_dyn_smem(score_sweep_kernel<NPL>, ringBytes);                                            \
+  score_sweep_kernel<NPL><<<dim3(d.B, 2), 32, ringBytes, stream>>>(arcs, costs, alphas, deltas,  \
+                                                                   g.stride, inLens, labLens, d.B, \
+                                                                   d.maxT, d.maxU, lossSum, ticket, halves)
+    TB200_BY_NPL_ANY(g.npl, CALL);
+#undef CALL
+    TB200_CHECK_LAUNCH();
+    return;
+  }
   ScopedKernel sk("alpha_sweep", stream);
   if (nat) {
     const NaturalTerms n{static_cast<const float*>(P), ebl, labels, d.V, d.blank};
@@ -1092,11 +1094,11 @@ void launch_sweep_forward(const void* E, const void* P, float* LN, const float* 
     return;
   }
   const int smem = ringBytes;
-#define CALL(NPL)                                                                                 \
-  allow_dyn_smem(alpha_sweep_kernel<NPL>, smem);                                                  \
-  alpha_sweep_kernel<NPL><<<dim3(d.B, 2), 32, smem, stream>>>(arcs, costs, alphas, deltas, g.stride, \
-                                                              g.nBlk, inLens, labLens, d.B, d.maxT, \
-                                                              d.maxU, lossSum, ticket, halves)
+#define CALL(NPL)                                                                                \
+  allow_dyn_smem(alpha_sweep_kernel<NPL>, smem);                                                 \
+  alpha_sweep_kernel<NPL><<<d.B, 32, smem, stream>>>(arcs, costs, alphas, deltas, g.stride,      \
+                                                     g.nDiag, inLens, labLens, d.B, d.maxT,      \
+                                                     d.maxU, lossSum, ticket)
   TB200_BY_NPL(g.npl, CALL);
 #undef CALL
   TB200_CHECK_LAUNCH();
@@ -1115,9 +1117,9 @@ void launch_sweep_backward(const SweepScratch& w, const float* P, const float* b
     const dim3 grid(div_up(g.nDiag, kFactorRows * kFactorWarps), d.B);
 #define CALL(NPL)                                                                              \
   gamma_factors_kernel<NPL><<<grid, 32 * kFactorWarps, 0, stream>>>(                           \
-      arcs, alphas, alphaDeltas, n, w.F, w.ticket, w.gradTickets, g.stride, g.nBlk, inLens, labLens, d.maxT, d.maxU)
+      arcs, alphas, alphaDeltas, n, w.F, w.ticket, w.gradTickets, g.stride, g.nDiag, inLens, labLens, d.maxT, d.maxU)
     const NaturalTerms n{P, blankEmissions, labels, d.V, d.blank};
-    TB200_BY_NPL(g.npl, CALL);
+    TB200_BY_NPL_ANY(g.npl, CALL);
 #undef CALL
     TB200_CHECK_LAUNCH();
   }
@@ -1126,14 +1128,8 @@ void launch_sweep_backward(const SweepScratch& w, const float* P, const float* b
     ScopedKernel sk("gamma_sweep", stream);
 #define CALL(NPL)                                                                              \
   allow_dyn_smem(gamma_sweep_kernel<NPL>, smem);                                               \
-  gamma_sweep_kernel<NPL><<<dim3(d.B, 2), 32, smem, stream>>>(w.F, alphas, w.g, g.stride, inLens, labLens, d.maxT, d.maxU)
-    if (g.npl <= 2) { if (g.npl == 1) { CALL(1); } else { CALL(2); } }
-    else if (g.npl <= 4) { CALL(4); }
-#undef CALL
-#define CALL(NPL)                                                                              \
-  allow_dyn_smem(gamma_sweep_natural_kernel<NPL>, smem);                                       \
-  gamma_sweep_natural_kernel<NPL><<<d.B, 32, smem, stream>>>(w.F, w.g, g.stride, inLens, labLens, d.maxT, d.maxU)
-    else { TB200_BY_NPL_NATURAL(g.npl, CALL); }
+  gamma_sweep_kernel<NPL><<<d.B, 32, smem, stream>>>(w.F, w.g, g.stride, inLens, labLens, d.maxT, d.maxU)
+    TB200_BY_NPL_ANY(g.npl, CALL);
 #undef CALL
     TB200_CHECK_LAUNCH();
   }
