@@ -134,7 +134,7 @@ def test_frames_cut_into_parts(B, T, U, V):
         assert not eg_t[b, int(il[b]):].any() and not pg_t[b, int(ll[b]) + 1:].any()
 
 
-@pytest.mark.parametrize("T,U,V,hi", [(70, 100, 100, 100), (33, 128, 130, 4), (95, 40, 64, 64), (64, 18, 128, 128),
+@pytest.mark.parametrize("T,U,V,hi", [(70, 100, 100, 100), (33, 128, 132, 4), (95, 40, 64, 64), (64, 18, 128, 128),
                                       (40, 151, 36, 36), (50, 201, 128, 3), (40, 60, 2048, 20)])
 def test_labels_that_are_not_staged(T, U, V, hi):
     """More labels in a block of columns than the gradient kernel stages, distinct and repeated."""

@@ -1,5 +1,6 @@
 // C ABI (include/transducer_b200.h) and the reference-compatible C++-linkage entry
 // points (include/transducer.h) on top of the kernel launchers.
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <sstream>
@@ -190,16 +191,18 @@ void need(size_t have, size_t want, const void* ws) {
 
 // Log-normalisers plus the row shifts.  With the SIMT kernels rowRef is the true row
 // maximum of E.
+// keepBits: where gradients follow, the weights behind the sweeps are rounded to TF32, and other log-normalisers,
+// however close, would flip some of those roundings (lattice_sweep.cu): the TF32 kernel at any size.
 // Returns true if the pass also produced the label / blank emissions (EL, ebl) it was offered.
 bool log_norms_impl(const void* E, const void* P, float* LN, float* rowRef, float* maxP,
                     const int* inLens, const int* labLens, const Dims& d, LogNormWs& ws,
                     bool fixup = true, const int* labels = nullptr, float* EL = nullptr,
-                    float* ebl = nullptr) {
+                    float* ebl = nullptr, bool keepBits = false) {
   if (d.B <= 0 || d.maxT <= 0 || d.maxU <= 0) return false;
   const bool can = lognorm_umma_supported(E, P, d);
   const int path = g_opt.lognorm_path;
-  const bool tensorCore = can && (path == 0 || path == 2);
-  if (path == 2 && !can)
+  const bool tensorCore = can && (path == 0 || path == 2 || path == 4);
+  if ((path == 2 || path == 4) && !can)
     throw std::invalid_argument(
         "tensor-core log-normaliser needs alphabetSize % 4 == 0, alphabetSize >= 32, "
         "maxLabelLength <= 256 and 16-byte aligned emissions");
@@ -220,7 +223,8 @@ bool log_norms_impl(const void* E, const void* P, float* LN, float* rowRef, floa
     const bool gathers = labels && EL && ebl && lognorm_umma_gathers(d) &&
                          (handOut == 2 || (handOut == 1 && bytesE > (size_t)96 << 20));
     launch_lognorm_umma(E, P, LN, rowRef, mp, inLens, labLens, d, ws.split,
-                        device_status_word(), fixup, g_stream, gathers ? labels : nullptr,
+                        device_status_word(), path == 4 || (path == 0 && !keepBits && lognorm_f16_pays(d)),
+                        fixup, g_stream, gathers ? labels : nullptr,
                         gathers ? EL : nullptr, gathers ? ebl : nullptr);
     return gathers;
   }
@@ -256,7 +260,7 @@ void* tb200_get_stream(void) { return g_stream; }
 
 int tb200_set_option(const char* key, int value) {
   if (!key) return fail(kErrInvalidArgument, "null option key");
-  if (!strcmp(key, "lognorm_path") && value >= 0 && value <= 3) g_opt.lognorm_path = value;
+  if (!strcmp(key, "lognorm_path") && value >= 0 && value <= 4) g_opt.lognorm_path = value;
   else if (!strcmp(key, "grads_path") && value >= 0 && value <= 2) g_opt.grads_path = value;
   else if (!strcmp(key, "grad_passes") && value >= 1 && value <= 3) g_opt.grad_passes = value;
   else if (!strcmp(key, "fused_gather") && value >= 0 && value <= 2) g_opt.fused_gather = value;
@@ -426,7 +430,8 @@ int loss_forward_any(const void* E, const void* P, const int* labels, const int*
     float* LN = sweep ? st.LN : fw.LN;
     // (nodes the tensor-core log-normaliser could not represent are recomputed by the re-layout)
     const bool gathered = log_norms_impl(E, P, LN, st.rowRef, st.maxP, inLens, labLens, d, ws,
-                                         /*fixup=*/false, labels, fw.EL, st.ebl);
+                                         /*fixup=*/false, labels, fw.EL, st.ebl,
+                                         /*keepBits=*/!score);
     TB200_CUDA_CHECK(cudaMemsetAsync(ws.ticket, 0, sizeof(unsigned) * (16 + (size_t)B), g_stream));
     if (lossSum && B == 0) TB200_CUDA_CHECK(cudaMemsetAsync(lossSum, 0, sizeof(float), g_stream));
     unsigned* ticket = lossSum ? ws.ticket : nullptr;

@@ -102,6 +102,9 @@ void launch_exp_rows(const float* P, float* expP, float* maxP, const int* labLen
 // at most 128 positions).  Usable when lognorm_umma_supported();
 // splitWs holds lognorm_umma_workspace_floats(d) floats; status is the device status word
 // (api_internal.h): [0] first device-side error code (0 = none), [1] nodes recomputed exactly.
+// f16: by lognorm_f16.cu, the TF32 kernel for the tiles that it marks only; lognorm_f16_pays: is
+// that the faster of the two for these sizes?
+bool lognorm_f16_pays(Dims d);
 bool lognorm_umma_supported(const void* E, const void* P, Dims d);
 size_t lognorm_umma_workspace_floats(Dims d);
 // Nodes whose factored sum left the fp32 range come out of the kernel as NaN; with `fixup` a
@@ -115,8 +118,24 @@ void launch_lognorm_fixup(const void* E, const void* P, float* LN, const int* in
 bool lognorm_umma_gathers(Dims d);
 void launch_lognorm_umma(const void* E, const void* P, float* LN, float* rowRef, float* maxP,
                          const int* inLens, const int* labLens, Dims d, float* splitWs,
-                         int* status, bool fixup, cudaStream_t stream,
+                         int* status, bool f16, bool fixup, cudaStream_t stream,
                          const int* labels = nullptr, float* EL = nullptr, float* ebl = nullptr);
+
+// ---- lognorm_f16.cu ------------------------------------------------------------
+// The workspace of launch_lognorm_umma, shared by both kernels.
+struct LogNormScratch {
+  float* operand;      // exp(P): fp16 pairs, or (TF32 kernel) two fp32 arrays
+  float* partial;      // partial sums of split tiles
+  float* rowSums;
+  float* sumP;         // [B,maxU]
+  unsigned* tickets;   // zero
+  int* marks;          // zero; 1 + B * tiles
+  int nSM;             // SMs of the device
+};
+// LN of every tile whose sums can be trusted; the others are marked (ws.marks) for the TF32 kernel.
+void launch_lognorm_f16(const void* E, const void* P, float* LN, float* rowRef, float* maxP,
+                        const int* inLens, const int* labLens, Dims d, const LogNormScratch& ws,
+                        int* status, cudaStream_t stream, const int* labels, float* EL, float* ebl);
 
 // ---- grads_umma.cu --------------------------------------------------------------
 // Tensor-core gradients: one pass over E produces egrads and pgrads.  Usable when

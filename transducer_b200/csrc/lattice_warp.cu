@@ -3,7 +3,7 @@
 // Lane l of the warp owns adjacent label positions; all nodes of a diagonal d = t + u are
 // independent, the one value per lane that crosses from the neighbouring lane arrives by a warp
 // shuffle, and the operands of a node, a pair, come by cp.async through the ring of pair_ring.cuh.
-// (Not from both ends, as the loss's sweeps: the scores are added in the reference's order.)
+// (Not from both ends, as the costs alone: the scores are added in the reference's order.)
 #include <algorithm>
 
 #include "kernels.h"

@@ -38,6 +38,7 @@
 #include <atomic>
 
 #include "kernels.h"
+#include "lognorm_items.cuh"
 #include "profile.h"
 #include "sm100.cuh"
 
@@ -128,14 +129,8 @@ CUtensorMap make_tmap_f32_rows(const void* base, uint64_t d0, uint64_t d1, uint6
 namespace {
 
 using namespace sm100;
+using namespace lognorm;
 
-constexpr int kTileM = 128;
-constexpr int kMaxSMs = 256;                      // slots for the partial sums of split tiles
-constexpr int kChunkK = 32;                       // floats per K-chunk = one 128-byte swizzle row
-// raw E chunk of a stage: 128 frames x 32 words, rows of 128 bytes (fp32) or 64 bytes (bf16)
-__host__ __device__ constexpr int raw_bytes(bool bf) { return kTileM * kChunkK * (bf ? 2 : 4); }
-constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kSumLo = 1e-30f, kSumHi = 1e30f;
 
 // ---------------------------------------------------------------------------------
 // exp(P - maxP) split into TF32 hi/lo as [B][nPad][kPad]: rows u < U_b, columns zero-padded to kPad
@@ -144,9 +139,15 @@ template <typename TIn>
 __global__ void __launch_bounds__(256) expp_split_kernel(
     const TIn* __restrict__ P, float* __restrict__ bHi, float* __restrict__ bLo,
     float* __restrict__ maxP, const int* __restrict__ labLens, int maxU, int V, int nPad,
-    int kPad) {
+    int kPad, const int* __restrict__ only, int tilesX) {
   __shared__ float red[8];
   const int b = blockIdx.y, u = blockIdx.x;
+  if (only) {   // the utterances with a marked tile
+    if (only[0] == 0) return;
+    int any = 0;
+    for (int x = threadIdx.x; x < tilesX; x += blockDim.x) any |= only[1 + b * tilesX + x];
+    if (!__syncthreads_or(any)) return;
+  }
   const int U = min(labLens[b] + 1, maxU);
   float* hi = bHi + ((i64)b * nPad + u) * kPad;
   float* lo = bLo + ((i64)b * nPad + u) * kPad;
@@ -213,6 +214,8 @@ struct LnParams {
   float* EL;         // [B, maxU, maxT], frames contiguous: EL[b,u,t] = E[b,t,labels[b,u]], u < U_b - 1
   float* ebl;        // [B, maxT]: E[b,t,blank]
   int blank;
+  // null, or [0] is any tile marked, [1 + b * tilesX + tile] is it: the others are left as they are
+  const int* only;
 };
 
 // Chunks per accumulation group.  The tensor core adds into its fp32 accumulator with
@@ -225,19 +228,6 @@ constexpr int kGroup = 2;
 //       group's wait for its tile and for its TMEM stores overlaps the other's exponentials.
 // NDRAIN drain warpgroups, each owning DCOLS accumulator columns (fp32 sums in registers).
 //
-// Work items.  A tile (128 frames of one utterance x the whole vocabulary) takes the same time
-// whatever it holds, and one CTA fits an SM, so n live tiles on nSM SMs cost ceil(n / nSM)
-// rounds: 454 tiles on 148 SMs pay for 592.  The tiles of the last, partly filled round are
-// therefore split along the vocabulary into k = min(8, nSM / rem) parts (rem = n mod nSM):
-// part 0 runs in the tile's own CTA, parts 1..k-1 in `worker` CTAs appended to the grid (the
-// hardware dispatches CTAs in index order, so they start exactly when the last round does).
-// Every part keeps the frame's shift of the whole tile (a part that does not begin at chunk 0
-// first fetches chunk 0 for it and feeds zeros to the tensor core for that chunk), writes its
-// partial sums to `partial`, and the part that finishes last adds the parts in index order.
-// The grid is (tilesX * B + nSM) x 1; lengths are on the device, so every CTA derives the
-// schedule from them itself (B <= 1024; larger batches are not split).
-constexpr int kMaxParts = 8;
-constexpr int kMaxLabels = 256;
 // BF: the emissions are bf16 (the raw chunk of a stage then has 64-byte rows, 64-byte swizzle).
 template <int NTW, int NDRAIN, int DCOLS, bool BF = false>
 __global__ void __launch_bounds__((4 * NTW + 4 * NDRAIN + 3) * 32, 1) lognorm_umma_kernel(
@@ -249,119 +239,11 @@ __global__ void __launch_bounds__((4 * NTW + 4 * NDRAIN + 3) * 32, 1) lognorm_um
   constexpr int kDrainCols = DCOLS;
   constexpr int kRawBytes = raw_bytes(BF);
   constexpr int kRowBytes = BF ? 64 : 128;
-  // 16 consecutive words of frame r's row of the raw chunk, starting at word 16 * half, as fp32
-  auto load16 = [](const uint8_t* row, int r, int half, float (&x)[16]) {
-    if constexpr (BF) {
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int jj = half * 2 + j;  // 16-byte piece (8 words) of the 64-byte row
-        const uint4 q = *reinterpret_cast<const uint4*>(row + ((jj ^ ((r >> 1) & 3)) << 4));
-        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          x[8 * j + 2 * k] = __uint_as_float(w[k] << 16);
-          x[8 * j + 2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u);
-        }
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int jj = half * 4 + j;  // 16-byte piece of the 128-byte row
-        const float4 v4 = *reinterpret_cast<const float4*>(row + ((jj ^ (r & 7)) << 4));
-        x[4 * j] = v4.x; x[4 * j + 1] = v4.y; x[4 * j + 2] = v4.z; x[4 * j + 3] = v4.w;
-      }
-    }
-  };
-  // word `off` (0..31) of frame r's row
-  auto load1 = [](const uint8_t* row, int r, int off) {
-    if constexpr (BF) {
-      const unsigned short h = *reinterpret_cast<const unsigned short*>(
-          row + (((off >> 3) ^ ((r >> 1) & 3)) << 4) + (off & 7) * 2);
-      return __uint_as_float((uint32_t)h << 16);
-    } else {
-      return *reinterpret_cast<const float*>(row + (((off >> 2) ^ (r & 7)) << 4) + (off & 3) * 4);
-    }
-  };
-  // ---- which work item is this CTA? (warp 0 scans the lengths; before any allocation) ----
-  __shared__ int sItem[6];  // b, tile, part, parts, split-tile index, valid
-  if (threadIdx.x < 32) {
-    const int lane0 = threadIdx.x;
-    const int perUtt = p.tilesX * p.halves;   // grid slots per utterance
-    const int nNatural = perUtt * p.B;
-    const bool worker = (int)blockIdx.x >= nNatural;
-    const int myB = worker ? -1 : (int)blockIdx.x / perUtt, myX = worker ? 0 : (int)blockIdx.x % perUtt;
-    // live work items of an utterance: tiles x column ranges that hold positions (item ix is
-    // range ix % ranges of tile ix / ranges, so the ranges of a tile run side by side and
-    // share its chunks of E in L2)
-    auto ranges = [&](int bb) {
-      const int Ub = min(p.labLens[bb] + 1, p.maxU);
-      return min(p.halves, (Ub + p.nPad - 1) / p.nPad);
-    };
-    auto liveTiles = [&](int bb) {
-      if (bb >= p.B) return 0;
-      const int Tb = min(p.inLens[bb], p.maxT), Ub = min(p.labLens[bb] + 1, p.maxU);
-      return (Tb > 0 && Ub > 0) ? ((Tb + kTileM - 1) / kTileM) * ranges(bb) : 0;
-    };
-    int n = 0, before = 0;  // live tiles in all, and in the utterances before mine
-    for (int b0 = 0; b0 < p.B; b0 += 32) {
-      const int v = liveTiles(b0 + lane0);
-      const int tot = __reduce_add_sync(0xffffffffu, v);
-      const int pre = __reduce_add_sync(0xffffffffu, (b0 + lane0 < myB) ? v : 0);
-      n += tot;
-      before += pre;
-    }
-    const int full = (n / p.nSM) * p.nSM, rem = n - full;
-    int k = (rem > 0 && p.B <= 1024) ? min(kMaxParts, p.nSM / rem) : 1;
-    k = min(k, ((p.V + kChunkK - 1) / kChunkK) / 16);  // a part is worth >= 16 chunks
-    if (k < 2) k = 1;
-    int ib = -1, ix = 0, part = 0, parts = 1, split = 0, valid = 0;
-    if (!worker) {
-      if (myX < liveTiles(myB)) {
-        valid = 1; ib = myB; ix = myX;
-        const int r = before + myX;
-        if (k > 1 && r >= full) { parts = k; split = r - full; }
-      }
-    } else if (k > 1) {
-      const int w = (int)blockIdx.x - nNatural;
-      if (w < rem * (k - 1)) {
-        split = w / (k - 1);
-        part = 1 + w % (k - 1);
-        parts = k;
-        // locate the tile of live rank full + split
-        const int target = full + split;
-        int run = 0;
-        for (int b0 = 0; b0 < p.B && !valid; b0 += 32) {
-          const int v = liveTiles(b0 + lane0);
-          int incl = v;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int up = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane0 >= o) incl += up;
-          }
-          const int lo = run + incl - v, hi = run + incl;  // my utterance holds ranks [lo, hi)
-          const unsigned hit = __ballot_sync(0xffffffffu, target >= lo && target < hi);
-          if (hit) {
-            const int src = __ffs(hit) - 1;
-            ib = b0 + src;
-            ix = target - __shfl_sync(0xffffffffu, lo, src);
-            valid = 1;
-          }
-          run += __shfl_sync(0xffffffffu, incl, 31);
-        }
-      }
-    }
-    if (lane0 == 0) {
-      sItem[0] = ib; sItem[1] = ix; sItem[2] = part; sItem[3] = parts; sItem[4] = split; sItem[5] = valid;
-    }
-  }
-  __syncthreads();
-  if (!sItem[5]) return;
-  const int b = sItem[0];
-  const int part = sItem[2], parts = sItem[3], splitIdx = sItem[4];
-  const int T = min(p.inLens[b], p.maxT), U = min(p.labLens[b] + 1, p.maxU);
-  const int nRanges = min(p.halves, (U + p.nPad - 1) / p.nPad);
-  const int t0 = (sItem[1] / nRanges) * kTileM;
-  const int uOff = (sItem[1] % nRanges) * p.nPad;   // first label position of my column range
+  if (p.only && p.only[0] == 0) return;   // (no tile is marked)
+  const LnItem it = ln_item(p.inLens, p.labLens, p.maxT, p.maxU, p.V, p.B, p.tilesX, p.halves, p.nPad, p.nSM);
+  if (it.b < 0 || (p.only && p.only[1 + it.b * p.tilesX + it.t0 / kTileM] == 0)) return;
+  const int b = it.b, T = it.T, U = it.U, t0 = it.t0, uOff = it.uOff;
+  const int part = it.part, parts = it.parts, splitIdx = it.split;
 
   extern __shared__ uint8_t smemRaw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) &
@@ -409,20 +291,9 @@ __global__ void __launch_bounds__((4 * NTW + 4 * NDRAIN + 3) * 32, 1) lognorm_um
     sMaxP[u] = (uOff + u < U) ? p.maxP[(i64)b * p.maxU + uOff + u] : 0.0f;
   const bool gather = p.EL != nullptr && uOff == 0;   // (one range hands out the emissions)
   const int nLab = gather ? min(U - 1, kMaxLabels) : 0;
-  if (gather) {  // rank sort by column (from a shared-memory copy); ties keep position order
+  if (gather) {
     __shared__ int sLab[kMaxLabels];
-    const int* lab = p.labels + (i64)b * (p.maxU - 1);
-    for (int i = threadIdx.x; i < nLab; i += kThreads) sLab[i] = lab[i];
-    __syncthreads();
-    for (int i = threadIdx.x; i < nLab; i += kThreads) {
-      const int mine = sLab[i];
-      int rank = 0;
-      for (int j = 0; j < nLab; ++j) {
-        const int o = sLab[j];
-        rank += (o < mine || (o == mine && j < i)) ? 1 : 0;
-      }
-      sKey[rank] = (mine << 8) | i;
-    }
+    sort_labels(p.labels + (i64)b * (p.maxU - 1), nLab, sLab, sKey);
   }
   if (warp == kMmaWarp) {
     tmem_alloc(&tmemBase, (uint32_t)p.tmemCols);
@@ -521,11 +392,10 @@ __global__ void __launch_bounds__((4 * NTW + 4 * NDRAIN + 3) * 32, 1) lognorm_um
       ok = __all_sync(0xffffffffu, ok);
       ref = sRef[r];
     }
-    int cur = 0;  // cursor into the sorted label list (the same in every thread)
-    // column of the next entry that this group has not passed yet, kept in a register so that a
-    // chunk without any costs one comparison and no shared-memory access
+    int cur = 0;  // cursor into the sorted label list (see hand_out)
     int nextCol = (gather && nLab > 0) ? (sKey[0] >> 8) : 0x7fffffff;
     float* elCol = gather ? p.EL + (i64)b * p.maxU * p.maxT + t0 + r : nullptr;  // my frame
+    float* eblAt = gather ? p.ebl + (i64)b * p.maxT + t0 + r : nullptr;
     int s = grp % S;
     uint32_t ph = (grp / S) & 1;
     for (int c = grp; c < nChunks && ok; c += NTW) {
@@ -541,7 +411,7 @@ __global__ void __launch_bounds__((4 * NTW + 4 * NDRAIN + 3) * 32, 1) lognorm_um
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           float x[16];
-          load16(row, r, half, x);
+          load_words16<BF>(row, r, half, x);
 #pragma unroll
           for (int j = 0; j < 16; ++j)
             if (half * 16 + j < kLeft) m = fmaxf(m, x[j]);
@@ -553,32 +423,15 @@ __global__ void __launch_bounds__((4 * NTW + 4 * NDRAIN + 3) * 32, 1) lognorm_um
         if (t0 + r < T && part == 0 && uOff == 0) p.rowRef[(i64)b * p.maxT + t0 + r] = ref;
       }
       const int col0 = chunkOf(c) * kChunkK;
-      if (gather && !refOnly && nextCol < col0 + kChunkK) {
-        // (uniform control flow: the list and the cursor are the same in all threads)
-        int key = sKey[cur];
-        while ((key >> 8) < col0 && ++cur < nLab) key = sKey[cur];   // the other group's chunks
-        while (cur < nLab && (key >> 8) < col0 + kChunkK) {
-          const int off = (key >> 8) - col0;
-          const float v = load1(row, r, off);
-          // (the 128 threads of the group write 128 consecutive floats of row u)
-          if (t0 + r < T) elCol[(i64)(key & 0xff) * p.maxT] = v;
-          if (++cur < nLab) key = sKey[cur];
-        }
-        nextCol = cur < nLab ? (key >> 8) : 0x7fffffff;
-      }
-      if (gather && !refOnly) {
-        if (p.blank >= col0 && p.blank < col0 + kChunkK) {
-          const int off = p.blank - col0;
-          const float v = load1(row, r, off);
-          if (t0 + r < T) p.ebl[(i64)b * p.maxT + t0 + r] = v;
-        }
-      }
+      if (gather && !refOnly)
+        hand_out([&](int off) { return load_word<BF>(row, r, off); }, col0, kChunkK, sKey, nLab, cur, nextCol,
+                 elCol, p.maxT, p.blank, eblAt, t0 + r < T);
       const float nref = -ref * kLog2e;
       const uint32_t dst = tA + laneAddr + (uint32_t)(s * 64);
 #pragma unroll
       for (int half = 0; half < 2; ++half) {  // 16 columns at a time (registers)
         float x[16];
-        load16(row, r, half, x);
+        load_words16<BF>(row, r, half, x);
         const int kLeftMine = refOnly ? 0 : kLeft - half * 16;
         uint32_t hi[16], lo[16];
         if (kLeftMine >= 16) {
@@ -771,35 +624,52 @@ LabelAxis label_axis(int maxU) {
   return LabelAxis{2, (int)round_up64((n + 1) / 2, 16)};
 }
 
-size_t lognorm_umma_workspace_floats(Dims d) {
-  const size_t nPad = (size_t)label_axis(d.maxU).rows();
-  const size_t kPad = (size_t)round_up64(d.V, kChunkK);
-  // exp(P) hi and lo; partial sums of split tiles (one slot per SM at most); their tickets
-  return 2 * (size_t)d.B * nPad * kPad + (size_t)kMaxSMs * kTileM * nPad + kMaxSMs;
+// Layout of the workspace: exp(P) hi and lo; partial sums of split tiles (one slot per SM at most) with
+// their frames' sums; sums of exp(P); tickets and marks (zeroed together).
+static size_t scratch(Dims d, float* base, LogNormScratch* ws) {
+  const size_t nPad = (size_t)label_axis(d.maxU).rows(), kPad = (size_t)round_up64(d.V, kChunkK);
+  const size_t B = (size_t)std::max(d.B, 0), maxU = (size_t)std::max(d.maxU, 0);
+  size_t at = 0;
+  auto take = [&](size_t n) {
+    float* q = base ? base + at : nullptr;
+    at += n;
+    return q;
+  };
+  LogNormScratch w{};
+  w.operand = take(2 * B * nPad * kPad);
+  w.partial = take((size_t)kMaxSMs * kTileM * nPad);
+  w.rowSums = take((size_t)kMaxSMs * kTileM * 2);
+  w.sumP = take(B * maxU);
+  w.tickets = reinterpret_cast<unsigned*>(take(kMaxSMs));
+  w.marks = reinterpret_cast<int*>(take(1 + B * (size_t)div_up(std::max(d.maxT, 0), kTileM)));
+  if (ws) *ws = w;
+  return at;
 }
+size_t lognorm_umma_workspace_floats(Dims d) { return scratch(d, nullptr, nullptr); }
 
 bool lognorm_umma_gathers(Dims d) { return d.maxU >= 1 && d.maxU <= kMaxLabels; }
 
-void launch_lognorm_umma(const void* E, const void* P, float* LN, float* rowRef, float* maxP,
-                         const int* inLens, const int* labLens, Dims d, float* splitWs,
-                         int* status, bool fixup, cudaStream_t stream, const int* labels,
-                         float* EL, float* ebl) {
-  if (d.B <= 0 || d.maxT <= 0 || d.maxU <= 0) return;
+// The TF32 kernel; only: see LnParams.
+static void launch_tf32(const void* E, const void* P, float* LN, float* rowRef, float* maxP,
+                        const int* inLens, const int* labLens, Dims d, const LogNormScratch& ws,
+                        int* status, cudaStream_t stream, const int* labels, float* EL, float* ebl,
+                        const int* only) {
   const LabelAxis axis = label_axis(d.maxU);
   const int nPad = axis.rows();          // rows of the exp(P) operand arrays
   const int nPart = axis.part;           // label positions per work item
   const int kPad = (int)round_up64(d.V, kChunkK);
   const bool bf = d.dtype == kDtypeBf16;
-  float* bHi = splitWs;
-  float* bLo = splitWs + (size_t)d.B * nPad * kPad;
+  const int tilesX = div_up(d.maxT, kTileM);
+  float* bHi = ws.operand;
+  float* bLo = ws.operand + (size_t)d.B * nPad * kPad;
   {
     ScopedKernel sk("expp_split", stream);
     if (bf)
       expp_split_kernel<bf16><<<dim3(nPad, d.B), 256, 0, stream>>>(
-          static_cast<const bf16*>(P), bHi, bLo, maxP, labLens, d.maxU, d.V, nPad, kPad);
+          static_cast<const bf16*>(P), bHi, bLo, maxP, labLens, d.maxU, d.V, nPad, kPad, only, tilesX);
     else
       expp_split_kernel<float><<<dim3(nPad, d.B), 256, 0, stream>>>(
-          static_cast<const float*>(P), bHi, bLo, maxP, labLens, d.maxU, d.V, nPad, kPad);
+          static_cast<const float*>(P), bHi, bLo, maxP, labLens, d.maxU, d.V, nPad, kPad, only, tilesX);
   }
   TB200_CHECK_LAUNCH();
 
@@ -818,15 +688,12 @@ void launch_lognorm_umma(const void* E, const void* P, float* LN, float* rowRef,
   p.status = status;
   p.maxT = d.maxT; p.maxU = d.maxU; p.V = d.V; p.nPad = nPart; p.halves = axis.ranges;
   p.labels = nullptr; p.EL = nullptr; p.ebl = nullptr; p.blank = d.blank;
-  int dev = 0, nSM = 0;
-  TB200_CUDA_CHECK(cudaGetDevice(&dev));
-  TB200_CUDA_CHECK(cudaDeviceGetAttribute(&nSM, cudaDevAttrMultiProcessorCount, dev));
   p.B = d.B;
-  p.tilesX = div_up(d.maxT, kTileM);
-  p.nSM = std::min(nSM, kMaxSMs);
-  p.partial = bLo + (size_t)d.B * nPad * kPad;
-  p.tickets = reinterpret_cast<unsigned*>(p.partial + (size_t)kMaxSMs * kTileM * nPad);
-  TB200_CUDA_CHECK(cudaMemsetAsync(p.tickets, 0, sizeof(unsigned) * kMaxSMs, stream));
+  p.tilesX = tilesX;
+  p.nSM = ws.nSM;
+  p.partial = ws.partial;
+  p.tickets = ws.tickets;
+  p.only = only;
   const int stageBytes = raw_bytes(bf) + 2 * nPart * kChunkK * 4;
   // Tensor memory (512 columns): two accumulators of nPart <= 128 columns (the MMA of one group
   // of chunks runs while the previous group is drained), then four operand stages of 64 columns.
@@ -846,7 +713,7 @@ void launch_lognorm_umma(const void* E, const void* P, float* LN, float* rowRef,
   dim3 grid((unsigned)(p.tilesX * p.halves * d.B + p.nSM));
   {
     ScopedKernel sk("lognorm_umma", stream);
-    if (labels != nullptr && EL != nullptr && ebl != nullptr && lognorm_umma_gathers(d)) {
+    if (labels != nullptr && EL != nullptr && ebl != nullptr) {
       p.labels = labels; p.EL = EL; p.ebl = ebl;
     }
     // 8 transform + 8 drain (64 columns each) warps, producer, two MMA issuers
@@ -861,6 +728,31 @@ void launch_lognorm_umma(const void* E, const void* P, float* LN, float* rowRef,
     }
   }
   TB200_CHECK_LAUNCH();
+}
+
+// The fp16 pairs need two launches more (for the marked tiles, mostly none: ~5 us).  Both kernels with
+// exp(P), us, TF32 / fp16: B = 8, T = 500, U = 50, V = 4096 (2^24 scores) 73 / 76; 8, 2000, 100, 1000 58 / 55;
+// 16, 1000, 100, 2048 91 / 84; 8, 2000, 100, 4000 131 / 112; 32, 2000, 100, 10000 929 / 765.
+bool lognorm_f16_pays(Dims d) { return (i64)d.B * d.maxT * d.V > (i64)1 << 24; }
+
+void launch_lognorm_umma(const void* E, const void* P, float* LN, float* rowRef, float* maxP,
+                         const int* inLens, const int* labLens, Dims d, float* splitWs,
+                         int* status, bool f16, bool fixup, cudaStream_t stream, const int* labels,
+                         float* EL, float* ebl) {
+  if (d.B <= 0 || d.maxT <= 0 || d.maxU <= 0) return;
+  if (!lognorm_umma_gathers(d)) labels = nullptr;
+  LogNormScratch ws;
+  const size_t floats = scratch(d, splitWs, &ws);
+  int dev = 0, nSM = 0;
+  TB200_CUDA_CHECK(cudaGetDevice(&dev));
+  TB200_CUDA_CHECK(cudaDeviceGetAttribute(&nSM, cudaDevAttrMultiProcessorCount, dev));
+  ws.nSM = std::min(nSM, kMaxSMs);
+  const size_t zeros = splitWs + floats - reinterpret_cast<float*>(ws.tickets);
+  TB200_CUDA_CHECK(cudaMemsetAsync(ws.tickets, 0, sizeof(float) * zeros, stream));
+  if (f16)
+    launch_lognorm_f16(E, P, LN, rowRef, maxP, inLens, labLens, d, ws, status, stream, labels, EL, ebl);
+  launch_tf32(E, P, LN, rowRef, maxP, inLens, labLens, d, ws, status, stream, f16 ? nullptr : labels, EL, ebl,
+              f16 ? ws.marks : nullptr);
   if (fixup) launch_lognorm_fixup(E, P, LN, inLens, labLens, d, stream);
 }
 
