@@ -134,6 +134,24 @@ def test_frames_cut_into_parts(B, T, U, V):
         assert not eg_t[b, int(il[b]):].any() and not pg_t[b, int(ll[b]) + 1:].any()
 
 
+@pytest.mark.parametrize("U", [128, 129, 136, 137, 144, 145, 159, 160, 161, 200])
+@pytest.mark.parametrize("T,V", [(1, 64), (33, 132), (95, 260)])
+def test_label_axes_around_one_launch(U, T, V):
+    """129 to 160 positions in one launch, more in two: every rounding of the axis, label lists of one and of two
+    warps more, ragged lengths that end in the first 128 positions and behind them."""
+    B = 4
+    E, P, labels, il, ll, deltas = make(B, T, U, V, seed=U + V)
+    ll[0], ll[1], ll[2], ll[3] = U - 1, min(128, U - 1), 127, 5
+    il[0], il[1], il[2], il[3] = T, T, max(1, T - 1), 0
+    case = (E, P, labels, il, ll, deltas)
+    _, eg_s, pg_s = grads(*case, path=1)
+    _, eg_t, pg_t = grads(*case, path=2)
+    assert (eg_t - eg_s).abs().max().item() <= 1e-3 * eg_s.abs().max().item()
+    assert (pg_t - pg_s).abs().max().item() <= 1e-3 * pg_s.abs().max().item()
+    for b in range(B):
+        assert not eg_t[b, int(il[b]):].any() and not pg_t[b, int(ll[b]) + 1:].any()
+
+
 @pytest.mark.parametrize("T,U,V,hi", [(70, 100, 100, 100), (33, 128, 132, 4), (95, 40, 64, 64), (64, 18, 128, 128),
                                       (40, 151, 36, 36), (50, 201, 128, 3), (40, 60, 2048, 20)])
 def test_labels_that_are_not_staged(T, U, V, hi):

@@ -73,7 +73,13 @@ constexpr int kStageRows = 2 + kMaxStagedLabels;  // row shifts, blank-arc sums,
 constexpr int kMaxRing = 4;
 
 constexpr int kTileFrames = 48;   // frames of a tile, roughly (the tile height depends on the label axis)
-constexpr int kMaxPos = 128;      // label positions of a launch
+// Label positions of a launch.  One launch for 129..160 of them, in tiles of 32 frames (all that tensor
+// memory leaves), reads E once and writes egrads once where two over parts of the axis do so twice:
+// B = 64, T = 750..1500, U' = 76..151, V = 4096 948 -> 805 us, label_overflow 17 -> 9.
+// An instance of its own: built for 160, the kernel takes 2 to 4 % longer on shorter axes.
+constexpr int kMaxPos = 128, kMaxPosWide = 160;
+bool wide(int maxU, int passes) { return passes == 2 && maxU > kMaxPos && maxU <= kMaxPosWide; }
+int launch_positions(int maxU, int passes) { return wide(maxU, passes) ? maxU : std::min(maxU, kMaxPos); }
 
 struct GradSplit {
   i64 whole;
@@ -95,14 +101,14 @@ struct GradParams {
   void* pgrads;
   int* status;
   int maxT, maxU, V, blank;
-  // Label axes of 129..256 positions run as two launches over the position ranges
+  // Longer label axes run as two launches over the position ranges
   // [uOff, uOff + 128): each computes its rows of pgrads and its share of egrads (the sum over
   // its positions and their label-arc terms); the first launch writes egrads (and carries the
   // blank-arc terms and the zero padding), the second ADDS its tiles to it (accumulate: the
   // stores become TMA reduce-adds).
   int uOff, accumulate;
   int ldT;      // maxT rounded up to 4: row length of nref / eBlank / emT
-  int ldW;      // columns of W (multiple of 32, <= 128)
+  int ldW;      // columns of W (multiple of 32, <= POS)
   int N2;       // GEMM2 N: maxU rounded up to 16 (<= ldW)
   int Ku;       // maxU rounded up to 8 = GEMM1 K
   int stagesE, stagesW;
@@ -112,7 +118,7 @@ struct GradParams {
   int blocksV;  // blocks of 128 vocabulary columns
   int whole;    // items (utterance, block) that one CTA processes alone
   int parts;    // CTAs of each of the others
-  float* partial;     // [items cut, parts, kMaxPos positions, 128 columns] their sums over their frames
+  float* partial;     // [items cut, parts, POS positions, 128 columns] their sums over their frames
   unsigned* tickets;  // [items cut] parts done: zero on entry, zero again on exit
 };
 
@@ -153,7 +159,8 @@ __device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) 
 // ESPLIT / PSPLIT: split exp(E) / exp(P) into TF32 hi + lo (two MMAs per k-step) instead
 // of rounding once.  BF: E, P and both gradients are bf16 in memory (converted exactly to fp32
 // on the way in, rounded to nearest on the way out; everything in between is the fp32 path).
-template <int TB, bool ESPLIT, bool PSPLIT, bool BF = false>
+// POS: label positions at most.
+template <int TB, bool ESPLIT, bool PSPLIT, bool BF, int POS>
 __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
     const __grid_constant__ GradMaps tm, const GradParams p) {
   using TIO = typename std::conditional<BF, bf16, float>::type;
@@ -169,8 +176,8 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
   const int b = item / p.blocksV, v0 = (item - b * p.blocksV) * kVBlock;
   const int T = min(p.inLens[b], p.maxT), Utot = min(p.labLens[b] + 1, p.maxU);
   // my range of label positions: local u <-> position uOff + u; U of them belong to the utterance
-  const int U = max(0, min(Utot - p.uOff, 128));
-  const int rowsMine = min(128, p.maxU - p.uOff);   // rows of pgrads this launch owns
+  const int U = max(0, min(Utot - p.uOff, POS));
+  const int rowsMine = min(POS, p.maxU - p.uOff);   // rows of pgrads this launch owns
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float delta = p.deltas ? p.deltas[b] : 1.0f;
   TIO* eg = static_cast<TIO*>(p.egrads) + (i64)b * p.maxT * p.V;
@@ -221,10 +228,10 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
   __shared__ uint64_t barPReady, barD2Done;
   __shared__ uint32_t tmemBase;
   __shared__ int abortFlag;
-  __shared__ int sWarpCnt[4];
-  __shared__ short sListU[128], sListV[128];
-  __shared__ int sLab[128];
-  __shared__ float sPb[128], sPl[128];
+  __shared__ int sWarpCnt[POS / 32];
+  __shared__ short sListU[POS], sListV[POS];
+  __shared__ int sLab[POS];
+  __shared__ float sPb[POS], sPl[POS];
   __shared__ int sLastPart, sSplit[3];   // (the split: not kept in registers through the loops)
 
   // (the blank-arc terms go with the launch that writes egrads)
@@ -257,7 +264,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
   // (kept in label-position order so repeated labels are combined deterministically).
   bool inBlock = false;
   int myLab = -1;
-  if (threadIdx.x < 128) {
+  if (threadIdx.x < POS) {
     const int u = threadIdx.x;
     if (u < U) {
       sPb[u] = p.pBlank[(i64)b * p.maxU + p.uOff + u];
@@ -276,7 +283,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (threadIdx.x < 128) {
+  if (threadIdx.x < POS) {
     const unsigned m = __ballot_sync(0xffffffffu, inBlock);
     int pos = __popc(m & ((1u << lane) - 1));
     for (int w = 0; w < warp; ++w) pos += sWarpCnt[w];
@@ -286,7 +293,9 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
     }
   }
   __syncthreads();
-  const int nList = sWarpCnt[0] + sWarpCnt[1] + sWarpCnt[2] + sWarpCnt[3];
+  int nList = 0;
+#pragma unroll
+  for (int w = 0; w < POS / 32; ++w) nList += sWarpCnt[w];
   const int nStaged = min(nList, kMaxStagedLabels);
 
   const uint32_t tBase = tmemBase;
@@ -373,7 +382,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
     }
   } else if (warp == kWarpWLoad) {
     // ---------------- W loader: both copies of W tile i into W stage i % SW ----------------
-    // Lanes 0..7: one 32-column box each (even lanes the K-major copy, odd the MN-major one).
+    // One 32-column box a lane (even lanes the K-major copy, odd the MN-major one).
     if (lane == 0) {
       tma_prefetch_desc(&tm.Wk);
       tma_prefetch_desc(&tm.Wmn);
@@ -391,7 +400,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
       if (lane == 0) mbar_arrive_expect_tx(&barWFull[s], (uint32_t)(2 * wBytes));
       __syncwarp();
       const int j = lane >> 1;
-      if (lane < 8 && j < nUB) {
+      if (lane < POS / 16 && j < nUB) {
         if (lane & 1) tma_load_3d(st + wBytes + j * kBoxBytes, &tm.Wmn, &barWFull[s], p.uOff + 32 * j, t0, b);
         else tma_load_3d(st + j * kBoxBytes, &tm.Wk, &barWFull[s], p.uOff + 32 * j, t0, b);
       }
@@ -428,7 +437,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
         const uint64_t bW0 = descW + (uint64_t)((uint32_t)(s * wStage) >> 4);
         const uint32_t d1 = tBase + cD1 + db * TB;
 #pragma unroll
-        for (int ks = 0; ks < 16; ++ks) {  // Ku <= 128: at most 16 k-steps, constants when unrolled
+        for (int ks = 0; ks < POS / 8; ++ks) {  // at most Ku / 8 k-steps, constants when unrolled
           if (ks < kSteps1) {
             const uint64_t bW = bW0 + (uint64_t)(((ks >> 2) * kBoxBytes + (ks & 3) * 32) >> 4);
             mma_tf32_ts(d1, tBase + cPhi + ks * 8, bW, idesc1, ks ? 1u : 0u);
@@ -664,10 +673,10 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
     if (ok) ok = mbar_wait(&barD2Done, 0, abortp, p.status, kStatusTimeoutMma);
     ok = __all_sync(0xffffffffu, ok);
     bool writer = ok;
-    const float* partials = p.partial + (size_t)cut * p.parts * (kMaxPos * kVBlock) + vl;
+    const float* partials = p.partial + (size_t)cut * p.parts * (POS * kVBlock) + vl;
     if (nParts > 1) {
       // my sums over my frames (NaN if they never came); the part that finishes last goes on
-      float* mine = p.partial + ((size_t)cut * p.parts + myPart) * (kMaxPos * kVBlock) + vl;
+      float* mine = p.partial + ((size_t)cut * p.parts + myPart) * (POS * kVBlock) + vl;
       if (ok) tc_fence_after();
       for (int u0 = 8 * share; u0 < p.Ku; u0 += 32) {
         uint32_t d2[8];
@@ -706,7 +715,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
             for (int z = 0; z < 4; ++z)
 #pragma unroll
               for (int j = 0; j < 8; ++j)
-                x[z][j] = __ldcg(partials + (size_t)min(z0 + z, nParts - 1) * (kMaxPos * kVBlock) + (u0 + j) * kVBlock);
+                x[z][j] = __ldcg(partials + (size_t)min(z0 + z, nParts - 1) * (POS * kVBlock) + (u0 + j) * kVBlock);
 #pragma unroll
             for (int z = 0; z < 4; ++z)
               if (z0 + z < nParts) {
@@ -770,15 +779,15 @@ int pow2_cols(int x) {
 // Measured (B = 8, T = 2000, U = 100, V = 100): 27 us, 35 with a thread per frame.  (Walking the unstaged
 // positions inside the gradient kernel's loop costs that kernel 7 % whether it has any or not.)
 constexpr int kOvfFrames = 32;
-template <typename TIO>
+template <typename TIO, int POS>
 __global__ void __launch_bounds__(128) label_overflow_kernel(
     const int* __restrict__ labels, const float* __restrict__ emT, TIO* __restrict__ egrads,
     const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT, int maxU, int V,
     int ldT, int uOff, int span, int framesPerCta) {
-  constexpr int kWords = (kMaxPos + 31) / 32;
+  constexpr int kWords = POS / 32;
   __shared__ unsigned sMask[kWords];
-  __shared__ short sU[kMaxPos], sV[kMaxPos], sNext[kMaxPos];
-  __shared__ float sEm[kMaxPos][kOvfFrames + 1];
+  __shared__ short sU[POS], sV[POS], sNext[POS];
+  __shared__ float sEm[POS][kOvfFrames + 1];
   const int b = blockIdx.y, v0 = blockIdx.x * kVBlock, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int T = min(inLens[b], maxT), tBeg = blockIdx.z * framesPerCta, tEnd = min(T, tBeg + framesPerCta);
   // the labelled positions of the launch's range: uOff + u, u < n
@@ -875,7 +884,7 @@ TileCfg pick_tile(int Ku, int ldW, int N2, int passes, int staticSmem, bool bf =
   return best;
 }
 
-template <int TB, bool ESPLIT, bool PSPLIT, bool BF = false>
+template <int TB, bool ESPLIT, bool PSPLIT, bool BF = false, int POS = kMaxPos>
 void launch_variant(const GradMaps& tm, GradParams p, TileCfg cfg, unsigned ctas, cudaStream_t stream) {
   const int eStage = e_stage_bytes(TB, BF);
   const int wStage = 2 * (p.ldW / 32) * TB * 128;
@@ -887,9 +896,9 @@ void launch_variant(const GradMaps& tm, GradParams p, TileCfg cfg, unsigned ctas
   p.tmemCols = pow2_cols(cols);
   size_t smem = (size_t)cfg.SE * eStage + (size_t)cfg.SW * wStage + 1024;
   if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it may hold all 512 TMEM columns
-  allow_dyn_smem(grads_umma_kernel<TB, ESPLIT, PSPLIT, BF>, 227 * 1024 - kStaticSmemBound);
+  allow_dyn_smem(grads_umma_kernel<TB, ESPLIT, PSPLIT, BF, POS>, 227 * 1024 - kStaticSmemBound);
   ScopedKernel sk("grads_umma", stream);
-  grads_umma_kernel<TB, ESPLIT, PSPLIT, BF><<<ctas, kGradThreads, smem, stream>>>(tm, p);
+  grads_umma_kernel<TB, ESPLIT, PSPLIT, BF, POS><<<ctas, kGradThreads, smem, stream>>>(tm, p);
 }
 
 }  // namespace
@@ -899,14 +908,13 @@ int grads_umma_ld_t(Dims d) { return (int)round_up64(d.maxT > 0 ? d.maxT : 1, 4)
 size_t grads_umma_partial_floats(Dims d) {
   if (d.B <= 0 || d.maxT <= 0 || d.V <= 0) return 0;
   const GradSplit s = grad_split(d);
-  return (size_t)s.cut * (s.parts > 1 ? s.parts : 0) * kMaxPos * kVBlock;
+  return (size_t)s.cut * (s.parts > 1 ? s.parts : 0) * (wide(d.maxU, 2) ? kMaxPosWide : kMaxPos) * kVBlock;
 }
 
 bool grads_umma_supported(const void* E, const void* P, const void* egrads,
                           const void* pgrads, Dims d, int passes) {
   const bool bf = d.dtype == kDtypeBf16;
-  // (label axes of 129..256 positions: two launches, the second adding to egrads -- fp32 only,
-  // a bf16 sum would be rounded twice)
+  // (two launches: the second adds to egrads -- fp32 only, a bf16 sum would be rounded twice)
   if (d.V % (bf ? 8 : 4) != 0 || d.V < 32 || d.maxU < 1 || d.maxU > (bf ? 128 : 256) || d.B > 65535 ||
       grad_split(d).ctas() > 0x7fffffff)
     return false;
@@ -916,7 +924,7 @@ bool grads_umma_supported(const void* E, const void* P, const void* egrads,
   // the same routing as for E: the SIMT kernels
   for (const void* ptr : {E, P, egrads, pgrads})
     if ((reinterpret_cast<uintptr_t>(ptr) & 15) != 0) return false;
-  const int n = std::min(d.maxU, 128);   // positions of the (first) launch
+  const int n = launch_positions(d.maxU, passes);   // of the (first) launch
   return pick_tile((int)round_up64(n, 8), (int)round_up64(n, 32), (int)round_up64(n, 16), passes,
                    kStaticSmemBound, bf).TB > 0;
 }
@@ -940,9 +948,9 @@ void launch_grads_umma(const void* E, const void* P, const float* maxP, const fl
   p.whole = (int)split.whole; p.parts = split.parts;
   p.partial = partial; p.tickets = tickets;
   const uint64_t V = d.V, T = d.maxT, B = d.B, ldWall = grads_umma_ld_w(d), ldT = p.ldT, U = d.maxU;
-  // one launch per range of 128 label positions (see GradParams::uOff)
-  for (int uOff = 0; uOff < d.maxU; uOff += 128) {
-    const int n = std::min(128, d.maxU - uOff);
+  const bool one = wide(d.maxU, passes);
+  for (int uOff = 0, n; uOff < d.maxU; uOff += n) {   // (see GradParams::uOff)
+    n = launch_positions(d.maxU - uOff, passes);
     p.uOff = uOff;
     p.accumulate = uOff > 0 ? 1 : 0;
     p.ldW = (int)round_up64(n, 32);
@@ -972,6 +980,9 @@ void launch_grads_umma(const void* E, const void* P, const float* maxP, const fl
       if (TB == 64) launch_variant<64, true, false, true>(tm, p, cfg, (unsigned)split.ctas(), stream);
       else if (TB == 48) launch_variant<48, true, false, true>(tm, p, cfg, (unsigned)split.ctas(), stream);
       else launch_variant<32, true, false, true>(tm, p, cfg, (unsigned)split.ctas(), stream);
+    } else if (one) {
+      if (TB != 32) throw std::logic_error("129..160 positions: tiles of 32 frames");   // (pick_tile)
+      launch_variant<32, true, false, false, kMaxPosWide>(tm, p, cfg, (unsigned)split.ctas(), stream);
     } else if (passes == 3) GO_TB(true, true);
     else if (passes == 2) GO_TB(true, false);
     else GO_TB(false, false);
@@ -985,12 +996,13 @@ void launch_grads_umma(const void* E, const void* P, const float* maxP, const fl
       // many blocks: almost every CTA returns at once -- keep them few)
       const int framesPerCta = d.V <= 1024 ? 2 * kOvfFrames : 1024;
       const dim3 grid(div_up(d.V, kVBlock), d.B, div_up(d.maxT, framesPerCta));
-      if (bf)
-        label_overflow_kernel<bf16><<<grid, kVBlock, 0, stream>>>(
-            labels, emT, static_cast<bf16*>(egrads), inLens, labLens, d.maxT, d.maxU, d.V, p.ldT, uOff, n, framesPerCta);
-      else
-        label_overflow_kernel<float><<<grid, kVBlock, 0, stream>>>(
-            labels, emT, static_cast<float*>(egrads), inLens, labLens, d.maxT, d.maxU, d.V, p.ldT, uOff, n, framesPerCta);
+#define GO(TIO, POS)                                                                          \
+  label_overflow_kernel<TIO, POS><<<grid, kVBlock, 0, stream>>>(                              \
+      labels, emT, static_cast<TIO*>(egrads), inLens, labLens, d.maxT, d.maxU, d.V, p.ldT, uOff, n, framesPerCta)
+      if (bf) GO(bf16, kMaxPos);
+      else if (one) GO(float, kMaxPosWide);
+      else GO(float, kMaxPos);
+#undef GO
       TB200_CHECK_LAUNCH();
     }
   }

@@ -145,7 +145,7 @@ int grads_umma_ld_t(Dims d);  // row length of nref / ebl / emT: maxT rounded up
 bool grads_umma_supported(const void* E, const void* P, const void* egrads,
                           const void* pgrads, Dims d, int passes);
 // E, P, egrads and pgrads are of d.dtype (bf16: passes = 2 only, label axes up to 128; fp32:
-// label axes up to 256 positions, those above 128 as two launches over halves of the axis).
+// label axes up to 256 positions, long ones as two launches over parts of the axis).
 // partial: scratch of grads_umma_partial_floats(d) floats; tickets: kGradTickets zeros, left zero.
 constexpr int kGradTickets = 148;   // one per SM
 size_t grads_umma_partial_floats(Dims d);
