@@ -563,19 +563,15 @@ __global__ void __launch_bounds__(32) alpha_natural_kernel(
 // is no arc (natural: from the pair rows of alpha_natural_kernel, by the accurate expf).  One warp
 // per 4 diagonals.  Bound by memory: a pair and an alpha (12 bytes) read, 8 written per node.
 constexpr int kFactorRows = 4, kFactorWarps = 8;
-static_assert(kGradTickets <= 32 * kFactorWarps, "one thread per ticket");
 template <int NPL>
 __global__ void __launch_bounds__(32 * kFactorWarps) gamma_factors_kernel(
     const float2* __restrict__ arcs, const float* __restrict__ alphas,
     const float* __restrict__ deltas, const NaturalTerms n, float2* __restrict__ F,
-    unsigned* __restrict__ occTicket, unsigned* __restrict__ gradTickets, i64 stride, int nDiag, const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT,
+    unsigned* __restrict__ occTicket, i64 stride, int nDiag, const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT,
     int maxU) {
   constexpr int ld = 32 * NPL, kPieces = NPL / 2;
   const int b = blockIdx.y, lane = threadIdx.x & 31;
-  if (blockIdx.x == 0) {   // the counters of the kernels behind this one
-    if (threadIdx.x == 0) occTicket[b] = 0u;
-    if (b == 0 && threadIdx.x < kGradTickets) gradTickets[threadIdx.x] = 0u;
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) occTicket[b] = 0u;
   const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU), S = T + U - 1;
   const int d0 = (blockIdx.x * kFactorWarps + (threadIdx.x >> 5)) * kFactorRows, u0 = NPL * lane;
   if (T <= 0 || U <= 0 || d0 >= S || u0 >= U) return;
@@ -651,11 +647,13 @@ __global__ void __launch_bounds__(32 * kFactorWarps) gamma_factors_kernel(
 // blank) down to 0.
 template <int NPL>
 __global__ void __launch_bounds__(32) gamma_sweep_kernel(
-    const float2* __restrict__ F, float* __restrict__ g, i64 stride, const int* __restrict__ inLens,
-    const int* __restrict__ labLens, int maxT, int maxU) {
+    const float2* __restrict__ F, float* __restrict__ g, unsigned* __restrict__ gradTickets, i64 stride,
+    const int* __restrict__ inLens, const int* __restrict__ labLens, int maxT, int maxU) {
   constexpr int ld = 32 * NPL;
   extern __shared__ __align__(128) uint8_t smemG[];
   const int b = blockIdx.x, lane = threadIdx.x;
+  if (b == 0)   // the counters of the gradient kernel behind this one
+    for (int i = lane; i < kGradTickets; i += 32) gradTickets[i] = 0u;
   const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
   if (T <= 0 || U <= 0) return;
   const int S = T + U - 1, nBlocks = (S + kDiag - 1) / kDiag, u0 = NPL * lane;
@@ -1117,7 +1115,7 @@ void launch_sweep_backward(const SweepScratch& w, const float* P, const float* b
     const dim3 grid(div_up(g.nDiag, kFactorRows * kFactorWarps), d.B);
 #define CALL(NPL)                                                                              \
   gamma_factors_kernel<NPL><<<grid, 32 * kFactorWarps, 0, stream>>>(                           \
-      arcs, alphas, alphaDeltas, n, w.F, w.ticket, w.gradTickets, g.stride, g.nDiag, inLens, labLens, d.maxT, d.maxU)
+      arcs, alphas, alphaDeltas, n, w.F, w.ticket, g.stride, g.nDiag, inLens, labLens, d.maxT, d.maxU)
     const NaturalTerms n{P, blankEmissions, labels, d.V, d.blank};
     TB200_BY_NPL_ANY(g.npl, CALL);
 #undef CALL
@@ -1128,7 +1126,8 @@ void launch_sweep_backward(const SweepScratch& w, const float* P, const float* b
     ScopedKernel sk("gamma_sweep", stream);
 #define CALL(NPL)                                                                              \
   allow_dyn_smem(gamma_sweep_kernel<NPL>, smem);                                               \
-  gamma_sweep_kernel<NPL><<<d.B, 32, smem, stream>>>(w.F, w.g, g.stride, inLens, labLens, d.maxT, d.maxU)
+  gamma_sweep_kernel<NPL><<<d.B, 32, smem, stream>>>(w.F, w.g, w.gradTickets, g.stride, inLens,   \
+                                                   labLens, d.maxT, d.maxU)
     TB200_BY_NPL_ANY(g.npl, CALL);
 #undef CALL
     TB200_CHECK_LAUNCH();
