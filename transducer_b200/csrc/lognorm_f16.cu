@@ -123,10 +123,10 @@ __device__ __forceinline__ void split_f16(float a, float b, uint32_t& hi, uint32
 // the rows' sums of exp(P - maxP).  Bound by memory: one read (the second comes from L2), one write.
 // ---------------------------------------------------------------------------------
 template <typename TIn>
-__global__ void __launch_bounds__(256) expp_f16_kernel(
+__global__ void __launch_bounds__(1024) expp_f16_kernel(
     const TIn* __restrict__ P, uint8_t* __restrict__ out, float* __restrict__ maxP,
     float* __restrict__ sumP, const int* __restrict__ labLens, int maxU, int V, int nPad, int kPad) {
-  __shared__ float red[8], redS[8];
+  __shared__ float red[32], redS[32];
   const int b = blockIdx.y, u = blockIdx.x;
   const int U = min(labLens[b] + 1, maxU);
   if (u >= U) {
@@ -145,8 +145,7 @@ __global__ void __launch_bounds__(256) expp_f16_kernel(
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
   __syncthreads();
   m = red[0];
-#pragma unroll
-  for (int k = 1; k < 8; ++k) m = fmaxf(m, red[k]);
+  for (int k = 1; k < (int)blockDim.x / 32; ++k) m = fmaxf(m, red[k]);
   float s = 0.0f;
   for (int v = threadIdx.x; v < kPad / 4; v += blockDim.x) {
     float xs[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -167,7 +166,7 @@ __global__ void __launch_bounds__(256) expp_f16_kernel(
   if ((threadIdx.x & 31) == 0) redS[threadIdx.x >> 5] = s;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int k = 1; k < 8; ++k) s += redS[k];
+    for (int k = 1; k < (int)blockDim.x / 32; ++k) s += redS[k];
     maxP[(i64)b * maxU + u] = m;
     sumP[(i64)b * maxU + u] = s;
   }
@@ -616,10 +615,10 @@ void launch_lognorm_f16(const void* E, const void* P, float* LN, float* rowRef, 
     ScopedKernel sk("expp_f16", stream);
     const dim3 grid(d.maxU, d.B);
     if (bf)
-      expp_f16_kernel<bf16><<<grid, 256, 0, stream>>>(static_cast<const bf16*>(P), operand, maxP,
+      expp_f16_kernel<bf16><<<grid, expp_threads(d.V), 0, stream>>>(static_cast<const bf16*>(P), operand, maxP,
                                                       ws.sumP, labLens, d.maxU, d.V, rows, kPad);
     else
-      expp_f16_kernel<float><<<grid, 256, 0, stream>>>(static_cast<const float*>(P), operand, maxP,
+      expp_f16_kernel<float><<<grid, expp_threads(d.V), 0, stream>>>(static_cast<const float*>(P), operand, maxP,
                                                        ws.sumP, labLens, d.maxU, d.V, rows, kPad);
   }
   TB200_CHECK_LAUNCH();

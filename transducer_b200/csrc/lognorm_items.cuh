@@ -7,6 +7,14 @@
 namespace tb200 {
 namespace lognorm {
 
+// Threads of the CTA that brings a row of P to exp(P) pairs, in two passes over it.  The 2048 threads of an SM
+// hold 8 rows with 256 of them, and the second pass finds the row in L2 only while 8 rows per SM leave
+// room there: fewer and larger CTAs for long rows.  Short rows want many.  us with 256 / 512 / 1024, TF32
+// pairs: B = 32, U' <= 101, V = 10000 77 / 67 / 91, V = 32000 273 / 256 / 216; fp16 pairs, B = 64, U' <= 151
+// V = 4096 62 / 85 / 142, V = 8192 108 / 119 / 185, U' <= 201 V = 16384 363 / 278 / 337, V = 24000 562 / 458 /
+// 487, V = 32000 745 / 667 / 602.
+inline int expp_threads(int V) { return V <= 8192 ? 256 : V <= 28000 ? 512 : 1024; }
+
 constexpr int kTileM = 128;    // frames per work item (UMMA M)
 constexpr int kChunkK = 32;    // words per chunk of the vocabulary
 constexpr int kMaxSMs = 256;   // slots for the partial sums of split tiles

@@ -136,11 +136,11 @@ using namespace lognorm;
 // exp(P - maxP) split into TF32 hi/lo as [B][nPad][kPad]: rows u < U_b, columns zero-padded to kPad
 // ---------------------------------------------------------------------------------
 template <typename TIn>
-__global__ void __launch_bounds__(256) expp_split_kernel(
+__global__ void __launch_bounds__(1024) expp_split_kernel(
     const TIn* __restrict__ P, float* __restrict__ bHi, float* __restrict__ bLo,
     float* __restrict__ maxP, const int* __restrict__ labLens, int maxU, int V, int nPad,
     int kPad, const int* __restrict__ only, int tilesX) {
-  __shared__ float red[8];
+  __shared__ float red[32];
   const int b = blockIdx.y, u = blockIdx.x;
   if (only) {   // the utterances with a marked tile
     if (only[0] == 0) return;
@@ -172,8 +172,7 @@ __global__ void __launch_bounds__(256) expp_split_kernel(
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
   __syncthreads();
   m = red[0];
-#pragma unroll
-  for (int k = 1; k < 8; ++k) m = fmaxf(m, red[k]);
+  for (int k = 1; k < (int)blockDim.x / 32; ++k) m = fmaxf(m, red[k]);
   for (int v = threadIdx.x; v < kPad / 4; v += blockDim.x) {
     float xs[4] = {0.0f, 0.0f, 0.0f, 0.0f}, h[4], l[4];
     if (4 * v < V) {
@@ -664,11 +663,13 @@ static void launch_tf32(const void* E, const void* P, float* LN, float* rowRef, 
   float* bLo = ws.operand + (size_t)d.B * nPad * kPad;
   {
     ScopedKernel sk("expp_split", stream);
+    // (mostly nothing is marked: small CTAs leave again sooner)
+    const int threads = only ? 256 : expp_threads(d.V);
     if (bf)
-      expp_split_kernel<bf16><<<dim3(nPad, d.B), 256, 0, stream>>>(
+      expp_split_kernel<bf16><<<dim3(nPad, d.B), threads, 0, stream>>>(
           static_cast<const bf16*>(P), bHi, bLo, maxP, labLens, d.maxU, d.V, nPad, kPad, only, tilesX);
     else
-      expp_split_kernel<float><<<dim3(nPad, d.B), 256, 0, stream>>>(
+      expp_split_kernel<float><<<dim3(nPad, d.B), threads, 0, stream>>>(
           static_cast<const float*>(P), bHi, bLo, maxP, labLens, d.maxU, d.V, nPad, kPad, only, tilesX);
   }
   TB200_CHECK_LAUNCH();
