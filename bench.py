@@ -696,7 +696,7 @@ NCU_TRAFFIC_BYTES = {
 
 def viterbi_algorithmic_bytes(w, il, ll):
     """Viterbi decode: E and P read once (shared by the log-normaliser and the max-plus pass),
-    three lattices written and read (log-normalisers, best label scores, packed records)."""
+    three lattices written and read (log-normalisers, best label scores, arc scores)."""
     sum_t = float(il.sum())
     sum_u = float((ll + 1).sum())
     sum_tu = float((il.double() * (ll.double() + 1)).sum())
@@ -716,6 +716,7 @@ def kernel_algorithmic_bytes(w, il, ll, elem_bytes=4):
         "lognorm_exact": 4.0 * V * (sum_t + sum_u) + 4.0 * sum_tu,
         "lognorm_factored": 4.0 * V * (sum_t + sum_u) + 4.0 * sum_tu,
         "lognorm_umma": eb * V * (sum_t + sum_u) + 4.0 * sum_tu,
+        "lognorm_f16": eb * V * (sum_t + sum_u) + 4.0 * sum_tu,
         "maxplus": 4.0 * V * (sum_t + sum_u) + 4.0 * sum_tu,
         "maxplus_pruned": 4.0 * V * sum_t + 4.0 * sum_tu,    # E rows in, scores out
         "maxplus_select_e": 4.0 * V * sum_t,
@@ -723,10 +724,11 @@ def kernel_algorithmic_bytes(w, il, ll, elem_bytes=4):
         "gamma_wavefront": 5 * 4.0 * sum_tu,
         "sweep_prep": 4 * 4.0 * sum_tu,     # LN and the label emission in, a pair out
         "alpha_sweep": 3 * 4.0 * sum_tu,    # a pair in, alpha out
+        "score_sweep": 2 * 4.0 * sum_tu,    # a pair in
         "gamma_factors": 5 * 4.0 * sum_tu,  # a pair and alpha in, the factors out
         "gamma_sweep": 3 * 4.0 * sum_tu,    # the factors in, g out
         "occupancy": 6 * 4.0 * sum_tu,      # factors, g and LN in, W and the label arcs out
-        "viterbi_warp": 4 * 4.0 * sum_tu,  # one float4 record per node in
+        "viterbi_warp": 2 * 4.0 * sum_tu,  # a pair per node in
         "egrad_simt": 4.0 * V * sum_t + 4.0 * V * n * w.T + 4.0 * V * sum_u,
         "pgrad_simt": 4.0 * V * sum_t + 4.0 * V * n * (w.U + 1) + 4.0 * V * sum_u,
         "grads_umma": eb * V * (sum_t + sum_u) + eb * V * n * (w.T + w.U + 1) + 4.0 * sum_tu,

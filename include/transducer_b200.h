@@ -51,8 +51,9 @@ void* tb200_get_stream(void);
 
 /* Tuning / test switches.  Keys:
  *   "lognorm_path"  0 auto, 1 exact SIMT logsumexp, 2 tensor-core factored GEMM, 3 fp32 factored
- *                   SIMT.  Auto takes 2 where TMA can address the inputs (alphabetSize % 4 == 0 and
- *                   >= 32, maxLabelLength <= 256, 16-byte aligned), else 1 or 3 by the number of nodes
+ *                   SIMT, 4 as 2 on fp16 pairs.  Auto takes 2 where TMA can address the inputs
+ *                   (alphabetSize % 4 == 0 and >= 32, maxLabelLength <= 256, 16-byte aligned), or
+ *                   4 for more than 2^24 scores if no gradients follow, else 1 or 3 by the number of nodes
  *   "grads_path"    0 auto, 1 SIMT, 2 tensor-core
  *   "grad_passes"   operand precision of the tensor-core gradient kernel.  The lattice
  *                   weights are always rounded once to TF32.  1: exp(E), exp(P) rounded
