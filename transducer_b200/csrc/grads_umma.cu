@@ -166,9 +166,9 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
   using TIO = typename std::conditional<BF, bf16, float>::type;
   constexpr int TBH = TB / 2;  // frames per owner half
   static_assert(TBH % 8 == 0, "tile halves move through TMEM in 8-column pieces");
-  int item = blockIdx.x, part = 0, parts = 1;
-  const int cutItem = item < p.whole ? 0 : (item - p.whole) / p.parts;
+  int item = blockIdx.x, part = 0, parts = 1, cutItem = 0;
   if (item >= p.whole) {
+    cutItem = (item - p.whole) / p.parts;
     part = item - p.whole - cutItem * p.parts;
     parts = p.parts;
     item = p.whole + cutItem;
@@ -196,10 +196,13 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
   }
   // my tiles: [tile0, tile0 + nTiles) of the utterance
   const int tilesAll = (T + TB - 1) / TB;
-  parts = min(parts, tilesAll);
-  if (part >= parts) return;
-  const int tile0 = (int)((i64)tilesAll * part / parts);
-  const int nTiles = (int)((i64)tilesAll * (part + 1) / parts) - tile0;
+  int tile0 = 0, nTiles = tilesAll;
+  if (parts > 1) {   // (at most 16 parts of 2^26 tiles.  Whole items, most of them, skip the divisions.)
+    parts = min(parts, tilesAll);
+    if (part >= parts) return;
+    tile0 = tilesAll * part / parts;
+    nTiles = tilesAll * (part + 1) / parts - tile0;
+  }
 
   extern __shared__ uint8_t smemRaw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) &
@@ -215,8 +218,11 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
   constexpr int kEStage = e_stage_bytes(TB, BF);   // E tile + kStageRows rows of scalars
   // Do the two halves of a group of column owners take alternate tiles, or halves of every tile?
   // Alternate where the ring and both pairs of tensor-memory operands make every tile of a half find
-  // its own ring slots and copies (all even); operand precision 3 leaves less.
-  const bool alt = SE == 4 && p.eBufs == 2 && p.dBufs == 2;
+  // its own ring slots and copies (all even; operand precision 3 leaves less), and where it is faster:
+  // halves / alternate, us, B = 32: tiles of 32 frames, U' = 151, V = 4096, T = 64 119 / 115, T = 512 243 / 235;
+  // of 48, U' = 101, V = 10000, T = 144 261 / 266, T = 240 307 / 307, T = 288 335 / 333, T = 2000 bf16 996 / 972;
+  // of 64, U' = 61, T = 64 160 / 165, T = 768 409 / 419.
+  const bool alt = (TB == 32 || (TB == 48 && nTiles >= 6)) && SE == 4 && p.eBufs == 2 && p.dBufs == 2;
   const int owners = alt ? kGroupWarps / 2 : kGroupWarps;   // warps of a group per tile
   const int wBytes = nUB * kBoxBytes;
   const int wStage = 2 * wBytes;               // K-major copy, MN-major copy
@@ -488,7 +494,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
     // gradient arithmetic.  Within a group the halves h = 0,1 take alternate tiles (or, see `alt`, split
     // the frames of a tile): half of what a tile costs a warp are round trips to barriers and to
     // tensor memory, ~1200 cycles whatever the frames (cycle stamps; without any copy to or from memory
-    // and without most of the MMAs the kernel was as slow).  Measured: B = 32, T = 1500..2000, U' = 61..101,
+    // and without most of the MMAs the kernel was as slow).  B = 32, T = 1500..2000, U' = 61..101,
     // V = 10000 1086 -> 1082 us, bf16 996 -> 972, B = 64, U' = 76..151, V = 4096 958 -> 947.  All 16 warps split the label positions
     // of the prologue and the epilogue.
     const int grp = warp >> 3, q = warp & 3, h = (warp >> 2) & 1;
