@@ -117,7 +117,7 @@ def test_unsupported_shape_is_refused_when_forced():
 
 # (utterances x blocks of 128 columns) that one CTA per item would leave most SMs to: their frames are cut
 # into parts; with short and empty utterances that have fewer tiles than there are parts
-@pytest.mark.parametrize("B,T,U,V", [(1, 96, 5, 128), (1, 97, 5, 128), (3, 700, 20, 100), (2, 2000, 101, 64),
+@pytest.mark.parametrize("B,T,U,V", [(1, 96, 5, 128), (1, 97, 5, 128), (1, 191, 5, 128), (1, 192, 5, 128), (3, 700, 20, 100), (2, 2000, 101, 64),
                                      (37, 200, 9, 520), (5, 300, 70, 4000), (150, 100, 5, 128), (2, 500, 151, 256)])
 def test_frames_cut_into_parts(B, T, U, V):
     E, P, labels, il, ll, deltas = make(B, T, U, V, seed=B + T, repeat_labels=V == 64)

@@ -134,7 +134,7 @@ GradSplit grad_split(Dims d) {
   const i64 n = (i64)div_up(d.V, kVBlock) * d.B;
   const int rem = (int)(n % kSMs);
   int parts = rem > 0 ? std::min(kMaxParts, kSMs / rem) : 1;
-  parts = std::min(parts, div_up(d.maxT, 2 * kTileFrames));
+  parts = std::min(parts, d.maxT / (2 * kTileFrames));
   if (parts < 2) return GradSplit{n, 0, 1};
   return GradSplit{n - rem, rem, parts};
 }
