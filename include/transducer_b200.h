@@ -53,7 +53,8 @@ void* tb200_get_stream(void);
  *   "lognorm_path"  0 auto, 1 exact SIMT logsumexp, 2 tensor-core factored GEMM, 3 fp32 factored
  *                   SIMT, 4 as 2 on fp16 pairs.  Auto takes 2 where TMA can address the inputs
  *                   (alphabetSize % 4 == 0 and >= 32, maxLabelLength <= 256, 16-byte aligned), or
- *                   4 for more than 2^24 scores if no gradients follow, else 1 or 3 by the number of nodes
+ *                   4 for more than 2^24 scores in calls that no gradients follow (tb200_loss_score,
+ *                   tb200_viterbi_decode), else 1 or 3 by the number of nodes
  *   "grads_path"    0 auto, 1 SIMT, 2 tensor-core
  *   "grad_passes"   operand precision of the tensor-core gradient kernel.  The lattice
  *                   weights are always rounded once to TF32.  1: exp(E), exp(P) rounded
@@ -169,7 +170,8 @@ int tb200_viterbi_static(const float* emissions, const float* predictions,
  * logsumexp_v(E[b,t,v] + P[b,u,v]) for every valid node (padding is not written).
  * Also returns the per-row shifts the factored gradient kernels reuse:
  * rowRef [B,maxT] (a per-frame reference value <= max_v E, not necessarily the
- * maximum) and maxP [B,maxU].  workspace: tb200_log_norms_workspace_bytes(). */
+ * maximum) and maxP [B,maxU].  The results may go into tb200_forward / tb200_backward: they are
+ * those of the training call at any size.  workspace: tb200_log_norms_workspace_bytes(). */
 size_t tb200_log_norms_workspace_bytes(int batchSize, int maxInputLength,
                                        int maxLabelLength, int alphabetSize);
 int tb200_log_norms(const float* emissions, const float* predictions, float* logNorms,

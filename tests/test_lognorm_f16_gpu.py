@@ -129,3 +129,13 @@ def test_bf16_emissions(B, T, U, V):
     finally:
         abi.set_option("lognorm_path", 0)
     assert torch.equal(a, b)
+
+
+def test_log_norms_that_gradients_may_follow():
+    """tb200_log_norms feeds the separate forward and backward calls: on more than 2^24 scores it stays with the
+    kernel that the training call takes, bit for bit."""
+    E, P, il, ll = make(2, 300, 30, 32000, seed=1)
+    assert E.numel() > 1 << 24
+    m = valid(il, ll, 300, 30)
+    auto, tf32, f16 = (norms(path, E, P, il, ll)[0][m] for path in (0, 2, 4))
+    assert torch.equal(auto, tf32) and not torch.equal(auto, f16)

@@ -191,13 +191,13 @@ void need(size_t have, size_t want, const void* ws) {
 
 // Log-normalisers plus the row shifts.  With the SIMT kernels rowRef is the true row
 // maximum of E.
-// keepBits: where gradients follow, the weights behind the sweeps are rounded to TF32, and other log-normalisers,
-// however close, would flip some of those roundings (lattice_sweep.cu): the TF32 kernel at any size.
+// keepBits: where gradients follow, or may follow, the weights behind the sweeps are rounded to TF32, and other
+// log-normalisers, however close, would flip some of those roundings (lattice_sweep.cu): the TF32 kernel at any size.
 // Returns true if the pass also produced the label / blank emissions (EL, ebl) it was offered.
 bool log_norms_impl(const void* E, const void* P, float* LN, float* rowRef, float* maxP,
                     const int* inLens, const int* labLens, const Dims& d, LogNormWs& ws,
                     bool fixup = true, const int* labels = nullptr, float* EL = nullptr,
-                    float* ebl = nullptr, bool keepBits = false) {
+                    float* ebl = nullptr, bool keepBits = true) {
   if (d.B <= 0 || d.maxT <= 0 || d.maxU <= 0) return false;
   const bool can = lognorm_umma_supported(E, P, d);
   const int path = g_opt.lognorm_path;
@@ -615,7 +615,8 @@ int tb200_viterbi_decode(const float* E, const float* P, const int* inLens,
     LogNormWs lw(c, d);
     // (nodes the log-normaliser could not represent are recomputed by the re-layout)
     const bool warp = viterbi_warp_supported(d);
-    log_norms_impl(E, P, ws.LN, ws.rowRef, ws.maxP, inLens, labLens, d, lw, /*fixup=*/!warp);
+    log_norms_impl(E, P, ws.LN, ws.rowRef, ws.maxP, inLens, labLens, d, lw, /*fixup=*/!warp, nullptr, nullptr,
+                   nullptr, /*keepBits=*/false);
     best_label_scores(E, P, ws.best, inLens, labLens, d, ws.prune);
     if (warp)
       launch_viterbi_warp(E, P, ws.LN, /*fix=*/true, ws.best, ws.nodes, ws.decBits, labels, inLens,
