@@ -144,6 +144,26 @@ def test_workspace_queries_are_pure_and_monotone():
     assert _lib.lib.tb200_viterbi_decode_workspace_bytes(2, 50, 11, 30) > 0
 
 
+def test_workspace_queries_do_not_grow_for_smaller_calls():
+    """A program sizes its workspace for the largest call and keeps it (the host pipeline for its last, smaller
+    chunk): no smaller call may ask for more, whatever round of CTAs its items happen to fill."""
+    lib = _lib.lib
+    queries = [lib.tb200_loss_backward_workspace_bytes, lib.tb200_loss_forward_workspace_bytes,
+               lib.tb200_loss_saved_bytes, lib.tb200_loss_score_workspace_bytes]
+    for f in queries:
+        for V in (100, 1000, 4736, 10000):
+            for T in (200, 900):
+                for U in (31, 128, 151, 200):
+                    sizes = [f(B, T, U, V) for B in range(1, 41)]
+                    assert sizes == sorted(sizes), (V, T, U)
+        for B, V in ((1, 4736), (8, 1000), (37, 1000)):
+            for U in (31, 151):
+                sizes = [f(B, T, U, V) for T in range(1, 1700, 13)]
+                assert sizes == sorted(sizes), (B, V, U)
+            sizes = [f(B, 700, U, V) for U in range(1, 257)]
+            assert sizes == sorted(sizes), (B, V)
+
+
 def test_host_pipeline_needs_a_gpu_and_host_tensors():
     """The host-buffer pipeline is part of the product path: no CUDA device, no result."""
     import torch

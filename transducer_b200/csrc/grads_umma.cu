@@ -129,12 +129,13 @@ struct GradParams {
 // that they start last.  Every part leaves its sums over the frames in `partial`, and the one that
 // finishes last adds them in frame order.  Measured, whole / cut: 8 items of 2000 frames (V = 100)
 // 88 / 31 us, 64 items 89 / 58, 632 items (V = 10000, 40 in the last round) 335 / 311.
+constexpr int kMaxGradParts = 16;
+int parts_by_frames(int maxT) { return std::min(kMaxGradParts, maxT / (2 * kTileFrames)); }
 GradSplit grad_split(Dims d) {
-  constexpr int kSMs = kGradTickets, kMaxParts = 16;
+  constexpr int kSMs = kGradTickets;
   const i64 n = (i64)div_up(d.V, kVBlock) * d.B;
   const int rem = (int)(n % kSMs);
-  int parts = rem > 0 ? std::min(kMaxParts, kSMs / rem) : 1;
-  parts = std::min(parts, d.maxT / (2 * kTileFrames));
+  const int parts = rem > 0 ? std::min(parts_by_frames(d.maxT), kSMs / rem) : 1;
   if (parts < 2) return GradSplit{n, 0, 1};
   return GradSplit{n - rem, rem, parts};
 }
@@ -923,10 +924,12 @@ void launch_variant(const GradMaps& tm, GradParams p, TileCfg cfg, unsigned ctas
 
 int grads_umma_ld_w(Dims d) { return (int)round_up64(d.maxU > 0 ? d.maxU : 1, 32); }
 int grads_umma_ld_t(Dims d) { return (int)round_up64(d.maxT > 0 ? d.maxT : 1, 4); }
+// Room for the parts of any call of at most these sizes, not only of this one (a workspace is laid out for
+// the largest call and serves smaller ones, whose last round may hold more items): at most one part per SM.
 size_t grads_umma_partial_floats(Dims d) {
-  if (d.B <= 0 || d.maxT <= 0 || d.V <= 0) return 0;
-  const GradSplit s = grad_split(d);
-  return (size_t)s.cut * (s.parts > 1 ? s.parts : 0) * (wide(d.maxU, 2) ? kMaxPosWide : kMaxPos) * kVBlock;
+  if (d.B <= 0 || d.maxT <= 0 || d.V <= 0 || parts_by_frames(d.maxT) < 2) return 0;
+  const i64 slots = std::min<i64>(kGradTickets, (i64)div_up(d.V, kVBlock) * d.B * parts_by_frames(d.maxT));
+  return (size_t)slots * (d.maxU > kMaxPos ? kMaxPosWide : kMaxPos) * kVBlock;
 }
 
 bool grads_umma_supported(const void* E, const void* P, const void* egrads,
