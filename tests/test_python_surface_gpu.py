@@ -174,6 +174,30 @@ def test_host_pipeline_moving_valid_rows_only_gives_the_same_outputs(dtype):
         assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
 
 
+@pytest.mark.parametrize("U", [60, 151])
+@pytest.mark.parametrize("sparse", [False, True])
+def test_host_pipeline_of_costs_alone_is_the_scoring_call(U, sparse):
+    """forward_only: the bits of TransducerLoss under no_grad on the same chunks, and no state of a training call."""
+    from transducer_b200 import HostLossPipeline
+    g = torch.Generator().manual_seed(U)
+    B, T, V = 5, 200, 512
+    E = torch.randn((B, T, V), generator=g).pin_memory()
+    P = torch.randn((B, U, V), generator=g).pin_memory()
+    labels = torch.randint(1, V, (B, U - 1), generator=g, dtype=torch.int32).pin_memory()
+    il = torch.randint(T // 2, T + 1, (B,), generator=g, dtype=torch.int32).pin_memory()
+    ll = torch.randint(0, U, (B,), generator=g, dtype=torch.int32).pin_memory()
+    costs = torch.full((B,), float("nan")).pin_memory()
+    pipe = HostLossPipeline(chunk=2, slots=2, forward_only=True, valid_rows_only=sparse)
+    loss_sum = pipe(E, P, labels, il, ll, costs, None, None)
+    torch.cuda.synchronize()
+    with torch.no_grad():
+        want = torch.cat([TransducerLoss()(*(x[i:i + 2].cuda() for x in (E, P, labels, il, ll)))
+                          for i in range(0, B, 2)]).cpu()
+    assert torch.equal(costs, want)
+    assert torch.allclose(loss_sum.cpu(), want.sum().reshape(1), rtol=1e-6)
+    assert all(slot.saved is None for slot in pipe.slots)
+
+
 def test_forward_backward_can_be_captured_in_a_cuda_graph():
     """The fused calls only enqueue work (kernels, memsets) on the chosen stream, so a training
     step can be captured once and replayed."""

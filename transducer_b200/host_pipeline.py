@@ -40,10 +40,15 @@ class _Slot(object):
         self.costs = torch.empty((n,), **f32)
         self.eg = None if forward_only else torch.empty((n, T, V), **io)
         self.pg = None if forward_only else torch.empty((n, U, V), **io)
-        self.saved_bytes = _transducer.loss_saved_bytes(n, T, U, V)
-        self.saved = torch.empty(max(self.saved_bytes, 1), **u8)
-        self.fwd_bytes = _transducer.loss_forward_workspace_bytes(n, T, U, V)
-        self.bwd_bytes = 0 if forward_only else _transducer.loss_backward_workspace_bytes(n, T, U, V)
+        if forward_only:
+            self.fwd_bytes = _transducer.loss_score_workspace_bytes(n, T, U, V)
+            self.saved_bytes = self.bwd_bytes = 0
+            self.saved = None
+        else:
+            self.saved_bytes = _transducer.loss_saved_bytes(n, T, U, V)
+            self.saved = torch.empty(max(self.saved_bytes, 1), **u8)
+            self.fwd_bytes = _transducer.loss_forward_workspace_bytes(n, T, U, V)
+            self.bwd_bytes = _transducer.loss_backward_workspace_bytes(n, T, U, V)
         self.ws = torch.empty(max(self.fwd_bytes, self.bwd_bytes, 1), **u8)
         self.shape = (n, T, U, V, forward_only, dtype)
 
@@ -152,11 +157,19 @@ class HostLossPipeline(object):
                     else:
                         slot.deltas[:n].copy_(deltas[lo:hi], non_blocking=True)
                     _transducer.set_stream(slot.stream.cuda_stream)
-                    loss_forward(
-                        slot.E.data_ptr(), slot.P.data_ptr(), slot.labels.data_ptr(),
-                        slot.il.data_ptr(), slot.ll.data_ptr(), slot.costs.data_ptr(),
-                        self.loss_parts[i:].data_ptr(), slot.saved.data_ptr(), slot.saved_bytes,
-                        n, T, U, V, self.blank, slot.ws.data_ptr(), slot.fwd_bytes)
+                    if self.forward_only:   # (as TransducerLoss under no_grad)
+                        _transducer.loss_score(
+                            slot.E.data_ptr(), slot.P.data_ptr(), slot.labels.data_ptr(),
+                            slot.il.data_ptr(), slot.ll.data_ptr(), slot.costs.data_ptr(),
+                            self.loss_parts[i:].data_ptr(), n, T, U, V, self.blank,
+                            slot.ws.data_ptr(), slot.fwd_bytes, bf)
+                    else:
+                        loss_forward(
+                            slot.E.data_ptr(), slot.P.data_ptr(), slot.labels.data_ptr(),
+                            slot.il.data_ptr(), slot.ll.data_ptr(), slot.costs.data_ptr(),
+                            self.loss_parts[i:].data_ptr(), slot.saved.data_ptr(),
+                            slot.saved_bytes, n, T, U, V, self.blank, slot.ws.data_ptr(),
+                            slot.fwd_bytes)
                     costs[lo:hi].copy_(slot.costs[:n], non_blocking=True)
                     if not self.forward_only:
                         loss_backward(
