@@ -73,6 +73,7 @@ constexpr int kStageRows = 2 + kMaxStagedLabels;  // row shifts, blank-arc sums,
 constexpr int kMaxRing = 4;
 
 constexpr int kTileFrames = 48;   // frames of a tile, roughly (the tile height depends on the label axis)
+constexpr int kAltTiles = 6;      // alternate tiles of 48 frames from here on, see `alt`
 // Label positions of a launch.  One launch for 129..160 of them, in tiles of 32 frames (all that tensor
 // memory leaves), reads E once and writes egrads once where two over parts of the axis do so twice:
 // B = 64, T = 750..1500, U' = 76..151, V = 4096 948 -> 805 us, label_overflow 17 -> 9.
@@ -129,13 +130,18 @@ struct GradParams {
 // that they start last.  Every part leaves its sums over the frames in `partial`, and the one that
 // finishes last adds them in frame order.  Measured, whole / cut: 8 items of 2000 frames (V = 100)
 // 88 / 31 us, 64 items 89 / 58, 632 items (V = 10000, 40 in the last round) 335 / 311.
+// Leaving and adding the sums takes ~7 us, so short utterances are not cut.  Whole / cut at 300, 500 and 700 frames:
+// 632 items in 3 parts 105 / 111, 132 / 134, 160 / 156 us; 64 items in 2 parts 25 / 27, 32 / 33, 39 / 33;
+// 2528 items, 12 of them in 3 to 7 parts 349 / 358, 461 / 467, 564 / 563; 8 items in 3 to 7 parts 19 / 17, 25 / 19, 30 / 19.
 constexpr int kMaxGradParts = 16;
-int parts_by_frames(int maxT) { return std::min(kMaxGradParts, maxT / (2 * kTileFrames)); }
+constexpr int kMinCutFrames = 576, kMinCutFramesFew = 288;   // few: with four parts each, the items still fit the SMs
 GradSplit grad_split(Dims d) {
   constexpr int kSMs = kGradTickets;
   const i64 n = (i64)div_up(d.V, kVBlock) * d.B;
   const int rem = (int)(n % kSMs);
-  const int parts = rem > 0 ? std::min(parts_by_frames(d.maxT), kSMs / rem) : 1;
+  int parts = 1;
+  if (rem > 0 && d.maxT >= (4 * n <= kSMs ? kMinCutFramesFew : kMinCutFrames))
+    parts = std::min({kMaxGradParts, kSMs / rem, d.maxT / (2 * kTileFrames)});
   if (parts < 2) return GradSplit{n, 0, 1};
   return GradSplit{n - rem, rem, parts};
 }
@@ -161,14 +167,17 @@ __device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) 
 // of rounding once.  BF: E, P and both gradients are bf16 in memory (converted exactly to fp32
 // on the way in, rounded to nearest on the way out; everything in between is the fp32 path).
 // POS: label positions at most.
-template <int TB, bool ESPLIT, bool PSPLIT, bool BF, int POS>
+// CUT: some items are cut (see grad_split).  ALT: the column owners' halves may take alternate tiles (see
+// `alt`).  Instances of their own: with either built in, utterances of a few tiles took 1 to 2 % longer
+// without making use of it (B = 32, T = 240, U' = 101, V = 10000: 302 us, 305 with the choice, 308 with the parts).
+template <int TB, bool ESPLIT, bool PSPLIT, bool BF, int POS, bool CUT, bool ALT>
 __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
     const __grid_constant__ GradMaps tm, const GradParams p) {
   using TIO = typename std::conditional<BF, bf16, float>::type;
   constexpr int TBH = TB / 2;  // frames per owner half
   static_assert(TBH % 8 == 0, "tile halves move through TMEM in 8-column pieces");
   int item = blockIdx.x, part = 0, parts = 1, cutItem = 0;
-  if (item >= p.whole) {
+  if (CUT && item >= p.whole) {
     cutItem = (item - p.whole) / p.parts;
     part = item - p.whole - cutItem * p.parts;
     parts = p.parts;
@@ -198,7 +207,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
   // my tiles: [tile0, tile0 + nTiles) of the utterance
   const int tilesAll = (T + TB - 1) / TB;
   int tile0 = 0, nTiles = tilesAll;
-  if (parts > 1) {   // (at most 16 parts of 2^26 tiles.  Whole items, most of them, skip the divisions.)
+  if (CUT && parts > 1) {   // (at most 16 parts of 2^26 tiles.  Whole items, most of them, skip the divisions.)
     parts = min(parts, tilesAll);
     if (part >= parts) return;
     tile0 = tilesAll * part / parts;
@@ -222,8 +231,8 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
   // its own ring slots and copies (all even; operand precision 3 leaves less), and where it is faster:
   // halves / alternate, us, B = 32: tiles of 32 frames, U' = 151, V = 4096, T = 64 119 / 115, T = 512 243 / 235;
   // of 48, U' = 101, V = 10000, T = 144 261 / 266, T = 240 307 / 307, T = 288 335 / 333, T = 2000 bf16 996 / 972;
-  // of 64, U' = 61, T = 64 160 / 165, T = 768 409 / 419.
-  const bool alt = (TB == 32 || (TB == 48 && nTiles >= 6)) && SE == 4 && p.eBufs == 2 && p.dBufs == 2;
+  // of 64, U' = 61, T = 64 160 / 165, T = 768 409 / 419 (not built).
+  const bool alt = ALT && (TB == 32 || nTiles >= kAltTiles) && SE == 4 && p.eBufs == 2 && p.dBufs == 2;
   const int owners = alt ? kGroupWarps / 2 : kGroupWarps;   // warps of a group per tile
   const int wBytes = nUB * kBoxBytes;
   const int wStage = 2 * wBytes;               // K-major copy, MN-major copy
@@ -245,9 +254,11 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
   const bool blankHere = !p.accumulate && p.blank >= v0 && p.blank < v0 + kVBlock;
 
   if (threadIdx.x == 0) {
-    sSplit[0] = cutItem;
-    sSplit[1] = part;
-    sSplit[2] = parts;
+    if constexpr (CUT) {
+      sSplit[0] = cutItem;
+      sSplit[1] = part;
+      sSplit[2] = parts;
+    }
     for (int s = 0; s < SE; ++s) {
       mbar_init(&barEFull[s], 1);
       mbar_init(&barStore[s], owners);        // gradient tile complete in shared memory
@@ -545,8 +556,10 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
       return reinterpret_cast<TIO*>(col + t * 128 + ((chunk ^ (t & 7)) << 4));
     };
 
-    const int first = alt ? h : 0, step = alt ? 2 : 1;                 // my tiles
-    const int hBeg = alt ? 0 : h, hEnd = alt ? 2 : h + 1;              // my halves of their frames
+    auto ownTiles = [&](auto alternate) {
+    constexpr bool kAlt = decltype(alternate)::value;
+    const int first = kAlt ? h : 0;                             // my tiles
+    constexpr int step = kAlt ? 2 : 1, kHalves = kAlt ? 2 : 1;  // my halves of their frames
     if (grp == 0) {
       // ---- exp group: raw E -> exp(E - ref), in place, and into TMEM as GEMM2's A operand ----
       int se = first, eb = first;  // E stage and expE^T copy of tile i
@@ -561,7 +574,8 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
         uint8_t* stE = smem + (size_t)se * kEStage;
         uint8_t* col = stE + colOff;
 #pragma unroll 1
-        for (int hh = hBeg; hh < hEnd; ++hh) {
+        for (int own = 0; own < kHalves; ++own) {
+          const int hh = kAlt ? own : h;
           // live frames in this half (may be <= 0); none for a column beyond the vocabulary
           const int tValid = vOk ? min(TB, T - (tile0 + i) * TB) - hh * TBH : 0;
           const float* nr = reinterpret_cast<const float*>(stE + kEBytes) + hh * TBH;
@@ -621,7 +635,8 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
         uint8_t* stE = smem + (size_t)se * kEStage;
         uint8_t* col = stE + colOff;
 #pragma unroll 1
-        for (int hh = hBeg; hh < hEnd; ++hh) {
+        for (int own = 0; own < kHalves; ++own) {
+          const int hh = kAlt ? own : h;
           // expE * D1, both from tensor memory (expE = hi + lo exactly)
           const uint32_t cEhi = cE + eb * kECols + hh * TBH, cElo = cEhi + TB;
           float d1[TBH];
@@ -639,7 +654,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
               d1[c + j] = x * __uint_as_float(r[j]);
             }
           }
-          if (hh == hEnd - 1) {
+          if (own == kHalves - 1) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) {
@@ -669,8 +684,20 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
         if ((db += step) >= DB) { db -= DB; dph ^= 1u; }
       }
     }
+    };
+    if constexpr (ALT) {
+      if (alt) ownTiles(std::true_type{});
+      else ownTiles(std::false_type{});
+    } else {
+      ownTiles(std::false_type{});
+    }
 
-    const int cut = ((volatile int*)sSplit)[0], myPart = ((volatile int*)sSplit)[1], nParts = ((volatile int*)sSplit)[2];
+    int cut = 0, myPart = 0, nParts = 1;
+    if constexpr (CUT) {
+      cut = ((volatile int*)sSplit)[0];
+      myPart = ((volatile int*)sSplit)[1];
+      nParts = ((volatile int*)sSplit)[2];
+    }
     // padded frames beyond the last tile: exact zeros
     if (vOk && !p.accumulate)
       for (int t = (T + TB - 1) / TB * TB + share + 4 * myPart; t < p.maxT; t += 4 * nParts)
@@ -681,7 +708,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
     ok = __all_sync(0xffffffffu, ok);
     bool writer = ok;
     const float* partials = p.partial + (size_t)cut * p.parts * (POS * kVBlock) + vl;
-    if (nParts > 1) {
+    if (CUT && nParts > 1) {
       // my sums over my frames (NaN if they never came); the part that finishes last goes on
       float* mine = p.partial + ((size_t)cut * p.parts + myPart) * (POS * kVBlock) + vl;
       if (ok) tc_fence_after();
@@ -733,7 +760,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
         tmem_wait_ld();
         writeRows(u0, d2, xh, xl);
       }
-    } else if (writer) {
+    } else if (CUT && writer) {
       tc_fence_after();
       for (int u0 = 8 * share; u0 < p.Ku; u0 += 32) {
         uint32_t d2[8], xh[8], xl[8];
@@ -915,9 +942,15 @@ void launch_variant(const GradMaps& tm, GradParams p, TileCfg cfg, unsigned ctas
   p.tmemCols = pow2_cols(cols);
   size_t smem = (size_t)cfg.SE * eStage + (size_t)cfg.SW * wStage + 1024;
   if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it may hold all 512 TMEM columns
-  allow_dyn_smem(grads_umma_kernel<TB, ESPLIT, PSPLIT, BF, POS>, 227 * 1024 - kStaticSmemBound);
-  ScopedKernel sk("grads_umma", stream);
-  grads_umma_kernel<TB, ESPLIT, PSPLIT, BF, POS><<<ctas, kGradThreads, smem, stream>>>(tm, p);
+  auto go = [&](auto kernel) {
+    allow_dyn_smem(kernel, 227 * 1024 - kStaticSmemBound);
+    ScopedKernel sk("grads_umma", stream);
+    kernel<<<ctas, kGradThreads, smem, stream>>>(tm, p);
+  };
+  constexpr bool kAlt = TB != 64;
+  if (p.parts > 1) go(grads_umma_kernel<TB, ESPLIT, PSPLIT, BF, POS, true, kAlt>);
+  else if (TB == 48 && p.maxT <= TB * (kAltTiles - 1)) go(grads_umma_kernel<TB, ESPLIT, PSPLIT, BF, POS, false, TB == 32>);
+  else go(grads_umma_kernel<TB, ESPLIT, PSPLIT, BF, POS, false, kAlt>);
 }
 
 }  // namespace
@@ -927,8 +960,9 @@ int grads_umma_ld_t(Dims d) { return (int)round_up64(d.maxT > 0 ? d.maxT : 1, 4)
 // Room for the parts of any call of at most these sizes, not only of this one (a workspace is laid out for
 // the largest call and serves smaller ones, whose last round may hold more items): at most one part per SM.
 size_t grads_umma_partial_floats(Dims d) {
-  if (d.B <= 0 || d.maxT <= 0 || d.V <= 0 || parts_by_frames(d.maxT) < 2) return 0;
-  const i64 slots = std::min<i64>(kGradTickets, (i64)div_up(d.V, kVBlock) * d.B * parts_by_frames(d.maxT));
+  if (d.B <= 0 || d.V <= 0 || d.maxT < kMinCutFramesFew) return 0;
+  const i64 slots = std::min<i64>(kGradTickets, (i64)div_up(d.V, kVBlock) * d.B *
+                                                    std::min(kMaxGradParts, d.maxT / (2 * kTileFrames)));
   return (size_t)slots * (d.maxU > kMaxPos ? kMaxPosWide : kMaxPos) * kVBlock;
 }
 
