@@ -185,7 +185,10 @@ int tb200_log_norms(const float* emissions, const float* predictions, float* log
  * (added in index order by the last CTA to finish).  What the reference keeps for
  * its backward pass as autograd-saved tensors (alphas, log_norms, expEs, ...,
  * torch_binding.py:52-55) is kept here in `saved`, an opaque device buffer of
- * tb200_loss_saved_bytes() owned by the caller; exp(E) is not among it. */
+ * tb200_loss_saved_bytes() owned by the caller; exp(E) is not among it.
+ * Words may be masked by -inf or by any low number.  An utterance whose every path goes through a
+ * masked word costs +inf, and its gradients are unspecified.  (Label axes of up to 128 positions: a cost beyond
+ * 3.8e29 is +inf.) */
 size_t tb200_loss_saved_bytes(int batchSize, int maxInputLength, int maxLabelLength,
                               int alphabetSize);
 size_t tb200_loss_forward_workspace_bytes(int batchSize, int maxInputLength,
@@ -198,8 +201,10 @@ int tb200_loss_forward(const float* emissions, const float* predictions,
                        int blank, void* workspace, size_t workspaceBytes);
 
 /* The costs alone, where no backward call will follow (torch_binding.py:25-58 under no_grad): nothing is
- * saved, and label axes of more than 128 positions need not keep to the rounding that their gradients
- * depend on.  workspace: tb200_loss_score_workspace_bytes().  _bf16: see tb200_loss_forward_bf16. */
+ * saved, and nothing keeps to the rounding that the gradients depend on, so the costs are those of
+ * tb200_loss_forward to rounding (1e-5 relative) only, whatever the sizes.  Masked words: as there, a cost beyond
+ * 3.8e29 is +inf up to 256 positions.  workspace: tb200_loss_score_workspace_bytes().  _bf16: see
+ * tb200_loss_forward_bf16. */
 size_t tb200_loss_score_workspace_bytes(int batchSize, int maxInputLength, int maxLabelLength,
                                         int alphabetSize);
 int tb200_loss_score(const float* emissions, const float* predictions, const int* labels,

@@ -61,11 +61,14 @@ using namespace sweep;
 __device__ __forceinline__ int middle(int S) { return (S / 2) & ~(kDiag - 1); }
 constexpr float kLn2F = 0.6931471805599453f;
 constexpr float kLog2e = 1.4426950408889634f;
-// "No such arc": a large negative finite number, the identity of the alpha recursion without -inf
-// arithmetic, so that the sweeps need no validity logic.
+// "No such arc": a large negative finite number (-5.97e29), the identity of the alpha recursion without -inf
+// arithmetic, so that the sweeps need no validity logic.  An exponent below kNoPath means that every path
+// has such an arc: the cost is +inf.
 constexpr unsigned kNoArcBits = 0xF0F0F0F0u;
+constexpr float kNoPath = -5.5e29f;
 
-// A log-probability as an arc term: a word masked by -inf makes no arc (NaN stays NaN).
+// A log-probability as an arc term: a word masked by -inf makes no arc (two of them into a node would make
+// NaN of their difference); NaN stays NaN.
 __device__ __forceinline__ float arc_term(float x) {
   float y;
   asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(x), "f"(__uint_as_float(kNoArcBits)));
@@ -231,7 +234,8 @@ __global__ void __launch_bounds__(32) alpha_sweep_kernel(
   // the last diagonal holds only the terminal node (T-1, U-1); its blank arc ends the path
 #pragma unroll
   for (int r = 0; r < NPL; ++r)
-    if (u0 + r == U - 1) finish_cost(costs, b, -(stayIn[r] + offset) * kLn2F, B, lossSum, ticket);
+    if (u0 + r == U - 1)
+      finish_cost(costs, b, stayIn[r] < kNoPath ? pos_inf() : -(stayIn[r] + offset) * kLn2F, B, lossSum, ticket);
 }
 
 // ---------------------------------------------------------------------------
@@ -388,7 +392,7 @@ __device__ __forceinline__ float beta_half(uint8_t* smem, const float2* arcs, fl
 }
 
 // Of a lane's nodes of the middle diagonal: 2^(alpha + beta - m), m the largest exponent of the warp, into
-// w; returns m, and the warp's sum of w in `total`.  No path at all (m ~ -6e29): total = 0, w = 0.
+// w; returns m, and the warp's sum of w in `total`.  No path at all (m < kNoPath): total = 0, w = 0.
 template <int NPL>
 __device__ __forceinline__ float meet(const float* al, const float* be, int lane, int U, float (&w)[NPL], float& total) {
   float m = -INFINITY;
@@ -403,7 +407,7 @@ __device__ __forceinline__ float meet(const float* al, const float* be, int lane
 #pragma unroll
   for (int r = 0; r < NPL; ++r) {
     const bool nan = w[r] != w[r];
-    w[r] = m > -1.0e28f || nan ? exp2f(w[r] - m) : 0.0f;
+    w[r] = m >= kNoPath || nan ? exp2f(w[r] - m) : 0.0f;
     s += w[r];
   }
   total = warp_sum(s);
@@ -720,7 +724,6 @@ struct PrepParams {
   const int* labLens;
   int maxT, maxU, V, blank, npl, ld, extra;
   bool nat;                  // for the natural sweeps
-  bool score;                // for score_sweep_kernel: words masked by -inf make no arc
   i64 stride;
 };
 
@@ -802,7 +805,7 @@ __global__ void __launch_bounds__(256) sweep_prep_kernel(const PrepParams p) {
       const float lnv = tLn[tt][lane];
       f.x = p.nat ? lnv : ((tEb[tt] + pbl) - lnv) * kLog2e;
       if (u < U - 1) f.y = p.nat ? tEl[tt][lane] : ((tEl[tt][lane] + plab) - lnv) * kLog2e;
-      if (p.score) f = make_float2(arc_term(f.x), arc_term(f.y));
+      if (!p.nat) f = make_float2(arc_term(f.x), arc_term(f.y));
     }
     arcs[(i64)d * p.ld] = f;
   }
@@ -1055,7 +1058,7 @@ void launch_sweep_forward(const void* E, const void* P, float* LN, const float* 
     q.E = E; q.P = P; q.LN = LN; q.ELrow = ELrow; q.ebl = ebl; q.arcs = arcs;
     q.labels = labels; q.inLens = inLens; q.labLens = labLens;
     q.maxT = d.maxT; q.maxU = d.maxU; q.V = d.V; q.blank = d.blank; q.npl = g.npl; q.ld = g.ld;
-    q.extra = div_up(d.maxU, 32); q.nat = nat; q.score = score; q.stride = g.stride;
+    q.extra = div_up(d.maxU, 32); q.nat = nat; q.stride = g.stride;
     const dim3 grid(div_up(d.maxU, 32), div_up(d.maxT, 32) + 2 * q.extra, d.B);
     ScopedKernel sk("sweep_prep", stream);
     if (d.dtype == kDtypeBf16) sweep_prep_kernel<bf16><<<grid, 256, 0, stream>>>(q);
