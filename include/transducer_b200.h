@@ -53,8 +53,10 @@ void* tb200_get_stream(void);
  *   "lognorm_path"  0 auto, 1 exact SIMT logsumexp, 2 tensor-core factored GEMM, 3 fp32 factored
  *                   SIMT, 4 as 2 on fp16 pairs.  Auto takes 2 where TMA can address the inputs
  *                   (alphabetSize % 4 == 0 and >= 32, maxLabelLength <= 256, 16-byte aligned), or
- *                   4 for more than 2^24 scores in calls that no gradients follow (tb200_loss_score,
- *                   tb200_viterbi_decode), else 1 or 3 by the number of nodes
+ *                   4 for more than 2^25 scores in calls that no gradients follow (tb200_loss_score,
+ *                   tb200_viterbi_decode), if a sample of the nodes says that the scores are close enough
+ *                   for it (a model that is sure of one word per frame and of another per position stays
+ *                   with 2; 4 itself computes such tiles twice), else 1 or 3 by the number of nodes
  *   "grads_path"    0 auto, 1 SIMT, 2 tensor-core
  *   "grad_passes"   operand precision of the tensor-core gradient kernel.  The lattice
  *                   weights are always rounded once to TF32.  1: exp(E), exp(P) rounded

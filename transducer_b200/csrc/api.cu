@@ -223,7 +223,10 @@ bool log_norms_impl(const void* E, const void* P, float* LN, float* rowRef, floa
     const bool gathers = labels && EL && ebl && lognorm_umma_gathers(d) &&
                          (handOut == 2 || (handOut == 1 && bytesE > (size_t)96 << 20));
     launch_lognorm_umma(E, P, LN, rowRef, mp, inLens, labLens, d, ws.split,
-                        device_status_word(), path == 4 || (path == 0 && !keepBits && lognorm_f16_pays(d)),
+                        device_status_word(),
+                        path == 4                                           ? PairFormat::f16
+                        : path == 0 && !keepBits && lognorm_f16_pays(d) ? PairFormat::f16_if_close
+                                                                            : PairFormat::tf32,
                         fixup, g_stream, gathers ? labels : nullptr,
                         gathers ? EL : nullptr, gathers ? ebl : nullptr);
     return gathers;

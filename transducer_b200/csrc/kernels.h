@@ -102,8 +102,10 @@ void launch_exp_rows(const float* P, float* expP, float* maxP, const int* labLen
 // at most 128 positions).  Usable when lognorm_umma_supported();
 // splitWs holds lognorm_umma_workspace_floats(d) floats; status is the device status word
 // (api_internal.h): [0] first device-side error code (0 = none), [1] nodes recomputed exactly.
-// f16: by lognorm_f16.cu, the TF32 kernel for the tiles that it marks only; lognorm_f16_pays: is
-// that the faster of the two for these sizes?
+// pairs: the TF32 kernel, or lognorm_f16.cu with the TF32 kernel for the tiles that it marks, or that
+// unless a sample of the scores says that most tiles would be marked.  lognorm_f16_pays: is the last
+// the fastest for these sizes?
+enum class PairFormat { tf32, f16, f16_if_close };
 bool lognorm_f16_pays(Dims d);
 bool lognorm_umma_supported(const void* E, const void* P, Dims d);
 size_t lognorm_umma_workspace_floats(Dims d);
@@ -118,7 +120,7 @@ void launch_lognorm_fixup(const void* E, const void* P, float* LN, const int* in
 bool lognorm_umma_gathers(Dims d);
 void launch_lognorm_umma(const void* E, const void* P, float* LN, float* rowRef, float* maxP,
                          const int* inLens, const int* labLens, Dims d, float* splitWs,
-                         int* status, bool f16, bool fixup, cudaStream_t stream,
+                         int* status, PairFormat pairs, bool fixup, cudaStream_t stream,
                          const int* labels = nullptr, float* EL = nullptr, float* ebl = nullptr);
 
 // ---- lognorm_f16.cu ------------------------------------------------------------
@@ -129,13 +131,14 @@ struct LogNormScratch {
   float* rowSums;
   float* sumP;         // [B,maxU]
   unsigned* tickets;   // zero
-  int* marks;          // zero; 1 + B * tiles
+  int* marks;          // zero; kMarkTiles + B * tiles
   int nSM;             // SMs of the device
 };
-// LN of every tile whose sums can be trusted; the others are marked (ws.marks) for the TF32 kernel.
+// LN of every tile whose sums can be trusted; the others are marked (ws.marks) for the TF32 kernel.  sample:
+// none at all, if a sample of the nodes says that most tiles would be.
 void launch_lognorm_f16(const void* E, const void* P, float* LN, float* rowRef, float* maxP,
                         const int* inLens, const int* labLens, Dims d, const LogNormScratch& ws,
-                        int* status, cudaStream_t stream, const int* labels, float* EL, float* ebl);
+                        int* status, bool sample, cudaStream_t stream, const int* labels, float* EL, float* ebl);
 
 // ---- grads_umma.cu --------------------------------------------------------------
 // Tensor-core gradients: one pass over E produces egrads and pgrads.  Usable when

@@ -20,8 +20,8 @@
 //     exceeds 2^-20 S, or whose S leaves [1e-30, 1e30], is marked.  Marked tiles are recomputed by the
 //     TF32 kernel behind this one (which returns at once when there are none).  N(0, 2) scores
 //     over 10000 words stay clear of that, as do words 6 above the rest; a frame and a position
-//     that each have one word 10 above all others, not the same one, do not, and then the call costs both
-//     kernels.
+//     that each have one word 10 above all others, not the same one, do not.  Where a sample of the
+//     nodes says so, the TF32 kernel has the whole call to itself (see spread_vote).
 //
 // Work item: 128 frames of one utterance (UMMA M=128) x up to 160 label positions (longer axes: two
 // column ranges) x the whole vocabulary in stages of 64 words.  Roles inside a CTA (one per SM):
@@ -60,6 +60,7 @@ constexpr int kStages = 3;           // of the ring; one transform group each
 constexpr int kStageK = 64;          // words of a stage
 constexpr int kScaleBits = 15;       // both operands' largest entries are brought to 2^15
 constexpr int kScaleSlots = 8;       // stages whose scales are kept (the ring and five)
+constexpr float kSpread = 9.5367431640625e-7f;   // 2^-20: a node's sum must reach this share of the bound's two
 constexpr int kMinExp = -96, kMaxExp = 110;   // of a stage's largest exponential
 // raw E of a stage: two boxes of 32 fp32 words or one of 64 bf16 words, rows of 128 bytes
 __host__ __device__ constexpr int stage_raw_bytes(bool bf) { return kTileM * kStageK * (bf ? 2 : 4); }
@@ -119,15 +120,92 @@ __device__ __forceinline__ void split_f16(float a, float b, uint32_t& hi, uint32
 }
 
 // ---------------------------------------------------------------------------------
+// Would most tiles be marked?  A frame and a position of a sharp model each have one word far above their others, mostly
+// not the same one, and then nearly every tile holds a node that fails, for a share of its nodes that is
+// small at first: with one random word per frame and one per position raised by g over N(0,1), 4096 words, 0 of 8
+// tiles at g = 9, some at 10, all at 11, for 0.1 % of the nodes.  Both kernels would run, so a few hundred nodes
+// spread over the batch are looked at first, in fp32, against a bound eight times as high: 0.1 % of them fail it at
+// g = 9, 2 % at 10, 9 % at 11.  One CTA a node, two rows read.  They are the first CTAs of the launch that brings P
+// to pairs, whose others stop as soon as the votes are there (nobody reads the pairs then).
+// ---------------------------------------------------------------------------------
+template <typename TIn>
+__device__ __forceinline__ void spread_vote(
+    const TIn* __restrict__ E, const TIn* __restrict__ P, const int* __restrict__ inLens,
+    const int* __restrict__ labLens, unsigned i, int B, int maxT, int maxU, int V, int* __restrict__ marks) {
+  __shared__ float red[32][5];
+  const int warps = blockDim.x >> 5;
+  const int b = (int)(i % (unsigned)B);
+  const int T = min(inLens[b], maxT), U = min(labLens[b] + 1, maxU);
+  if (T <= 0 || U <= 0) return;
+  // node i / B of the utterance: two sequences that fill [0, 1) evenly (multiples of the golden ratio, of sqrt 2)
+  const unsigned k = i / (unsigned)B + 1u;
+  const int t = (int)__umulhi((k + 7u * (unsigned)b) * 2654435769u, (unsigned)T);
+  const int u = (int)__umulhi((k + 5u * (unsigned)b) * 1779033704u, (unsigned)U);
+  const TIn* e = E + ((i64)b * maxT + t) * V;
+  const TIn* p = P + ((i64)b * maxU + u) * V;
+  // sums relative to the largest words so far (in units of log2; words masked below that count for nothing)
+  float mE = -1e30f, mP = -1e30f, s = 0.0f, sE = 0.0f, sP = 0.0f;
+  auto rescale = [&](float toE, float toP) {
+    const float fE = ex2_approx(mE - toE), fP = ex2_approx(mP - toP);
+    sE *= fE;
+    sP *= fP;
+    s *= fE * fP;
+    mE = toE;
+    mP = toP;
+  };
+#pragma unroll 4
+  for (int v = 4 * threadIdx.x; v < V; v += 4 * blockDim.x) {   // (V % 4 == 0)
+    const float4 x4 = ld4(e + v), y4 = ld4(p + v);
+    const float x[4] = {x4.x, x4.y, x4.z, x4.w}, y[4] = {y4.x, y4.y, y4.z, y4.w};
+    rescale(fmaxf(mE, fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3])) * kLog2e),
+            fmaxf(mP, fmaxf(fmaxf(y[0], y[1]), fmaxf(y[2], y[3])) * kLog2e));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float a = ex2_approx(fmaf(x[j], kLog2e, -mE)), c = ex2_approx(fmaf(y[j], kLog2e, -mP));
+      sE += a;
+      sP += c;
+      s = fmaf(a, c, s);
+    }
+  }
+  rescale(warp_max(mE), warp_max(mP));
+  s = warp_sum(s);
+  sE = warp_sum(sE);
+  sP = warp_sum(sP);
+  if ((threadIdx.x & 31) == 0) {
+    float* mine = red[threadIdx.x >> 5];
+    mine[0] = mE; mine[1] = mP; mine[2] = sE; mine[3] = sP; mine[4] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  const float* mine = red[min((int)threadIdx.x, warps - 1)];
+  const bool one = (int)threadIdx.x < warps;
+  mE = mine[0]; mP = mine[1]; sE = one ? mine[2] : 0.0f; sP = one ? mine[3] : 0.0f; s = one ? mine[4] : 0.0f;
+  rescale(warp_max(mE), warp_max(mP));
+  s = warp_sum(s);
+  sE = warp_sum(sE);
+  sP = warp_sum(sP);
+  // (no votes from rows without a word and from NaN: their tiles are marked in any case)
+  if (threadIdx.x == 0 && sE > 0.0f && sP > 0.0f && s < 8.0f * kSpread * (sE + sP)) atomicAdd(&marks[kMarkVotes], 1);
+}
+
+// ---------------------------------------------------------------------------------
 // exp(P - maxP) * 2^15 as rows of [B][nPad][stage][hi 64 | lo 64] halves, zero beyond V; maxP and
 // the rows' sums of exp(P - maxP).  Bound by memory: one read (the second comes from L2), one write.
 // ---------------------------------------------------------------------------------
+// The first `samples` CTAs vote (see spread_vote).
 template <typename TIn>
 __global__ void __launch_bounds__(1024) expp_f16_kernel(
-    const TIn* __restrict__ P, uint8_t* __restrict__ out, float* __restrict__ maxP,
-    float* __restrict__ sumP, const int* __restrict__ labLens, int maxU, int V, int nPad, int kPad) {
+    const TIn* __restrict__ E, const TIn* __restrict__ P, uint8_t* __restrict__ out, float* __restrict__ maxP,
+    float* __restrict__ sumP, const int* __restrict__ inLens, const int* __restrict__ labLens, int samples, int B,
+    int maxT, int maxU, int V, int nPad, int kPad, int* marks) {
   __shared__ float red[32], redS[32];
-  const int b = blockIdx.y, u = blockIdx.x;
+  if ((int)blockIdx.x < samples) {
+    spread_vote(E, P, inLens, labLens, blockIdx.x, B, maxT, maxU, V, marks);
+    return;
+  }
+  if (samples > 0 && __syncthreads_or(threadIdx.x == 0 && *(volatile const int*)(marks + kMarkVotes) >= kVotes)) return;
+  const unsigned pos = blockIdx.x - samples;
+  const int b = (int)(pos / (unsigned)maxU), u = (int)(pos % (unsigned)maxU);
   const int U = min(labLens[b] + 1, maxU);
   if (u >= U) {
     // (rows beyond the utterance's label axis only feed accumulator columns that nobody reads)
@@ -189,7 +267,7 @@ struct F16Params {
   float* partial;        // [nSM][kTileM][nPad] partial sums of split tiles
   float* rowSums;        // [nSM][2][kTileM] their sums and maxima of exp(E)
   unsigned* tickets;     // [nSM] parts finished per split tile (zero on entry, zero again on exit)
-  int* marks;            // [0] any, [1 + b * tilesX + tile] (zero on entry)
+  int* marks;            // (see kMarkAny)
   const int* labels;     // label / blank emissions handed out (null: not wanted), see hand_out
   float* EL;
   float* ebl;
@@ -203,6 +281,7 @@ __global__ void __launch_bounds__((4 * kStages + 4 * ND + 4) * 32, 1) lognorm_f1
   static_assert(DCOLS % 8 == 0, "columns move in eights");
   constexpr int kDrainWarp0 = 4 * kStages, kLoadE = kDrainWarp0 + 4 * ND, kLoadP = kLoadE + 1, kMmaWarp = kLoadP + 1;
   constexpr int kRaw = stage_raw_bytes(BF);
+  if (all_marked(p.marks)) return;
   const LnItem it = ln_item(p.inLens, p.labLens, p.maxT, p.maxU, p.V, p.B, p.tilesX, p.halves, p.nPad, p.nSM);
   if (it.b < 0) return;
   const int b = it.b, T = it.T, U = it.U, t0 = it.t0, uOff = it.uOff;
@@ -566,13 +645,13 @@ __global__ void __launch_bounds__((4 * kStages + 4 * ND + 4) * 32, 1) lognorm_f1
             const float acc = sum[j];
             out[u] = (logf(acc) + ref) + sMaxP[c0 + j];
             marked |= !(acc >= kSumLo && acc <= kSumHi &&
-                        acc >= 9.5367431640625e-7f * fmaf(maxE, sSumP[c0 + j], sumE));   // 2^-20
+                        acc >= kSpread * fmaf(maxE, sSumP[c0 + j], sumE));
           }
         }
       }
       if (marked) {
-        p.marks[1 + b * p.tilesX + t0 / kTileM] = 1;
-        p.marks[0] = 1;
+        p.marks[kMarkTiles + b * p.tilesX + t0 / kTileM] = 1;
+        p.marks[kMarkAny] = 1;
       }
     }
   }
@@ -606,20 +685,20 @@ LabelAxis label_axis(int maxU) {
 
 void launch_lognorm_f16(const void* E, const void* P, float* LN, float* rowRef, float* maxP,
                         const int* inLens, const int* labLens, Dims d, const LogNormScratch& ws,
-                        int* status, cudaStream_t stream, const int* labels, float* EL, float* ebl) {
+                        int* status, bool sample, cudaStream_t stream, const int* labels, float* EL, float* ebl) {
   const LabelAxis axis = label_axis(d.maxU);
   const int rows = axis.rows(), kPad = (int)round_up64(d.V, kStageK);
   const bool bf = d.dtype == kDtypeBf16;
   uint8_t* operand = reinterpret_cast<uint8_t*>(ws.operand);
   {
     ScopedKernel sk("expp_f16", stream);
-    const dim3 grid(d.maxU, d.B);
-    if (bf)
-      expp_f16_kernel<bf16><<<grid, expp_threads(d.V), 0, stream>>>(static_cast<const bf16*>(P), operand, maxP,
-                                                      ws.sumP, labLens, d.maxU, d.V, rows, kPad);
-    else
-      expp_f16_kernel<float><<<grid, expp_threads(d.V), 0, stream>>>(static_cast<const float*>(P), operand, maxP,
-                                                       ws.sumP, labLens, d.maxU, d.V, rows, kPad);
+    const int samples = !sample ? 0 : d.V <= 8192 ? 4 * ws.nSM : 2 * ws.nSM;
+    auto go = [&](auto k, auto* e, auto* p) {
+      k<<<(unsigned)samples + (unsigned)d.maxU * (unsigned)d.B, expp_threads(d.V), 0, stream>>>(
+          e, p, operand, maxP, ws.sumP, inLens, labLens, samples, d.B, d.maxT, d.maxU, d.V, rows, kPad, ws.marks);
+    };
+    if (bf) go(expp_f16_kernel<bf16>, static_cast<const bf16*>(E), static_cast<const bf16*>(P));
+    else go(expp_f16_kernel<float>, static_cast<const float*>(E), static_cast<const float*>(P));
   }
   TB200_CHECK_LAUNCH();
   const CUtensorMap tmE =

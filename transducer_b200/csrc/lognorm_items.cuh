@@ -22,6 +22,12 @@ constexpr int kMaxParts = 8;
 constexpr int kMaxLabels = 256;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kSumLo = 1e-30f, kSumHi = 1e30f;   // sums outside are not trusted
+
+// Marks of the fp16 kernel for the TF32 kernel behind it: any tile marked, votes of the sampled nodes, a word per
+// tile.  Enough votes (kVotes, see spread_kernel) leave every tile to the TF32 kernel.
+constexpr int kMarkAny = 0, kMarkVotes = 1, kMarkTiles = 2;
+constexpr int kVotes = 2;
+__device__ __forceinline__ bool all_marked(const int* marks) { return marks[kMarkVotes] >= kVotes; }
 // raw E chunk of a stage: 128 frames x 32 words, rows of 128 bytes (fp32) or 64 bytes (bf16)
 __host__ __device__ constexpr int raw_bytes(bool bf) { return kTileM * kChunkK * (bf ? 2 : 4); }
 

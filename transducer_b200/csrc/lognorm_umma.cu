@@ -142,10 +142,10 @@ __global__ void __launch_bounds__(1024) expp_split_kernel(
     int kPad, const int* __restrict__ only, int tilesX) {
   __shared__ float red[32];
   const int b = blockIdx.y, u = blockIdx.x;
-  if (only) {   // the utterances with a marked tile
-    if (only[0] == 0) return;
+  if (only && !all_marked(only)) {   // the utterances with a marked tile
+    if (only[kMarkAny] == 0) return;
     int any = 0;
-    for (int x = threadIdx.x; x < tilesX; x += blockDim.x) any |= only[1 + b * tilesX + x];
+    for (int x = threadIdx.x; x < tilesX; x += blockDim.x) any |= only[kMarkTiles + b * tilesX + x];
     if (!__syncthreads_or(any)) return;
   }
   const int U = min(labLens[b] + 1, maxU);
@@ -238,9 +238,10 @@ __global__ void __launch_bounds__((4 * NTW + 4 * NDRAIN + 3) * 32, 1) lognorm_um
   constexpr int kDrainCols = DCOLS;
   constexpr int kRawBytes = raw_bytes(BF);
   constexpr int kRowBytes = BF ? 64 : 128;
-  if (p.only && p.only[0] == 0) return;   // (no tile is marked)
+  const bool all = p.only == nullptr || all_marked(p.only);
+  if (!all && p.only[kMarkAny] == 0) return;   // (no tile is marked)
   const LnItem it = ln_item(p.inLens, p.labLens, p.maxT, p.maxU, p.V, p.B, p.tilesX, p.halves, p.nPad, p.nSM);
-  if (it.b < 0 || (p.only && p.only[1 + it.b * p.tilesX + it.t0 / kTileM] == 0)) return;
+  if (it.b < 0 || (!all && p.only[kMarkTiles + it.b * p.tilesX + it.t0 / kTileM] == 0)) return;
   const int b = it.b, T = it.T, U = it.U, t0 = it.t0, uOff = it.uOff;
   const int part = it.part, parts = it.parts, splitIdx = it.split;
 
@@ -640,7 +641,7 @@ static size_t scratch(Dims d, float* base, LogNormScratch* ws) {
   w.rowSums = take((size_t)kMaxSMs * kTileM * 2);
   w.sumP = take(B * maxU);
   w.tickets = reinterpret_cast<unsigned*>(take(kMaxSMs));
-  w.marks = reinterpret_cast<int*>(take(1 + B * (size_t)div_up(std::max(d.maxT, 0), kTileM)));
+  w.marks = reinterpret_cast<int*>(take(kMarkTiles + B * (size_t)div_up(std::max(d.maxT, 0), kTileM)));
   if (ws) *ws = w;
   return at;
 }
@@ -731,14 +732,17 @@ static void launch_tf32(const void* E, const void* P, float* LN, float* rowRef, 
   TB200_CHECK_LAUNCH();
 }
 
-// The fp16 pairs need two launches more (for the marked tiles, mostly none: ~5 us).  Both kernels with
-// exp(P), us, TF32 / fp16: B = 8, T = 500, U = 50, V = 4096 (2^24 scores) 73 / 76; 8, 2000, 100, 1000 58 / 55;
-// 16, 1000, 100, 2048 91 / 84; 8, 2000, 100, 4000 131 / 112; 32, 2000, 100, 10000 929 / 765.
-bool lognorm_f16_pays(Dims d) { return (i64)d.B * d.maxT * d.V > (i64)1 << 24; }
+// The fp16 pairs need two launches more, for the marked tiles, which mostly find nothing to do (6 and 8 us at 8
+// utterances, 11 and 15 at 64).  Whole scoring call, us, TF32 / fp16 if close, on N(0,1) scores and with one random
+// word per frame and position raised by 11: B = 8, T = 500, U = 50, V = 4096 (2^24 scores) 112 / 115, 106 / 118; 16,
+// 1000, 100, 2048 (2^25) 140 / 140, 139 / 156; 8, 2000, 100, 4000 212 / 202, 212 / 228; 8, 2000, 100, 8000 297 / 266,
+// 298 / 319; 32, 2000, 100, 10000 854 / 709, 914 / 962; 64, 1500, 150, 4096 1010 / 680, 1010 / 1090 (without the votes
+// the last three took 458, 1520 and 1560 on the raised ones).
+bool lognorm_f16_pays(Dims d) { return (i64)d.B * d.maxT * d.V > (i64)1 << 25; }
 
 void launch_lognorm_umma(const void* E, const void* P, float* LN, float* rowRef, float* maxP,
                          const int* inLens, const int* labLens, Dims d, float* splitWs,
-                         int* status, bool f16, bool fixup, cudaStream_t stream, const int* labels,
+                         int* status, PairFormat pairs, bool fixup, cudaStream_t stream, const int* labels,
                          float* EL, float* ebl) {
   if (d.B <= 0 || d.maxT <= 0 || d.maxU <= 0) return;
   if (!lognorm_umma_gathers(d)) labels = nullptr;
@@ -750,9 +754,12 @@ void launch_lognorm_umma(const void* E, const void* P, float* LN, float* rowRef,
   ws.nSM = std::min(nSM, kMaxSMs);
   const size_t zeros = splitWs + floats - reinterpret_cast<float*>(ws.tickets);
   TB200_CUDA_CHECK(cudaMemsetAsync(ws.tickets, 0, sizeof(float) * zeros, stream));
+  const bool f16 = pairs != PairFormat::tf32;
   if (f16)
-    launch_lognorm_f16(E, P, LN, rowRef, maxP, inLens, labLens, d, ws, status, stream, labels, EL, ebl);
-  launch_tf32(E, P, LN, rowRef, maxP, inLens, labLens, d, ws, status, stream, f16 ? nullptr : labels, EL, ebl,
+    launch_lognorm_f16(E, P, LN, rowRef, maxP, inLens, labLens, d, ws, status, pairs == PairFormat::f16_if_close,
+                       stream, labels, EL, ebl);
+  // (marked tiles hand their emissions out again: the same numbers)
+  launch_tf32(E, P, LN, rowRef, maxP, inLens, labLens, d, ws, status, stream, labels, EL, ebl,
               f16 ? ws.marks : nullptr);
   if (fixup) launch_lognorm_fixup(E, P, LN, inLens, labLens, d, stream);
 }
