@@ -507,8 +507,8 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
     // the frames of a tile): half of what a tile costs a warp are round trips to barriers and to
     // tensor memory, ~1200 cycles whatever the frames (cycle stamps; without any copy to or from memory
     // and without most of the MMAs the kernel was as slow).  B = 32, T = 1500..2000, U' = 61..101,
-    // V = 10000 1086 -> 1082 us, bf16 996 -> 972, B = 64, U' = 76..151, V = 4096 958 -> 947.  All 16 warps split the label positions
-    // of the prologue and the epilogue.
+    // V = 10000 1086 -> 1082 us, bf16 996 -> 972, B = 64, U' = 76..151, V = 4096 958 -> 947.  All 16 warps
+    // split the label positions of the prologue and the epilogue.
     const int grp = warp >> 3, q = warp & 3, h = (warp >> 2) & 1;
     const int share = grp * 2 + h;  // 0..3: of the prologue / epilogue
     const int vl = q * 32 + lane;
@@ -798,10 +798,16 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
   if (warp == kWarpMma1) tmem_dealloc(tBase, (uint32_t)p.tmemCols);
   if (*abortp && threadIdx.x < kVBlock && v0 + (int)threadIdx.x < p.V) {
     // a wait ran out (recorded in the status word): whatever this CTA wrote is incomplete, so
-    // its whole slice of both gradients becomes NaN rather than a plausible-looking number
+    // its slice of both gradients becomes NaN rather than a plausible-looking number.  Of a cut item
+    // these are this part's frames (the others have theirs from other CTAs) and, through the sums, pgrads.
     const float bad = __int_as_float(0x7fc00000);
     const int v = v0 + threadIdx.x;
-    for (int t = 0; t < p.maxT; ++t) from_f32(eg[(i64)t * p.V + v], bad);
+    int tBeg = 0, tEnd = p.maxT;
+    if (CUT && sSplit[2] > 1) {
+      tBeg = tilesAll * sSplit[1] / sSplit[2] * TB;
+      tEnd = min(tilesAll * (sSplit[1] + 1) / sSplit[2] * TB, p.maxT);
+    }
+    for (int t = tBeg; t < tEnd; ++t) from_f32(eg[(i64)t * p.V + v], bad);
     for (int u = 0; u < rowsMine; ++u) from_f32(pg[(i64)u * p.V + v], bad);
   }
 }
