@@ -547,7 +547,7 @@ int loss_backward_any(const void* E, const void* P, const int* labels, const int
                         g_stream);
       launch_lattice_unskew(ws.Ws, ws.EMs, ws.W, ldW, ws.em, inLens, labLens, g, d, g_stream);
     }
-    if (tensorCore) {   // (label axes of 129..256 positions: once per half of the axis)
+    if (tensorCore) {   // (label axes of more than 160 positions: one launch per part of the axis)
       launch_grads_umma(E, P, st.maxP, ws.W, ws.emT, ws.nref, ws.ebl, ws.pBlank, ws.pLabel, labels,
                         deltas, egrads, pgrads, inLens, labLens, d, passes, ws.gradPartial,
                         ws.sweep.gradTickets, device_status_word(), g_stream);

@@ -35,7 +35,7 @@
 // node) up to the middle diagonal M and beta (all paths from a node) down to it, the total is the sum
 // over M of alpha beta.  The two halves are two warps that know nothing of each other, both chains are
 // half as long, nothing but their ends is stored, and every label axis runs on rebased logarithms.  B = 64,
-// T = 500..1000, U' = 101..201: 242 -> 71 us.
+// T = 500..1000, U' = 101..201: 242 -> 64 us.
 // With gradients to follow each recursion keeps to one warp from one end.  The weights W of the gradient
 // products are rounded to TF32 behind the sweeps, and any other order of operations in front of that
 // rounding flips some of them by one step, 2^-10 of a weight near one.  Where a blank is nearly certain

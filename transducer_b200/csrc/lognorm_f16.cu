@@ -4,8 +4,8 @@
 //
 // (transducer/torch_binding.py:35-40: row maxima, exp, bmm, log) in one pass over E, as
 // lognorm_umma.cu does with TF32 pairs.  There a product of two fp32 numbers is three kind::tf32
-// MMAs; here every factor is hi + lo with both halves fp16 (round-to-nearest: 22 bits, the dropped
-// lo * lo is below 2^-24) and the three products are kind::f16 MMAs, which take half the time for
+// MMAs; here every factor is hi + lo with both halves fp16 (round-to-nearest: 22 bits, and the dropped
+// lo * lo is at most 2^-22 of the product too, of either sign) and the three products are kind::f16 MMAs, which take half the time for
 // half the operand bytes.  Distance to float64 of the two, N(0,1..2) scores over 64..8000 words: rms
 // 3e-7..5e-7 here, 1.5e-6 there (half as many truncating accumulation steps besides).  What fp16 lacks is
 // range, so

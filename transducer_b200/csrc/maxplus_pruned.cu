@@ -577,7 +577,7 @@ int fallback_capacity(Dims d) {
   const i64 nodes = (i64)d.B * d.maxT * (d.maxU - 1);
   return (int)std::min<i64>(1 << 22, std::max<i64>(4096, nodes / 64));
 }
-// one row fits a selection warp's staging area, two rows a group of the evaluation kernel,
+// one row fits a selection warp's staging area and a group's buffer in the evaluation kernel,
 // and an index fits the 16 bits of a list head
 constexpr int kMaxWords = 16384;
 

@@ -12,7 +12,9 @@ of the two directions instead of their sum.
 
 No counterpart in the reference (its wrapper takes device tensors only,
 transducer/torch_binding.py:23-58).  Same arithmetic, same kernels, same results as
-`TransducerLoss` on the whole batch: utterances do not interact.
+`TransducerLoss` on the whole batch: utterances do not interact.  (forward_only: as
+`TransducerLoss` under no_grad on each chunk; on another number of utterances the sums may be
+rounded differently.)
 """
 import torch
 
