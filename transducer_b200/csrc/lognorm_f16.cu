@@ -194,7 +194,7 @@ __device__ __forceinline__ void spread_vote(
 // ---------------------------------------------------------------------------------
 // The first `samples` CTAs vote (see spread_vote).
 template <typename TIn>
-__global__ void __launch_bounds__(1024) expp_f16_kernel(
+__global__ void __launch_bounds__(1024, 2) expp_f16_kernel(
     const TIn* __restrict__ E, const TIn* __restrict__ P, uint8_t* __restrict__ out, float* __restrict__ maxP,
     float* __restrict__ sumP, const int* __restrict__ inLens, const int* __restrict__ labLens, int samples, int B,
     int maxT, int maxU, int V, int nPad, int kPad, int* marks) {
@@ -203,9 +203,10 @@ __global__ void __launch_bounds__(1024) expp_f16_kernel(
     spread_vote(E, P, inLens, labLens, blockIdx.x, B, maxT, maxU, V, marks);
     return;
   }
-  if (samples > 0 && __syncthreads_or(threadIdx.x == 0 && *(volatile const int*)(marks + kMarkVotes) >= kVotes)) return;
   const unsigned pos = blockIdx.x - samples;
   const int b = (int)(pos / (unsigned)maxU), u = (int)(pos % (unsigned)maxU);
+  // (an old number from L1 will do: if not this CTA, a later one sees them)
+  const int votes = samples > 0 ? marks[kMarkVotes] : 0;
   const int U = min(labLens[b] + 1, maxU);
   if (u >= U) {
     // (rows beyond the utterance's label axis only feed accumulator columns that nobody reads)
@@ -215,13 +216,14 @@ __global__ void __launch_bounds__(1024) expp_f16_kernel(
   const TIn* p = P + ((i64)b * maxU + u) * V;
   uint8_t* row = out + ((i64)b * nPad + u) * kPad * 4;
   float m = neg_inf();
-  for (int v = threadIdx.x; v < V / 4; v += blockDim.x) {
-    const float4 x = ld4(p + 4 * v);
-    m = fmaxf(fmaxf(m, fmaxf(x.x, x.y)), fmaxf(x.z, x.w));
-  }
+  if (votes < kVotes)
+    for (int v = threadIdx.x; v < V / 4; v += blockDim.x) {
+      const float4 x = ld4(p + 4 * v);
+      m = fmaxf(fmaxf(m, fmaxf(x.x, x.y)), fmaxf(x.z, x.w));
+    }
   m = warp_max(m);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
+  if (__syncthreads_or(votes >= kVotes)) return;
   m = red[0];
   for (int k = 1; k < (int)blockDim.x / 32; ++k) m = fmaxf(m, red[k]);
   float s = 0.0f;
@@ -692,7 +694,7 @@ void launch_lognorm_f16(const void* E, const void* P, float* LN, float* rowRef, 
   uint8_t* operand = reinterpret_cast<uint8_t*>(ws.operand);
   {
     ScopedKernel sk("expp_f16", stream);
-    const int samples = !sample ? 0 : d.V <= 8192 ? 4 * ws.nSM : 2 * ws.nSM;
+    const int samples = !sample ? 0 : d.V <= 8192 ? 4 * ws.nSM : ws.nSM;   // (half of the first round's CTAs at most)
     auto go = [&](auto k, auto* e, auto* p) {
       k<<<(unsigned)samples + (unsigned)d.maxU * (unsigned)d.B, expp_threads(d.V), 0, stream>>>(
           e, p, operand, maxP, ws.sumP, inLens, labLens, samples, d.B, d.maxT, d.maxU, d.V, rows, kPad, ws.marks);
