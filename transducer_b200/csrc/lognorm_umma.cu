@@ -735,9 +735,9 @@ static void launch_tf32(const void* E, const void* P, float* LN, float* rowRef, 
 // The fp16 pairs need two launches more, for the marked tiles, which mostly find nothing to do (6 and 8 us at 8
 // utterances, 11 and 15 at 64).  Whole scoring call, us, TF32 / fp16 if close, on N(0,1) scores and with one random
 // word per frame and position raised by 11: B = 8, T = 500, U = 50, V = 4096 (2^24 scores) 112 / 115, 106 / 118; 16,
-// 1000, 100, 2048 (2^25) 140 / 140, 139 / 156; 8, 2000, 100, 4000 212 / 202, 212 / 228; 8, 2000, 100, 8000 297 / 266,
-// 298 / 319; 32, 2000, 100, 10000 854 / 709, 914 / 962; 64, 1500, 150, 4096 1010 / 680, 1010 / 1090 (without the votes
-// the last three took 458, 1520 and 1560 on the raised ones).
+// 1000, 100, 2048 (2^25) 140 / 140, 139 / 156; 8, 2000, 100, 4000 214 / 204, 210 / 225; 8, 2000, 100, 8000 296 / 264,
+// 297 / 316; 32, 2000, 100, 10000 880 / 740, 915 / 960; 64, 1500, 150, 4096 1000 / 685, 1000 / 1060 (without the votes
+// the last three took 458, 1530 and 1540 on the raised ones).
 bool lognorm_f16_pays(Dims d) { return (i64)d.B * d.maxT * d.V > (i64)1 << 25; }
 
 void launch_lognorm_umma(const void* E, const void* P, float* LN, float* rowRef, float* maxP,
