@@ -84,3 +84,25 @@ def test_accuracy_of_sharp_scores(V, gap, std):
     want = truth(E, P)
     rms = {path: (norms(path, E, P, il, ll)[0].double() - want).pow(2).mean().sqrt().item() for path in (2, 4)}
     assert rms[4] <= rms[2]
+
+
+def test_a_captured_call_decides_at_every_replay():
+    E, P, *rest = make(4, 700, 30, 16000)
+    close, sharp = (E, P), (E.clone(), P.clone())
+    raise_words(*sharp, 12.0)
+    want = [costs(0, [*kind, *rest]) for kind in (close, sharp)]
+    held = [E.clone(), P.clone()]
+    loss = TransducerLoss(validate_lengths=False)
+    stream = torch.cuda.Stream()
+    with torch.no_grad(), torch.cuda.stream(stream):
+        loss(*held, *rest)
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            out = loss(*held, *rest)
+    for i in (0, 1, 0, 1):
+        held[0].copy_((close, sharp)[i][0])
+        held[1].copy_((close, sharp)[i][1])
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want[i])

@@ -664,8 +664,8 @@ static void launch_tf32(const void* E, const void* P, float* LN, float* rowRef, 
   float* bLo = ws.operand + (size_t)d.B * nPad * kPad;
   {
     ScopedKernel sk("expp_split", stream);
-    // (mostly nothing is marked: small CTAs leave again sooner)
-    const int threads = only ? 256 : expp_threads(d.V);
+    // (mostly nothing is marked: smaller CTAs leave again sooner)
+    const int threads = only ? std::min(512, expp_threads(d.V)) : expp_threads(d.V);
     if (bf)
       expp_split_kernel<bf16><<<dim3(nPad, d.B), threads, 0, stream>>>(
           static_cast<const bf16*>(P), bHi, bLo, maxP, labLens, d.maxU, d.V, nPad, kPad, only, tilesX);
