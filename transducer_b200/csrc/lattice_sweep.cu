@@ -27,7 +27,7 @@
 // Measured (T = 2000, U' = 101, device time, B = 8 / 32): alpha 132 us (147 with bulk copies issued and
 // waited for by the sweeping warp); reverse sweep 12 / 27 us for the factors + 60 us for the recursion
 // (152 us when helper warps of the same CTA prepared the factors and carried away the results).
-// B = 64, T = 750..1500, U' = 151: alpha 195 us, factors 65 + recursion 76 us, operands 105 us, against
+// B = 64, T = 750..1500, U' = 151: alpha 195 us, factors 69 + recursion 76 us, operands 105 us, against
 // 384, 512 and (lattices re-laid out twice) 168 us of the block-wide kernels, which take a barrier
 // per diagonal.  B = 8, T = 4000, U' = 251: alpha 855 us, block-wide 954.
 //
@@ -72,6 +72,13 @@ constexpr float kNoPath = -5.5e29f;
 __device__ __forceinline__ float arc_term(float x) {
   float y;
   asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(x), "f"(__uint_as_float(kNoArcBits)));
+  return y;
+}
+
+// -inf becomes the lowest number; NaN stays NaN.
+__device__ __forceinline__ float not_below_lowest(float x) {
+  float y;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(x), "f"(-3.402823466e38f));
   return y;
 }
 
@@ -588,6 +595,11 @@ __global__ void __launch_bounds__(32 * kFactorWarps) gamma_factors_kernel(
     const i64 row = (i64)min(d0 + i, S - 1) * ld;
     load_row<NPL>(al + row, lane, a[i]);
     aN[i] = al[row + next];
+    if constexpr (natural(NPL)) {   // (nodes that nothing leads to: no differences of infinities)
+#pragma unroll
+      for (int r = 0; r < NPL; ++r) a[i][r] = not_below_lowest(a[i][r]);
+      aN[i] = not_below_lowest(aN[i]);
+    }
     if (i < kFactorRows) {
       const float2* ar = arcs + (i64)b * stride + row;
 #pragma unroll
