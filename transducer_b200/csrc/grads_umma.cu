@@ -556,10 +556,9 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
       return reinterpret_cast<TIO*>(col + t * 128 + ((chunk ^ (t & 7)) << 4));
     };
 
-    auto ownTiles = [&](auto alternate) {
-    constexpr bool kAlt = decltype(alternate)::value;
-    const int first = kAlt ? h : 0;                             // my tiles
-    constexpr int step = kAlt ? 2 : 1, kHalves = kAlt ? 2 : 1;  // my halves of their frames
+    // (constants without ALT)
+    const int first = alt ? h : 0, step = alt ? 2 : 1;                 // my tiles
+    const int hBeg = alt ? 0 : h, hEnd = alt ? 2 : h + 1;              // my halves of their frames
     if (grp == 0) {
       // ---- exp group: raw E -> exp(E - ref), in place, and into TMEM as GEMM2's A operand ----
       int se = first, eb = first;  // E stage and expE^T copy of tile i
@@ -574,8 +573,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
         uint8_t* stE = smem + (size_t)se * kEStage;
         uint8_t* col = stE + colOff;
 #pragma unroll 1
-        for (int own = 0; own < kHalves; ++own) {
-          const int hh = kAlt ? own : h;
+        for (int hh = hBeg; hh < hEnd; ++hh) {
           // live frames in this half (may be <= 0); none for a column beyond the vocabulary
           const int tValid = vOk ? min(TB, T - (tile0 + i) * TB) - hh * TBH : 0;
           const float* nr = reinterpret_cast<const float*>(stE + kEBytes) + hh * TBH;
@@ -635,8 +633,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
         uint8_t* stE = smem + (size_t)se * kEStage;
         uint8_t* col = stE + colOff;
 #pragma unroll 1
-        for (int own = 0; own < kHalves; ++own) {
-          const int hh = kAlt ? own : h;
+        for (int hh = hBeg; hh < hEnd; ++hh) {
           // expE * D1, both from tensor memory (expE = hi + lo exactly)
           const uint32_t cEhi = cE + eb * kECols + hh * TBH, cElo = cEhi + TB;
           float d1[TBH];
@@ -654,7 +651,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
               d1[c + j] = x * __uint_as_float(r[j]);
             }
           }
-          if (own == kHalves - 1) {
+          if (hh == hEnd - 1) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) {
@@ -683,13 +680,6 @@ __global__ void __launch_bounds__(kGradThreads, 1) grads_umma_kernel(
         if ((eb += step) >= EB) { eb -= EB; eph ^= 1u; }
         if ((db += step) >= DB) { db -= DB; dph ^= 1u; }
       }
-    }
-    };
-    if constexpr (ALT) {
-      if (alt) ownTiles(std::true_type{});
-      else ownTiles(std::false_type{});
-    } else {
-      ownTiles(std::false_type{});
     }
 
     int cut = 0, myPart = 0, nParts = 1;
