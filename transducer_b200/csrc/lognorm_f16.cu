@@ -283,9 +283,9 @@ __global__ void __launch_bounds__((4 * kStages + 4 * ND + 4) * 32, 1) lognorm_f1
   static_assert(DCOLS % 8 == 0, "columns move in eights");
   constexpr int kDrainWarp0 = 4 * kStages, kLoadE = kDrainWarp0 + 4 * ND, kLoadP = kLoadE + 1, kMmaWarp = kLoadP + 1;
   constexpr int kRaw = stage_raw_bytes(BF);
-  if (all_marked(p.marks)) return;
+  const bool none = all_marked(p.marks);   // (looked at behind the lengths)
   const LnItem it = ln_item(p.inLens, p.labLens, p.maxT, p.maxU, p.V, p.B, p.tilesX, p.halves, p.nPad, p.nSM);
-  if (it.b < 0) return;
+  if (it.b < 0 || none) return;
   const int b = it.b, T = it.T, U = it.U, t0 = it.t0, uOff = it.uOff;
   const int part = it.part, parts = it.parts, splitIdx = it.split;
 
